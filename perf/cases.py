@@ -221,3 +221,93 @@ def tolerance(case):
     # same quantisation points 2.7e-3.  The router's sums in another order (library GEMM instead of the fused kernel)
     # change a result by 1e-4 at most.
     return {"rel": 1e-2}
+
+
+def _activate(name, z):
+    gate, up = (z[:, 0::2], z[:, 1::2]) if is_glu(ActivationType(name)) else (z, None)
+    act = {"swiglu": torch.nn.functional.silu, "silu": torch.nn.functional.silu, "geglu": torch.nn.functional.gelu,
+           "gelu": torch.nn.functional.gelu, "reglu": torch.relu, "relu": torch.relu,
+           "relu_sq": lambda v: torch.relu(v).square()}[name](gate)
+    return act if up is None else act * up
+
+
+def _experts64(case, x, w1, b1, w2, b2, tokens, experts, scores, dout):
+    """Output of the experts and, with dout, the gradients of x, w1, b1, w2, b2 and scores, expert by expert."""
+    train = dout is not None
+    out = torch.zeros_like(x)
+    dx, ds = (torch.zeros_like(x), torch.zeros_like(scores)) if train else (None, None)
+    dw = [None if w is None else torch.zeros(w.shape, dtype=torch.float64, device=x.device) if train else None
+          for w in (w1, b1, w2, b2)]
+    for e in range(case["E"]):
+        pairs = (experts == e).nonzero()[:, 0]
+        if pairs.numel() == 0:
+            continue
+        rows, s = tokens[pairs].long(), scores[pairs, None]
+        up, down, xe = w1[e].double(), w2[e].double(), x[rows]
+        z = (xe @ up.T + (0 if b1 is None else b1[e].double())).requires_grad_(train)
+        with torch.enable_grad():
+            y1 = _activate(case["activation"], z)
+        y2 = y1.detach() @ down.T + (0 if b2 is None else b2[e].double())
+        out.index_add_(0, rows, s * y2)
+        if train:
+            dy2 = dout[rows]
+            ds[pairs] = (dy2 * y2).sum(-1)
+            dy2 = dy2 * s
+            dz, = torch.autograd.grad(y1, z, dy2 @ down)
+            dx.index_add_(0, rows, dz @ up)
+            dw[0][e], dw[2][e] = dz.T @ xe, dy2.T @ y1.detach()
+            if b1 is not None:
+                dw[1][e], dw[3][e] = dz.sum(0), dy2.sum(0)
+    return out, dx, dw, ds
+
+
+@torch.no_grad()
+def exact(case, seed):
+    """The layer in 64 bits, routed on the logits rounded to the activations' type as the layer defines them (near-ties
+    would otherwise go to other experts).  FP8 cases: the layer without quantisation, which is what they approximate.
+    Token rounding has none: which pairs it keeps hangs on ties among 16-bit probabilities."""
+    kind, T, E, K = case["kind"], case["T"], case["E"], case["K"]
+    if kind == "rounding" or work(case)["flops"] > 3e13:
+        return None
+    state = prepare(case, seed)
+    x = state["x"].detach().double()
+    train = state["train"]
+    dout = state["dout"].double() if train else None
+    if kind == "pairs":
+        w1, w2 = (p.detach() for p in state["params"])
+        tokens, experts, scores = state["tokens"], state["experts"], state["scores"].detach().double()
+        out, dx, dw, ds = _experts64(case, x, w1, None, w2, None, tokens, experts, scores, dout)
+        return dict(out=out, count=torch.bincount(experts, minlength=E).int(), grads=(dx, ds, dw[0], dw[2]))
+    if "moe" in state:
+        named = {n: p.detach() for n, p in state["moe"].named_parameters()}
+        order = [n for n, _ in state["moe"].named_parameters()]
+    else:
+        order = ["router.weight", "c_fc.weight", "c_proj.weight"]
+        named = {n: p.detach() for n, p in zip(order, state["params"])}
+    router = named["router.weight"].double()
+    w1, b1, w2, b2 = (named.get(n) for n in ("c_fc.weight", "c_fc.bias", "c_proj.weight", "c_proj.bias"))
+    logits = (x @ router.T).to(state["x"].dtype).double()
+    top, chosen = logits.sort(dim=-1, descending=True, stable=True)
+    top, chosen = top[:, :K], chosen[:, :K]
+    scores = torch.softmax(top, -1)
+    experts = chosen.reshape(-1)
+    count = torch.bincount(experts, minlength=E)
+    tokens = torch.arange(T, device=x.device).repeat_interleave(K)
+    out, dx, dw, ds = _experts64(case, x, w1, b1, w2, b2, tokens, experts, scores.reshape(-1), dout)
+    if not train:
+        return dict(out=out) if kind == "infer" else dict(out=out, count=count.int())
+    ds = ds.view(T, K)
+    dlogits = torch.zeros_like(logits).scatter_(1, chosen, scores * (ds - (ds * scores).sum(-1, keepdim=True)))
+    if kind == "train":
+        # E <share, p> with p the mean of the full softmax over the tokens (its sum is 1) and share the tokens' shares
+        share, probs = count / count.sum(), torch.softmax(logits, -1)
+        aux = E * (probs.mean(0) * share).sum()
+        dprobs = (AUX_WEIGHT * E / T) * (share - (probs.mean(0) * share).sum())
+        dlogits += probs * (dprobs - (probs * dprobs).sum(-1, keepdim=True))
+    dx += dlogits @ router
+    grads = {"router.weight": dlogits.T @ x, "c_fc.weight": dw[0], "c_fc.bias": dw[1], "c_proj.weight": dw[2],
+             "c_proj.bias": dw[3]}
+    grads = (dx, *[grads[n] for n in order])
+    if kind == "train":
+        return dict(out=out, aux=aux, grads=grads)
+    return dict(out=out, count=count.int(), grads=grads)
