@@ -88,34 +88,48 @@ __device__ __forceinline__ void prefetch_l2_lines(const void* p, int lines) {
   for (int i = 0; i < lines; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(c + 128 * i));
 }
 
-// value and derivative of the elementwise function behind every activation of the layer
-__device__ __forceinline__ void act_value_grad(int act, float x, float& a, float& da) {
+// The elementwise functions behind the layer's activations: value a and derivative da at x.
+enum ActFn : int { FN_SILU = 0, FN_GELU = 1, FN_RELU_SQ = 2, FN_RELU = 3 };
+
+template <int FN>
+__device__ __forceinline__ void act_value_grad(float x, float& a, float& da) {
+  if constexpr (FN == FN_SILU) {
+    const float sig = sigmoid_f(x);
+    a = x * sig;
+    da = sig * (1.f + x * (1.f - sig));
+  } else if constexpr (FN == FN_GELU) {  // exact (erf) GELU
+    const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
+    a = x * cdf;
+    da = cdf + x * 0.3989422804014327f * __expf(-0.5f * x * x);
+  } else if constexpr (FN == FN_RELU_SQ) {
+    const float r = fmaxf(x, 0.f);
+    a = r * r;
+    da = 2.f * r;
+  } else {
+    a = fmaxf(x, 0.f);
+    da = x > 0.f ? 1.f : 0.f;
+  }
+}
+
+template <int FN, bool GATED>
+struct ActKind {
+  static constexpr int fn = FN;
+  static constexpr bool gated = GATED;
+};
+
+// f(ActKind) for an Activation code, once per tile: with the switch inside the element loop the values of a row form
+// one serial chain of branches and function latencies (measured at T 8191, H 1024, I 512, E 32, K 4 with GELU, together
+// with rows stored one per lane by four warps: dH 196 us, up projection 134 us).
+template <class F>
+__device__ __forceinline__ auto act_dispatch(int act, F&& f) {
   switch (act) {
-    case ACT_SWIGLU:
-    case ACT_SILU: {
-      const float sig = sigmoid_f(x);
-      a = x * sig;
-      da = sig * (1.f + x * (1.f - sig));
-      break;
-    }
-    case ACT_GEGLU:
-    case ACT_GELU: {  // exact (erf) GELU
-      const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
-      a = x * cdf;
-      da = cdf + x * 0.3989422804014327f * __expf(-0.5f * x * x);
-      break;
-    }
-    case ACT_RELU_SQ: {
-      const float r = fmaxf(x, 0.f);
-      a = r * r;
-      da = 2.f * r;
-      break;
-    }
-    default: {  // ACT_REGLU, ACT_RELU
-      a = fmaxf(x, 0.f);
-      da = x > 0.f ? 1.f : 0.f;
-      break;
-    }
+    case ACT_SWIGLU: return f(ActKind<FN_SILU, true>{});
+    case ACT_GEGLU: return f(ActKind<FN_GELU, true>{});
+    case ACT_REGLU: return f(ActKind<FN_RELU, true>{});
+    case ACT_RELU_SQ: return f(ActKind<FN_RELU_SQ, false>{});
+    case ACT_RELU: return f(ActKind<FN_RELU, false>{});
+    case ACT_GELU: return f(ActKind<FN_GELU, false>{});
+    default: return f(ActKind<FN_SILU, false>{});
   }
 }
 
@@ -131,65 +145,6 @@ __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float (&
   }
 }
 
-// Warp-cooperative row I/O through a warp's staging rows (32 rows of PITCH bytes).  Lane l owns row l of a 32-row
-// block; global memory is touched with consecutive lanes on consecutive 16-byte pieces of one row, so an instruction
-// moves whole 64- or 128-byte row segments.  Rows at or beyond row_end are skipped.  Every lane must call.
-template <int PITCH>
-__device__ __forceinline__ void warp_store_rows64(uint32_t stage, int lane, const uint32_t (&w)[16], __nv_bfloat16* out,
-                                                  long long ld, int row_base, int row_end, int col) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) st_shared_v4(stage + lane * PITCH + 16 * q, w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int rr = 8 * i + (lane >> 2);
-    const uint4 v = ld_shared_v4(stage + rr * PITCH + 16 * (lane & 3));
-    if (row_base + rr < row_end) *reinterpret_cast<uint4*>(out + (row_base + rr) * ld + col + 8 * (lane & 3)) = v;
-  }
-  __syncwarp();
-}
-
-template <int PITCH>
-__device__ __forceinline__ void warp_store_rows128(uint32_t stage, int lane, const uint32_t (&w)[32], __nv_bfloat16* out,
-                                                   long long ld, int row_base, int row_end, int col) {
-  static_assert(PITCH >= 128 + 16, "128-byte payload");
-#pragma unroll
-  for (int q = 0; q < 8; ++q) st_shared_v4(stage + lane * PITCH + 16 * q, w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int rr = 4 * i + (lane >> 3);
-    const uint4 v = ld_shared_v4(stage + rr * PITCH + 16 * (lane & 7));
-    if (row_base + rr < row_end) *reinterpret_cast<uint4*>(out + (row_base + rr) * ld + col + 8 * (lane & 7)) = v;
-  }
-  __syncwarp();
-}
-
-// The inverse: 32 rows x 128 bytes read with whole-row-segment loads; lane l ends with row l (zeros past row_end).
-template <int PITCH>
-__device__ __forceinline__ void warp_load_rows128(uint32_t stage, int lane, uint32_t (&w)[32], const __nv_bfloat16* src,
-                                                  long long ld, int row_base, int row_end, int col) {
-  static_assert(PITCH >= 128 + 16, "128-byte payload");
-  uint4 v[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int rr = 4 * i + (lane >> 3);
-    v[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (row_base + rr < row_end)
-      v[i] = *reinterpret_cast<const uint4*>(src + (row_base + rr) * ld + col + 8 * (lane & 7));
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    st_shared_v4(stage + (4 * i + (lane >> 3)) * PITCH + 16 * (lane & 7), v[i].x, v[i].y, v[i].z, v[i].w);
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const uint4 t = ld_shared_v4(stage + lane * PITCH + 16 * q);
-    w[4 * q] = t.x; w[4 * q + 1] = t.y; w[4 * q + 2] = t.z; w[4 * q + 3] = t.w;
-  }
-  __syncwarp();
-}
-
 // eight packed bf16 values plus the eight at dst (fp32 sums, rounded once)
 __device__ __forceinline__ uint4 add_bf16x8(uint4 a, const uint4* dst) {
   const uint4 b = *dst;
@@ -202,6 +157,45 @@ __device__ __forceinline__ uint4 add_bf16x8(uint4 a, const uint4* dst) {
     o[i] = pack_bf16(x.x + y.x, x.y + y.y);
   }
   return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// Warp-cooperative row I/O through a warp's staging rows (32 rows of 64 bytes, 2 KiB).  Lane l owns row l of a 32-row
+// block; global memory is touched with consecutive lanes on consecutive 16-byte pieces of one row, so an instruction
+// moves whole 64-byte segments.  Rows at or beyond row_end are skipped.  Every lane must call.
+// The four pieces of a row are permuted by its row pair, so that both directions are free of bank conflicts (eight lanes
+// write the same piece of eight rows, or read two whole rows): with 80-byte rows the reads took twice the shared-memory
+// cycles, of which the tensor cores' operands leave few.
+constexpr int STAGE_ROWS_BYTES = 32 * 64;
+__device__ __forceinline__ uint32_t stage_piece(uint32_t stage, int row, int piece) {
+  return stage + row * 64 + 16 * (piece ^ ((row >> 1) & 3));
+}
+
+// dst(rr) gives the address of the 64-byte segment of the block's row rr, or nullptr (called by every lane).
+template <class Dst>
+__device__ __forceinline__ void warp_store_segments64(uint32_t stage, int lane, const uint32_t (&w)[16], bool accumulate,
+                                                      Dst&& dst) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) st_shared_v4(stage_piece(stage, lane, q), w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int rr = 8 * i + (lane >> 2);
+    const uint4 v = ld_shared_v4(stage_piece(stage, rr, lane & 3));
+    __nv_bfloat16* d = dst(rr);
+    if (d != nullptr) {
+      uint4* d4 = reinterpret_cast<uint4*>(d + 8 * (lane & 3));
+      *d4 = accumulate ? add_bf16x8(v, d4) : v;
+    }
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ void warp_store_rows64(uint32_t stage, int lane, const uint32_t (&w)[16], __nv_bfloat16* out,
+                                                  long long ld, int row_base, int row_end, int col,
+                                                  bool accumulate = false) {
+  warp_store_segments64(stage, lane, w, accumulate, [&](int rr) {
+    return row_base + rr < row_end ? out + (row_base + rr) * ld + col : nullptr;
+  });
 }
 
 // acc (+ bias) as 32 floats
@@ -225,8 +219,6 @@ __device__ __forceinline__ void load_biased(const GemmParams& p, int expert, int
   }
 }
 
-// One 32-column piece of one accumulator row: v[j] = acc[r, n + j] (fp32 bits).  `r` is the grouped row
-// (ragged-M) or the output row inside the expert's matrix (ragged-K); only called for rows that exist.
 // dSwiGLU on 32 accumulator columns (= 64 columns of dz).  acc[., i] = dy1[r, i]; z[r, 2i] = gate, z[r, 2i+1] = up.
 // Writes dz (bf16), y1 * score, accumulates ds.  KEEP: the 32 packed bf16x2 words of dz replace v and amax collects
 // max |dz| over the bf16 values (for a caller that also quantises dz).
@@ -270,8 +262,7 @@ __device__ __forceinline__ void dswiglu_chunk(const GemmParams& p, int r, int n,
   }
 }
 
-// 64-byte variant of warp_load_rows128 (staging rows of PITCH >= 80 bytes).
-template <int PITCH>
+// The inverse: 32 rows x 64 bytes read with whole-row-segment loads; lane l ends with row l (zeros past row_end).
 __device__ __forceinline__ void warp_load_rows64(uint32_t stage, int lane, uint32_t (&w)[16], const __nv_bfloat16* src,
                                                  long long ld, int row_base, int row_end, int col) {
   uint4 v[4];
@@ -284,11 +275,11 @@ __device__ __forceinline__ void warp_load_rows64(uint32_t stage, int lane, uint3
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    st_shared_v4(stage + (8 * i + (lane >> 2)) * PITCH + 16 * (lane & 3), v[i].x, v[i].y, v[i].z, v[i].w);
+    st_shared_v4(stage_piece(stage, 8 * i + (lane >> 2), lane & 3), v[i].x, v[i].y, v[i].z, v[i].w);
   __syncwarp();
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const uint4 t = ld_shared_v4(stage + lane * PITCH + 16 * q);
+    const uint4 t = ld_shared_v4(stage_piece(stage, lane, q));
     w[4 * q] = t.x; w[4 * q + 1] = t.y; w[4 * q + 2] = t.z; w[4 * q + 3] = t.w;
   }
   __syncwarp();
@@ -297,13 +288,13 @@ __device__ __forceinline__ void warp_load_rows64(uint32_t stage, int lane, uint3
 // dswiglu_chunk with the row traffic (z in, dz and y1 * score out) going through the warp's staging rows as 64-byte
 // row segments.  Every lane of the warp must call (lane l owns row row_base + l; rows at or past row_end read zeros
 // and store nothing).  Same arithmetic, same results.
-template <bool KEEP, int PITCH>
+template <bool KEEP>
 __device__ __forceinline__ void dswiglu_chunk_staged(const GemmParams& p, uint32_t stage, int lane, int row_base,
                                                      int row_end, int n, uint32_t (&v)[32], float score, float& ds_acc,
                                                      float& amax) {
   uint32_t za[16], zb[16], ys[16];
-  warp_load_rows64<PITCH>(stage, lane, za, p.z, 2ll * p.N, row_base, row_end, 2 * n);
-  warp_load_rows64<PITCH>(stage, lane, zb, p.z, 2ll * p.N, row_base, row_end, 2 * n + 32);
+  warp_load_rows64(stage, lane, za, p.z, 2ll * p.N, row_base, row_end, 2 * n);
+  warp_load_rows64(stage, lane, zb, p.z, 2ll * p.N, row_base, row_end, 2 * n + 32);
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
     uint32_t& zw = i < 16 ? za[i] : zb[i - 16];
@@ -321,9 +312,9 @@ __device__ __forceinline__ void dswiglu_chunk_staged(const GemmParams& p, uint32
   }
 #pragma unroll
   for (int j = 0; j < 16; ++j) ys[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-  warp_store_rows64<PITCH>(stage, lane, za, p.out0, p.ld0, row_base, row_end, 2 * n);
-  warp_store_rows64<PITCH>(stage, lane, zb, p.out0, p.ld0, row_base, row_end, 2 * n + 32);
-  warp_store_rows64<PITCH>(stage, lane, ys, p.out1, p.ld1, row_base, row_end, n);
+  warp_store_rows64(stage, lane, za, p.out0, p.ld0, row_base, row_end, 2 * n);
+  warp_store_rows64(stage, lane, zb, p.out0, p.ld0, row_base, row_end, 2 * n + 32);
+  warp_store_rows64(stage, lane, ys, p.out1, p.ld1, row_base, row_end, n);
   if constexpr (KEEP) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
@@ -334,6 +325,7 @@ __device__ __forceinline__ void dswiglu_chunk_staged(const GemmParams& p, uint32
   }
 }
 
+// One 32-column piece of one accumulator row, stored by the lane that holds it: v[j] = acc[r, n + j].  FP8 kernels.
 template <int EPI, bool RAGGED_K>
 __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int expert, int r, int n, uint32_t (&v)[32],
                                        float score, float& ds_acc) {
@@ -383,86 +375,6 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int expert, 
   } else if constexpr (EPI == EPI_DSWIGLU) {
     float unused = 0.f;
     dswiglu_chunk<false>(p, r, n, v, score, ds_acc, unused);
-  } else if constexpr (EPI == EPI_STORE_BIAS) {
-    float f[32];
-    load_biased(p, expert, n, v, f);
-    store_bf16x32(p.out0 + r * p.ld0 + n, f);
-  } else if constexpr (EPI == EPI_ACT) {
-    float f[32];
-    load_biased(p, expert, n, v, f);
-    if (p.out0 != nullptr) store_bf16x32(p.out0 + r * p.ld0 + n, f);
-    if (act_is_gated(p.act)) {
-      float y[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        float a, da;
-        act_value_grad(p.act, f[2 * j], a, da);
-        y[j] = a * f[2 * j + 1];
-      }
-      __nv_bfloat16* dst1 = p.out1 + r * p.ld1 + (n >> 1);
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        reinterpret_cast<uint4*>(dst1)[j] = make_uint4(pack_bf16(y[8 * j], y[8 * j + 1]), pack_bf16(y[8 * j + 2], y[8 * j + 3]),
-                                                       pack_bf16(y[8 * j + 4], y[8 * j + 5]), pack_bf16(y[8 * j + 6], y[8 * j + 7]));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        float a, da;
-        act_value_grad(p.act, f[j], a, da);
-        f[j] = a;
-      }
-      store_bf16x32(p.out1 + r * p.ld1 + n, f);
-    }
-  } else if constexpr (EPI == EPI_DACT) {
-    // acc[., i] = dy1[r, i]
-    if (act_is_gated(p.act)) {
-      const uint4* zsrc = reinterpret_cast<const uint4*>(p.z + static_cast<long long>(r) * (2ll * p.N) + 2 * n);
-      __nv_bfloat16* dz_dst = p.out0 + r * p.ld0 + 2 * n;
-      __nv_bfloat16* ys_dst = p.out1 + r * p.ld1 + n;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint4 za = zsrc[2 * j], zb = zsrc[2 * j + 1];
-        const uint32_t zw[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
-        uint32_t dzw[8];
-        float ys[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const __nv_bfloat162 gu = *reinterpret_cast<const __nv_bfloat162*>(&zw[i]);
-          const float g = __low2float(gu), u = __high2float(gu);
-          const float dy = __uint_as_float(v[8 * j + i]);
-          float a, da;
-          act_value_grad(p.act, g, a, da);
-          const float y1 = a * u;
-          ds_acc += dy * y1;
-          dzw[i] = pack_bf16(dy * u * da * score, dy * a * score);
-          ys[i] = y1 * score;
-        }
-        reinterpret_cast<uint4*>(dz_dst)[2 * j] = make_uint4(dzw[0], dzw[1], dzw[2], dzw[3]);
-        reinterpret_cast<uint4*>(dz_dst)[2 * j + 1] = make_uint4(dzw[4], dzw[5], dzw[6], dzw[7]);
-        reinterpret_cast<uint4*>(ys_dst)[j] = make_uint4(pack_bf16(ys[0], ys[1]), pack_bf16(ys[2], ys[3]),
-                                                         pack_bf16(ys[4], ys[5]), pack_bf16(ys[6], ys[7]));
-      }
-    } else {
-      const uint4* zsrc = reinterpret_cast<const uint4*>(p.z + static_cast<long long>(r) * p.N + n);
-      float dzf[32], ysf[32];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint4 zq = zsrc[j];
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&zq);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float zval = (i & 1) ? __high2float(h[i >> 1]) : __low2float(h[i >> 1]);
-          const float dy = __uint_as_float(v[8 * j + i]);
-          float a, da;
-          act_value_grad(p.act, zval, a, da);
-          ds_acc += dy * a;
-          dzf[8 * j + i] = dy * da * score;
-          ysf[8 * j + i] = a * score;
-        }
-      }
-      store_bf16x32(p.out0 + r * p.ld0 + n, dzf);
-      store_bf16x32(p.out1 + r * p.ld1 + n, ysf);
-    }
   } else if constexpr (EPI == EPI_STORE_ROWS) {
     __nv_bfloat16* dst = p.out0 + static_cast<long long>(p.gather[r]) * p.ld0 + n;
     float f[32];
@@ -481,6 +393,204 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int expert, 
                    "f"(score * __uint_as_float(v[4 * j + 0])), "f"(score * __uint_as_float(v[4 * j + 1])),
                    "f"(score * __uint_as_float(v[4 * j + 2])), "f"(score * __uint_as_float(v[4 * j + 3]))
                    : "memory");
+    }
+  }
+}
+
+// The backward activation epilogue of one warp: CHUNKS x 32 accumulator columns (dy1) of its 32 rows.  Reads the saved
+// pre-activation z, writes dz and y1 * score, adds to the row's partial of ds.  acc[., i] = dy1[r, i]; gated: z[r, 2i] =
+// gate, z[r, 2i+1] = up.  All row traffic goes through the warp's staging rows in whole 64-byte segments, and the next
+// chunk's z is in flight while this one is worked on: the first one's before the accumulator is waited for.  Lane l owns
+// row row_base + l; rows at or past row_end read zeros and store nothing.
+// Bound by latency, not by arithmetic: four warps without the z pipeline needed 25 us for a 256 x 256 tile (dH of
+// T 24576, H 1536, I 256, E 128, K 8: 284 us), more than the MMAs of a reduction of 4096.
+template <int FN, bool GATED, int CHUNKS, class Wait, class Release>
+__device__ __forceinline__ bool dact_columns(const GemmParams& p, uint32_t stage, int lane, int row_base, int row_end,
+                                             int n_first, uint32_t t_addr, float score, float& ds_acc, Wait&& wait_acc,
+                                             Release&& release_acc) {
+  constexpr int ZW = GATED ? 2 : 1;          // z columns per accumulator column
+  constexpr int ROWS = GATED ? 4 : 8;        // rows that one load instruction of the warp covers
+  constexpr int PIECES = 32 / ROWS;          // 16-byte pieces per row and chunk
+  const __nv_bfloat16* z = p.z + 8 * (lane % PIECES);
+  const long long z_ld = static_cast<long long>(ZW) * p.N;
+  uint4 vz[4 * ZW];
+  auto fetch_z = [&](int n) {
+#pragma unroll
+    for (int i = 0; i < 4 * ZW; ++i) {
+      const int r = row_base + ROWS * i + lane / PIECES;
+      vz[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < row_end) vz[i] = *reinterpret_cast<const uint4*>(z + r * z_ld + ZW * n);
+    }
+  };
+  if (n_first < p.N) {
+    fetch_z(n_first);
+    // the other chunks' pieces of this lane's row: have the L2 fetch them meanwhile
+    if (row_base + lane < row_end)
+      prefetch_l2_lines(p.z + (row_base + lane) * z_ld + ZW * n_first, min(CHUNKS * 32, p.N - n_first) * ZW * 2 / 128);
+  }
+  if (!wait_acc()) return false;
+  if (n_first >= p.N) release_acc();
+#pragma unroll 1
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int n = n_first + 32 * c;
+    if (n >= p.N) break;
+    uint32_t v[32], zw[16 * ZW];
+    tmem_ld32(t_addr + 32 * c, v);
+#pragma unroll
+    for (int h = 0; h < ZW; ++h) {  // 64 bytes of every row at a time
+#pragma unroll
+      for (int i = 0; i < 4 * ZW; ++i)
+        if (!GATED || ((lane >> 2) & 1) == h)
+          st_shared_v4(stage_piece(stage, ROWS * i + lane / PIECES, lane & 3), vz[i].x, vz[i].y, vz[i].z, vz[i].w);
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 t = ld_shared_v4(stage_piece(stage, lane, q));
+        zw[16 * h + 4 * q] = t.x; zw[16 * h + 4 * q + 1] = t.y; zw[16 * h + 4 * q + 2] = t.z; zw[16 * h + 4 * q + 3] = t.w;
+      }
+      __syncwarp();
+    }
+    const bool more = c + 1 < CHUNKS && n + 32 < p.N;
+    if (more) fetch_z(n + 32);
+    tmem_ld_wait();
+    if (!more) release_acc();
+    uint32_t out[16];
+    if constexpr (GATED) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const __nv_bfloat162 gu = *reinterpret_cast<const __nv_bfloat162*>(&zw[i]);
+        const float g = __low2float(gu), u = __high2float(gu);
+        const float dy = __uint_as_float(v[i]);
+        float a, da;
+        act_value_grad<FN>(g, a, da);
+        const float y1 = a * u;
+        ds_acc += dy * y1;
+        zw[i] = pack_bf16(dy * u * da * score, dy * a * score);
+        v[i] = __float_as_uint(y1 * score);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) out[j] = zw[16 * h + j];
+        warp_store_rows64(stage, lane, out, p.out0, p.ld0, row_base, row_end, 2 * n + 32 * h);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const __nv_bfloat162 zz = *reinterpret_cast<const __nv_bfloat162*>(&zw[i]);
+        const float d0 = __uint_as_float(v[2 * i]), d1 = __uint_as_float(v[2 * i + 1]);
+        float a0, da0, a1, da1;
+        act_value_grad<FN>(__low2float(zz), a0, da0);
+        act_value_grad<FN>(__high2float(zz), a1, da1);
+        ds_acc += d0 * a0;
+        ds_acc += d1 * a1;
+        out[i] = pack_bf16(d0 * da0 * score, d1 * da1 * score);
+        v[2 * i] = __float_as_uint(a0 * score);
+        v[2 * i + 1] = __float_as_uint(a1 * score);
+      }
+      warp_store_rows64(stage, lane, out, p.out0, p.ld0, row_base, row_end, n);
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) out[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+    warp_store_rows64(stage, lane, out, p.out1, p.ld1, row_base, row_end, n);
+  }
+  return true;
+}
+
+// The forward activation epilogue of one warp, laid out like dact_columns: z = acc (+ bias) unless p.out0 is null,
+// y1 = act(z) (gated: act(even) * odd; two chunks make one 64-byte segment of y1, N is a multiple of 128).
+template <int FN, bool GATED, int CHUNKS, class Release>
+__device__ __forceinline__ void act_columns(const GemmParams& p, int expert, uint32_t stage, int lane, int row_base,
+                                            int row_end, int n_first, uint32_t t_addr, Release&& release_acc) {
+  if (n_first >= p.N) release_acc();
+  uint32_t first_half[8];
+#pragma unroll 1
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int n = n_first + 32 * c;
+    if (n >= p.N) break;
+    uint32_t v[32], out[16];
+    tmem_ld32(t_addr + 32 * c, v);
+    tmem_ld_wait();
+    if (c + 1 == CHUNKS || n + 32 >= p.N) release_acc();
+    float f[32];
+    load_biased(p, expert, n, v, f);
+    if (p.out0 != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) out[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
+      warp_store_rows64(stage, lane, out, p.out0, p.ld0, row_base, row_end, n);
+    }
+    if constexpr (GATED) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float a, da;
+        act_value_grad<FN>(f[2 * j], a, da);
+        f[j] = a * f[2 * j + 1];
+      }
+      if ((c & 1) == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) first_half[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          out[j] = first_half[j];
+          out[8 + j] = pack_bf16(f[2 * j], f[2 * j + 1]);
+        }
+        warp_store_rows64(stage, lane, out, p.out1, p.ld1, row_base, row_end, (n - 32) >> 1);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float a0, a1, da;
+        act_value_grad<FN>(f[2 * j], a0, da);
+        act_value_grad<FN>(f[2 * j + 1], a1, da);
+        out[j] = pack_bf16(a0, a1);
+      }
+      warp_store_rows64(stage, lane, out, p.out1, p.ld1, row_base, row_end, n);
+    }
+  }
+}
+
+// One 32-column piece of a warp's 32 accumulator rows for the epilogues that store it as it is: v[j] = acc[r, n + j] of
+// lane l's row r = row_base + l (ragged-K: the output row inside the expert's matrix).  Every lane must call.
+// `dst_row`: EPI_STORE_ROWS, the lane's source row.
+template <int EPI, bool RAGGED_K>
+__device__ __forceinline__ void store_chunk(const GemmParams& p, int expert, uint32_t stage, int lane, int row_base,
+                                            int row_end, int n, const uint32_t (&v)[32], float score, int dst_row) {
+  if constexpr (EPI == EPI_SCATTER) {
+    if (row_base + lane >= row_end) return;
+    float* dst = p.acc_out + static_cast<long long>(dst_row) * p.N + n;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * j),
+                   "f"(score * __uint_as_float(v[4 * j + 0])), "f"(score * __uint_as_float(v[4 * j + 1])),
+                   "f"(score * __uint_as_float(v[4 * j + 2])), "f"(score * __uint_as_float(v[4 * j + 3]))
+                   : "memory");
+    }
+  } else {
+    float f[32];
+    if constexpr (EPI == EPI_STORE_BIAS) {
+      load_biased(p, expert, n, v, f);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+    }
+    if constexpr (EPI == EPI_STORE_ROWS) {
+      if (p.scores != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) f[j] = score * __bfloat162float(__float2bfloat16_rn(f[j]));
+      }
+    }
+    uint32_t w[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) w[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
+    if constexpr (EPI == EPI_STORE_ROWS) {
+      warp_store_segments64(stage, lane, w, false, [&](int rr) {
+        const int row = __shfl_sync(0xffffffffu, dst_row, rr);
+        return row_base + rr < row_end ? p.out0 + row * p.ld0 + n : nullptr;
+      });
+    } else {
+      warp_store_rows64(stage, lane, w, p.out0 + (RAGGED_K ? expert * p.out0_expert_stride : 0ll), p.ld0, row_base,
+                               row_end, n, EPI == EPI_STORE && p.accumulate);
     }
   }
 }

@@ -69,17 +69,18 @@ static bool use_dual_tiles() {
   return v;
 }
 
-template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI, int EW, int GW,
+template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI, int GW,
           int DUAL = pair::DUAL_NONE>
 static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
-  auto kernel = pair::grouped_gemm_pair_kernel<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, EW, GW, DUAL>;
+  auto kernel = pair::grouped_gemm_pair_kernel<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, GW, DUAL>;
+  constexpr bool kSplit = pair::splits_registers(EPI, DUAL);
   static PerDeviceFlag configured;
   const int dev = current_device();
   if (dev < 0) return SMOE_ERR_DRIVER;
   if (!configured.test(dev)) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES) != cudaSuccess)
       return SMOE_ERR_LAUNCH;
-    if (DUAL != pair::DUAL_NONE) {
+    if (kSplit) {
       // the kernel re-partitions registers between its warpgroups (setmaxnreg 56 / 200 around 128): that only
       // balances if it was compiled to exactly 128 registers per thread -- refuse to launch otherwise
       cudaFuncAttributes fa;
@@ -91,7 +92,7 @@ static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   if (sms < 2) return SMOE_ERR_DRIVER;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1), 1, 1);
-  cfg.blockDim = dim3(pair::threads(EW, GW, DUAL != pair::DUAL_NONE), 1, 1);
+  cfg.blockDim = dim3(pair::threads(GW, kSplit), 1, 1);
   cfg.dynamicSmemBytes = pair::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -104,13 +105,12 @@ static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   return cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p) == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 
-// Kernels without a gathered operand: 4 epilogue warps.  Kernels with one: dual tiles (8 epilogue + 4 gather
-// warps) where they pay, else single tiles with 4 epilogue + 8 gather warps.
+// Kernels without a gathered operand work on single tiles, kernels with one on dual tiles where they pay.
 template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
   constexpr bool kGather = A_GATHER || B_GATHER;
   if constexpr (!kGather) {
-    return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 4, 0>(tmA, tmB, p, stream);
+    return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 0>(tmA, tmB, p, stream);
   } else {
     // not when the doubled dimension is so far from a multiple of 512 that the half-empty last unit wastes more
     // than an eighth of the MMA work (e.g. N = 768)
@@ -119,14 +119,17 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
     // The activation-gradient epilogues keep single tiles: with both accumulators belonging to one unit the next
     // unit's second MMA group waits for the first accumulator's dSwiGLU pass.  Measured at the benchmark shape with
     // that pass staged through shared memory like the single-tile one: step 17.75-17.97 ms dual against 17.88-18.13 ms
-    // single in alternating runs, the kernel alone 2.26-2.69 against 2.09-2.58 ms -- no gain worth a second variant.
-    if constexpr (EPI != EPI_DSWIGLU && EPI != EPI_DACT) {
+    // single in alternating runs, the kernel alone 2.26-2.69 against 2.09-2.58 ms -- no gain worth a second variant.  The general forward epilogue is
+    // too long to be worked off from registers, and must not hold accumulators that the next unit needs.
+    if constexpr (EPI != EPI_DSWIGLU && EPI != EPI_DACT && EPI != EPI_ACT) {
     if (use_dual_tiles() && fits) {
       constexpr int kDual = A_GATHER ? pair::DUAL_N : pair::DUAL_M;
-      return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 8, 4, kDual>(tmA, tmB, p, stream);
+      return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 4, kDual>(tmA, tmB, p, stream);
     }
     }
-    return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 4, 8>(tmA, tmB, p, stream);
+    // plain stores leave registers for eight gather warps (four: dW2 at H 1536, I 256, 1536 rows per expert 206 us, eight 175)
+    constexpr int kGatherWarps = EPI == EPI_STORE ? 8 : 4;
+    return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, kGatherWarps>(tmA, tmB, p, stream);
   }
 }
 

@@ -74,10 +74,9 @@ struct SharedStorage {
 
 // Output staging: 32 rows x 80 bytes per epilogue warp, so that bf16 outputs leave as 64-byte row segments (8 rows
 // per store instruction) instead of one row per lane (see warp_store_rows64 in epilogue.cuh).
-constexpr int STAGE_OUT_PITCH = 80;
-constexpr int STAGE_OUT_BYTES = EPI_WARPS * 32 * STAGE_OUT_PITCH;  // 20 KiB
+constexpr int STAGE_OUT_BYTES = EPI_WARPS * STAGE_ROWS_BYTES;  // 16 KiB
 constexpr int SMEM_BYTES = 1024 + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + SF_SETS * SF_SET_BYTES +
-                           ((sizeof(SharedStorage) + 15) & ~15) + STAGE_OUT_BYTES;
+                           ((sizeof(SharedStorage) + 127) & ~127) + STAGE_OUT_BYTES;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
 
 // Instruction descriptor of the block-scaled kinds: no accumulator-format field (always fp32); scale-factor
@@ -126,7 +125,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   uint8_t* sB = smem + STAGES * A_STAGE_BYTES;
   uint8_t* sSF = smem + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES);
   SharedStorage& ss = *reinterpret_cast<SharedStorage*>(sSF + SF_SETS * SF_SET_BYTES);
-  uint8_t* stage_out = reinterpret_cast<uint8_t*>(&ss) + ((sizeof(SharedStorage) + 15) & ~15);
+  uint8_t* stage_out = reinterpret_cast<uint8_t*>(&ss) + ((sizeof(SharedStorage) + 127) & ~127);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -370,7 +369,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     const int quad = warp & 3;
     const int col_half = (warp - FIRST_EPI_WARP) >> 2;
     const int row_in_tile = quad * 32 + lane;
-    const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * (32 * STAGE_OUT_PITCH);
+    const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * STAGE_ROWS_BYTES;
     uint32_t acc_phase = 0;
     bool ok = true;
     Tile tile;
@@ -408,9 +407,9 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
           if (cols_ok) {  // warp-uniform; rows past the expert's end read zeros and store nothing
             auto quantise_block = [&](uint32_t (&a)[32], uint32_t (&b)[32], int n) {
               float amax = 0.f;
-              dswiglu_chunk_staged<true, STAGE_OUT_PITCH>(p, my_stage, lane, r - lane, tile.row_end, n, a, score, ds_acc,
+              dswiglu_chunk_staged<true>(p, my_stage, lane, r - lane, tile.row_end, n, a, score, ds_acc,
                                                           amax);
-              dswiglu_chunk_staged<true, STAGE_OUT_PITCH>(p, my_stage, lane, r - lane, tile.row_end, n + 32, b, score,
+              dswiglu_chunk_staged<true>(p, my_stage, lane, r - lane, tile.row_end, n + 32, b, score,
                                                           ds_acc, amax);
               if (!row_ok) return;
               float inv;
@@ -453,7 +452,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
               uint32_t zp[16];
 #pragma unroll
               for (int j = 0; j < 16; ++j) zp[j] = pack_bf16(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
-              warp_store_rows64<STAGE_OUT_PITCH>(my_stage, lane, zp, p.out0, p.ld0, r - lane, tile.row_end, n);
+              warp_store_rows64(my_stage, lane, zp, p.out0, p.ld0, r - lane, tile.row_end, n);
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j) {  // gate = even column, up = odd column
@@ -497,11 +496,11 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         if (!done && cols_ok) {
           done = true;
           float unused = 0.f;
-          dswiglu_chunk_staged<false, STAGE_OUT_PITCH>(p, my_stage, lane, r - lane, tile.row_end, ncol0, v0, score, ds_acc, unused);
-          dswiglu_chunk_staged<false, STAGE_OUT_PITCH>(p, my_stage, lane, r - lane, tile.row_end, ncol0 + 32, v1, score, ds_acc, unused);
+          dswiglu_chunk_staged<false>(p, my_stage, lane, r - lane, tile.row_end, ncol0, v0, score, ds_acc, unused);
+          dswiglu_chunk_staged<false>(p, my_stage, lane, r - lane, tile.row_end, ncol0 + 32, v1, score, ds_acc, unused);
           if (ncol0 + 64 < p.N) {
-            dswiglu_chunk_staged<false, STAGE_OUT_PITCH>(p, my_stage, lane, r - lane, tile.row_end, ncol0 + 64, v2, score, ds_acc, unused);
-            dswiglu_chunk_staged<false, STAGE_OUT_PITCH>(p, my_stage, lane, r - lane, tile.row_end, ncol0 + 96, v3, score, ds_acc, unused);
+            dswiglu_chunk_staged<false>(p, my_stage, lane, r - lane, tile.row_end, ncol0 + 64, v2, score, ds_acc, unused);
+            dswiglu_chunk_staged<false>(p, my_stage, lane, r - lane, tile.row_end, ncol0 + 96, v3, score, ds_acc, unused);
           }
         }
       }
@@ -512,7 +511,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
             uint32_t w[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) w[j] = pack_bf16(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
-            warp_store_rows64<STAGE_OUT_PITCH>(my_stage, lane, w, p.out0, p.ld0, r - lane, tile.row_end, n);
+            warp_store_rows64(my_stage, lane, w, p.out0, p.ld0, r - lane, tile.row_end, n);
           };
           store32(v0, ncol0);
           store32(v1, ncol0 + 32);

@@ -14,8 +14,8 @@
 //   0        TMA producer for the operands that are not gathered (both CTAs; completion bytes are counted
 //            on the leader CTA's "full" barrier)
 //   1        leader CTA: MMA issuer.  other CTA: idle
-//   2..      EW epilogue warps (4 or 8)
-//   2+EW..   GW gather warps (0, 4 or 8): the routed rows of the gathered operand by TMA tile::gather4, issued
+//   2..      8 epilogue warps (each 32 rows x 128 columns)
+//   10..     GW gather warps (0, 4 or 8): the routed rows of the gathered operand by TMA tile::gather4, issued
 //            from 32 threads spread over these warps (gather4 operations issued by one warp are serialised)
 //
 // Barriers.  full[s]: leader only; one arrival (the leader's expect_tx), tx = TMA bytes of both CTAs,
@@ -39,11 +39,16 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;       // 16 KiB
 constexpr int B_STAGE_BYTES = BN_CTA * BK * 2;   // 16 KiB
 constexpr int CHUNK_BYTES = BK * 128;            // 64-element MN chunk: BK rows x 128 B
 constexpr int MAX_EXPERTS = 1024;
+constexpr int EPI_WARPS = 8;
 
-// DUAL kernels keep warps 2 and 3 idle so that every role fills whole warpgroups (setmaxnreg is a warpgroup-wide
-// instruction): warps 0-3 producer / MMA, 4-11 epilogue, 12-15 gather.
-__host__ __device__ constexpr int threads(int epi_warps, int gather_warps, bool dual = false) {
-  return 32 * ((dual ? 4 : 2) + epi_warps + gather_warps);
+// Kernels whose epilogue warps need more than 128 registers (a whole accumulator piece held by each thread, or z of two
+// chunks beside the activation's arithmetic) move registers to them with setmaxnreg.  That is a warpgroup-wide
+// instruction, so these keep warps 2 and 3 idle: warps 0-3 producer / MMA, 4-11 epilogue, 12-15 gather.
+__host__ __device__ constexpr bool splits_registers(int epi, int dual) {
+  return dual != 0 || epi == EPI_DSWIGLU || epi == EPI_DACT || epi == EPI_ACT;
+}
+__host__ __device__ constexpr int threads(int gather_warps, bool split) {
+  return 32 * ((split ? 4 : 2) + EPI_WARPS + gather_warps);
 }
 
 struct SharedStorage {
@@ -53,20 +58,16 @@ struct SharedStorage {
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
+  int off[MAX_EXPERTS + 1];            // first grouped row of every expert
   int m_tile_prefix[MAX_EXPERTS + 1];  // ragged-M: exclusive prefix of ceil(count / 256) per expert
 };
 
-// Output staging of the plain-store epilogues: each epilogue warp owns 32 rows x (payload + 16 B pad).  A thread
-// writes its accumulator row there, the warp reads it back so that consecutive lanes hold consecutive 16-byte pieces
-// of one row, and stores whole 64- or 128-byte row segments: 4 or 8 requests to L2 per store instruction instead of
-// 32 (with one row per lane the epilogue sent about as many requests to L2 as the main loop's operand fetches and
-// competed with them).  Single tiles (4 epilogue warps): 128-byte payload; dual tiles (8 warps): 64-byte payload.
-constexpr int STAGE_OUT_PITCH_WIDE = 144;    // 128 B payload: row r starts 36 words after row r-1 -> conflict-free
-constexpr int STAGE_OUT_PITCH_NARROW = 80;   // 64 B payload
-constexpr int STAGE_OUT_BYTES = 8 * 32 * STAGE_OUT_PITCH_NARROW;  // 20480 >= 4 * 32 * 144
-static_assert(4 * 32 * STAGE_OUT_PITCH_WIDE <= STAGE_OUT_BYTES, "staging area");
+// Output staging of the epilogues: each epilogue warp has 32 rows of 64 bytes (epilogue.cuh), through which a tile leaves
+// in whole 64-byte row segments: 8 requests to L2 per store instruction instead of 32 (with one row per lane the epilogue
+// sent about as many requests to L2 as the main loop's operand fetches and competed with them).
+constexpr int STAGE_OUT_BYTES = EPI_WARPS * STAGE_ROWS_BYTES;
 constexpr int SMEM_BYTES =
-    1024 + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + ((sizeof(SharedStorage) + 15) & ~15) + STAGE_OUT_BYTES;
+    1024 + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + ((sizeof(SharedStorage) + 127) & ~127) + STAGE_OUT_BYTES;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
 
 struct Tile {
@@ -80,78 +81,93 @@ struct Tile {
 
 enum { DUAL_NONE = 0, DUAL_N = 1, DUAL_M = 2 };
 
-// num_n counts work units along N (DUAL_N: 512 columns each).
-template <bool RAGGED_K, int DUAL = DUAL_NONE>
-__device__ __forceinline__ bool decode_tile(const GemmParams& p, const SharedStorage& ss, long long t, int num_n,
-                                            uint32_t rank, Tile& tile) {
-  constexpr int UNIT_N = DUAL == DUAL_N ? 2 * BN : BN;
-  constexpr int UNIT_M = DUAL == DUAL_M ? 4 * BM : 2 * BM;
-  if constexpr (!RAGGED_K) {
-    const int total_m = ss.m_tile_prefix[p.E];
-    if (t >= static_cast<long long>(total_m) * num_n) return false;
-    const int mi = static_cast<int>(t / num_n);
-    const int ni = static_cast<int>(t % num_n);
-    int lo = 0, hi = p.E;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (ss.m_tile_prefix[mid] <= mi) lo = mid; else hi = mid;
+// The work units of one cluster, in the order in which every role of its CTAs walks them.  Each warp keeps its own
+// walker; all lanes must call next().  All state is in registers and shared memory: with 64-bit divisions, a binary
+// search and two dependent global loads per unit, finding a unit took longer than the MMAs of a short reduction.
+// Units go expert by expert, row tiles outermost, and are dealt out round-robin.
+template <bool RAGGED_K, int DUAL>
+struct UnitWalker {
+  static constexpr int UNIT_N = DUAL == DUAL_N ? 2 * BN : BN;
+  static constexpr int UNIT_M = DUAL == DUAL_M ? 4 * BM : 2 * BM;
+  const GemmParams& p;
+  const SharedStorage& ss;
+  const int cluster, clusters, lane, num_n;
+  int total;         // units of the whole grid
+  int per_expert;    // ragged-K: units per expert
+  int round = 0;
+  int mi, ni, e = 0;  // ragged-M: row tile, unit along N and expert of the next unit
+  int step_m, step_n;
+
+  __device__ __forceinline__ UnitWalker(const GemmParams& p_, const SharedStorage& ss_, int lane_)
+      : p(p_), ss(ss_), cluster(blockIdx.x >> 1), clusters(gridDim.x >> 1), lane(lane_),
+        num_n((p_.N + UNIT_N - 1) / UNIT_N) {
+    if constexpr (RAGGED_K) {
+      per_expert = (p.M + UNIT_M - 1) / UNIT_M * num_n;
+      total = per_expert * p.E;
+    } else {
+      total = ss.m_tile_prefix[p.E] * num_n;
+      mi = cluster / num_n;
+      ni = cluster % num_n;
+      step_m = clusters / num_n;
+      step_n = clusters % num_n;
     }
-    tile.e = lo;
-    tile.row0 = p.off[lo] + (mi - ss.m_tile_prefix[lo]) * (2 * BM) + static_cast<int>(rank) * BM;
-    tile.row_end = p.off[lo + 1];
-    tile.n0 = ni * UNIT_N;
-    tile.k_begin = 0;
-    tile.k_end = p.K;
-    tile.num_kb = p.K / BK;
+  }
+  __device__ __forceinline__ int unit_of_round() const {
+    return round * clusters + cluster;
+  }
+  // Number of k-blocks of the next unit, or -1 when there is none (all that the MMA issuer wants to know).
+  __device__ __forceinline__ int next_num_kb() {
+    const int t = unit_of_round();
+    if (t >= total) return -1;
+    ++round;
+    if constexpr (!RAGGED_K) {
+      return p.K / BK;
+    } else {
+      const int ex = t / per_expert;
+      return (ss.off[ex + 1] - ss.off[ex] + BK - 1) / BK;
+    }
+  }
+  __device__ __forceinline__ bool next(uint32_t rank, Tile& tile) {
+    const int t = unit_of_round();
+    if (t >= total) return false;
+    ++round;
+    if constexpr (!RAGGED_K) {
+      while (true) {  // the first expert whose tiles end beyond mi, 32 experts at a time
+        const int i = e + 1 + lane;
+        const unsigned before = __ballot_sync(0xffffffffu, i <= p.E && ss.m_tile_prefix[i] <= mi);
+        e += __popc(before);
+        if (before != 0xffffffffu) break;
+      }
+      tile.e = e;
+      tile.row0 = ss.off[e] + (mi - ss.m_tile_prefix[e]) * (2 * BM) + static_cast<int>(rank) * BM;
+      tile.row_end = ss.off[e + 1];
+      tile.n0 = ni * UNIT_N;
+      tile.k_begin = 0;
+      tile.k_end = p.K;
+      tile.num_kb = p.K / BK;
+      mi += step_m;
+      ni += step_n;
+      if (ni >= num_n) {
+        ni -= num_n;
+        ++mi;
+      }
+    } else {
+      const int i = t / per_expert, rem = t - i * per_expert, m = rem / num_n;
+      tile.e = i;
+      tile.row0 = m * UNIT_M + static_cast<int>(rank) * BM;
+      tile.row_end = p.M;
+      tile.n0 = (rem - m * num_n) * UNIT_N;
+      tile.k_begin = ss.off[tile.e];
+      tile.k_end = ss.off[tile.e + 1];
+      tile.num_kb = (tile.k_end - tile.k_begin + BK - 1) / BK;
+    }
     return true;
-  } else {
-    const int num_m = (p.M + UNIT_M - 1) / UNIT_M;
-    const long long per_e = static_cast<long long>(num_m) * num_n;
-    if (t >= per_e * p.E) return false;
-    const int e = static_cast<int>(t / per_e);
-    const int rem = static_cast<int>(t % per_e);
-    tile.e = e;
-    tile.row0 = (rem / num_n) * UNIT_M + static_cast<int>(rank) * BM;
-    tile.row_end = p.M;
-    tile.n0 = (rem % num_n) * UNIT_N;
-    tile.k_begin = p.off[e];
-    tile.k_end = p.off[e + 1];
-    tile.num_kb = (tile.k_end - tile.k_begin + BK - 1) / BK;
-    return true;
   }
-}
+};
 
-// What the MMA issuer needs to know about work unit t: whether it exists and how many k-blocks it has.  The full
-// decode_tile (a 64-bit division, a binary search and two dependent global loads) would sit between the last MMA of
-// one tile and the first of the next; for ragged-M the k-block count is a constant, for ragged-K the expert's token
-// range is fetched one unit ahead by the caller.
-template <bool RAGGED_K, int DUAL>
-__device__ __forceinline__ long long num_units(const GemmParams& p, const SharedStorage& ss, int num_n) {
-  if constexpr (!RAGGED_K) {
-    return static_cast<long long>(ss.m_tile_prefix[p.E]) * num_n;
-  } else {
-    constexpr int UNIT_M = DUAL == DUAL_M ? 4 * BM : 2 * BM;
-    const int num_m = (p.M + UNIT_M - 1) / UNIT_M;
-    return static_cast<long long>(num_m) * num_n * p.E;
-  }
-}
-
-template <bool RAGGED_K, int DUAL>
-__device__ __forceinline__ int unit_num_kb(const GemmParams& p, long long t, long long total, int num_n) {
-  if (t >= total) return 0;
-  if constexpr (!RAGGED_K) {
-    return p.K / BK;
-  } else {
-    constexpr int UNIT_M = DUAL == DUAL_M ? 4 * BM : 2 * BM;
-    const int num_m = (p.M + UNIT_M - 1) / UNIT_M;
-    const int e = static_cast<int>(t / (static_cast<long long>(num_m) * num_n));
-    return (p.off[e + 1] - p.off[e] + BK - 1) / BK;
-  }
-}
-
-template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI, int EW, int GW,
+template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI, int GW,
           int DUAL = DUAL_NONE>
-__global__ void __launch_bounds__(threads(EW, GW, DUAL != 0), 1)
+__global__ void __launch_bounds__(threads(GW, splits_registers(EPI, DUAL)), 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const GemmParams p) {
   // DUAL: four stages of three 16 KiB tiles (A, B and the second plain tile X) instead of six stages of two
@@ -165,27 +181,23 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   uint8_t* sB = smem + NSTAGES * A_STAGE_BYTES;
   uint8_t* sX = sB + NSTAGES * B_STAGE_BYTES;
   SharedStorage& ss = *reinterpret_cast<SharedStorage*>(smem + NSTAGES * (A_STAGE_BYTES + B_STAGE_BYTES + X_STAGE_BYTES));
-  uint8_t* stage_out = reinterpret_cast<uint8_t*>(&ss) + ((sizeof(SharedStorage) + 15) & ~15);
+  uint8_t* stage_out = reinterpret_cast<uint8_t*>(&ss) + ((sizeof(SharedStorage) + 127) & ~127);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool leader = rank == 0;
-  const long long first_tile = blockIdx.x >> 1;
-  const long long tile_step = gridDim.x >> 1;
   volatile int* abort_flag = &ss.abort_flag;
-  constexpr int UNIT_N = DUAL == DUAL_N ? 2 * BN : BN;
-  const int num_n = (p.N + UNIT_N - 1) / UNIT_N;
 
   constexpr bool kGather = A_GATHER || B_GATHER;
   static_assert(!(A_GATHER && B_GATHER), "at most one operand is gathered");
   static_assert(!kGather || GW > 0, "a gathered operand needs gather warps");
-  static_assert(EW == 4 || EW == 8, "4 or 8 epilogue warps");
-  static_assert(GW == 0 || GW == 4 || GW == 8 || GW == 16, "0, 4, 8 or 16 gather warps");
+  static_assert(GW == 0 || GW == 4 || GW == 8, "0, 4 or 8 gather warps");
   constexpr int GATHER_THREADS = 32 * GW;
-  constexpr int FIRST_EPI_WARP = DUAL != DUAL_NONE ? 4 : 2;
-  constexpr int FIRST_GATHER_WARP = FIRST_EPI_WARP + EW;
-  static_assert(DUAL == DUAL_NONE || (EW == 8 && GW == 4), "dual tiles: 8 epilogue warps, 4 gather warps (512 threads)");
+  constexpr bool SPLIT_REGS = splits_registers(EPI, DUAL);
+  constexpr int FIRST_EPI_WARP = SPLIT_REGS ? 4 : 2;
+  constexpr int FIRST_GATHER_WARP = FIRST_EPI_WARP + EPI_WARPS;
+  static_assert(!SPLIT_REGS || GW == 4, "4 gather warps (512 threads)");
   constexpr uint32_t kTmaBytesPerCta = A_STAGE_BYTES + B_STAGE_BYTES + X_STAGE_BYTES;  // gathered rows included
 
   // ---- set-up -------------------------------------------------------------------------------
@@ -196,7 +208,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&ss.acc_full[a]), 1);
-      mbar_init(smem_u32(&ss.acc_empty[a]), 2 * EW);
+      mbar_init(smem_u32(&ss.acc_empty[a]), 2 * EPI_WARPS);
     }
     ss.abort_flag = 0;
     fence_mbar_init();
@@ -209,6 +221,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     tmem_alloc(smem_u32(&ss.tmem_base), 2 * BN);  // all 512 columns: both CTAs get the same base
     tmem_relinquish();
   }
+  for (int e = threadIdx.x; e <= p.E; e += blockDim.x) ss.off[e] = p.off[e];
   if constexpr (!RAGGED_K) {
     if (warp == 2) {
       int running = 0;
@@ -234,11 +247,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 
-  // DUAL: the epilogue warps hold 128 accumulator values per thread; registers move to them from the other roles
+  // SPLIT_REGS: registers move to the epilogue warps from the other roles
   // (512 threads x 128 registers at launch; two warpgroups give up 72 registers per thread, two take 72).  Each
   // role branch starts with its own setmaxnreg so that the register limit is known along the whole branch.
   if (warp < FIRST_EPI_WARP) {
-  if constexpr (DUAL != DUAL_NONE) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  if constexpr (SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   // ---- TMA producer -------------------------------------------------------------------------
   if (warp == 0) {
     if constexpr (kTmaBytesPerCta > 0) {
@@ -246,9 +259,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       uint32_t phase = 0;
       bool ok = true;
       Tile tile;
-      for (long long t = first_tile; ok && decode_tile<RAGGED_K, DUAL>(p, ss, t, num_n, rank, tile); t += tile_step) {
+      UnitWalker<RAGGED_K, DUAL> walk(p, ss, lane);
+      while (ok && walk.next(rank, tile)) {
         for (int kb = 0; kb < tile.num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);  // the leader's barrier
           const uint32_t a_dst = smem_u32(sA + stage * A_STAGE_BYTES);
           const uint32_t b_dst = smem_u32(sB + stage * B_STAGE_BYTES);
@@ -294,7 +308,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
   // ---- MMA issuer (leader) / gather relay (other CTA) ----------------------------------------
   else if (warp == 1) {
-    if (leader) {
+    if (leader && lane == 0) {  // one thread: nothing in this loop is warp-wide
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       constexpr uint32_t a_lbo = A_MN ? CHUNK_BYTES : 16;
       constexpr uint32_t b_lbo = B_MN ? CHUNK_BYTES : 16;
@@ -305,11 +319,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      const long long total_units = num_units<RAGGED_K, DUAL>(p, ss, num_n);
-      int next_kb = unit_num_kb<RAGGED_K, DUAL>(p, first_tile, total_units, num_n);
-      for (long long t = first_tile; ok && t < total_units; t += tile_step) {
-        const int num_kb = next_kb;
-        next_kb = unit_num_kb<RAGGED_K, DUAL>(p, t + tile_step, total_units, num_n);  // loads overlap this unit's MMAs
+      UnitWalker<RAGGED_K, DUAL> walk(p, ss, lane);
+      for (int num_kb = walk.next_num_kb(); ok && num_kb >= 0; num_kb = walk.next_num_kb()) {
         if (num_kb == 0) continue;
         if constexpr (DUAL == DUAL_NONE) {
           if (!mbar_wait(smem_u32(&ss.acc_empty[acc]), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
@@ -325,63 +336,53 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           tc_fence_after();
           const uint64_t a_desc = make_smem_desc(smem_u32(sA + stage * A_STAGE_BYTES), a_lbo, 1024);
           const uint64_t b_desc = make_smem_desc(smem_u32(sB + stage * B_STAGE_BYTES), b_lbo, 1024);
-          if (lane == 0) {
 #pragma unroll
-            for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
-              umma_bf16_pair(d_tmem, a_desc + ((k4 * a_kstep) >> 4), b_desc + ((k4 * b_kstep) >> 4), idesc,
-                             (kb > 0 || k4 > 0) ? 1u : 0u);
-            }
+          for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
+            umma_bf16_pair(d_tmem, a_desc + ((k4 * a_kstep) >> 4), b_desc + ((k4 * b_kstep) >> 4), idesc,
+                           (kb > 0 || k4 > 0) ? 1u : 0u);
           }
           if constexpr (DUAL != DUAL_NONE) {
             if (kb == 0) {  // the second accumulator of the previous unit has been copied out
-              __syncwarp();
               if (!mbar_wait(smem_u32(&ss.acc_empty[1]), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
               tc_fence_after();
             }
           }
-          if (lane == 0) {
-            if constexpr (DUAL == DUAL_N) {
-              const uint64_t x_desc = make_smem_desc(smem_u32(sX + stage * X_STAGE_BYTES), b_lbo, 1024);
+          if constexpr (DUAL == DUAL_N) {
+            const uint64_t x_desc = make_smem_desc(smem_u32(sX + stage * X_STAGE_BYTES), b_lbo, 1024);
 #pragma unroll
-              for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
-                umma_bf16_pair(d_tmem + BN, a_desc + ((k4 * a_kstep) >> 4), x_desc + ((k4 * b_kstep) >> 4), idesc,
-                               (kb > 0 || k4 > 0) ? 1u : 0u);
-              }
+            for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
+              umma_bf16_pair(d_tmem + BN, a_desc + ((k4 * a_kstep) >> 4), x_desc + ((k4 * b_kstep) >> 4), idesc,
+                             (kb > 0 || k4 > 0) ? 1u : 0u);
             }
-            if constexpr (DUAL == DUAL_M) {
-              const uint64_t x_desc = make_smem_desc(smem_u32(sX + stage * X_STAGE_BYTES), a_lbo, 1024);
-#pragma unroll
-              for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
-                umma_bf16_pair(d_tmem + BN, x_desc + ((k4 * a_kstep) >> 4), b_desc + ((k4 * b_kstep) >> 4), idesc,
-                               (kb > 0 || k4 > 0) ? 1u : 0u);
-              }
-            }
-            umma_commit_pair(smem_u32(&ss.empty[stage]), 3);  // frees the stage in both CTAs
           }
-          __syncwarp();
+          if constexpr (DUAL == DUAL_M) {
+            const uint64_t x_desc = make_smem_desc(smem_u32(sX + stage * X_STAGE_BYTES), a_lbo, 1024);
+#pragma unroll
+            for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
+              umma_bf16_pair(d_tmem + BN, x_desc + ((k4 * a_kstep) >> 4), b_desc + ((k4 * b_kstep) >> 4), idesc,
+                             (kb > 0 || k4 > 0) ? 1u : 0u);
+            }
+          }
+          umma_commit_pair(smem_u32(&ss.empty[stage]), 3);  // frees the stage in both CTAs
           if (++stage == NSTAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         if constexpr (DUAL == DUAL_NONE) {
-          if (lane == 0) umma_commit_pair(smem_u32(&ss.acc_full[acc]), 3);
-          __syncwarp();
+          umma_commit_pair(smem_u32(&ss.acc_full[acc]), 3);
           if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
         } else {
-          if (lane == 0) {
-            umma_commit_pair(smem_u32(&ss.acc_full[0]), 3);
-            umma_commit_pair(smem_u32(&ss.acc_full[1]), 3);
-          }
-          __syncwarp();
+          umma_commit_pair(smem_u32(&ss.acc_full[0]), 3);
+          umma_commit_pair(smem_u32(&ss.acc_full[1]), 3);
           acc_phase ^= 1u;
         }
       }
-      if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_MMA);
+      if (!ok && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_MMA);
     }
   }
-  }  // warps below FIRST_EPI_WARP (DUAL: warps 2 and 3 idle)
+  }  // warps below FIRST_EPI_WARP (SPLIT_REGS: warps 2 and 3 idle)
   // ---- gather producers ----------------------------------------------------------------------
   else if (warp >= FIRST_GATHER_WARP) {
-    if constexpr (DUAL != DUAL_NONE) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if constexpr (SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if constexpr (kGather) {
       const int gt = threadIdx.x - 32 * FIRST_GATHER_WARP;
       int stage = 0;
@@ -397,7 +398,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         const CUtensorMap* tm = A_GATHER ? &tmA : &tmB;
         uint8_t* stage_base = A_GATHER ? sA : sB;
         constexpr int STAGE_BYTES = A_GATHER ? A_STAGE_BYTES : B_STAGE_BYTES;
-        for (long long t = first_tile; ok && decode_tile<RAGGED_K, DUAL>(p, ss, t, num_n, rank, tile); t += tile_step) {
+        UnitWalker<RAGGED_K, DUAL> walk(p, ss, lane);
+        while (ok && walk.next(rank, tile)) {
           if constexpr (!RAGGED_K) {
             int r4[4];
 #pragma unroll
@@ -406,7 +408,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
               r4[i] = (r < p.total_rows) ? p.gather[r] : 0;
             }
             for (int kb = 0; kb < tile.num_kb; ++kb) {
-              if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+              if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
               if (issuer)
                 tma_gather4_pair(tm, map_to_cta(smem_u32(&ss.full[stage]), 0),
                                  smem_u32(stage_base + stage * STAGE_BYTES) + j * 512, kb * BK, r4[0], r4[1], r4[2],
@@ -426,7 +428,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             };
             load_idx(0, cur);
             load_idx(1, nxt);
-            for (int kb = 0; kb < tile.num_kb; ++kb) {
+            for (int kb = 0; kb < tile.num_kb; ++kb) {  // (nothing here is warp-wide)
               if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
               if (issuer)
                 tma_gather4_pair(tm, map_to_cta(smem_u32(&ss.full[stage]), 0),
@@ -445,17 +447,17 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
   // ---- epilogue -----------------------------------------------------------------------------
   else {
-    if constexpr (DUAL != DUAL_NONE) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    if constexpr (SPLIT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
     const int quad = warp & 3;
-    constexpr int COL_SPLIT = EW / 4;
-    constexpr int COLS_PER_WARP = BN / COL_SPLIT;
+    constexpr int COLS_PER_WARP = BN * 4 / EPI_WARPS;
     const int col_half = (warp - FIRST_EPI_WARP) >> 2;
     const int row_in_tile = quad * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
     Tile tile;
-    for (long long t = first_tile; ok && decode_tile<RAGGED_K, DUAL>(p, ss, t, num_n, rank, tile); t += tile_step) {
+    UnitWalker<RAGGED_K, DUAL> walk(p, ss, lane);
+    while (ok && walk.next(rank, tile)) {
       const bool have_acc = tile.num_kb > 0;
       constexpr int SUBTILES = DUAL == DUAL_NONE ? 1 : 2;
       if constexpr (DUAL != DUAL_NONE && EPI == EPI_STORE) {
@@ -468,7 +470,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 #pragma unroll
         for (int sub = 0; sub < 2; ++sub) {
           if (have_acc) {
-            if (!mbar_wait(smem_u32(&ss.acc_full[sub]), acc_phase, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&ss.acc_full[sub]), acc_phase, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t t_addr = tmem_base + sub * BN + (static_cast<uint32_t>(quad * 32) << 16);
 #pragma unroll
@@ -496,7 +498,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (!ok) break;
         {
           // stores: 64-byte row segments through this warp's staging rows (8 rows per store instruction)
-          const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * (32 * STAGE_OUT_PITCH_NARROW);
+          const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * STAGE_ROWS_BYTES;
 #pragma unroll
           for (int sub = 0; sub < 2; ++sub) {
             const int row_base = tile.row0 + (DUAL == DUAL_M ? sub * 2 * BM : 0) + quad * 32;
@@ -506,23 +508,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             for (int c = 0; c < CHUNKS; ++c) {
               const int n = n0 + (col_half * CHUNKS + c) * 32;
               if (n >= p.N) break;
+              uint32_t w[16];
 #pragma unroll
-              for (int q = 0; q < 4; ++q)
-                st_shared_v4(my_stage + lane * STAGE_OUT_PITCH_NARROW + 16 * q, packed[sub][c * 16 + 4 * q],
-                             packed[sub][c * 16 + 4 * q + 1], packed[sub][c * 16 + 4 * q + 2],
-                             packed[sub][c * 16 + 4 * q + 3]);
-              __syncwarp();
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int rr = 8 * i + (lane >> 2);
-                const uint4 w = ld_shared_v4(my_stage + rr * STAGE_OUT_PITCH_NARROW + 16 * (lane & 3));
-                const int r = row_base + rr;
-                if (r < tile.row_end) {
-                  uint4* dst = reinterpret_cast<uint4*>(out + r * p.ld0 + n + 8 * (lane & 3));
-                  *dst = p.accumulate ? add_bf16x8(w, dst) : w;
-                }
-              }
-              __syncwarp();
+              for (int j = 0; j < 16; ++j) w[j] = packed[sub][c * 16 + j];
+              warp_store_rows64(my_stage, lane, w, out, p.ld0, row_base, tile.row_end, n, p.accumulate);
             }
           }
         }
@@ -540,34 +529,39 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           if (row_ok && (EPI != EPI_STORE_ROWS || p.scores != nullptr))
             score = load_score(p.scores, p.scores_are_bf16, p.s_scatter[r]);
         }
-        if constexpr (EPI == EPI_DSWIGLU || EPI == EPI_DACT) {
-          // the epilogue reads this thread's piece of the saved pre-activation row: have the L2 fetch it while the
-          // unit's MMAs are still running
-          if (row_ok && n0 + col_half * COLS_PER_WARP < p.N) {
-            const int zw = (EPI == EPI_DACT && !act_is_gated(p.act)) ? 1 : 2;  // z columns per accumulator column
-            prefetch_l2_lines(p.z + static_cast<long long>(r) * (zw * p.N) + zw * (n0 + col_half * COLS_PER_WARP),
-                              zw * COLS_PER_WARP * 2 / 128);
+        const auto wait_acc = [&] {
+          if (have_acc) {
+            if (!mbar_wait_warp(smem_u32(&ss.acc_full[acc]), acc_phase, abort_flag)) return false;
+            tc_fence_after();
           }
-        }
-        if (have_acc) {
-          if (!mbar_wait(smem_u32(&ss.acc_full[acc]), acc_phase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
+          return true;
+        };
+        // Hands the accumulator back as soon as the last of it is in registers.  Relaxed: what has to be ordered before
+        // it, the tensor-memory reads, is (tcgen05.wait::ld and the fence); a release would also wait for the tile's
+        // global stores, 1800 to 2500 cycles of the 6000 that a plain-store tile took.
+        const auto release_acc = [&] {
+          if (have_acc) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ss.acc_empty[acc]), 0));
+          }
+        };
+        if constexpr (EPI != EPI_DSWIGLU && EPI != EPI_DACT) {  // those wait once their first loads are in flight
+          if (!wait_acc()) { ok = false; break; }
         }
         float ds_acc = 0.f;
         const uint32_t t_addr = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
         if constexpr (DUAL != DUAL_NONE) {
           // Copy this warp's columns of the accumulator into registers and hand the accumulator back at once: the
           // next unit's MMAs need both accumulators, so the epilogue arithmetic and stores must not hold them.
-          static_assert(DUAL == DUAL_NONE || COLS_PER_WARP == 128, "dual tiles use 8 epilogue warps");
+          static_assert(EPI == EPI_SWIGLU || EPI == EPI_STORE, "dual tiles: SwiGLU, and plain stores (done above)");
           constexpr int CHUNKS = COLS_PER_WARP / 32;
           uint32_t v[CHUNKS][32];
           if (have_acc) {
 #pragma unroll
             for (int c = 0; c < CHUNKS; ++c) tmem_ld32(t_addr + (col_half * CHUNKS + c) * 32, v[c]);
             tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ss.acc_empty[acc]), 0));
+            release_acc();
           } else {
 #pragma unroll
             for (int c = 0; c < CHUNKS; ++c)
@@ -578,7 +572,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             // z (unless not wanted) and y1 = silu(gate) * up leave through the warp's staging rows as 64-byte row
             // segments: one per 32 accumulator columns for z, one per 64 for y1 (N = 2I is a multiple of 128, so
             // chunks come in pairs)
-            const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * (32 * STAGE_OUT_PITCH_NARROW);
+            const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * STAGE_ROWS_BYTES;
             const int row_base = r - lane;
             uint32_t yp[16];
 #pragma unroll
@@ -597,137 +591,73 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
               for (int j = 0; j < 8; ++j)
                 yp[(c & 1) * 8 + j] = pack_bf16(__uint_as_float(v[c][2 * j]), __uint_as_float(v[c][2 * j + 1]));
               if (p.out0 != nullptr)
-                warp_store_rows64<STAGE_OUT_PITCH_NARROW>(my_stage, lane, zp, p.out0, p.ld0, row_base, tile.row_end, n);
+                warp_store_rows64(my_stage, lane, zp, p.out0, p.ld0, row_base, tile.row_end, n);
               if (c & 1)
-                warp_store_rows64<STAGE_OUT_PITCH_NARROW>(my_stage, lane, yp, p.out1, p.ld1, row_base, tile.row_end,
+                warp_store_rows64(my_stage, lane, yp, p.out1, p.ld1, row_base, tile.row_end,
                                                           (n - 32) >> 1);
             }
-          } else if (row_ok) {
-#pragma unroll
-            for (int c = 0; c < CHUNKS; ++c) {
-              const int n = n0 + (col_half * CHUNKS + c) * 32;
-              if (n < p.N) epilogue_chunk<EPI, RAGGED_K>(p, tile.e, r, n, v[c], score, ds_acc);
-            }
-          }
-        } else if constexpr (EPI == EPI_DSWIGLU && EW == 4) {
-          // dSwiGLU of single tiles, 32 accumulator columns at a time: the 128-byte piece of the saved pre-activation
-          // row comes in, and the dz (128 B) and y1*s (64 B) pieces go out, through this warp's staging rows with
-          // whole-row-segment accesses; the arithmetic stays one row per thread.
-          const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * (32 * STAGE_OUT_PITCH_WIDE);
-          const int row_base = tile.row0 + quad * 32;
-#pragma unroll 1
-          for (int c = 0; c < COLS_PER_WARP / 32; ++c) {
-            const int n = n0 + c * 32;
-            if (n >= p.N) break;
-            uint32_t v[32], zw[32];
-            if (have_acc) tmem_ld32(t_addr + c * 32, v);
-            warp_load_rows128<STAGE_OUT_PITCH_WIDE>(my_stage, lane, zw, p.z, 2ll * p.N, row_base, tile.row_end, 2 * n);
-            if (have_acc) {
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = 0u;
-            }
-            uint32_t ys[16];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const __nv_bfloat162 gu = *reinterpret_cast<const __nv_bfloat162*>(&zw[i]);
-              const float g = __low2float(gu), u = __high2float(gu);
-              const float dy = __uint_as_float(v[i]);
-              const float sig = sigmoid_f(g);
-              const float silu = g * sig;
-              const float y1 = silu * u;
-              ds_acc += dy * y1;
-              const float dg = dy * u * (sig * (1.f + g * (1.f - sig))) * score;
-              const float du = dy * silu * score;
-              zw[i] = pack_bf16(dg, du);
-              v[i] = __float_as_uint(y1 * score);
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) ys[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-            warp_store_rows128<STAGE_OUT_PITCH_WIDE>(my_stage, lane, zw, p.out0, p.ld0, row_base, tile.row_end, 2 * n);
-            warp_store_rows64<STAGE_OUT_PITCH_WIDE>(my_stage, lane, ys, p.out1, p.ld1, row_base, tile.row_end, n);
-          }
-        } else if constexpr (EPI == EPI_STORE && EW == 4) {
-          // plain stores of single tiles: two 32-column chunks (a 128-byte row segment) at a time through this warp's
-          // staging rows, 4 full rows per store instruction
-          const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * (32 * STAGE_OUT_PITCH_WIDE);
-          const int row_base = tile.row0 + quad * 32;
-          __nv_bfloat16* out = p.out0 + (RAGGED_K ? tile.e * p.out0_expert_stride : 0ll);
-#pragma unroll 1
-          for (int c = 0; c < COLS_PER_WARP / 32; c += 2) {
-            const int n = n0 + c * 32;
-            if (n >= p.N) break;  // N is a multiple of 64: both chunks exist or neither
-            uint32_t v0[32], v1[32];
-            if (have_acc) {
-              tmem_ld32(t_addr + c * 32, v0);
-              tmem_ld32(t_addr + (c + 1) * 32, v1);
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v0[j] = v1[j] = 0u;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              st_shared_v4(my_stage + lane * STAGE_OUT_PITCH_WIDE + 16 * q,
-                           pack_bf16(__uint_as_float(v0[8 * q]), __uint_as_float(v0[8 * q + 1])),
-                           pack_bf16(__uint_as_float(v0[8 * q + 2]), __uint_as_float(v0[8 * q + 3])),
-                           pack_bf16(__uint_as_float(v0[8 * q + 4]), __uint_as_float(v0[8 * q + 5])),
-                           pack_bf16(__uint_as_float(v0[8 * q + 6]), __uint_as_float(v0[8 * q + 7])));
-              st_shared_v4(my_stage + lane * STAGE_OUT_PITCH_WIDE + 64 + 16 * q,
-                           pack_bf16(__uint_as_float(v1[8 * q]), __uint_as_float(v1[8 * q + 1])),
-                           pack_bf16(__uint_as_float(v1[8 * q + 2]), __uint_as_float(v1[8 * q + 3])),
-                           pack_bf16(__uint_as_float(v1[8 * q + 4]), __uint_as_float(v1[8 * q + 5])),
-                           pack_bf16(__uint_as_float(v1[8 * q + 6]), __uint_as_float(v1[8 * q + 7])));
-            }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int rr = 4 * i + (lane >> 3);
-              const uint4 w = ld_shared_v4(my_stage + rr * STAGE_OUT_PITCH_WIDE + 16 * (lane & 7));
-              const int rw = row_base + rr;
-              if (rw < tile.row_end) {
-                uint4* dst = reinterpret_cast<uint4*>(out + rw * p.ld0 + n + 8 * (lane & 7));
-                *dst = p.accumulate ? add_bf16x8(w, dst) : w;
-              }
-            }
-            __syncwarp();
           }
         } else {
-#pragma unroll 1
-          for (int c = col_half * (COLS_PER_WARP / 32); c < (col_half + 1) * (COLS_PER_WARP / 32); ++c) {
-            const int n = n0 + c * 32;
-            if (n >= p.N) break;
-            uint32_t v[32];
-            if (have_acc) {
-              tmem_ld32(t_addr + c * 32, v);
-              tmem_ld_wait();
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = 0u;
+          // Single tiles: each warp's 128 columns 32 at a time, row traffic in whole 64-byte segments through its staging
+          // rows.  Eight warps, not four: with a short reduction the epilogue of a tile is longer than its main loop, and
+          // it is latency (tensor memory, shared memory, the stores) that its warps wait for.  Four warps took 4.1 us per
+          // plain-store tile and 25 us per dSwiGLU tile: down projection, dX and dH at T 24576, H 1536, I 256, E 128,
+          // K 8 278, 327 and 284 us against 1.1, 2.2 and 6.5 us of MMAs per tile.
+          const uint32_t my_stage = smem_u32(stage_out) + (warp - FIRST_EPI_WARP) * STAGE_ROWS_BYTES;
+          const int row_base = r - lane;
+          const int n_first = n0 + col_half * COLS_PER_WARP;
+          constexpr int CHUNKS = COLS_PER_WARP / 32;
+          const uint32_t t_cols = t_addr + col_half * COLS_PER_WARP;
+          if constexpr (EPI == EPI_DSWIGLU) {
+            ok = dact_columns<FN_SILU, true, CHUNKS>(p, my_stage, lane, row_base, tile.row_end, n_first,
+                                                                      t_cols, score, ds_acc, wait_acc, release_acc);
+          } else if constexpr (EPI == EPI_DACT) {
+            ok = act_dispatch(p.act, [&](auto kind) {
+              using Kind = decltype(kind);
+              return dact_columns<Kind::fn, Kind::gated, CHUNKS>(
+                  p, my_stage, lane, row_base, tile.row_end, n_first, t_cols, score, ds_acc, wait_acc, release_acc);
+            });
+          } else if constexpr (EPI == EPI_SWIGLU) {
+            act_columns<FN_SILU, true, CHUNKS>(p, tile.e, my_stage, lane, row_base, tile.row_end, n_first,
+                                                                t_cols, release_acc);
+          } else if constexpr (EPI == EPI_ACT) {
+            act_dispatch(p.act, [&](auto kind) {
+              using Kind = decltype(kind);
+              act_columns<Kind::fn, Kind::gated, CHUNKS>(p, tile.e, my_stage, lane, row_base,
+                                                                          tile.row_end, n_first, t_cols, release_acc);
+            });
+          } else {
+            int dst_row = 0;
+            if constexpr (EPI == EPI_STORE_ROWS || EPI == EPI_SCATTER) {
+              if (row_ok) dst_row = p.gather[r];
             }
-            if (!row_ok) continue;
-            epilogue_chunk<EPI, RAGGED_K>(p, tile.e, r, n, v, score, ds_acc);
+            if (n_first >= p.N) release_acc();
+#pragma unroll 1
+            for (int c = 0; c < CHUNKS; ++c) {
+              const int n = n_first + 32 * c;
+              if (n >= p.N) break;
+              uint32_t v[32];
+              if (have_acc) {
+                tmem_ld32(t_cols + 32 * c, v);
+                tmem_ld_wait();
+                if (c + 1 == CHUNKS || n + 32 >= p.N) release_acc();
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = 0u;
+              }
+              store_chunk<EPI, RAGGED_K>(p, tile.e, my_stage, lane, row_base, tile.row_end, n, v, score,
+                                                          dst_row);
+            }
           }
+          if (!ok) break;
         }
         if constexpr (EPI == EPI_DSWIGLU || EPI == EPI_DACT) {
           if (row_ok && n0 < p.N) {
-            float* dsp = p.ds_partial + static_cast<long long>(2 * (n0 / BN)) * p.total_rows + r;
-            if constexpr (COL_SPLIT == 2) {
-              dsp[static_cast<long long>(col_half) * p.total_rows] = ds_acc;
-            } else {
-              dsp[0] = ds_acc;
-              dsp[p.total_rows] = 0.f;
-            }
+            p.ds_partial[static_cast<long long>(2 * (n0 / BN) + col_half) * p.total_rows + r] = ds_acc;
           }
         }
         if constexpr (DUAL == DUAL_NONE) {
-          if (have_acc) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ss.acc_empty[acc]), 0));
-            if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
-          }
+          if (have_acc && ++acc == 2) { acc = 0; acc_phase ^= 1u; }
         }
       }
       if constexpr (DUAL != DUAL_NONE) {
@@ -746,6 +676,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   __syncthreads();
   cluster_sync_all();  // neither CTA leaves while the other may still signal its barriers or read its smem
   if (warp == 1) {
+    __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * BN);
   }

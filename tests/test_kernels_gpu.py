@@ -601,3 +601,56 @@ def test_stream_flag_write_then_wait(smoe):
     assert lib.smoe_stream_wait_values(flags.data_ptr(), 0, 99, consumer.cuda_stream) == 0
     assert lib.smoe_stream_write_value(None, 1, consumer.cuda_stream) != 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("act", ["swiglu", "geglu", "reglu", "relu_sq", "relu", "gelu", "silu"])
+@pytest.mark.parametrize("I", [128, 384])
+def test_general_epilogues_at_tile_edges(smoe, act, I):
+    """Counts around a tile's 256 rows (0, 1, 31, 255, 256, 257, 290) and widths that leave half of a tile's columns
+    empty: the up projection's z and y1 and the backward epilogue's dz, y1 * s and ds, against fp32.  bf16 outputs of
+    fp32 sums: one rounding (2^-9) plus the activation's own input rounding, BF16_TOL as for the other kernels."""
+    from sonicmoe.enums import ActivationType, is_glu
+    from sonicmoe.functional import _ACT_CODE
+
+    smoe, lib = smoe[0], smoe[0].lib
+    H, counts = 320, [0, 1, 31, 255, 256, 257, 290]
+    E, TK = len(counts), sum(counts)
+    T = 300
+    kind = ActivationType(act)
+    gated = is_glu(kind)
+    half = I // 2 if gated else I  # output width; gated: half = 64 or 192
+    g = torch.Generator().manual_seed(I + len(act))
+    x, dout = torch.randn(T, H, generator=g).bfloat16(), torch.randn(T, H, generator=g).bfloat16()
+    w1 = (torch.randn(E, I, H, generator=g) * 0.05).bfloat16()
+    w2 = (torch.randn(E, H, half, generator=g) * 0.05).bfloat16()
+    b1 = (torch.randn(E, I, generator=g) * 0.1).bfloat16()
+    score = torch.rand(TK, generator=g)
+    tok = torch.randint(0, T, (TK,), generator=g, dtype=torch.int32)
+    slot = torch.randperm(TK, generator=g).to(torch.int32)
+    expert = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    off = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int32)
+    d = [t.cuda() for t in (x, dout, w1, w2, b1, score, tok, slot, off)]
+    dx_, dd, dw1, dw2, db1, ds_, dt, dsl, do = d
+    z = torch.full((TK, I), float("nan"), dtype=torch.bfloat16, device="cuda")
+    y1 = torch.full((TK, half), float("nan"), dtype=torch.bfloat16, device="cuda")
+    st = smoe.device_state(z.device).status.data_ptr()
+    s = torch.cuda.current_stream().cuda_stream
+    assert lib.smoe_up_projection_forward_act(dx_.data_ptr(), dw1.data_ptr(), db1.data_ptr(), z.data_ptr(), y1.data_ptr(),
+                                              do.data_ptr(), dt.data_ptr(), T, H, I, E, TK, _ACT_CODE[kind], st, s) == 0
+    dz, ys = torch.full_like(z, float("nan")), torch.full_like(y1, float("nan"))
+    part = torch.full((lib.smoe_ds_partial_columns(half), TK), float("nan"), device="cuda")
+    assert lib.smoe_down_projection_backward_dact(
+        dd.data_ptr(), dw2.data_ptr(), z.data_ptr(), ds_.data_ptr(), 0, dz.data_ptr(), ys.data_ptr(), part.data_ptr(),
+        do.data_ptr(), dt.data_ptr(), dsl.data_ptr(), T, H, half, E, TK, _ACT_CODE[kind], st, s) == 0
+    torch.cuda.synchronize()
+    smoe.check_status()
+    pre = torch.einsum("rh,rih->ri", x[tok.long()].float(), w1[expert].float()) + b1[expert].float()
+    assert rel(z, pre) < BF16_TOL
+    assert rel(y1, orc.activation(act, pre)) < BF16_TOL
+    zz = z.float().cpu().requires_grad_(True)  # the kernel's own z, so that only its arithmetic is compared
+    y = orc.activation(act, zz)
+    dy = torch.einsum("rh,rhi->ri", dout[tok.long()].float(), w2[expert].float())
+    sc = score[slot.long()]
+    assert rel(dz, torch.autograd.grad(y, zz, dy * sc[:, None])[0]) < BF16_TOL
+    assert rel(ys, y.detach() * sc[:, None]) < BF16_TOL
+    assert rel(part.sum(0), (y.detach() * dy).sum(-1)) < BF16_TOL
