@@ -59,7 +59,9 @@ struct SharedStorage {
   uint32_t tmem_base;
   int abort_flag;
   int off[MAX_EXPERTS + 1];            // first grouped row of every expert
-  int m_tile_prefix[MAX_EXPERTS + 1];  // ragged-M: exclusive prefix of ceil(count / 256) per expert
+  int m_tile_prefix[MAX_EXPERTS + 1];  // ragged-M: exclusive prefix of ceil(count / 256) per expert; ragged-K: counts
+  int expert_order[MAX_EXPERTS];       // ragged-K with a skewed load: experts by descending count
+  int most_rows;                       // ragged-K: the largest count
 };
 
 // Output staging of the epilogues: each epilogue warp has 32 rows of 64 bytes (epilogue.cuh), through which a tile leaves
@@ -81,10 +83,44 @@ struct Tile {
 
 enum { DUAL_NONE = 0, DUAL_N = 1, DUAL_M = 2 };
 
+// Ragged-K: whether one expert has more than twice the mean number of rows.  Ordering is quadratic in the experts, so it
+// stops at 512 (1 us per 128).
+__device__ __forceinline__ bool is_skewed(const GemmParams& p, const SharedStorage& ss) {
+  return p.E <= 512 && static_cast<long long>(ss.most_rows) * p.E > 2ll * p.total_rows;
+}
+
+// Ragged-K: fills expert_order if the load is skewed (ties: lower expert first).  Called by the whole block; most_rows was
+// zeroed before an earlier barrier, and the arrays are complete after the caller's next one.
+__device__ __forceinline__ void order_experts(const GemmParams& p, SharedStorage& ss) {
+  int* count = ss.m_tile_prefix;
+  for (int e = threadIdx.x; e < p.E; e += blockDim.x) {
+    count[e] = p.off[e + 1] - p.off[e];
+    atomicMax(&ss.most_rows, count[e]);
+  }
+  __syncthreads();
+  if (!is_skewed(p, ss)) return;
+  for (int e = threadIdx.x; e < p.E; e += blockDim.x) {
+    const int mine = count[e];
+    int rank = 0;
+#pragma unroll 8
+    for (int f = 0; f < p.E; ++f) {
+      const int c = count[f];
+      rank += (c > mine || (c == mine && f < e)) ? 1 : 0;
+    }
+    ss.expert_order[rank] = e;
+  }
+}
+
 // The work units of one cluster, in the order in which every role of its CTAs walks them.  Each warp keeps its own
 // walker; all lanes must call next().  All state is in registers and shared memory: with 64-bit divisions, a binary
 // search and two dependent global loads per unit, finding a unit took longer than the MMAs of a short reduction.
 // Units go expert by expert, row tiles outermost, and are dealt out round-robin.
+// Ragged-K with a skewed load: a unit is as long as its expert's token count, so the experts go in descending order of
+// their counts and every other round is dealt out in reverse, which evens out the clusters' sums: at 65536 tokens, top-4 of
+// 64 experts, loads falling with the square of the rank, the longest cluster has 1379 k-blocks (dW2) where the mean is
+// 1336 and plain round-robin gave 2356; dW2 1489 -> 1040 us, dW1 1818 -> 1315 us.  Even loads keep the plain order, which
+// is 3 % faster there (dW1 of the 128-expert benchmark layer 3560 against 3666 us): the line is a largest count of twice
+// the mean, below which round-robin is at most one such unit off.
 template <bool RAGGED_K, int DUAL>
 struct UnitWalker {
   static constexpr int UNIT_N = DUAL == DUAL_N ? 2 * BN : BN;
@@ -94,6 +130,7 @@ struct UnitWalker {
   const int cluster, clusters, lane, num_n;
   int total;         // units of the whole grid
   int per_expert;    // ragged-K: units per expert
+  bool skewed;       // ragged-K: dealt out by descending count
   int round = 0;
   int mi, ni, e = 0;  // ragged-M: row tile, unit along N and expert of the next unit
   int step_m, step_n;
@@ -104,6 +141,7 @@ struct UnitWalker {
     if constexpr (RAGGED_K) {
       per_expert = (p.M + UNIT_M - 1) / UNIT_M * num_n;
       total = per_expert * p.E;
+      skewed = is_skewed(p, ss);
     } else {
       total = ss.m_tile_prefix[p.E] * num_n;
       mi = cluster / num_n;
@@ -113,7 +151,7 @@ struct UnitWalker {
     }
   }
   __device__ __forceinline__ int unit_of_round() const {
-    return round * clusters + cluster;
+    return round * clusters + (RAGGED_K && skewed && (round & 1) ? clusters - 1 - cluster : cluster);
   }
   // Number of k-blocks of the next unit, or -1 when there is none (all that the MMA issuer wants to know).
   __device__ __forceinline__ int next_num_kb() {
@@ -123,7 +161,7 @@ struct UnitWalker {
     if constexpr (!RAGGED_K) {
       return p.K / BK;
     } else {
-      const int ex = t / per_expert;
+      const int i = t / per_expert, ex = skewed ? ss.expert_order[i] : i;
       return (ss.off[ex + 1] - ss.off[ex] + BK - 1) / BK;
     }
   }
@@ -153,7 +191,7 @@ struct UnitWalker {
       }
     } else {
       const int i = t / per_expert, rem = t - i * per_expert, m = rem / num_n;
-      tile.e = i;
+      tile.e = skewed ? ss.expert_order[i] : i;
       tile.row0 = m * UNIT_M + static_cast<int>(rank) * BM;
       tile.row_end = p.M;
       tile.n0 = (rem - m * num_n) * UNIT_N;
@@ -222,7 +260,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     tmem_relinquish();
   }
   for (int e = threadIdx.x; e <= p.E; e += blockDim.x) ss.off[e] = p.off[e];
-  if constexpr (!RAGGED_K) {
+  if constexpr (RAGGED_K) {
+    if (threadIdx.x == 0) ss.most_rows = 0;
+    __syncthreads();
+    order_experts(p, ss);
+  } else {
     if (warp == 2) {
       int running = 0;
       for (int base = 0; base < p.E; base += 32) {
