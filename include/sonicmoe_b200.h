@@ -365,6 +365,21 @@ int smoe_router_backward(void* dlogits, const void* logits, const float* dscores
                          const int* indices, const float* g_colsum, const void* g_logits, int T, int E, int K,
                          void* stream);
 
+/* The two above with the load-balancing loss: aux (1) fp32 = E <mean, share>, mean = prob_colsum / its sum, share =
+ * expert_count / its sum (denominators at least 1e-12; sonicmoe/moe.py:261-274), and aux_grad (E) fp32 = its gradient by
+ * prob_colsum; both or neither.  Backward: *g_aux (a device word, optional) is the gradient of aux; g_aux * aux_grad is
+ * added to g_colsum. */
+int smoe_router_forward_aux(const void* x, const void* router_w, void* logits, float* scores, int* indices,
+                            int* expert_count, float* prob_colsum, float* aux, float* aux_grad, void* workspace, int T,
+                            int H, int E, int K, int* status, void* stream);
+int smoe_router_backward_aux(void* dlogits, const void* logits, const float* dscores, const float* scores,
+                             const int* indices, const float* g_colsum, const void* g_logits, const float* g_aux,
+                             const float* aux_grad, int T, int E, int K, void* stream);
+/* The load-balancing loss of logits (T,E) bf16 and counts that other kernels made, E <= 256; its gradient is
+ * smoe_router_backward_aux with only logits, g_aux and aux_grad.  workspace: smoe_router_forward_workspace_bytes(E). */
+int smoe_switch_loss(const void* logits, const int* expert_count, float* aux, float* aux_grad, void* workspace, int T,
+                     int E, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Expert parallelism over peer memory (one node, NVLink / NVSwitch).  The reference has no distributed
  * code (sonicmoe/moe.py:260 skips even the aux-loss reduction), so these have no counterpart there; they

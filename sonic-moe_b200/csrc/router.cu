@@ -34,7 +34,7 @@ constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int MAX_E = 256;
 constexpr int THREADS = 192;
-constexpr int MAX_STAGES = 6;
+constexpr int MAX_STAGES = 16;
 
 struct Shared {
   uint64_t full[MAX_STAGES];
@@ -49,6 +49,7 @@ struct Shared {
 
 struct Params {
   int T, H, E, K;
+  int tile_rows, split;  // router_forward_small_kernel: tokens per tile, CTAs that share its experts
   int stages;
   int acc_cols;  // tensor-memory columns per accumulator (power of two >= E)
   __nv_bfloat16* logits;  // (T, E)
@@ -67,6 +68,26 @@ __device__ __forceinline__ uint32_t order_key(float v) {  // larger key = better
 }
 __device__ __forceinline__ float key_value(uint32_t k) {
   const uint32_t b = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
+  return __uint_as_float(b);
+}
+
+// Shared memory of router_forward_small_kernel (offsets from its 1024-byte aligned start).
+struct SmallLayout {
+  int stage, logits, pitch, sums, shared, total;
+  __host__ __device__ SmallLayout(int tile_rows, int split, int E, int stages) {
+    stage = (tile_rows + E / split) * BK * 2;  // E / split is a multiple of 16: 1024-byte aligned
+    // the MMA reads 128 rows of A from the last stage on, whatever is behind its tile_rows
+    logits = stages * stage + (BM - tile_rows) * BK * 2;
+    pitch = 2 * E + 16;                        // bf16 rows; the pad spreads 16-byte writes of eight rows over the banks
+    sums = logits + tile_rows / split * pitch;  // a multiple of 16
+    shared = (sums + THREADS / 32 * E * 4 + 15) & ~15;
+    total = 1024 + shared + static_cast<int>(sizeof(Shared));
+  }
+};
+
+// value of a key whose upper half holds a bf16's order key
+__device__ __forceinline__ float half_key_value(uint32_t k) {
+  const uint32_t b = (k & 0x80000000u) ? (k & 0x7FFF0000u) : (~k & 0xFFFF0000u);
   return __uint_as_float(b);
 }
 
@@ -296,26 +317,318 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   }
 }
 
-// count[e] and colsum[e]: the CTAs' partials added up in CTA order.
-__global__ void __launch_bounds__(256) router_finish_kernel(const float* __restrict__ colsum_partial,
-                                                            const int* __restrict__ hist_partial, int blocks, int E,
-                                                            float* __restrict__ colsum, int* __restrict__ count) {
-  const int e = threadIdx.x;
-  if (e >= E) return;
+// Few tokens: smaller tiles, so that the chip is not left idle.  With one CTA per 128 tokens the walk over H, a ring of TMA
+// loads at one SM's rate, and the serial winner lists of one thread per token are all of the time (T 1, H 2048, E 64: 23 us;
+// T 64, H 4096, E 128: 49 us; T 1027, H 4096, E 256: 101 us).  Here a cluster of S CTAs takes R = 32, 64 or 128 tokens and
+// CTA r multiplies them with its E / S experts over all of H: every logit is the same sum in the same order as in the
+// kernel above, so the two agree bit for bit (a split of H would flip the rounding of a logit now and then, and with it
+// near ties).  The rows, rounded to bf16, go to the CTAs that own the tokens (CTA d takes R / S of them) over distributed
+// shared memory, and each token is worked on by a warp: lanes hold the columns, the K best are K warp-wide maxima of
+// (value, lower column first): 14, 27 and 32 us at the sizes above, and 42 instead of 51 at T 8192, H 4096, E 128.  What is
+// left is the chain of H / 64 loads and multiplications.  The MMA has 128 rows whatever R is: rows from R on multiply whatever is in shared memory
+// there, and are not read back.
+template <int PER_LANE>
+__global__ void __launch_bounds__(THREADS, 1)
+router_forward_small_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
+                            const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const SmallLayout lay(p.tile_rows, p.split, p.E, p.stages);
+  Shared& ss = *reinterpret_cast<Shared*>(smem + lay.shared);
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  volatile int* abort_flag = &ss.abort_flag;
+  const int rank = static_cast<int>(cluster_ctarank());
+  const int tile = blockIdx.x / p.split;
+  const int num_kb = p.H / BK;
+  const int cols = p.E / p.split;           // experts of this CTA
+  const int owned = p.tile_rows / p.split;  // tokens that each CTA of the cluster finishes
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(smem_u32(&ss.full[s]), 1);
+      mbar_init(smem_u32(&ss.empty[s]), 1);
+    }
+    mbar_init(smem_u32(&ss.acc_full[0]), 1);
+    ss.abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW);
+  }
+  for (int e = threadIdx.x; e < MAX_E; e += THREADS) ss.hist[e] = 0;
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&ss.tmem_base), p.acc_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // every CTA of the cluster runs before anything is written to its shared memory
+  tc_fence_after();
+  const uint32_t tmem_base = ss.tmem_base;
+
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+        const uint32_t bar = smem_u32(&ss.full[stage]);
+        const uint32_t a_dst = smem_u32(smem + stage * lay.stage);
+        mbar_arrive_expect_tx(bar, lay.stage);
+        tma_load_2d(&tmX, bar, a_dst, kb * BK, tile * p.tile_rows);
+        tma_load_2d(&tmW, bar, a_dst + p.tile_rows * BK * 2, kb * BK, rank * cols);
+        if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+      }
+      if (!ok && p.status) atomicCAS(p.status, SMOE_ST_OK, SMOE_ST_TIMEOUT_PRODUCER);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = make_idesc_bf16(BM, cols, false, false);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(smem + stage * lay.stage);
+        const uint64_t a_desc = make_smem_desc(a_addr, 16, 1024);
+        const uint64_t b_desc = make_smem_desc(a_addr + p.tile_rows * BK * 2, 16, 1024);
+#pragma unroll
+        for (int k4 = 0; k4 < BK / UMMA_K; ++k4)
+          umma_bf16(tmem_base, a_desc + ((k4 * UMMA_K * 2) >> 4), b_desc + ((k4 * UMMA_K * 2) >> 4), idesc,
+                    (kb > 0 || k4 > 0) ? 1u : 0u);
+        umma_commit(smem_u32(&ss.empty[stage]));
+        if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+      }
+      if (ok) umma_commit(smem_u32(&ss.acc_full[0]));
+      else if (p.status) atomicCAS(p.status, SMOE_ST_OK, SMOE_ST_TIMEOUT_MMA);
+    }
+  } else {
+    ok = mbar_wait_warp(smem_u32(&ss.acc_full[0]), 0, abort_flag);
+    tc_fence_after();
+    const int row = (warp & 3) * 32 + lane;
+    if (!ok) {
+      if (lane == 0 && p.status) atomicCAS(p.status, SMOE_ST_OK, SMOE_ST_TIMEOUT_EPILOGUE);
+    } else if ((warp & 3) * 32 < p.tile_rows) {
+      const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+      const uint32_t dst =
+          map_to_cta(smem_u32(smem + lay.logits + (row % owned) * lay.pitch + rank * cols * 2), row / owned);
+      for (int c = 0; c < cols; c += 16) {
+        uint32_t v[16];
+        tmem_ld16(t_addr + c, v);
+        tmem_ld_wait();
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+          w[j] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        st_cluster_v4(dst + 2 * c, w[0], w[1], w[2], w[3]);
+        st_cluster_v4(dst + 2 * c + 16, w[4], w[5], w[6], w[7]);
+      }
+      tc_fence_before();
+    }
+  }
+  __syncwarp();
+  if (*abort_flag != 0) {  // let this CTA's loads in flight land
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+  __syncwarp();
+  cluster_sync_all();  // all rows of the owned tokens are here; after this no CTA touches another's shared memory
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, p.acc_cols);
+  }
+
+  float colsum[PER_LANE];
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) colsum[j] = 0.f;
+  for (int i = warp; i < owned; i += THREADS / 32) {
+    const int row = tile * p.tile_rows + rank * owned + i;
+    if (row >= p.T) break;
+    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(smem + lay.logits + i * lay.pitch);
+    uint32_t key[PER_LANE];
+    float f[PER_LANE];
+    float m = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const int col = lane + 32 * j;
+      key[j] = 0u;
+      f[j] = -INFINITY;
+      if (col < p.E) {
+        const __nv_bfloat16 h = src[col];
+        p.logits[static_cast<long long>(row) * p.E + col] = h;
+        f[j] = __bfloat162float(h);
+        // a bf16 value's order key is exact in its upper half; the lower half prefers the lower column
+        key[j] = (order_key(f[j]) & 0xFFFF0000u) | static_cast<uint32_t>(0xFFFF - col);
+        m = fmaxf(m, f[j]);
+      }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+    // full softmax of the row
+    float prob[PER_LANE], s = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      prob[j] = lane + 32 * j < p.E ? __expf(f[j] - m) : 0.f;
+      s += prob[j];
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    const float inv_s = 1.f / s;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) colsum[j] += prob[j] * inv_s;
+    // lane k keeps the k-th best
+    uint32_t mine = 0u, best0 = 0u;
+    for (int k = 0; k < p.K; ++k) {
+      uint32_t local = key[0];
+#pragma unroll
+      for (int j = 1; j < PER_LANE; ++j) local = max(local, key[j]);
+      const uint32_t best = __reduce_max_sync(0xffffffffu, local);
+      if (k == 0) best0 = best;
+      if (lane == k) mine = best;
+#pragma unroll
+      for (int j = 0; j < PER_LANE; ++j)
+        if (key[j] == best) key[j] = 0u;
+    }
+    const float vmax = half_key_value(best0);
+    const float ex = lane < p.K ? expf(half_key_value(mine) - vmax) : 0.f;
+    float sum = 0.f;
+    for (int k = 0; k < p.K; ++k) sum += __shfl_sync(0xffffffffu, ex, k);
+    if (lane < p.K) {
+      const int col = 0xFFFF - static_cast<int>(mine & 0xFFFFu);
+      p.scores[static_cast<long long>(row) * p.K + lane] = ex / sum;
+      p.indices[static_cast<long long>(row) * p.K + lane] = col;
+      atomicAdd(&ss.hist[col], 1);
+    }
+  }
+  // the warps' column sums, then this CTA's partial results
+  float* sums = reinterpret_cast<float*>(smem + lay.sums);
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j)
+    if (lane + 32 * j < p.E) sums[warp * p.E + lane + 32 * j] = colsum[j];
+  __syncthreads();
+  for (int col = threadIdx.x; col < p.E; col += THREADS) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) s += sums[w * p.E + col];
+    p.colsum_partial[static_cast<long long>(blockIdx.x) * p.E + col] = s;
+    p.hist_partial[static_cast<long long>(blockIdx.x) * p.E + col] = ss.hist[col];
+  }
+}
+
+// count[e] and colsum[e]: the CTAs' partials added up in a fixed order (each column by 1024 / 256 groups of threads, each
+// over its share of the CTAs); without hist_partial, count is an input.  With `aux` also the load-balancing loss E <mean, share>, mean = colsum / sum(colsum) and
+// share = count / sum(count) (denominators at least 1e-12), and its gradient by colsum, E (share - <mean, share>) /
+// sum(colsum): two norms, divisions and a product over E values that took ten launches forward and fifteen backward.
+__global__ void __launch_bounds__(1024) router_finish_kernel(const float* __restrict__ colsum_partial,
+                                                             const int* __restrict__ hist_partial, int blocks, int E,
+                                                             float* __restrict__ colsum, int* __restrict__ count,
+                                                             float* __restrict__ aux, float* __restrict__ aux_grad) {
+  __shared__ float part_s[4][MAX_E];
+  __shared__ int part_c[4][MAX_E];
+  __shared__ float red[3][8];
+  const int e = threadIdx.x & (MAX_E - 1), group = threadIdx.x / MAX_E;
   float s = 0.f;
   int c = 0;
-  for (int b = 0; b < blocks; ++b) {
-    s += colsum_partial[static_cast<long long>(b) * E + e];
-    c += hist_partial[static_cast<long long>(b) * E + e];
+  if (e < E) {
+    const int begin = blocks * group / 4, end = blocks * (group + 1) / 4;
+#pragma unroll 8
+    for (int b = begin; b < end; ++b) {
+      s += colsum_partial[static_cast<long long>(b) * E + e];
+      if (hist_partial != nullptr) c += hist_partial[static_cast<long long>(b) * E + e];
+    }
+    if (hist_partial == nullptr && group == 0) c = count[e];
   }
-  colsum[e] = s;
-  count[e] = c;
+  part_s[group][e] = s;
+  part_c[group][e] = c;
+  __syncthreads();
+  s = ((part_s[0][e] + part_s[1][e]) + part_s[2][e]) + part_s[3][e];
+  c = part_c[0][e] + part_c[1][e] + part_c[2][e] + part_c[3][e];
+  if (group == 0 && e < E) {
+    if (colsum != nullptr) colsum[e] = s;
+    if (hist_partial != nullptr) count[e] = c;
+  }
+  if (aux == nullptr) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float sums = fabsf(s), counts = static_cast<float>(c);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    sums += __shfl_xor_sync(0xffffffffu, sums, d);
+    counts += __shfl_xor_sync(0xffffffffu, counts, d);
+  }
+  if (group == 0 && lane == 0) {
+    red[0][warp] = sums;
+    red[1][warp] = counts;
+  }
+  __syncthreads();
+  sums = counts = 0.f;
+#pragma unroll
+  for (int w = 0; w < MAX_E / 32; ++w) {
+    sums += red[0][w];
+    counts += red[1][w];
+  }
+  sums = fmaxf(sums, 1e-12f);
+  const float share = static_cast<float>(c) / fmaxf(counts, 1e-12f);
+  float dot = s / sums * share;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, d);
+  if (group == 0 && lane == 0) red[2][warp] = dot;
+  __syncthreads();
+  dot = 0.f;
+#pragma unroll
+  for (int w = 0; w < MAX_E / 32; ++w) dot += red[2][w];
+  if (threadIdx.x == 0) *aux = static_cast<float>(E) * dot;
+  if (group == 0 && e < E) aux_grad[e] = static_cast<float>(E) * (share - dot) / sums;
+}
+
+// Column sums of softmax(logits) for logits that another kernel made: one warp per row, partial sums per CTA.
+template <int PER_LANE>
+__global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16* __restrict__ logits, int rows, int E,
+                                                             float* __restrict__ colsum_partial) {
+  __shared__ float sums[8][MAX_E];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float colsum[PER_LANE];
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) colsum[j] = 0.f;
+  for (long long row = blockIdx.x * 8ll + warp; row < rows; row += gridDim.x * 8ll) {
+    float l[PER_LANE], m = -INFINITY, s = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const int col = lane + 32 * j;
+      l[j] = col < E ? __bfloat162float(logits[row * E + col]) : -INFINITY;
+      m = fmaxf(m, l[j]);
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      l[j] = lane + 32 * j < E ? __expf(l[j] - m) : 0.f;
+      s += l[j];
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    const float inv = 1.f / s;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) colsum[j] += l[j] * inv;
+  }
+#pragma unroll
+  for (int j = 0; j < PER_LANE; ++j) sums[warp][lane + 32 * j] = colsum[j];
+  __syncthreads();
+  for (int col = threadIdx.x; col < E; col += 256) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += sums[w][col];
+    colsum_partial[static_cast<long long>(blockIdx.x) * E + col] = s;
+  }
 }
 
 // dlogits[t, e] = g_logits[t, e]                                      (optional)
 //              + s_k (g_k - sum_j g_j s_j) for e = idx[t, k]           (gradient through the K winners' softmax)
 //              + p[t, e] (c_e - sum_j p[t, j] c_j)                     (optional: gradient c of the column sums of
-//                                                                       the full softmax p of the row)
+//                                                                       the full softmax p of the row);
+//                                                                       c = g_colsum + *g_aux * aux_grad
 // One warp per row; the row's probabilities are recomputed from the saved bf16 logits.
 template <int PER_LANE>
 __global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __restrict__ dlogits,
@@ -324,8 +637,10 @@ __global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __r
                                                               const float* __restrict__ score,
                                                               const int* __restrict__ indices,
                                                               const float* __restrict__ g_colsum,
-                                                              const __nv_bfloat16* __restrict__ g_logits, int rows,
-                                                              int E, int K) {
+                                                              const __nv_bfloat16* __restrict__ g_logits,
+                                                              const float* __restrict__ g_aux,
+                                                              const float* __restrict__ aux_grad, int rows, int E,
+                                                              int K) {
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -335,12 +650,15 @@ __global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __r
     const int col = lane + 32 * j;
     out[j] = (g_logits != nullptr && col < E) ? __bfloat162float(g_logits[row * E + col]) : 0.f;
   }
-  if (g_colsum != nullptr) {
-    float l[PER_LANE];
+  if (g_colsum != nullptr || g_aux != nullptr) {
+    float l[PER_LANE], c[PER_LANE];
     float m = -INFINITY;
+    const float scale = g_aux != nullptr ? *g_aux : 0.f;
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) {
       const int col = lane + 32 * j;
+      c[j] = (g_colsum != nullptr && col < E) ? g_colsum[col] : 0.f;
+      if (g_aux != nullptr && col < E) c[j] += scale * aux_grad[col];
       l[j] = col < E ? __bfloat162float(logits[row * E + col]) : -INFINITY;
       m = fmaxf(m, l[j]);
     }
@@ -352,7 +670,7 @@ __global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __r
       const int col = lane + 32 * j;
       l[j] = col < E ? __expf(l[j] - m) : 0.f;
       s += l[j];
-      dot += col < E ? l[j] * g_colsum[col] : 0.f;
+      dot += l[j] * c[j];
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -364,7 +682,7 @@ __global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __r
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) {
       const int col = lane + 32 * j;
-      if (col < E) out[j] += l[j] * inv * (g_colsum[col] - dot);
+      if (col < E) out[j] += l[j] * inv * (c[j] - dot);
     }
   }
   if (dscore != nullptr) {
@@ -423,6 +741,25 @@ static int encode_rows(CUtensorMap* map, const void* base, uint64_t rows, uint64
   return r == CUDA_SUCCESS ? SMOE_OK : SMOE_ERR_TENSORMAP;
 }
 
+// Tile of router_forward_small_kernel: what a CTA loads per k-block is (rows + E / split) lines, so the smallest such tile
+// whose CTAs all fit on the chip at once; one with the large kernel's 128 rows and all experts means that kernel (from
+// 9473 tokens on at 148 SMs, where tiles of half its traffic would take a second wave).
+static void small_tile(int T, int E, int sms, int& rows, int& split) {
+  rows = BM;
+  split = 1;
+  int best = BM + E;
+  for (int r = 32; r <= BM; r *= 2) {
+    for (int s = 1; s <= 8 && s <= r; s *= 2) {
+      if (E % (16 * s) != 0 || (T + r - 1) / r * s > sms) continue;
+      if (r + E / s < best) {
+        best = r + E / s;
+        rows = r;
+        split = s;
+      }
+    }
+  }
+}
+
 static bool unsupported(int T, int H, int E, int K) {
   return T < 0 || H <= 0 || (H % BK) != 0 || E < 32 || E > MAX_E || (E % 32) != 0 || K <= 0 || K > 16 || K > E;
 }
@@ -445,25 +782,40 @@ size_t smoe_router_forward_workspace_bytes(int E) {
 int smoe_router_forward(const void* x, const void* router_w, void* logits, float* scores, int* indices,
                         int* expert_count, float* prob_colsum, void* workspace, int T, int H, int E, int K,
                         int* status, void* stream) {
+  return smoe_router_forward_aux(x, router_w, logits, scores, indices, expert_count, prob_colsum, nullptr, nullptr,
+                                 workspace, T, H, E, K, status, stream);
+}
+
+int smoe_router_forward_aux(const void* x, const void* router_w, void* logits, float* scores, int* indices,
+                            int* expert_count, float* prob_colsum, float* aux, float* aux_grad, void* workspace, int T,
+                            int H, int E, int K, int* status, void* stream) {
+  if ((aux == nullptr) != (aux_grad == nullptr)) return SMOE_ERR_SHAPE;
   if (unsupported(T, H, E, K)) return SMOE_ERR_SHAPE;
   if (workspace == nullptr) return SMOE_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int sms = num_sms();
   if (sms <= 0) return SMOE_ERR_DRIVER;
   const int tiles = (T + BM - 1) / BM;
-  const int grid = tiles < sms ? tiles : sms;
+  int grid = tiles < sms ? tiles : sms;
   float* colsum_partial = static_cast<float*>(workspace);
   int* hist_partial = reinterpret_cast<int*>(colsum_partial + static_cast<size_t>(sms) * E);
   if (T > 0) {
-    CUtensorMap tmX, tmW;
-    int rc = encode_rows(&tmX, x, T, H, BM);
-    if (rc != SMOE_OK) return rc;
-    rc = encode_rows(&tmW, router_w, E, H, E);
-    if (rc != SMOE_OK) return rc;
     Params p = {};
     p.T = T; p.H = H; p.E = E; p.K = K;
+    small_tile(T, E, sms, p.tile_rows, p.split);
+    const bool small = p.tile_rows < BM || p.split > 1;
+    CUtensorMap tmX, tmW;
+    int rc = encode_rows(&tmX, x, T, H, p.tile_rows);
+    if (rc != SMOE_OK) return rc;
+    rc = encode_rows(&tmW, router_w, E, H, E / p.split);
+    if (rc != SMOE_OK) return rc;
+    const int cols = E / p.split;
     p.stages = E <= 128 ? 6 : 4;
-    p.acc_cols = E <= 32 ? 32 : E <= 64 ? 64 : E <= 128 ? 128 : 256;
+    if (small) {  // as many as 128 KiB hold
+      p.stages = 128 * 1024 / ((p.tile_rows + cols) * BK * 2);
+      p.stages = p.stages > MAX_STAGES ? MAX_STAGES : p.stages;
+    }
+    p.acc_cols = cols <= 32 ? 32 : cols <= 64 ? 64 : cols <= 128 ? 128 : 256;
     p.logits = static_cast<__nv_bfloat16*>(logits);
     p.scores = scores; p.indices = indices;
     p.colsum_partial = colsum_partial; p.hist_partial = hist_partial;
@@ -471,8 +823,30 @@ int smoe_router_forward(const void* x, const void* router_w, void* logits, float
     const int smem = 1024 + p.stages * (A_STAGE_BYTES + E * BK * 2) + static_cast<int>(sizeof(Shared));
     const int dev = current_device();
     if (dev < 0) return SMOE_ERR_DRIVER;
-    static PerDeviceFlag configured8, configured16;
-    if (K <= 8) {
+    static PerDeviceFlag configured8, configured16, configured_small4, configured_small8;
+    if (small) {
+      grid = (T + p.tile_rows - 1) / p.tile_rows * p.split;
+      auto kernel = E <= 128 ? router_forward_small_kernel<4> : router_forward_small_kernel<8>;
+      PerDeviceFlag& configured = E <= 128 ? configured_small4 : configured_small8;
+      if (!configured.test(dev)) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+          return SMOE_ERR_LAUNCH;
+        configured.set(dev);
+      }
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+      cfg.blockDim = dim3(THREADS, 1, 1);
+      cfg.dynamicSmemBytes = SmallLayout(p.tile_rows, p.split, E, p.stages).total;
+      cfg.stream = st;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = static_cast<unsigned>(p.split);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (cudaLaunchKernelEx(&cfg, kernel, tmX, tmW, p) != cudaSuccess) return SMOE_ERR_LAUNCH;
+    } else if (K <= 8) {
       if (!configured8.test(dev)) {
         if (cudaFuncSetAttribute(router_forward_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
             cudaSuccess)
@@ -491,14 +865,48 @@ int smoe_router_forward(const void* x, const void* router_w, void* logits, float
     }
     if (cudaGetLastError() != cudaSuccess) return SMOE_ERR_LAUNCH;
   }
-  router_finish_kernel<<<1, 256, 0, st>>>(colsum_partial, hist_partial, T > 0 ? grid : 0, E, prob_colsum, expert_count);
+  router_finish_kernel<<<1, 1024, 0, st>>>(colsum_partial, hist_partial, T > 0 ? grid : 0, E, prob_colsum, expert_count,
+                                           aux, aux_grad);
+  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+}
+
+int smoe_switch_loss(const void* logits, const int* expert_count, float* aux, float* aux_grad, void* workspace, int T,
+                     int E, void* stream) {
+  if (T < 0 || E <= 0 || E > MAX_E) return SMOE_ERR_SHAPE;
+  if (workspace == nullptr) return SMOE_ERR_WORKSPACE;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int sms = num_sms();
+  if (sms <= 0) return SMOE_ERR_DRIVER;
+  const int blocks = T == 0 ? 0 : (T + 7) / 8 < sms ? (T + 7) / 8 : sms;
+  float* colsum_partial = static_cast<float*>(workspace);
+  const __nv_bfloat16* l = static_cast<const __nv_bfloat16*>(logits);
+  if (blocks > 0) {
+    const int per_lane = (E + 31) / 32;
+    if (per_lane <= 1)
+      softmax_colsum_kernel<1><<<blocks, 256, 0, st>>>(l, T, E, colsum_partial);
+    else if (per_lane <= 4)
+      softmax_colsum_kernel<4><<<blocks, 256, 0, st>>>(l, T, E, colsum_partial);
+    else
+      softmax_colsum_kernel<8><<<blocks, 256, 0, st>>>(l, T, E, colsum_partial);
+    if (cudaGetLastError() != cudaSuccess) return SMOE_ERR_LAUNCH;
+  }
+  router_finish_kernel<<<1, 1024, 0, st>>>(colsum_partial, nullptr, blocks, E, nullptr, const_cast<int*>(expert_count),
+                                           aux, aux_grad);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 
 int smoe_router_backward(void* dlogits, const void* logits, const float* dscores, const float* scores,
                          const int* indices, const float* g_colsum, const void* g_logits, int T, int E, int K,
                          void* stream) {
+  return smoe_router_backward_aux(dlogits, logits, dscores, scores, indices, g_colsum, g_logits, nullptr, nullptr, T, E,
+                                  K, stream);
+}
+
+int smoe_router_backward_aux(void* dlogits, const void* logits, const float* dscores, const float* scores,
+                             const int* indices, const float* g_colsum, const void* g_logits, const float* g_aux,
+                             const float* aux_grad, int T, int E, int K, void* stream) {
   if (T < 0 || E <= 0 || E > MAX_E || K <= 0 || K > E) return SMOE_ERR_SHAPE;
+  if (g_aux != nullptr && (aux_grad == nullptr || (T > 0 && logits == nullptr))) return SMOE_ERR_SHAPE;
   if (dscores != nullptr && (scores == nullptr || indices == nullptr)) return SMOE_ERR_SHAPE;
   if (g_colsum != nullptr && logits == nullptr) return SMOE_ERR_SHAPE;
   if (T == 0) return SMOE_OK;
@@ -509,11 +917,14 @@ int smoe_router_backward(void* dlogits, const void* logits, const float* dscores
   const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(g_logits);
   const int per_lane = (E + 31) / 32;
   if (per_lane <= 2)
-    router_backward_kernel<2><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, T, E, K);
+    router_backward_kernel<2><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E,
+                                                  K);
   else if (per_lane <= 4)
-    router_backward_kernel<4><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, T, E, K);
+    router_backward_kernel<4><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E,
+                                                  K);
   else
-    router_backward_kernel<8><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, T, E, K);
+    router_backward_kernel<8><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E,
+                                                  K);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

@@ -273,10 +273,11 @@ def layer_router_logits(x: torch.Tensor, router_w: torch.Tensor, K: int) -> torc
 
 
 class _FusedRouter(torch.autograd.Function):
-    """(logits (T,E) bf16, scores (T,K) fp32, indices (T,K) int32, expert_frequency (E) int32, prob_colsum (E) fp32)
-    from one pass over x: router GEMM, top-K + softmax over the winners, token counts and the column sums of the
-    full softmax, in one kernel.  Routing is decided on the bf16 logits this returns.  Backward: one kernel turns
-    the gradients of logits, scores and prob_colsum into dlogits; the two router GEMMs stay library calls, as the
+    """(logits (T,E) bf16, scores (T,K) fp32, indices (T,K) int32, expert_frequency (E) int32, prob_colsum (E) fp32,
+    load-balancing loss () fp32) from one pass over x: router GEMM, top-K + softmax over the winners, token counts and
+    the column sums of the full softmax, in one kernel, and the loss in the small one that adds up its CTAs' sums.
+    Routing is decided on the bf16 logits this returns.  Backward: one kernel turns
+    the gradients of logits, scores, prob_colsum and the loss into dlogits; the two router GEMMs stay library calls, as the
     forward one does in the reference (sonicmoe/functional/__init__.py:438-446, sonicmoe/moe.py:251-274)."""
 
     @staticmethod
@@ -293,19 +294,22 @@ class _FusedRouter(torch.autograd.Function):
             indices = torch.empty(T, K, dtype=torch.int32, device=dev)
             freq = torch.empty(E, dtype=torch.int32, device=dev)
             colsum = torch.empty(E, dtype=torch.float32, device=dev)
+            aux = torch.empty((), dtype=torch.float32, device=dev)
+            aux_grad = torch.empty(E, dtype=torch.float32, device=dev)
             ws = st.router_workspace(E)
-            check(lib.smoe_router_forward(x.data_ptr(), router_w.data_ptr(), logits.data_ptr(), scores.data_ptr(),
-                                          indices.data_ptr(), freq.data_ptr(), colsum.data_ptr(), ws.data_ptr(),
-                                          T, H, E, K, st.status.data_ptr(), stream_ptr(dev)), "router_forward")
-        ctx.save_for_backward(x, router_w, logits, scores, indices)
+            check(lib.smoe_router_forward_aux(x.data_ptr(), router_w.data_ptr(), logits.data_ptr(), scores.data_ptr(),
+                                              indices.data_ptr(), freq.data_ptr(), colsum.data_ptr(), aux.data_ptr(),
+                                              aux_grad.data_ptr(), ws.data_ptr(), T, H, E, K, st.status.data_ptr(),
+                                              stream_ptr(dev)), "router_forward")
+        ctx.save_for_backward(x, router_w, logits, scores, indices, aux_grad)
         ctx.mark_non_differentiable(indices, freq)
         ctx.set_materialize_grads(False)
-        return logits, scores, indices, freq, colsum
+        return logits, scores, indices, freq, colsum, aux
 
     @staticmethod
-    def backward(ctx, g_logits, g_scores, _gi, _gf, g_colsum):
-        x, router_w, logits, scores, indices = ctx.saved_tensors
-        if g_logits is None and g_scores is None and g_colsum is None:
+    def backward(ctx, g_logits, g_scores, _gi, _gf, g_colsum, g_aux):
+        x, router_w, logits, scores, indices, aux_grad = ctx.saved_tensors
+        if g_logits is None and g_scores is None and g_colsum is None and g_aux is None:
             return None, None, None
         T, E = logits.shape
         K = scores.shape[1]
@@ -316,14 +320,56 @@ class _FusedRouter(torch.autograd.Function):
             g_scores = g_scores.contiguous().float()
         if g_colsum is not None:
             g_colsum = g_colsum.contiguous().float()
+        if g_aux is not None:
+            g_aux = g_aux.float()
         with torch.cuda.device(dev):
             dlogits = torch.empty_like(logits)
-            check(lib.smoe_router_backward(dlogits.data_ptr(), logits.data_ptr(), ptr(g_scores), scores.data_ptr(),
-                                           indices.data_ptr(), ptr(g_colsum), ptr(g_logits), T, E, K,
-                                           stream_ptr(dev)), "router_backward")
+            check(lib.smoe_router_backward_aux(dlogits.data_ptr(), logits.data_ptr(), ptr(g_scores), scores.data_ptr(),
+                                               indices.data_ptr(), ptr(g_colsum), ptr(g_logits), ptr(g_aux),
+                                               aux_grad.data_ptr(), T, E, K, stream_ptr(dev)), "router_backward")
         dx = dlogits @ router_w if ctx.needs_input_grad[0] else None
         dw = dlogits.t() @ x if ctx.needs_input_grad[1] else None
         return dx, dw, None
+
+
+class _SwitchLoss(torch.autograd.Function):
+    """The load-balancing loss of bf16 logits (T,E), E <= 256, and token counts that other kernels made."""
+
+    @staticmethod
+    def forward(ctx, logits, freq):
+        logits = logits.contiguous()
+        T, E = logits.shape
+        dev = logits.device
+        with torch.cuda.device(dev):
+            aux = torch.empty((), dtype=torch.float32, device=dev)
+            aux_grad = torch.empty(E, dtype=torch.float32, device=dev)
+            ws = torch.empty(lib.smoe_router_forward_workspace_bytes(E), dtype=torch.uint8, device=dev)
+            check(lib.smoe_switch_loss(logits.data_ptr(), freq.data_ptr(), aux.data_ptr(), aux_grad.data_ptr(),
+                                       ws.data_ptr(), T, E, stream_ptr(dev)), "switch_loss")
+        ctx.save_for_backward(logits, aux_grad)
+        return aux
+
+    @staticmethod
+    def backward(ctx, g_aux):
+        logits, aux_grad = ctx.saved_tensors
+        T, E = logits.shape
+        dev = logits.device
+        g_aux = g_aux.float()
+        with torch.cuda.device(dev):
+            dlogits = torch.empty_like(logits)
+            check(lib.smoe_router_backward_aux(dlogits.data_ptr(), logits.data_ptr(), None, None, None, None, None,
+                                               g_aux.data_ptr(), aux_grad.data_ptr(), T, E, 1, stream_ptr(dev)),
+                  "router_backward")
+        return dlogits, None
+
+
+def switch_loss(logits: torch.Tensor, expert_frequency: torch.Tensor) -> torch.Tensor | None:
+    """E <normalised mean of softmax(logits), normalised expert_frequency>, or None where the kernels do not apply."""
+    if not (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.shape[1] <= 256
+            and expert_frequency.dtype == torch.int32 and expert_frequency.device == logits.device
+            and expert_frequency.is_contiguous() and not torch.compiler.is_compiling()):
+        return None
+    return _SwitchLoss.apply(logits, expert_frequency)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -626,14 +672,20 @@ def moe_TC_softmax_topk_layer_with_router_stats(x, router_w, w1, b1, w2, b2, K, 
                                                 is_inference_mode_enabled=False):
     """`moe_TC_softmax_topk_layer` plus a fourth result: the column sums (E,) fp32 of softmax(router_logits) when the
     fused routing kernel produced them (what the load-balancing loss needs), else None."""
+    return _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inference_mode_enabled)[:4]
+
+
+def _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inference_mode_enabled):
+    """(o, router_logits, expert_frequency, column sums of softmax(router_logits), load-balancing loss); the last two
+    are None where the fused routing kernel does not apply."""
     activation_type = _check_experts_args(x, w1, w2, b1, b2, activation_type)
     E = router_w.size(0)
     T = x.size(0)
     inference = is_inference_mode_enabled or not torch.is_grad_enabled()
     if fused_router_applies(x, router_w, K):
-        router_logits, scores, indices, _freq, colsum = _FusedRouter.apply(x, router_w, K)
+        router_logits, scores, indices, _freq, colsum, aux = _FusedRouter.apply(x, router_w, K)
     else:
-        colsum = None
+        colsum = aux = None
         # a router kept in fp32 (an extension over the reference) computes its logits in fp32
         router_logits = F.linear(x if x.dtype == router_w.dtype else x.to(router_w.dtype), router_w)
         if torch.compiler.is_compiling() and b1 is None and activation_type == ActivationType.SWIGLU:
@@ -641,11 +693,11 @@ def moe_TC_softmax_topk_layer_with_router_stats(x, router_w, w1, b1, w2, b2, K, 
             from .compiled_ops import layer_with_custom_ops
 
             o, freq = layer_with_custom_ops(x, router_logits, w1, w2, K, E, inference)
-            return o, router_logits, freq, None
+            return o, router_logits, freq, None, None
         scores, indices = topk_softmax(router_logits, K)
     route = _route_metadata(indices.reshape(-1), None, E, K)
     o = _experts(x, w1, b1, w2, b2, scores.reshape(-1), route, T, inference, activation_type)
-    return o, router_logits, route.expert_frequency, colsum
+    return o, router_logits, route.expert_frequency, colsum, aux
 
 
 def moe_general_routing_inputs(

@@ -169,3 +169,45 @@ def test_layer_with_fused_router_matches_separate_router(built_library):
     assert rel(res[True][1], res[False][1]) < 1e-4
     for a, b in zip(res[True], res[False]):
         assert rel(a, b) < 2e-2
+
+
+@pytest.mark.parametrize("T,H,E,K", [
+    (1, 2048, 64, 4), (127, 4096, 128, 8), (2048, 512, 256, 16),        # eight CTAs per tile
+    (1030, 64, 64, 1), (200, 128, 96, 2), (260, 320, 160, 6),           # reductions of 1, 2 and 5 k-blocks
+    (2049, 1024, 32, 8), (4096, 768, 192, 16),                          # four
+    (4097, 512, 128, 8), (9472, 256, 64, 4), (9473, 256, 64, 4),        # two, and one above the last split
+])
+def test_router_forward_small_tiles(built_library, T, H, E, K):
+    """The small-tile form around the token counts at which its tile changes: what test_router_forward asks of a shape."""
+    test_router_forward(built_library, T, H, E, K)
+
+
+@pytest.mark.parametrize("T,E,fused", [(1, 64, True), (1000, 64, True), (6000, 256, True), (0, 32, True),
+                                       (1, 8, False), (777, 8, False), (3001, 40, False), (500, 256, False), (0, 8, False)])
+def test_switch_loss(built_library, T, E, fused):
+    """The load-balancing loss and its gradient by the logits against the formula in 64 bits: fp32 sums and the fast
+    exponential (2^-22 relative) leave 1e-5, the bf16 gradient one rounding (2^-9)."""
+    from sonicmoe.functional import _FusedRouter, switch_loss
+
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    K = 2
+    if fused:
+        x = torch.randn(T, 128, generator=g, device="cuda").bfloat16()
+        w = (torch.randn(E, 128, generator=g, device="cuda") * 0.1).bfloat16().requires_grad_(True)
+        logits, _, _, freq, _, aux = _FusedRouter.apply(x, w, K)
+        wrt = w
+    else:
+        logits = torch.randn(T, E, generator=g, device="cuda").bfloat16().requires_grad_(True)
+        freq = torch.bincount(torch.randint(0, E, (T * K,), generator=g, device="cuda"), minlength=E).int()
+        aux = switch_loss(logits, freq)
+        wrt = logits
+    (grad,) = torch.autograd.grad(aux, wrt, torch.tensor(3.0, device="cuda"))
+    if T == 0:
+        assert aux.item() == 0 and not grad.float().abs().sum().item()
+        return
+    lf = logits.detach().double().requires_grad_(True)
+    mean = torch.softmax(lf, -1).sum(0)
+    want = E * (mean / mean.sum() * (freq.double() / freq.sum())).sum()
+    (glogits,) = torch.autograd.grad(want * 3.0, lf)
+    assert abs(aux.item() / want.item() - 1) < 1e-5
+    assert rel(grad, glogits.T @ x.double() if fused else glogits) < 1e-2
