@@ -53,6 +53,8 @@ struct GemmParams {
   int* status;              // device word, 0 = ok
   int accumulate;           // plain-store epilogues: add to what out0 holds (bf16, fp32 sum, one rounding) instead of
                             // overwriting it -- weight gradients summed over several chunks of tokens
+  int min_rows;             // ragged-M tiles: experts with at most this many rows are left to another launch
+  int max_rows;             // kernel for experts with few rows: those with more are left to another launch
   // general epilogues
   const __nv_bfloat16* bias;  // (E, N) added to the accumulator, or nullptr
   int act;                    // Activation code
@@ -62,6 +64,20 @@ struct GemmParams {
   uint8_t* q_scale;           // (total_rows, q_scale_ld)
   long long q_scale_ld;
 };
+
+// Whether the experts with more than `limit` rows hold at least half of all rows.  Then the 256 x 256 tiles take all experts
+// and the kernel for experts with few rows finds nothing to do: most of the others have next to none, and a wave of each
+// kernel would cost more than tiles for all of them (T 640, top-8 of 128 experts, loads falling with the square of the rank:
+// up projection 208 us divided, 170 by tiles).  One warp, all lanes; both kernels come to the same answer.
+__device__ __forceinline__ bool tiles_take_all(const GemmParams& p, int limit, int lane) {
+  int above = 0;
+  for (int e = lane; e < p.E; e += 32) {
+    const int rows = p.off[e + 1] - p.off[e];
+    if (rows > limit) above += rows;
+  }
+  above = __reduce_add_sync(0xffffffffu, above);
+  return 2ll * above >= p.total_rows;
+}
 
 __device__ __forceinline__ float load_score(const void* scores, int is_bf16, int slot) {
   return is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(scores)[slot])

@@ -1,6 +1,7 @@
 // Host side of the grouped GEMMs: tensor-map construction and the C-ABI launchers.
 #include "device_cache.cuh"
 #include "gemm_pair.cuh"
+#include "gemm_skinny.cuh"
 
 #include <cstdlib>
 #include <mutex>
@@ -133,6 +134,42 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
   }
 }
 
+// Rows per unit of the kernel for experts with few rows (gemm_skinny.cuh), or 0 for the 256 x 256 tiles.  The line is the
+// mean number of rows per expert, all that the host knows of the load; an expert with more rows than a unit reads its
+// weights again, mostly from L2.  Up / down projection at H 4096, I 1024, E 128, us, units of 32 / 64 / 128 rows / tiles:
+// mean 4 339, 344, 353, 406 / 180, 183, 188, 197; mean 16 350, 350, 360, 409 / 195, 186, 193, 201; mean 32 533, 375, 377,
+// 407 / 234, 191, 195, 205; mean 64 867, 551, 387, 412 / 389, 244, 201, 209; mean 128 1546, 862, 594, 426 / 680, 391,
+// 252, 219.
+static int skinny_rows(int TK, int E) {
+  const double mean = static_cast<double>(TK) / E;
+  return mean <= 12 ? 32 : mean <= 40 ? 64 : mean <= 96 ? 128 : 0;
+}
+
+// A skewed load has experts with many rows beside many with few: above this many routed rows the experts that take more
+// than two units go to a second launch, of the 256 x 256 tiles (about 4 us when it finds nothing to do).  T 640, top-8 of
+// 128 experts, loads falling with the square of the rank, up / down projection: 166 / 90 us with tiles alone, 299 / 143
+// with units alone (tiles_take_all() gives such a load to the tiles).  Below it, all rows in one expert still cost less than that launch and a wave of its tiles.
+constexpr int SKINNY_ONLY_ROWS = 2048;
+static int skinny_max_rows(int TK, int nt) { return TK > SKINNY_ONLY_ROWS ? 2 * nt : TK; }
+
+template <bool GATHER, bool SWIGLU>
+static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p, int nt, cudaStream_t stream) {
+  auto kernel = skinny::skinny_gemm_kernel<GATHER, SWIGLU>;
+  static PerDeviceFlag configured;
+  const int dev = current_device();
+  if (dev < 0) return SMOE_ERR_DRIVER;
+  if (!configured.test(dev)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+      return SMOE_ERR_LAUNCH;
+    configured.set(dev);
+  }
+  const int sms = num_sms();
+  if (sms <= 0) return SMOE_ERR_DRIVER;
+  const int stages = skinny::num_stages(nt);
+  kernel<<<sms, skinny::threads(GATHER), skinny::smem_bytes(nt, stages), stream>>>(tmW, tmX, p, nt, stages);
+  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+}
+
 // An empty batch (T == 0, hence TK == 0) is valid: the entry points return at once (weight-gradient entry points
 // after zero-filling their output).  What is refused: negative sizes, or routed rows without any token.
 static bool bad_tokens(int T, int TK) { return T < 0 || TK < 0 || (T == 0 && TK > 0); }
@@ -161,12 +198,18 @@ int smoe_up_projection_forward(const void* x, const void* w1, void* z, void* y1,
   CUtensorMap tmA, tmB;
   SMOE_TRY(encode_2d(&tmA, x, T, H, H, 1, BK));                        // gather4 rows of x
   SMOE_TRY(encode_2d(&tmB, w1, (uint64_t)E * 2 * I, H, H, pair::BN_CTA, BK));    // W1[e] rows = output features, K-major
+  static_assert(pair::BN_CTA == skinny::BM, "one weight map for both kernels");
   GemmParams p = {};
   p.E = E; p.N = 2 * I; p.K = H; p.total_rows = TK; p.gather_rows = T; p.b_rows_per_expert = 2 * I;
   p.off = expert_offset; p.gather = x_gather_idx;
   p.out0 = static_cast<__nv_bfloat16*>(z); p.ld0 = 2 * I;
   p.out1 = static_cast<__nv_bfloat16*>(y1); p.ld1 = I;
   p.status = status;
+  if (const int nt = skinny_rows(TK, E)) {
+    p.max_rows = p.min_rows = skinny_max_rows(TK, nt);
+    SMOE_TRY((launch_skinny<true, true>(tmB, tmA, p, nt, static_cast<cudaStream_t>(stream))));
+    if (p.max_rows == TK) return SMOE_OK;
+  }
   return launch<false, true, false, false, false, EPI_SWIGLU>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
 }
 
@@ -182,6 +225,13 @@ int smoe_down_projection_forward(const void* y1, const void* w2, void* y2, const
   p.off = expert_offset;
   p.out0 = static_cast<__nv_bfloat16*>(y2); p.ld0 = H;
   p.status = status;
+  if (const int nt = skinny_rows(TK, E)) {
+    CUtensorMap tmX;
+    SMOE_TRY(encode_2d(&tmX, y1, TK, I, I, skinny::BOX_ROWS, BK));
+    p.max_rows = p.min_rows = skinny_max_rows(TK, nt);
+    SMOE_TRY((launch_skinny<false, false>(tmB, tmX, p, nt, static_cast<cudaStream_t>(stream))));
+    if (p.max_rows == TK) return SMOE_OK;
+  }
   return launch<false, false, false, false, false, EPI_STORE>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
 }
 

@@ -59,7 +59,7 @@ struct SharedStorage {
   uint32_t tmem_base;
   int abort_flag;
   int off[MAX_EXPERTS + 1];            // first grouped row of every expert
-  int m_tile_prefix[MAX_EXPERTS + 1];  // ragged-M: exclusive prefix of ceil(count / 256) per expert; ragged-K: counts
+  int m_tile_prefix[MAX_EXPERTS + 1];  // ragged-M: exclusive prefix of the experts' row tiles; ragged-K: counts
   int expert_order[MAX_EXPERTS];       // ragged-K with a skewed load: experts by descending count
   int most_rows;                       // ragged-K: the largest count
 };
@@ -266,11 +266,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     order_experts(p, ss);
   } else {
     if (warp == 2) {
+      const int min_rows = p.min_rows > 0 && !tiles_take_all(p, p.min_rows, lane) ? p.min_rows : 0;
       int running = 0;
       for (int base = 0; base < p.E; base += 32) {
         const int e = base + lane;
         int v = 0;
-        if (e < p.E) v = (p.off[e + 1] - p.off[e] + 2 * BM - 1) / (2 * BM);
+        if (e < p.E) {
+          const int rows = p.off[e + 1] - p.off[e];
+          v = rows > min_rows ? (rows + 2 * BM - 1) / (2 * BM) : 0;
+        }
         int incl = v;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {

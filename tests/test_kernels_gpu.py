@@ -654,3 +654,46 @@ def test_general_epilogues_at_tile_edges(smoe, act, I):
     assert rel(dz, torch.autograd.grad(y, zz, dy * sc[:, None])[0]) < BF16_TOL
     assert rel(ys, y.detach() * sc[:, None]) < BF16_TOL
     assert rel(part.sum(0), (y.detach() * dy).sum(-1)) < BF16_TOL
+
+
+@pytest.mark.parametrize("counts", [
+    [0, 1, 3, 4, 5, 16, 17, 31, 32, 33, 70, 0],   # mean below 20: 32-row units, experts with several of them
+    [0, 1, 15, 63, 64, 65, 130, 20],              # 64
+    [0, 127, 128, 129, 33, 97, 250, 1],           # 128
+    [0, 1500, 63, 128, 129, 64, 300, 1] + [2] * 70,  # above 2048 rows, most of them in few experts: tiles for all
+    [0, 500, 63, 128, 129, 64, 200, 1] + [25] * 70,  # those above two units go to the tiles
+    [1],
+])
+@pytest.mark.parametrize("H,I", [(192, 64), (512, 192), (64, 128)])
+def test_few_rows_per_expert(smoe, counts, H, I):
+    """Up projection (with and without z) and down projection around the row counts of a unit of the kernel for experts
+    with few rows, with a last feature block that is half empty (H 192, 64), against fp32."""
+    lib = smoe[0].lib
+    E, TK, T = len(counts), sum(counts), 50
+    g = torch.Generator().manual_seed(H + I + E)
+    x = torch.randn(T, H, generator=g).bfloat16()
+    w1 = (torch.randn(E, 2 * I, H, generator=g) * 0.05).bfloat16()
+    w2 = (torch.randn(E, H, I, generator=g) * 0.05).bfloat16()
+    tok = torch.randint(0, T, (TK,), generator=g, dtype=torch.int32)
+    expert = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))
+    off = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int32)
+    xd, w1d, w2d, td, od = [t.cuda() for t in (x, w1, w2, tok, off)]
+    nan = dict(fill_value=float("nan"), dtype=torch.bfloat16, device="cuda")
+    z, y1, y1b, y2 = (torch.full((TK + 1, n), **nan) for n in (2 * I, I, I, H))
+    st = smoe[0].device_state(z.device).status.data_ptr()
+    s = torch.cuda.current_stream().cuda_stream
+    assert lib.smoe_up_projection_forward(xd.data_ptr(), w1d.data_ptr(), z.data_ptr(), y1.data_ptr(), od.data_ptr(),
+                                          td.data_ptr(), T, H, I, E, TK, st, s) == 0
+    assert lib.smoe_up_projection_forward(xd.data_ptr(), w1d.data_ptr(), None, y1b.data_ptr(), od.data_ptr(),
+                                          td.data_ptr(), T, H, I, E, TK, st, s) == 0
+    assert lib.smoe_down_projection_forward(y1.data_ptr(), w2d.data_ptr(), y2.data_ptr(), od.data_ptr(), H, I, E, TK, st,
+                                            s) == 0
+    torch.cuda.synchronize()
+    smoe[0].check_status()
+    pre = torch.einsum("rh,rih->ri", x[tok.long()].float(), w1[expert].float())
+    assert rel(z[:TK], pre) < BF16_TOL
+    assert rel(y1[:TK], orc.activation("swiglu", pre)) < BF16_TOL
+    assert torch.equal(y1[:TK], y1b[:TK])
+    assert rel(y2[:TK], torch.einsum("ri,rhi->rh", y1[:TK].float().cpu(), w2[expert].float())) < BF16_TOL
+    for t in (z, y1, y1b, y2):  # nothing behind the last row
+        assert t[TK].isnan().all()
