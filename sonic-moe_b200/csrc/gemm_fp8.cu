@@ -177,15 +177,25 @@ __global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat1
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long base = (static_cast<long long>(e) * rows + static_cast<long long>(rb) * 128) * cols + cb * 128;
   const int nrows = min(128, rows - rb * 128);
+  // warp w has rows 16w .. 16w+15 of the block, half a warp per row and load, all of them in flight together; they stay in
+  // registers for the conversion.  Bound by memory: 8-byte loads in two dependent passes ran at 4.2 TB/s (1.02 ms for the
+  // weights of 32 experts, H 7168, I 2048; now 0.74 ms, 5.7 TB/s).
+  const int piece = lane & 15;
+  uint4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = warp * 16 + 2 * i + (lane >> 4);
+    v[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (r < nrows) v[i] = reinterpret_cast<const uint4*>(w + base + static_cast<long long>(r) * cols)[piece];
+  }
   float amax = 0.f;
-  // pass 1: warp w scans rows 16w .. 16w+15 of the block (a lane covers 4 columns)
-  for (int rr = 0; rr < 16; ++rr) {
-    const int r = warp * 16 + rr;
-    if (r < nrows) {
-      const uint2 v = reinterpret_cast<const uint2*>(w + base + static_cast<long long>(r) * cols)[lane];
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-      const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-      amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[i]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = __bfloat1622float2(h[j]);
+      amax = fmaxf(amax, fmaxf(fabsf(a.x), fabsf(a.y)));
     }
   }
 #pragma unroll
@@ -198,20 +208,20 @@ __global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat1
   const float s = amax > 0.f ? amax / 448.f : 1.f;
   float inv = 1.f;
   const uint8_t byte = POW2 ? pow2_scale(amax, inv) : 0;
-  // pass 2: the block is still in L1/L2
-  for (int rr = 0; rr < 16; ++rr) {
-    const int r = warp * 16 + rr;
-    if (r < nrows) {
-      const uint2 v = reinterpret_cast<const uint2*>(w + base + static_cast<long long>(r) * cols)[lane];
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-      const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-      uint32_t packed;
-      if (POW2)
-        packed = to_e4m3(a.x * inv) | (to_e4m3(a.y * inv) << 8) | (to_e4m3(b.x * inv) << 16) | (to_e4m3(b.y * inv) << 24);
-      else
-        packed = to_e4m3(a.x / s) | (to_e4m3(a.y / s) << 8) | (to_e4m3(b.x / s) << 16) | (to_e4m3(b.y / s) << 24);
-      reinterpret_cast<uint32_t*>(q + base + static_cast<long long>(r) * cols)[lane] = packed;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = warp * 16 + 2 * i + (lane >> 4);
+    if (r >= nrows) continue;
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[i]);
+    uint32_t packed[2] = {0u, 0u};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = __bfloat1622float2(h[j]);
+      const uint32_t two = POW2 ? (to_e4m3(a.x * inv) | (to_e4m3(a.y * inv) << 8))
+                                : (to_e4m3(a.x / s) | (to_e4m3(a.y / s) << 8));
+      packed[j >> 1] |= two << (16 * (j & 1));
     }
+    reinterpret_cast<uint2*>(q + base + static_cast<long long>(r) * cols)[piece] = make_uint2(packed[0], packed[1]);
   }
   if (threadIdx.x == 0) {
     const long long idx = (static_cast<long long>(e) * gridDim.y + rb) * gridDim.x + cb;
