@@ -105,4 +105,6 @@ def forward_token_choice_rounding(x: torch.Tensor, router_w: torch.Tensor, E: in
     topk_val = topk_val / topk_val.sum(dim=-1, keepdim=True)
     scores = probs.scatter(-1, idx64, topk_val)
     tokens, experts, _ = select_pairs(scores.detach(), topk_idx, routing)
-    return scores[tokens.long(), experts.long()].contiguous(), tokens, experts
+    # by flat position: the backward of a two-index lookup sorts its indices first, which the pairs, each there once, do
+    # not need
+    return scores.reshape(-1).gather(0, tokens.long() * E + experts), tokens, experts
