@@ -380,6 +380,15 @@ int smoe_router_backward_aux(void* dlogits, const void* logits, const float* dsc
 int smoe_switch_loss(const void* logits, const int* expert_count, float* aux, float* aux_grad, void* workspace, int T,
                      int E, void* stream);
 
+/* Inference forward of the bias-free SwiGLU layer with top-K routing in one call: smoe_router_forward_aux,
+ * smoe_route_metadata, smoe_up_projection_forward without z, smoe_down_projection_forward and smoe_gather_sum (K == 1:
+ * smoe_down_projection_forward_rows), with their requirements, in this order on the stream.  scratch:
+ * smoe_layer_forward_scratch_bytes(T, H, I, E, K) bytes of device memory, 256-byte aligned, that the call alone uses. */
+size_t smoe_layer_forward_scratch_bytes(int T, int H, int I, int E, int K);
+int smoe_layer_forward(const void* x, const void* router_w, const void* w1, const void* w2, void* o, void* logits,
+                       int* expert_count, float* prob_colsum, float* aux, void* scratch, int T, int H, int I, int E,
+                       int K, int* status, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Expert parallelism over peer memory (one node, NVLink / NVSwitch).  The reference has no distributed
  * code (sonicmoe/moe.py:260 skips even the aux-loss reduction), so these have no counterpart there; they

@@ -88,6 +88,8 @@ SIGNATURES: dict[str, tuple] = {
     "smoe_router_forward_aux": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, P, P]),
     "smoe_router_backward_aux": (I, [P, P, P, P, P, P, P, P, P, I, I, I, P]),
     "smoe_switch_loss": (I, [P, P, P, P, P, I, I, P]),
+    "smoe_layer_forward_scratch_bytes": (c_size_t, [I, I, I, I, I]),
+    "smoe_layer_forward": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P]),
     "smoe_peer_alloc": (I, [c_size_t, P]),
     "smoe_peer_free": (I, [P]),
     "smoe_peer_export": (I, [P, P]),
@@ -122,7 +124,7 @@ lib = _load()
 
 
 # kernels one successful entry-point call launches (1 unless listed)
-_KERNELS_PER_CALL = {"route_metadata": 3, "count_cumsum": 2, "router_forward": 2, "switch_loss": 2}
+_KERNELS_PER_CALL = {"route_metadata": 3, "count_cumsum": 2, "router_forward": 2, "switch_loss": 2, "layer_forward": 8}
 _launches = 0
 
 

@@ -23,6 +23,7 @@ from dataclasses import dataclass
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from .. import _lib
 from .._lib import check, lib, ptr, stream_ptr
@@ -675,6 +676,29 @@ def moe_TC_softmax_topk_layer_with_router_stats(x, router_w, w1, b1, w2, b2, K, 
     return _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inference_mode_enabled)[:4]
 
 
+def _layer_forward(x, router_w, w1, w2, K):
+    """The results of `_layer_with_aux` for a bias-free SwiGLU layer with the fused router where no gradient is wanted:
+    one call of the library, one piece of scratch."""
+    dev = x.device
+    T, H = x.shape
+    E = router_w.shape[0]
+    x, router_w = x.contiguous(), router_w.contiguous()
+    w1e, w2e = _expert_major(w1), _expert_major(w2)
+    I = w2e.shape[2]
+    with torch.cuda.device(dev):
+        o = torch.empty_like(x)
+        logits = torch.empty(T, E, dtype=torch.bfloat16, device=dev)
+        freq = torch.empty(E, dtype=torch.int32, device=dev)
+        colsum = torch.empty(E, dtype=torch.float32, device=dev)
+        aux = torch.empty((), dtype=torch.float32, device=dev)
+        scratch = torch.empty(lib.smoe_layer_forward_scratch_bytes(T, H, I, E, K), dtype=torch.uint8, device=dev)
+        check(lib.smoe_layer_forward(
+            x.data_ptr(), router_w.data_ptr(), w1e.data_ptr(), w2e.data_ptr(), o.data_ptr(), logits.data_ptr(),
+            freq.data_ptr(), colsum.data_ptr(), aux.data_ptr(), scratch.data_ptr(), T, H, I, E, K,
+            _lib.device_state(dev).status.data_ptr(), stream_ptr(dev)), "layer_forward")
+    return o, logits, freq, colsum, aux
+
+
 def _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inference_mode_enabled):
     """(o, router_logits, expert_frequency, column sums of softmax(router_logits), load-balancing loss); the last two
     are None where the fused routing kernel does not apply."""
@@ -682,7 +706,12 @@ def _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inferenc
     E = router_w.size(0)
     T = x.size(0)
     inference = is_inference_mode_enabled or not torch.is_grad_enabled()
-    if fused_router_applies(x, router_w, K):
+    fused = fused_router_applies(x, router_w, K)
+    if (fused and T > 0 and b1 is None and activation_type == ActivationType.SWIGLU and not _FUSED_COMBINE
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in (x, router_w, w1, w2)))
+            and not torch.jit.is_tracing() and forward_ad._current_level < 0):
+        return _layer_forward(x, router_w, w1, w2, K)
+    if fused:
         router_logits, scores, indices, _freq, colsum, aux = _FusedRouter.apply(x, router_w, K)
     else:
         colsum = aux = None

@@ -348,3 +348,33 @@ def test_chunks_share_weight_gradient_buffers(built_library, kind):
             assert rel(a, c) < tol and rel(b, c) < tol
             if len(bounds) == 3:
                 assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T,E,K", [(1, 32, 1), (1, 64, 4), (130, 32, 1), (777, 64, 4), (3000, 32, 8)])
+def test_forward_without_gradients_matches_training_forward(built_library, T, E, K):
+    """The one-call inference forward against the forward pass of a training step: the same kernels, so the same bits."""
+    import sonicmoe
+    from sonicmoe import _lib
+    from sonicmoe.enums import ActivationType
+
+    H, I = 256, 128
+    inp = orc.make_inputs(T, H, I, E, K, seed=T, dtype=torch.bfloat16)
+    m = sonicmoe.MoE(E, K, H, I, ActivationType.SWIGLU, False, 0.05).cuda().to(torch.bfloat16)
+    x = inp["x"].cuda()
+    o_ref, aux_ref = m(x)
+    assert o_ref.requires_grad
+    with torch.no_grad():
+        o, aux = m(x)
+        side = torch.cuda.Stream()  # its scratch is its own: a second stream gives the same
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            o_side, _ = m(x)
+        torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(o, o_ref) and torch.equal(aux, aux_ref) and torch.equal(o_side, o_ref)
+    assert not o.requires_grad
+    out, logits, freq = sonicmoe.moe_TC_softmax_topk_layer(
+        x, m.router.weight.detach(), m.c_fc.weight.detach().permute(1, 2, 0), None,
+        m.c_proj.weight.detach().permute(1, 2, 0), None, K, 0, ActivationType.SWIGLU, True)
+    assert torch.equal(out, o_ref) and logits.shape == (T, E) and int(freq.sum()) == T * K
