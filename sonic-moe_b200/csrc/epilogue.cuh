@@ -10,7 +10,7 @@ enum Epilogue : int {
   EPI_SWIGLU = 1,   // out0[r, n] = bf16(acc) (unless out0 == nullptr); out1[r, n/2] = silu(acc[2j]) * acc[2j+1]
   EPI_DSWIGLU = 2,  // acc = dy1; reads z, score; writes dz (out0), y1*s (out1), per-row partial of ds
   EPI_SCATTER = 3,  // red.add fp32: acc_out[token(r), n] += score(r) * acc
-  // general forms: any activation of the layer, optional per-expert bias (GemmParams::act, ::bias)
+  // general forms: any activation of the layer, optional per-expert bias (EPI + 16 * Activation, GemmParams::bias)
   EPI_ACT = 4,         // z = acc + b1 -> out0 (unless nullptr); y1 = act(z) (gated: act(z_even) * z_odd) -> out1
   EPI_DACT = 5,        // acc = dy1; reads z, score; writes dz (out0), y1*s (out1), per-row partial of ds
   EPI_STORE_BIAS = 6,  // out0[r, n] = bf16(acc + bias[e, n])
@@ -19,7 +19,7 @@ enum Epilogue : int {
                        // routed row each, with the rounding points of the store + gather_sum pair it replaces
 };
 
-// Activation codes (GemmParams::act).  The first three are gated: the pre-activation has 2I columns,
+// Activation codes.  The first three are gated: the pre-activation has 2I columns,
 // gate = even column, up = odd column.
 enum Activation : int { ACT_SWIGLU = 0, ACT_GEGLU = 1, ACT_REGLU = 2, ACT_RELU_SQ = 3, ACT_RELU = 4, ACT_GELU = 5,
                         ACT_SILU = 6 };
@@ -57,7 +57,6 @@ struct GemmParams {
   int max_rows;             // kernel for experts with few rows: those with more are left to another launch
   // general epilogues
   const __nv_bfloat16* bias;  // (E, N) added to the accumulator, or nullptr
-  int act;                    // Activation code
   // EPI_DSWIGLU of the hardware-scaled FP8 kernel: dz also leaves the epilogue quantised (E4M3, one UE8M0 scale
   // byte per row and 128 columns), nullptr = not wanted
   uint8_t* q_out;             // (total_rows, 2N)
@@ -127,26 +126,15 @@ __device__ __forceinline__ void act_value_grad(float x, float& a, float& da) {
   }
 }
 
-template <int FN, bool GATED>
-struct ActKind {
-  static constexpr int fn = FN;
-  static constexpr bool gated = GATED;
-};
-
-// f(ActKind) for an Activation code, once per tile: with the switch inside the element loop the values of a row form
-// one serial chain of branches and function latencies (measured at T 8191, H 1024, I 512, E 32, K 4 with GELU, together
-// with rows stored one per lane by four warps: dH 196 us, up projection 134 us).
-template <class F>
-__device__ __forceinline__ auto act_dispatch(int act, F&& f) {
-  switch (act) {
-    case ACT_SWIGLU: return f(ActKind<FN_SILU, true>{});
-    case ACT_GEGLU: return f(ActKind<FN_GELU, true>{});
-    case ACT_REGLU: return f(ActKind<FN_RELU, true>{});
-    case ACT_RELU_SQ: return f(ActKind<FN_RELU_SQ, false>{});
-    case ACT_RELU: return f(ActKind<FN_RELU, false>{});
-    case ACT_GELU: return f(ActKind<FN_GELU, false>{});
-    default: return f(ActKind<FN_SILU, false>{});
-  }
+// The general epilogues are compiled once per activation (GEMM template argument EPI + 16 * Activation): with a switch
+// inside the element loop the values of a row formed one serial chain of branches and function latencies, and with one
+// around the tile's loop the widest variant's spills slowed all of them (dH of T 8191, H 1024, I 512, E 32, K 4 with GELU:
+// 196 us, 119 us, and 64 as it is).
+__host__ __device__ constexpr int epi_base(int epi_code) { return epi_code % 16; }
+__host__ __device__ constexpr int act_fn(int act) {
+  return act == ACT_GEGLU || act == ACT_GELU ? FN_GELU
+         : act == ACT_RELU_SQ                ? FN_RELU_SQ
+         : act == ACT_REGLU || act == ACT_RELU ? FN_RELU : FN_SILU;
 }
 
 __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float (&f)[32]) {

@@ -122,7 +122,7 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
     // that pass staged through shared memory like the single-tile one: step 17.75-17.97 ms dual against 17.88-18.13 ms
     // single in alternating runs, the kernel alone 2.26-2.69 against 2.09-2.58 ms -- no gain worth a second variant.  The general forward epilogue is
     // too long to be worked off from registers, and must not hold accumulators that the next unit needs.
-    if constexpr (EPI != EPI_DSWIGLU && EPI != EPI_DACT && EPI != EPI_ACT) {
+    if constexpr (EPI != EPI_DSWIGLU && epi_base(EPI) != EPI_DACT && epi_base(EPI) != EPI_ACT) {
     if (use_dual_tiles() && fits) {
       constexpr int kDual = A_GATHER ? pair::DUAL_N : pair::DUAL_M;
       return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 4, kDual>(tmA, tmB, p, stream);
@@ -132,6 +132,22 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
     constexpr int kGatherWarps = EPI == EPI_STORE ? 8 : 4;
     return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, kGatherWarps>(tmA, tmB, p, stream);
   }
+}
+
+// The kernel of a general epilogue (gathered rows, weights K-major or MN-major) compiled for this activation.
+template <bool B_MN, int EPI>
+static int launch_activation(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int activation,
+                             cudaStream_t stream) {
+  switch (activation) {
+    case ACT_SWIGLU: return launch<false, true, false, false, B_MN, EPI + 16 * ACT_SWIGLU>(tmA, tmB, p, stream);
+    case ACT_GEGLU: return launch<false, true, false, false, B_MN, EPI + 16 * ACT_GEGLU>(tmA, tmB, p, stream);
+    case ACT_REGLU: return launch<false, true, false, false, B_MN, EPI + 16 * ACT_REGLU>(tmA, tmB, p, stream);
+    case ACT_RELU_SQ: return launch<false, true, false, false, B_MN, EPI + 16 * ACT_RELU_SQ>(tmA, tmB, p, stream);
+    case ACT_RELU: return launch<false, true, false, false, B_MN, EPI + 16 * ACT_RELU>(tmA, tmB, p, stream);
+    case ACT_GELU: return launch<false, true, false, false, B_MN, EPI + 16 * ACT_GELU>(tmA, tmB, p, stream);
+    case ACT_SILU: return launch<false, true, false, false, B_MN, EPI + 16 * ACT_SILU>(tmA, tmB, p, stream);
+  }
+  return SMOE_ERR_SHAPE;
 }
 
 // Rows per unit of the kernel for experts with few rows (gemm_skinny.cuh), or 0 for the 256 x 256 tiles.  The line is the
@@ -308,9 +324,9 @@ int smoe_up_projection_forward_act(const void* x, const void* w1, const void* b1
   p.off = expert_offset; p.gather = x_gather_idx;
   p.out0 = static_cast<__nv_bfloat16*>(z); p.ld0 = N1;
   p.out1 = static_cast<__nv_bfloat16*>(y1); p.ld1 = act_is_gated(activation) ? N1 / 2 : N1;
-  p.bias = static_cast<const __nv_bfloat16*>(b1); p.act = activation;
+  p.bias = static_cast<const __nv_bfloat16*>(b1);
   p.status = status;
-  return launch<false, true, false, false, false, EPI_ACT>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
+  return launch_activation<false, EPI_ACT>(tmA, tmB, p, activation, static_cast<cudaStream_t>(stream));
 }
 
 int smoe_down_projection_forward_bias(const void* y1, const void* w2, const void* b2, void* y2,
@@ -349,9 +365,8 @@ int smoe_down_projection_backward_dact(const void* dout, const void* w2, const v
   p.out1 = static_cast<__nv_bfloat16*>(y1s); p.ld1 = I;
   p.z = static_cast<const __nv_bfloat16*>(z);
   p.scores = scores; p.scores_are_bf16 = scores_are_bf16; p.ds_partial = ds_partial;
-  p.act = activation;
   p.status = status;
-  return launch<false, true, false, false, true, EPI_DACT>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
+  return launch_activation<true, EPI_DACT>(tmA, tmB, p, activation, static_cast<cudaStream_t>(stream));
 }
 
 int smoe_ds_partial_columns(int I) { return 2 * ((I + BN - 1) / BN); }

@@ -45,7 +45,7 @@ constexpr int EPI_WARPS = 8;
 // chunks beside the activation's arithmetic) move registers to them with setmaxnreg.  That is a warpgroup-wide
 // instruction, so these keep warps 2 and 3 idle: warps 0-3 producer / MMA, 4-11 epilogue, 12-15 gather.
 __host__ __device__ constexpr bool splits_registers(int epi, int dual) {
-  return dual != 0 || epi == EPI_DSWIGLU || epi == EPI_DACT || epi == EPI_ACT;
+  return dual != 0 || epi_base(epi) == EPI_DSWIGLU || epi_base(epi) == EPI_DACT || epi_base(epi) == EPI_ACT;
 }
 __host__ __device__ constexpr int threads(int gather_warps, bool split) {
   return 32 * ((split ? 4 : 2) + EPI_WARPS + gather_warps);
@@ -203,11 +203,13 @@ struct UnitWalker {
   }
 };
 
-template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI, int GW,
+template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI_CODE, int GW,
           int DUAL = DUAL_NONE>
-__global__ void __launch_bounds__(threads(GW, splits_registers(EPI, DUAL)), 1)
+__global__ void __launch_bounds__(threads(GW, splits_registers(EPI_CODE, DUAL)), 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const GemmParams p) {
+  constexpr int EPI = epi_base(EPI_CODE);
+  constexpr int ACT = EPI_CODE / 16;  // general epilogues: the Activation
   // DUAL: four stages of three 16 KiB tiles (A, B and the second plain tile X) instead of six stages of two
   constexpr int NSTAGES = DUAL != DUAL_NONE ? 4 : STAGES;
   constexpr int X_STAGE_BYTES = DUAL != DUAL_NONE ? A_STAGE_BYTES : 0;
@@ -658,20 +660,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             ok = dact_columns<FN_SILU, true, CHUNKS>(p, my_stage, lane, row_base, tile.row_end, n_first,
                                                                       t_cols, score, ds_acc, wait_acc, release_acc);
           } else if constexpr (EPI == EPI_DACT) {
-            ok = act_dispatch(p.act, [&](auto kind) {
-              using Kind = decltype(kind);
-              return dact_columns<Kind::fn, Kind::gated, CHUNKS>(
-                  p, my_stage, lane, row_base, tile.row_end, n_first, t_cols, score, ds_acc, wait_acc, release_acc);
-            });
+            ok = dact_columns<act_fn(ACT), act_is_gated(ACT), CHUNKS>(p, my_stage, lane, row_base, tile.row_end, n_first,
+                                                                      t_cols, score, ds_acc, wait_acc, release_acc);
           } else if constexpr (EPI == EPI_SWIGLU) {
             act_columns<FN_SILU, true, CHUNKS>(p, tile.e, my_stage, lane, row_base, tile.row_end, n_first,
                                                                 t_cols, release_acc);
           } else if constexpr (EPI == EPI_ACT) {
-            act_dispatch(p.act, [&](auto kind) {
-              using Kind = decltype(kind);
-              act_columns<Kind::fn, Kind::gated, CHUNKS>(p, tile.e, my_stage, lane, row_base,
-                                                                          tile.row_end, n_first, t_cols, release_acc);
-            });
+            act_columns<act_fn(ACT), act_is_gated(ACT), CHUNKS>(p, tile.e, my_stage, lane, row_base, tile.row_end, n_first,
+                                                                t_cols, release_acc);
           } else {
             int dst_row = 0;
             if constexpr (EPI == EPI_STORE_ROWS || EPI == EPI_SCATTER) {
