@@ -319,7 +319,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           const int k0 = RAGGED_K ? (tile.k_begin + kb * BK) : kb * BK;
           if constexpr (!A_GATHER) {
             if constexpr (!A_MN) {
-              if (lane == 0) tma_load_2d_pair(&tmA, bar, a_dst, k0, tile.row0);
+              // no rows at all in this CTA's half of the tile: read past the tensor's end, which delivers zeros
+              if (lane == 0)
+                tma_load_2d_pair(&tmA, bar, a_dst, k0, tile.row0 < tile.row_end ? tile.row0 : p.total_rows);
             } else {
               if (lane < BM / 64) tma_load_2d_pair(&tmA, bar, a_dst + lane * CHUNK_BYTES, tile.row0 + 64 * lane, k0);
             }
@@ -453,7 +455,9 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const int r = tile.row0 + 4 * j + i;
-              r4[i] = (r < p.total_rows) ? p.gather[r] : 0;
+              r4[i] = (r < tile.row_end) ? p.gather[r] : p.gather_rows;  // rows that do not exist: zeros
+              // (they cost no traffic and next to no power; multiplying other rows in their place took 2.5 % longer where a
+              // fifth of the tiles' rows do not exist, up projection of 512 rows per expert 980 -> 959 us)
             }
             for (int kb = 0; kb < tile.num_kb; ++kb) {
               if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
