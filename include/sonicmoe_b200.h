@@ -258,7 +258,9 @@ int smoe_ds_add_bias_term(const void* dout, const void* b2, const int* expert_of
 /* q (rows, cols) uint8 E4M3 and scale (rows, cols/128) fp32 from x (rows, cols) bf16; cols % 128 == 0. */
 int smoe_fp8_quantize_rows(const void* x, void* q, float* scale, long long rows, int cols, void* stream);
 
-/* q (batch, rows, cols) and scale (batch, ceil(rows/128), cols/128) from w (batch, rows, cols) bf16. */
+/* q (batch, rows, cols) and scale (batch, ceil(rows/128), cols/128) from w (batch, rows, cols) bf16.  A w that is
+ * only 8-byte aligned (a view into a larger buffer) and a q that is only 4-byte aligned are taken as well; the same
+ * holds for smoe_mxfp8_quantize_blocks. */
 int smoe_fp8_quantize_blocks(const void* w, void* q, float* scale, int batch, int rows, int cols, void* stream);
 
 /* As smoe_up_projection_forward with xq (T,H) + x_scale (T,H/128), w1q (E,2I,H) + w1_scale (E,2I/128,H/128);

@@ -168,7 +168,8 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16*
 
 // One CTA per 128 x 128 block of a (batch, rows, cols) tensor; rows need not be a multiple of 128.
 // POW2: the scale is a UE8M0 byte (smallest power of two >= amax / 448), else fp32 amax / 448.
-template <bool POW2>
+// WIDE: w is 16-byte and q 8-byte aligned; otherwise (a view into a larger buffer) w is 8-byte and q 4-byte aligned.
+template <bool POW2, bool WIDE>
 __global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat16* __restrict__ w,
                                                               uint8_t* __restrict__ q, void* __restrict__ scale,
                                                               int rows, int cols) {
@@ -186,7 +187,15 @@ __global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat1
   for (int i = 0; i < 8; ++i) {
     const int r = warp * 16 + 2 * i + (lane >> 4);
     v[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (r < nrows) v[i] = reinterpret_cast<const uint4*>(w + base + static_cast<long long>(r) * cols)[piece];
+    if (r < nrows) {
+      const __nv_bfloat16* src = w + base + static_cast<long long>(r) * cols + 8 * piece;
+      if constexpr (WIDE) {
+        v[i] = *reinterpret_cast<const uint4*>(src);
+      } else {
+        const uint2 a = reinterpret_cast<const uint2*>(src)[0], b = reinterpret_cast<const uint2*>(src)[1];
+        v[i] = make_uint4(a.x, a.y, b.x, b.y);
+      }
+    }
   }
   float amax = 0.f;
 #pragma unroll
@@ -221,13 +230,32 @@ __global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat1
                                 : (to_e4m3(a.x / s) | (to_e4m3(a.y / s) << 8));
       packed[j >> 1] |= two << (16 * (j & 1));
     }
-    reinterpret_cast<uint2*>(q + base + static_cast<long long>(r) * cols)[piece] = make_uint2(packed[0], packed[1]);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(q + base + static_cast<long long>(r) * cols) + 2 * piece;
+    if constexpr (WIDE) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[1]);
+    } else {
+      dst[0] = packed[0];
+      dst[1] = packed[1];
+    }
   }
   if (threadIdx.x == 0) {
     const long long idx = (static_cast<long long>(e) * gridDim.y + rb) * gridDim.x + cb;
     if (POW2) static_cast<uint8_t*>(scale)[idx] = byte;
     else static_cast<float*>(scale)[idx] = s;
   }
+}
+
+template <bool POW2>
+static int quantize_blocks(const void* w, void* q, void* scale, int batch, int rows, int cols, void* stream) {
+  if (batch <= 0 || rows <= 0 || cols <= 0 || (cols % 128) != 0) return SMOE_ERR_SHAPE;
+  const uintptr_t wa = reinterpret_cast<uintptr_t>(w), qa = reinterpret_cast<uintptr_t>(q);
+  if (wa % 8 != 0 || qa % 4 != 0) return SMOE_ERR_ALIGNMENT;
+  if (!POW2 && reinterpret_cast<uintptr_t>(scale) % 4 != 0) return SMOE_ERR_ALIGNMENT;
+  const dim3 grid(cols / 128, (rows + 127) / 128, batch);
+  const auto kernel = wa % 16 == 0 && qa % 8 == 0 ? quantize_blocks_kernel<POW2, true> : quantize_blocks_kernel<POW2, false>;
+  kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(w),
+                                                              static_cast<uint8_t*>(q), scale, rows, cols);
+  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 
 }  // namespace fp8
@@ -255,11 +283,7 @@ int smoe_fp8_quantize_rows(const void* x, void* q, float* scale, long long rows,
 }
 
 int smoe_fp8_quantize_blocks(const void* w, void* q, float* scale, int batch, int rows, int cols, void* stream) {
-  if (batch <= 0 || rows <= 0 || cols <= 0 || (cols % 128) != 0) return SMOE_ERR_SHAPE;
-  const dim3 grid(cols / 128, (rows + 127) / 128, batch);
-  quantize_blocks_kernel<false><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(w), static_cast<uint8_t*>(q), scale, rows, cols);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return quantize_blocks<false>(w, q, scale, batch, rows, cols, stream);
 }
 
 int smoe_fp8_up_projection_forward(const void* xq, const float* x_scale, const void* w1q, const float* w1_scale,
@@ -355,11 +379,7 @@ int smoe_mxfp8_quantize_rows(const void* x, void* q, void* scale, long long rows
 }
 
 int smoe_mxfp8_quantize_blocks(const void* w, void* q, void* scale, int batch, int rows, int cols, void* stream) {
-  if (batch <= 0 || rows <= 0 || cols <= 0 || (cols % 128) != 0) return SMOE_ERR_SHAPE;
-  const dim3 grid(cols / 128, (rows + 127) / 128, batch);
-  quantize_blocks_kernel<true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(w), static_cast<uint8_t*>(q), scale, rows, cols);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return quantize_blocks<true>(w, q, scale, batch, rows, cols, stream);
 }
 
 static mx8::ScaleBytes mx_scales(const void* a, int a_cols, const void* b, long long b_expert, long long b_n,

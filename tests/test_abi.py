@@ -52,3 +52,14 @@ def test_queries_and_argument_checks_without_gpu(built_library):
     # empty problems are no-ops
     assert lib.smoe_topk_softmax(None, 0, None, None, 0, 8, 2, None) == 0
     assert lib.smoe_up_projection_forward(None, None, None, None, None, None, 16, 128, 64, 8, 0, None, None) == 0
+
+
+def test_block_quantiser_refuses_misaligned_pointers(built_library):
+    """Refused before anything is launched (the addresses here belong to nothing)."""
+    from sonicmoe._lib import lib
+
+    for quantise in (lib.smoe_fp8_quantize_blocks, lib.smoe_mxfp8_quantize_blocks):
+        assert quantise(4096 + 2, 8192, 8192, 1, 128, 128, None) == -2
+        assert quantise(4096 + 4, 8192, 8192, 1, 128, 128, None) == -2
+        assert quantise(4096, 8192 + 2, 8192, 1, 128, 128, None) == -2
+    assert lib.smoe_fp8_quantize_blocks(4096, 8192, 8192 + 2, 1, 128, 128, None) == -2

@@ -62,6 +62,20 @@ def test_quantize_blocks(built_library, E, rows, cols):
     assert rel(dequant_blocks(q, s), w) < 0.04
 
 
+@pytest.mark.parametrize("fmt", ["fp32", "ue8m0"])
+@pytest.mark.parametrize("offset", [4, 8, 12])
+def test_quantize_blocks_of_a_view(built_library, fmt, offset):
+    """Weights that are a view into a larger buffer, 8-byte but not 16-byte aligned: the same bytes as from a copy."""
+    from sonicmoe.functional import fp8
+
+    E, rows, cols = 2, 200, 256
+    g = torch.Generator().manual_seed(offset)
+    flat = (torch.randn(offset + E * rows * cols, generator=g) * 0.02).bfloat16().cuda()
+    view = flat[offset:].view(E, rows, cols)
+    got, want = fp8.quantize_blocks(view, fmt), fp8.quantize_blocks(view.clone(), fmt)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 128), (1000, 256), (4096, 1024), (333, 640)])
 def test_quantize_rows_pow2(built_library, rows, cols):
     from oracle import fp8_sim
