@@ -33,6 +33,8 @@ struct Scratch {
   }
 };
 
+bool aligned(const void* p, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
+
 }  // namespace
 
 #define SMOE_TRY(expr)              \
@@ -51,8 +53,22 @@ size_t smoe_layer_forward_scratch_bytes(int T, int H, int I, int E, int K) {
 int smoe_layer_forward(const void* x, const void* router_w, const void* w1, const void* w2, void* o, void* logits,
                        int* expert_count, float* prob_colsum, float* aux, void* scratch, int T, int H, int I, int E,
                        int K, int* status, void* stream) {
-  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || K <= 0 || static_cast<long long>(T) * K > 0x7fffffffll) return SMOE_ERR_SHAPE;
+  // what any of the calls below would refuse is refused before the first of them launches something
+  if (T <= 0 || !smoe_router_forward_supported(H, E, K) || I <= 0 || I % 64 != 0 ||
+      static_cast<long long>(T) * K > 0x7fffffffll)
+    return SMOE_ERR_SHAPE;
+  const void* const wide[] = {x, router_w, w1, w2, o, logits};  // TMA sources, and rows stored in 16-byte pieces
+  for (const void* ptr : wide) {
+    if (ptr == nullptr) return SMOE_ERR_SHAPE;
+    if (!aligned(ptr, 16)) return SMOE_ERR_ALIGNMENT;
+  }
+  const void* const words[] = {expert_count, prob_colsum, aux};
+  for (const void* ptr : words) {
+    if (ptr == nullptr) return SMOE_ERR_SHAPE;
+    if (!aligned(ptr, 4)) return SMOE_ERR_ALIGNMENT;
+  }
   if (scratch == nullptr) return SMOE_ERR_WORKSPACE;
+  if (!aligned(scratch, 256)) return SMOE_ERR_ALIGNMENT;
   const Scratch at(T, H, I, E, K);
   char* base = static_cast<char*>(scratch);
   const auto ints = [base](size_t o_) { return reinterpret_cast<int*>(base + o_); };

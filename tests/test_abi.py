@@ -63,3 +63,20 @@ def test_block_quantiser_refuses_misaligned_pointers(built_library):
         assert quantise(4096 + 4, 8192, 8192, 1, 128, 128, None) == -2
         assert quantise(4096, 8192 + 2, 8192, 1, 128, 128, None) == -2
     assert lib.smoe_fp8_quantize_blocks(4096, 8192, 8192 + 2, 1, 128, 128, None) == -2
+
+
+def test_layer_forward_refuses_before_the_first_launch(built_library):
+    """Sizes and pointers that only a later kernel of the call would refuse (the addresses here belong to nothing)."""
+    from sonicmoe._lib import lib
+
+    def call(T=4, H=128, I=64, E=32, K=2, **bad):
+        names = ["x", "router_w", "w1", "w2", "o", "logits", "expert_count", "prob_colsum", "aux", "scratch"]
+        return lib.smoe_layer_forward(*[bad.get(n, 4096) for n in names], T, H, I, E, K, None, None)
+
+    assert call(I=100) == -1 and call(I=0) == -1 and call(H=100) == -1 and call(E=8) == -1 and call(K=17) == -1
+    assert call(T=0) == -1 and call(T=2 ** 30, K=2) == -1
+    for name in ("x", "router_w", "w1", "w2", "o", "logits"):
+        assert call(**{name: 4096 + 8}) == -2 and call(**{name: None}) == -1, name
+    for name in ("expert_count", "prob_colsum", "aux"):
+        assert call(**{name: 4096 + 2}) == -2 and call(**{name: None}) == -1, name
+    assert call(scratch=4096 + 16) == -2 and call(scratch=None) == -7
