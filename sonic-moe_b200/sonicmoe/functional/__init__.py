@@ -410,6 +410,12 @@ def _check_experts_args(x, w1, w2, b1, b2, activation_type):
     return activation_type
 
 
+def _check_router_args(x, router_w, w1):
+    """The kernels take the number of experts from the router and read that many experts' weights."""
+    if router_w.shape != (w1.shape[2], x.shape[1]):
+        raise ValueError(f"inconsistent shapes: x {tuple(x.shape)}, router {tuple(router_w.shape)}, w1 {tuple(w1.shape)}")
+
+
 def _experts(x, w1, b1, w2, b2, scores_flat, route, T, inference, activation_type):
     """Routed experts: the tuned bias-free SwiGLU kernels, or the general ones for a bias / another activation."""
     if b1 is None and activation_type == ActivationType.SWIGLU:
@@ -702,6 +708,7 @@ def _layer_forward(x, router_w, w1, w2, K):
 def _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inference_mode_enabled):
     """(o, router_logits, expert_frequency, column sums of softmax(router_logits), load-balancing loss); the last two
     are None where the fused routing kernel does not apply."""
+    _check_router_args(x, router_w, w1)
     activation_type = _check_experts_args(x, w1, w2, b1, b2, activation_type)
     E = router_w.size(0)
     T = x.size(0)

@@ -259,9 +259,10 @@ def moe_fp8_softmax_topk_layer(x, router_w, w1, b1, w2, b2, K, stream_id=0,
                                is_inference_mode_enabled: bool = False, scale_format: str | None = None):
     """``moe_TC_softmax_topk_layer`` with the expert GEMMs of forward and activation gradients in FP8
     (``scale_format``: "fp32", "ue8m0" or None for the module default)."""
-    from . import _check_experts_args, _route_metadata, topk_softmax
+    from . import _check_experts_args, _check_router_args, _route_metadata, topk_softmax
 
     refuse_unsupported(b1, b2, activation_type)
+    _check_router_args(x, router_w, w1)
     activation_type = _check_experts_args(x, w1, w2, b1, b2, activation_type)
     H = x.shape[1]
     if H % BLOCK != 0 or (w1.shape[0] // 2) % BLOCK != 0:

@@ -169,3 +169,15 @@ def test_weight_grad_sum_bookkeeping():
     out1, out2 = shared.finish_chunk()
     assert out1 is d1 and out2 is d2
     assert shared.dw1 is None and shared.dw2 is None and shared.remaining == 0
+
+
+def test_router_and_expert_weights_must_agree(built_library):
+    """One number of experts, one hidden size: checked before anything reads a weight."""
+    from sonicmoe.functional import moe_TC_softmax_topk_layer
+    from sonicmoe.functional.fp8 import moe_fp8_softmax_topk_layer
+
+    x, w1, w2 = torch.zeros(4, 128), torch.zeros(256, 128, 32), torch.zeros(128, 128, 32)
+    for layer in (moe_TC_softmax_topk_layer, moe_fp8_softmax_topk_layer):
+        for router in (torch.zeros(64, 128), torch.zeros(16, 128), torch.zeros(32, 64), torch.zeros(32, 256)):
+            with pytest.raises(ValueError):
+                layer(x, router, w1, None, w2, None, 2)
