@@ -266,7 +266,7 @@ def time_kernels(moe, x, dout, cfg, peaks, reps=5):
         r_idx = torch.empty(T, K, dtype=torch.int32, device=dev)
         r_cnt = torch.empty(E, dtype=torch.int32, device=dev)
         r_col = torch.empty(E, dtype=torch.float32, device=dev)
-        r_ws = _lib.device_state(dev).router_workspace(E)
+        r_ws = _lib.workspace(lib.smoe_router_forward_workspace_bytes(E), dev)
         hbm_ops["router_forward_fused"] = (T * H * 2 + E * H * 2 + T * E * 2 + T * K * 8, lambda: lib.smoe_router_forward(
             x.data_ptr(), rw.data_ptr(), r_logits.data_ptr(), r_scores.data_ptr(), r_idx.data_ptr(), r_cnt.data_ptr(),
             r_col.data_ptr(), r_ws.data_ptr(), T, H, E, K, st, stream))
@@ -275,7 +275,7 @@ def time_kernels(moe, x, dout, cfg, peaks, reps=5):
         hbm_ops["router_backward"] = (2 * T * E * 2 + T * K * 12, lambda: lib.smoe_router_backward(
             d_logits.data_ptr(), logits.data_ptr(), g_sc.data_ptr(), sc.data_ptr(), idx.data_ptr(), None, None, T, E, K,
             stream))
-    m_ws = _lib.device_state(dev).route_workspace(E)
+    m_ws = _lib.workspace(lib.smoe_route_metadata_workspace_bytes(E), dev)
     m_out = torch.empty(3, TK, dtype=torch.int32, device=dev)
     m_cnt = torch.empty(E, dtype=torch.int32, device=dev)
     m_off = torch.empty(E + 1, dtype=torch.int32, device=dev)

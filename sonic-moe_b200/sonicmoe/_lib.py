@@ -140,6 +140,11 @@ def launch_count() -> int:
     return _launches
 
 
+def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
+    """Scratch of one library call, from the current stream's pool."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
 def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
@@ -163,25 +168,11 @@ def require_cuda(t: torch.Tensor, name: str) -> None:
 
 
 class _DeviceState:
-    """Per-device scratch owned by the Python side: the GEMM status word and the routing workspace."""
+    """What the Python side keeps per device: the GEMM status word.  Workspaces belong to the call that needs them, so that
+    layers may run on several streams and threads of a device."""
 
     def __init__(self, device: torch.device) -> None:
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
-        self.route_ws = torch.empty(0, dtype=torch.int32, device=device)
-        self.router_ws = torch.empty(0, dtype=torch.uint8, device=device)
-
-    def route_workspace(self, E: int) -> torch.Tensor:
-        need = lib.smoe_route_metadata_workspace_bytes(E) // 4
-        if self.route_ws.numel() < need:
-            self.route_ws = torch.empty(need, dtype=torch.int32, device=self.status.device)
-        return self.route_ws
-
-
-    def router_workspace(self, E: int) -> torch.Tensor:
-        need = lib.smoe_router_forward_workspace_bytes(E)
-        if self.router_ws.numel() < need:
-            self.router_ws = torch.empty(need, dtype=torch.uint8, device=self.status.device)
-        return self.router_ws
 
 
 _states: dict[int, _DeviceState] = {}

@@ -25,7 +25,7 @@ def count_cumsum(x: torch.Tensor, E: int, do_cumsum: bool = True):
         count = torch.empty(E, dtype=torch.int32, device=dev)
         cumsum = torch.empty(E, dtype=torch.int32, device=dev) if do_cumsum else None
         # bins beyond 4096 are counted with global atomics and need no scratch
-        ws = _lib.device_state(dev).route_workspace(E) if E <= 4096 else None
+        ws = _lib.workspace(_lib.lib.smoe_count_cumsum_workspace_bytes(E), dev) if E <= 4096 else None
         rc = _lib.lib.smoe_count_cumsum(
             x.data_ptr(), _lib.dtype_code(x.dtype), x.numel(), E, count.data_ptr(), _lib.ptr(cumsum),
             _lib.ptr(ws), _lib.stream_ptr(dev),

@@ -148,7 +148,7 @@ def _route_metadata(expert_idx: torch.Tensor, token_idx: torch.Tensor | None, E:
         freq = torch.empty(E, dtype=torch.int32, device=dev)
         off = torch.empty(E + 1, dtype=torch.int32, device=dev)
         idx3 = torch.empty(3, n, dtype=torch.int32, device=dev)
-        ws = _lib.device_state(dev).route_workspace(E)
+        ws = _lib.workspace(lib.smoe_route_metadata_workspace_bytes(E), dev)
         rc = lib.smoe_route_metadata(
             expert_idx.data_ptr(), ptr(token_idx), n, E, max(K, 1), freq.data_ptr(), off.data_ptr(),
             idx3[0].data_ptr(), idx3[1].data_ptr(), idx3[2].data_ptr(), ws.data_ptr(), stream_ptr(dev),
@@ -297,7 +297,7 @@ class _FusedRouter(torch.autograd.Function):
             colsum = torch.empty(E, dtype=torch.float32, device=dev)
             aux = torch.empty((), dtype=torch.float32, device=dev)
             aux_grad = torch.empty(E, dtype=torch.float32, device=dev)
-            ws = st.router_workspace(E)
+            ws = _lib.workspace(lib.smoe_router_forward_workspace_bytes(E), dev)
             check(lib.smoe_router_forward_aux(x.data_ptr(), router_w.data_ptr(), logits.data_ptr(), scores.data_ptr(),
                                               indices.data_ptr(), freq.data_ptr(), colsum.data_ptr(), aux.data_ptr(),
                                               aux_grad.data_ptr(), ws.data_ptr(), T, H, E, K, st.status.data_ptr(),
@@ -344,7 +344,7 @@ class _SwitchLoss(torch.autograd.Function):
         with torch.cuda.device(dev):
             aux = torch.empty((), dtype=torch.float32, device=dev)
             aux_grad = torch.empty(E, dtype=torch.float32, device=dev)
-            ws = torch.empty(lib.smoe_router_forward_workspace_bytes(E), dtype=torch.uint8, device=dev)
+            ws = _lib.workspace(lib.smoe_router_forward_workspace_bytes(E), dev)
             check(lib.smoe_switch_loss(logits.data_ptr(), freq.data_ptr(), aux.data_ptr(), aux_grad.data_ptr(),
                                        ws.data_ptr(), T, E, stream_ptr(dev)), "switch_loss")
         ctx.save_for_backward(logits, aux_grad)
@@ -697,7 +697,7 @@ def _layer_forward(x, router_w, w1, w2, K):
         freq = torch.empty(E, dtype=torch.int32, device=dev)
         colsum = torch.empty(E, dtype=torch.float32, device=dev)
         aux = torch.empty((), dtype=torch.float32, device=dev)
-        scratch = torch.empty(lib.smoe_layer_forward_scratch_bytes(T, H, I, E, K), dtype=torch.uint8, device=dev)
+        scratch = _lib.workspace(lib.smoe_layer_forward_scratch_bytes(T, H, I, E, K), dev)
         check(lib.smoe_layer_forward(
             x.data_ptr(), router_w.data_ptr(), w1e.data_ptr(), w2e.data_ptr(), o.data_ptr(), logits.data_ptr(),
             freq.data_ptr(), colsum.data_ptr(), aux.data_ptr(), scratch.data_ptr(), T, H, I, E, K,

@@ -74,7 +74,7 @@ def select_pairs(scores: torch.Tensor, topk_idx: torch.Tensor, routing: str, til
     extra = {"down": 0, "up": tile - 1, "nr": tile // 2}[routing]
     capacity = min(T * E, T * K + E * extra)
     with torch.cuda.device(dev):
-        ws = torch.empty(lib.smoe_token_rounding_workspace_bytes(T, E), dtype=torch.uint8, device=dev)
+        ws = _lib.workspace(lib.smoe_token_rounding_workspace_bytes(T, E), dev)
         count = torch.empty(E, dtype=torch.int32, device=dev)
         tokens = torch.empty(capacity, dtype=torch.int32, device=dev)
         experts = torch.empty(capacity, dtype=torch.int32, device=dev)

@@ -181,3 +181,41 @@ def test_router_and_expert_weights_must_agree(built_library):
         for router in (torch.zeros(64, 128), torch.zeros(16, 128), torch.zeros(32, 64), torch.zeros(32, 256)):
             with pytest.raises(ValueError):
                 layer(x, router, w1, None, w2, None, 2)
+
+
+@pytest.mark.parametrize("entry,position", [("route_metadata", 10), ("router_forward_aux", 9)])
+def test_calls_that_overlap_have_workspaces_of_their_own(built_library, monkeypatch, entry, position):
+    """A second call that runs inside the first, as one of another thread or stream may: their scratch must differ."""
+    import contextlib
+
+    from sonicmoe import _lib, functional as fn
+
+    real, spaces = _lib.lib, []
+
+    def call():
+        if entry == "route_metadata":
+            fn._route_metadata(torch.zeros(64, dtype=torch.int32), None, 32, 2)
+        else:
+            fn._FusedRouter.apply(torch.zeros(32, 64).bfloat16(), torch.zeros(32, 64).bfloat16(), 2)
+
+    class Library:
+        def __getattr__(self, name):
+            if name != "smoe_" + entry:
+                return getattr(real, name)
+
+            def kernel(*args):
+                spaces.append(args[position])
+                if len(spaces) == 1:
+                    call()
+                return 0
+
+            return kernel
+
+    state = _lib._DeviceState(torch.device("cpu"))
+    monkeypatch.setattr(fn, "lib", Library())
+    monkeypatch.setattr(fn, "stream_ptr", lambda device: 0)
+    monkeypatch.setattr(_lib, "require_cuda", lambda t, name: None)
+    monkeypatch.setattr(_lib, "device_state", lambda device: state)
+    monkeypatch.setattr(torch.cuda, "device", lambda device: contextlib.nullcontext())
+    call()
+    assert len(spaces) == 2 and all(spaces) and spaces[0] != spaces[1]

@@ -378,3 +378,38 @@ def test_forward_without_gradients_matches_training_forward(built_library, T, E,
         x, m.router.weight.detach(), m.c_fc.weight.detach().permute(1, 2, 0), None,
         m.c_proj.weight.detach().permute(1, 2, 0), None, K, 0, ActivationType.SWIGLU, True)
     assert torch.equal(out, o_ref) and logits.shape == (T, E) and int(freq.sum()) == T * K
+
+
+def test_training_steps_on_two_streams_at_a_time(built_library):
+    """Forward and backward passes of two layers on two streams, not ordered with each other, against the same one after
+    the other."""
+    import sonicmoe
+    from sonicmoe import _lib
+    from sonicmoe.enums import ActivationType
+
+    T, H, I, K, rounds = 2048, 256, 128, 4, 8
+    layers = []
+    for n, E in enumerate((32, 64)):  # the second needs larger workspaces
+        inp = orc.make_inputs(T, H, I, E, K, seed=n, dtype=torch.bfloat16)
+        m = sonicmoe.MoE(E, K, H, I, ActivationType.SWIGLU, False, 0.05).cuda().to(torch.bfloat16)
+        layers.append((m, inp["x"].cuda().requires_grad_(True), inp["dout"].cuda()))
+
+    def step(m, x, dout):
+        o, aux = m(x)
+        return [o, aux, *torch.autograd.grad([o, aux], [x, *m.parameters()], [dout, torch.ones_like(aux)])]
+
+    want = [step(*layer) for layer in layers]
+    streams = [torch.cuda.Stream() for _ in layers]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    got = [[], []]
+    for _ in range(rounds):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(step(*layers[i]))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for i in range(2):
+        for result in got[i]:
+            for a, b in zip(result, want[i]):
+                assert torch.equal(a, b)
