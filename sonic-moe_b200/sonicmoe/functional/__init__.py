@@ -333,12 +333,20 @@ class _FusedRouter(torch.autograd.Function):
         return dx, dw, None
 
 
+def switch_loss_formula(probs: torch.Tensor, expert_frequency: torch.Tensor) -> torch.Tensor:
+    """E <normalised mean of the rows of probs (T,E), normalised expert_frequency>."""
+    share = F.normalize(expert_frequency.float(), p=1, dim=0)
+    mean_prob = F.normalize(probs.sum(0), p=1, dim=0)
+    return probs.size(-1) * (mean_prob * share).sum()
+
+
 class _SwitchLoss(torch.autograd.Function):
-    """The load-balancing loss of bf16 logits (T,E), E <= 256, and token counts that other kernels made."""
+    """The load-balancing loss of bf16 logits (T,E), E <= 256, and token counts that other kernels made.  A backward pass
+    that is itself recorded (create_graph) differentiates the loss's formula instead, so that higher derivatives exist."""
 
     @staticmethod
     def forward(ctx, logits, freq):
-        logits = logits.contiguous()
+        logits_in, logits = logits, logits.contiguous()
         T, E = logits.shape
         dev = logits.device
         with torch.cuda.device(dev):
@@ -347,12 +355,16 @@ class _SwitchLoss(torch.autograd.Function):
             ws = _lib.workspace(lib.smoe_router_forward_workspace_bytes(E), dev)
             check(lib.smoe_switch_loss(logits.data_ptr(), freq.data_ptr(), aux.data_ptr(), aux_grad.data_ptr(),
                                        ws.data_ptr(), T, E, stream_ptr(dev)), "switch_loss")
-        ctx.save_for_backward(logits, aux_grad)
+        ctx.save_for_backward(logits_in, freq, aux_grad)
         return aux
 
     @staticmethod
     def backward(ctx, g_aux):
-        logits, aux_grad = ctx.saved_tensors
+        logits, freq, aux_grad = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            aux = switch_loss_formula(F.softmax(logits, dim=-1, dtype=torch.float32), freq)
+            return torch.autograd.grad(aux, logits, g_aux, create_graph=True)[0], None
+        logits = logits.contiguous()
         T, E = logits.shape
         dev = logits.device
         g_aux = g_aux.float()
@@ -365,7 +377,7 @@ class _SwitchLoss(torch.autograd.Function):
 
 
 def switch_loss(logits: torch.Tensor, expert_frequency: torch.Tensor) -> torch.Tensor | None:
-    """E <normalised mean of softmax(logits), normalised expert_frequency>, or None where the kernels do not apply."""
+    """`switch_loss_formula` of softmax(logits) by kernels, or None where they do not apply."""
     if not (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.shape[1] <= 256
             and expert_frequency.dtype == torch.int32 and expert_frequency.device == logits.device
             and expert_frequency.is_contiguous() and not torch.compiler.is_compiling()):

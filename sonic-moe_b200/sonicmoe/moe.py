@@ -14,7 +14,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from .enums import ActivationType, KernelBackendMoE, is_glu
-from .functional import _layer_with_aux, moe_TC_softmax_topk_layer, switch_loss
+from .functional import _layer_with_aux, moe_TC_softmax_topk_layer, switch_loss, switch_loss_formula
 
 
 def _glu_halves(z: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
@@ -131,7 +131,8 @@ class MoE(nn.Module):
             raise ValueError(f"kernel backend {kernel_backend_moe} is not provided by this build")
 
         out = out.view(original_shape)
-        if aux_loss is None and kernel_backend_moe == KernelBackendMoE.sonicmoe:
+        replaced = getattr(self._compute_switch_loss, "__func__", None) is not MoE._compute_switch_loss
+        if aux_loss is None and kernel_backend_moe == KernelBackendMoE.sonicmoe and not replaced:
             aux_loss = switch_loss(router_logits, expert_frequency)
         if aux_loss is None:
             aux_loss = self._compute_switch_loss(
@@ -147,10 +148,7 @@ class MoE(nn.Module):
 
         Expert frequencies are per rank: nothing is reduced across data-parallel workers.
         """
-        probs = probs.view(-1, probs.size(-1))
-        share = F.normalize(expert_frequency.float(), p=1, dim=0)
-        mean_prob = F.normalize(probs.sum(0), p=1, dim=0)
-        return logits.size(-1) * (mean_prob * share).sum()
+        return switch_loss_formula(probs.view(-1, probs.size(-1)), expert_frequency)
 
     # ---- plain PyTorch definition of the layer (KernelBackendMoE.torch) ------------------------------
     def _torch_forward(self, x: torch.Tensor):

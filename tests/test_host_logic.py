@@ -219,3 +219,53 @@ def test_calls_that_overlap_have_workspaces_of_their_own(built_library, monkeypa
     monkeypatch.setattr(torch.cuda, "device", lambda device: contextlib.nullcontext())
     call()
     assert len(spaces) == 2 and all(spaces) and spaces[0] != spaces[1]
+
+
+def test_recorded_backward_of_the_load_balancing_loss(built_library, monkeypatch):
+    """Second derivatives through the loss that kernels compute, against those of its formula."""
+    import contextlib
+
+    from sonicmoe import _lib, functional as fn
+
+    class Library:  # the kernels' results play no part in a recorded backward pass
+        def __getattr__(self, name):
+            return getattr(_lib.lib, name) if name.endswith("bytes") else lambda *args: 0
+
+    monkeypatch.setattr(fn, "lib", Library())
+    monkeypatch.setattr(fn, "stream_ptr", lambda device: 0)
+    monkeypatch.setattr(torch.cuda, "device", lambda device: contextlib.nullcontext())
+    T, E = 24, 8
+    x = torch.randn(T, 16, generator=torch.Generator().manual_seed(0)).requires_grad_(True)
+    w = torch.randn(E, 16, generator=torch.Generator().manual_seed(1)).requires_grad_(True)
+    freq = torch.arange(E, dtype=torch.int32)
+    results = []
+    for loss in (fn._SwitchLoss.apply,
+                 lambda logits, n: fn.switch_loss_formula(torch.softmax(logits, -1, dtype=torch.float32), n)):
+        for logits in ((x @ w.T).bfloat16(), (w @ x.T).bfloat16().T):  # a transposed view as well
+            first = torch.autograd.grad(loss(logits, freq), [x, w], create_graph=True)
+            second = torch.autograd.grad(sum(g.square().sum() for g in first), [x, w])
+            results.append([*first, *second])
+    for got, want in zip(results[:2], results[2:]):
+        for a, b in zip(got, want):
+            assert b.abs().max() > 0 and torch.equal(a, b)
+
+
+def test_own_load_balancing_loss_is_used(built_library, monkeypatch):
+    """A subclass's (or an instance's) `_compute_switch_loss` takes the place of the loss kernels."""
+    import sonicmoe.moe as module
+
+    m, inp = _module()
+    T, E = 96, 8
+    layer = (torch.zeros(T, 128), torch.zeros(T, E), torch.full((E,), 24, dtype=torch.int32), None, None)
+    monkeypatch.setattr(module, "_layer_with_aux", lambda *args: layer)
+    monkeypatch.setattr(module, "switch_loss", lambda logits, freq: torch.tensor(1.0))
+    assert m(inp["x"])[1].item() == 1.0
+
+    class Own(module.MoE):
+        def _compute_switch_loss(self, logits, probs, expert_frequency):
+            return probs.sum() * 0 + 2.0
+
+    m.__class__ = Own
+    assert m(inp["x"])[1].item() == 2.0
+    m._compute_switch_loss = lambda logits, probs, expert_frequency: torch.tensor(3.0)
+    assert m(inp["x"])[1].item() == 3.0
