@@ -583,7 +583,9 @@ __global__ void __launch_bounds__(1024) router_finish_kernel(const float* __rest
   if (group == 0 && e < E) aux_grad[e] = static_cast<float>(E) * (share - dot) / sums;
 }
 
-// Column sums of softmax(logits) for logits that another kernel made: one warp per row, partial sums per CTA.
+// Column sums of softmax(logits) for logits that another kernel made: one warp per row, partial sums per CTA.  The
+// accurate exponential and division: the fast ones are off by |x| 2^-24 of a probability, which shows in the loss when the
+// tokens go to experts of small probability.
 template <int PER_LANE>
 __global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16* __restrict__ logits, int rows, int E,
                                                              float* __restrict__ colsum_partial) {
@@ -604,14 +606,13 @@ __global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16
     for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) {
-      l[j] = lane + 32 * j < E ? __expf(l[j] - m) : 0.f;
+      l[j] = lane + 32 * j < E ? expf(l[j] - m) : 0.f;
       s += l[j];
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    const float inv = 1.f / s;
 #pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) colsum[j] += l[j] * inv;
+    for (int j = 0; j < PER_LANE; ++j) colsum[j] += l[j] / s;
   }
 #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) sums[warp][lane + 32 * j] = colsum[j];
@@ -629,8 +630,9 @@ __global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16
 //              + p[t, e] (c_e - sum_j p[t, j] c_j)                     (optional: gradient c of the column sums of
 //                                                                       the full softmax p of the row);
 //                                                                       c = g_colsum + *g_aux * aux_grad
-// One warp per row; the row's probabilities are recomputed from the saved bf16 logits.
-template <int PER_LANE>
+// One warp per row; the row's probabilities are recomputed from the saved bf16 logits, with the exponential that the forward
+// pass used: the fast one behind the router kernels, the accurate one (EXACT) behind softmax_colsum_kernel.
+template <int PER_LANE, bool EXACT>
 __global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __restrict__ dlogits,
                                                               const __nv_bfloat16* __restrict__ logits,
                                                               const float* __restrict__ dscore,
@@ -668,7 +670,7 @@ __global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __r
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) {
       const int col = lane + 32 * j;
-      l[j] = col < E ? __expf(l[j] - m) : 0.f;
+      l[j] = col < E ? (EXACT ? expf(l[j] - m) : __expf(l[j] - m)) : 0.f;
       s += l[j];
       dot += l[j] * c[j];
     }
@@ -915,16 +917,13 @@ int smoe_router_backward_aux(void* dlogits, const void* logits, const float* dsc
   __nv_bfloat16* d = static_cast<__nv_bfloat16*>(dlogits);
   const __nv_bfloat16* l = static_cast<const __nv_bfloat16*>(logits);
   const __nv_bfloat16* g = static_cast<const __nv_bfloat16*>(g_logits);
+  // the gradient of smoe_switch_loss alone
+  const bool exact = dscores == nullptr && g_colsum == nullptr && g_logits == nullptr;
   const int per_lane = (E + 31) / 32;
-  if (per_lane <= 2)
-    router_backward_kernel<2><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E,
-                                                  K);
-  else if (per_lane <= 4)
-    router_backward_kernel<4><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E,
-                                                  K);
-  else
-    router_backward_kernel<8><<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E,
-                                                  K);
+  const auto kernel = per_lane <= 2   ? (exact ? router_backward_kernel<2, true> : router_backward_kernel<2, false>)
+                      : per_lane <= 4 ? (exact ? router_backward_kernel<4, true> : router_backward_kernel<4, false>)
+                                      : (exact ? router_backward_kernel<8, true> : router_backward_kernel<8, false>);
+  kernel<<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E, K);
   return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
 }
 

@@ -211,3 +211,19 @@ def test_switch_loss(built_library, T, E, fused):
     (glogits,) = torch.autograd.grad(want * 3.0, lf)
     assert abs(aux.item() / want.item() - 1) < 1e-5
     assert rel(grad, glogits.T @ x.double() if fused else glogits) < 1e-2
+
+
+@pytest.mark.parametrize("E", [8, 33, 256])
+def test_switch_loss_of_small_probabilities(built_library, E):
+    """All tokens at an expert of small probability p = exp(-depth): the loss is E p to fp32 accuracy.  Bound: the
+    exponential 2^-23, the division, 8 + 8 + 4 sums of equal terms and the final products 2^-24 each: 1.6e-6."""
+    from sonicmoe import functional as fn
+
+    T = 64
+    freq = torch.zeros(E, dtype=torch.int32, device="cuda")
+    freq[1] = T
+    for depth in range(20, 84):
+        logits = torch.full((T, E), -100.0, dtype=torch.bfloat16, device="cuda")
+        logits[:, 0], logits[:, 1] = 0, -depth
+        want = E * torch.softmax(logits[0].double(), 0)[1].item()
+        assert abs(fn.switch_loss(logits, freq).item() - want) <= 1.6e-6 * want, depth
