@@ -561,15 +561,17 @@ template <int EPI, bool RAGGED_K>
 __device__ __forceinline__ void store_chunk(const GemmParams& p, int expert, uint32_t stage, int lane, int row_base,
                                             int row_end, int n, const uint32_t (&v)[32], float score, int dst_row) {
   if constexpr (EPI == EPI_SCATTER) {
-    if (row_base + lane >= row_end) return;
-    float* dst = p.acc_out + static_cast<long long>(dst_row) * p.N + n;
+    if (row_base + lane < row_end) {
+      float* dst = p.acc_out + static_cast<long long>(dst_row) * p.N + n;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * j),
-                   "f"(score * __uint_as_float(v[4 * j + 0])), "f"(score * __uint_as_float(v[4 * j + 1])),
-                   "f"(score * __uint_as_float(v[4 * j + 2])), "f"(score * __uint_as_float(v[4 * j + 3]))
-                   : "memory");
+      for (int j = 0; j < 8; ++j) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * j),
+                     "f"(score * __uint_as_float(v[4 * j + 0])), "f"(score * __uint_as_float(v[4 * j + 1])),
+                     "f"(score * __uint_as_float(v[4 * j + 2])), "f"(score * __uint_as_float(v[4 * j + 3]))
+                     : "memory");
+      }
     }
+    __syncwarp();  // the next piece's tensor-memory read is warp-wide
   } else {
     float f[32];
     if constexpr (EPI == EPI_STORE_BIAS) {
