@@ -224,11 +224,9 @@ __device__ __forceinline__ void load_biased(const GemmParams& p, int expert, int
 }
 
 // dSwiGLU on 32 accumulator columns (= 64 columns of dz).  acc[., i] = dy1[r, i]; z[r, 2i] = gate, z[r, 2i+1] = up.
-// Writes dz (bf16), y1 * score, accumulates ds.  KEEP: the 32 packed bf16x2 words of dz replace v and amax collects
-// max |dz| over the bf16 values (for a caller that also quantises dz).
-template <bool KEEP>
-__device__ __forceinline__ void dswiglu_chunk(const GemmParams& p, int r, int n, uint32_t (&v)[32], float score,
-                                              float& ds_acc, float& amax) {
+// Writes dz (bf16), y1 * score, accumulates ds.
+__device__ __forceinline__ void dswiglu_chunk(const GemmParams& p, int r, int n, const uint32_t (&v)[32], float score,
+                                              float& ds_acc) {
   const uint4* zsrc = reinterpret_cast<const uint4*>(p.z + static_cast<long long>(r) * (2ll * p.N) + 2 * n);
   __nv_bfloat16* dz_dst = p.out0 + r * p.ld0 + 2 * n;
   __nv_bfloat16* ys_dst = p.out1 + r * p.ld1 + n;
@@ -256,13 +254,6 @@ __device__ __forceinline__ void dswiglu_chunk(const GemmParams& p, int r, int n,
     reinterpret_cast<uint4*>(dz_dst)[2 * j + 1] = make_uint4(dzw[4], dzw[5], dzw[6], dzw[7]);
     reinterpret_cast<uint4*>(ys_dst)[j] = make_uint4(pack_bf16(ys[0], ys[1]), pack_bf16(ys[2], ys[3]),
                                                      pack_bf16(ys[4], ys[5]), pack_bf16(ys[6], ys[7]));
-    if constexpr (KEEP) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        v[8 * j + i] = dzw[i];
-        amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(dzw[i] << 16)), fabsf(__uint_as_float(dzw[i] & 0xFFFF0000u))));
-      }
-    }
   }
 }
 
@@ -291,7 +282,8 @@ __device__ __forceinline__ void warp_load_rows64(uint32_t stage, int lane, uint3
 
 // dswiglu_chunk with the row traffic (z in, dz and y1 * score out) going through the warp's staging rows as 64-byte
 // row segments.  Every lane of the warp must call (lane l owns row row_base + l; rows at or past row_end read zeros
-// and store nothing).  Same arithmetic, same results.
+// and store nothing).  Same arithmetic, same results.  KEEP: the 32 packed bf16x2 words of dz replace v and amax collects
+// max |dz| over the bf16 values (for a caller that also quantises dz).
 template <bool KEEP>
 __device__ __forceinline__ void dswiglu_chunk_staged(const GemmParams& p, uint32_t stage, int lane, int row_base,
                                                      int row_end, int n, uint32_t (&v)[32], float score, float& ds_acc,
@@ -330,11 +322,11 @@ __device__ __forceinline__ void dswiglu_chunk_staged(const GemmParams& p, uint32
 }
 
 // One 32-column piece of one accumulator row, stored by the lane that holds it: v[j] = acc[r, n + j].  FP8 kernels.
-template <int EPI, bool RAGGED_K>
-__device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int expert, int r, int n, uint32_t (&v)[32],
-                                       float score, float& ds_acc) {
+template <int EPI>
+__device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int r, int n, uint32_t (&v)[32], float score,
+                                               float& ds_acc) {
   if constexpr (EPI == EPI_STORE) {
-    __nv_bfloat16* dst = p.out0 + (RAGGED_K ? expert * p.out0_expert_stride : 0ll) + r * p.ld0 + n;
+    __nv_bfloat16* dst = p.out0 + r * p.ld0 + n;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       uint4 w;
@@ -342,8 +334,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int expert, 
       w.y = pack_bf16(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]));
       w.z = pack_bf16(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]));
       w.w = pack_bf16(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]));
-      uint4* d4 = reinterpret_cast<uint4*>(dst) + j;
-      *d4 = p.accumulate ? add_bf16x8(w, d4) : w;
+      reinterpret_cast<uint4*>(dst)[j] = w;
     }
   } else if constexpr (EPI == EPI_SWIGLU) {
     if (p.out0 != nullptr) {
@@ -377,8 +368,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int expert, 
       reinterpret_cast<uint4*>(dst1)[j] = w;
     }
   } else if constexpr (EPI == EPI_DSWIGLU) {
-    float unused = 0.f;
-    dswiglu_chunk<false>(p, r, n, v, score, ds_acc, unused);
+    dswiglu_chunk(p, r, n, v, score, ds_acc);
   } else if constexpr (EPI == EPI_STORE_ROWS) {
     __nv_bfloat16* dst = p.out0 + static_cast<long long>(p.gather[r]) * p.ld0 + n;
     float f[32];
@@ -389,15 +379,6 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, int expert, 
       for (int j = 0; j < 32; ++j) f[j] = score * __bfloat162float(__float2bfloat16_rn(f[j]));
     }
     store_bf16x32(dst, f);
-  } else if constexpr (EPI == EPI_SCATTER) {
-    float* dst = p.acc_out + static_cast<long long>(p.gather[r]) * p.N + n;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * j),
-                   "f"(score * __uint_as_float(v[4 * j + 0])), "f"(score * __uint_as_float(v[4 * j + 1])),
-                   "f"(score * __uint_as_float(v[4 * j + 2])), "f"(score * __uint_as_float(v[4 * j + 3]))
-                   : "memory");
-    }
   }
 }
 

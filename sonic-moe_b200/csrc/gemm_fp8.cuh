@@ -327,7 +327,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           uint32_t v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(acc[c * 32 + i]);
-          epilogue_chunk<EPI, false>(p, tile.e, r, ncol0 + c * 32, v, score, ds_acc);
+          epilogue_chunk<EPI>(p, r, ncol0 + c * 32, v, score, ds_acc);
         }
       }
       if constexpr (EPI == EPI_DSWIGLU) {

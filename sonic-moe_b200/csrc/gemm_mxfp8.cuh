@@ -520,10 +520,10 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         }
       }
       if (!done && row_ok && cols_ok) {
-        epilogue_chunk<EPI, false>(p, tile.e, r, ncol0, v0, score, ds_acc);
-        epilogue_chunk<EPI, false>(p, tile.e, r, ncol0 + 32, v1, score, ds_acc);
-        epilogue_chunk<EPI, false>(p, tile.e, r, ncol0 + 64, v2, score, ds_acc);
-        epilogue_chunk<EPI, false>(p, tile.e, r, ncol0 + 96, v3, score, ds_acc);
+        epilogue_chunk<EPI>(p, r, ncol0, v0, score, ds_acc);
+        epilogue_chunk<EPI>(p, r, ncol0 + 32, v1, score, ds_acc);
+        epilogue_chunk<EPI>(p, r, ncol0 + 64, v2, score, ds_acc);
+        epilogue_chunk<EPI>(p, r, ncol0 + 96, v3, score, ds_acc);
       }
       if constexpr (EPI == EPI_DSWIGLU) {
         // every partial row the reduction reads is written, also the one past the last column block (zero)
