@@ -46,6 +46,9 @@ enum { SMOE_F32 = 0, SMOE_BF16 = 1, SMOE_I32 = 2, SMOE_I64 = 3 };
 /* Library version, for the loader to check that it found the right build. */
 int smoe_abi_version(void);
 
+/* Kernels that this process has launched through the library so far (launches recorded by a stream capture count once). */
+long long smoe_kernel_launches(void);
+
 /* ---------------------------------------------------------------------------------------------
  * Router: top-k, softmax over the winners, histogram / prefix sum, grouped-row index vectors
  * ------------------------------------------------------------------------------------------- */

@@ -1,10 +1,14 @@
-// Per-device host-side caches.  cudaFuncSetAttribute and the SM count are facts of one device, and one
+// Host-side state of the library: per-device caches and the launch counter.
+//
+// Per-device caches.  cudaFuncSetAttribute and the SM count are facts of one device, and one
 // process may drive several devices through this library (threads, one module per GPU), so nothing here is
 // cached per process.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <atomic>
+
+#include "../../include/sonicmoe_b200.h"
 
 namespace smoe {
 
@@ -37,5 +41,16 @@ inline int num_sms() {
   }
   return v;
 }
+
+// Kernels that the library has launched in this process, of all devices and threads (smoe_kernel_launches).
+inline std::atomic<long long> kernel_launches{0};
+
+// The entry points' return code after `kernels` launches, which are counted if none of them failed.
+inline int launched(cudaError_t rc, int kernels = 1) {
+  if (rc != cudaSuccess) return SMOE_ERR_LAUNCH;
+  kernel_launches.fetch_add(kernels, std::memory_order_relaxed);
+  return SMOE_OK;
+}
+inline int launch_rc(int kernels = 1) { return launched(cudaGetLastError(), kernels); }
 
 }  // namespace smoe

@@ -103,7 +103,7 @@ static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p) == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launched(cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p));
 }
 
 // Kernels without a gathered operand work on single tiles, kernels with one on dual tiles where they pay.
@@ -183,7 +183,7 @@ static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, const G
   if (sms <= 0) return SMOE_ERR_DRIVER;
   const int stages = skinny::num_stages(nt);
   kernel<<<sms, skinny::threads(GATHER), skinny::smem_bytes(nt, stages), stream>>>(tmW, tmX, p, nt, stages);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc();
 }
 
 // An empty batch (T == 0, hence TK == 0) is valid: the entry points return at once (weight-gradient entry points

@@ -80,7 +80,7 @@ static int launch_kernel(Kernel kernel, PerDeviceFlag& configured, int smem_byte
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p, sc) == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launched(cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p, sc));
 }
 
 template <bool A_GATHER, bool B_MN, int EPI>
@@ -255,7 +255,7 @@ static int quantize_blocks(const void* w, void* q, void* scale, int batch, int r
   const auto kernel = wa % 16 == 0 && qa % 8 == 0 ? quantize_blocks_kernel<POW2, true> : quantize_blocks_kernel<POW2, false>;
   kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(w),
                                                               static_cast<uint8_t*>(q), scale, rows, cols);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc();
 }
 
 }  // namespace fp8
@@ -279,7 +279,7 @@ int smoe_fp8_quantize_rows(const void* x, void* q, float* scale, long long rows,
   const long long warps = rows * ((nblk + 3) / 4);
   quantize_rows_kernel<false><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale, rows, cols, nblk);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc();
 }
 
 int smoe_fp8_quantize_blocks(const void* w, void* q, float* scale, int batch, int rows, int cols, void* stream) {
@@ -375,7 +375,7 @@ int smoe_mxfp8_quantize_rows(const void* x, void* q, void* scale, long long rows
   const long long warps = rows * (ld / 4);
   quantize_rows_kernel<true><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale, rows, cols, ld);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc();
 }
 
 int smoe_mxfp8_quantize_blocks(const void* w, void* q, void* scale, int batch, int rows, int cols, void* stream) {

@@ -12,6 +12,7 @@
 #include <mutex>
 
 #include "../../include/sonicmoe_b200.h"
+#include "device_cache.cuh"
 
 namespace smoe {
 
@@ -205,7 +206,7 @@ int smoe_gather_sum_to_peers(const void* src, const void* weights, int weights_d
         s_, static_cast<const __nv_bfloat16*>(weights), reverse_idx, token_offset, T, H, K, first_row, seg);
   else
     return SMOE_ERR_DTYPE;
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc();
 }
 
 }  // extern "C"

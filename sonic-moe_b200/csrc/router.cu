@@ -869,7 +869,7 @@ int smoe_router_forward_aux(const void* x, const void* router_w, void* logits, f
   }
   router_finish_kernel<<<1, 1024, 0, st>>>(colsum_partial, hist_partial, T > 0 ? grid : 0, E, prob_colsum, expert_count,
                                            aux, aux_grad);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc(T > 0 ? 2 : 1);
 }
 
 int smoe_switch_loss(const void* logits, const int* expert_count, float* aux, float* aux_grad, void* workspace, int T,
@@ -894,7 +894,7 @@ int smoe_switch_loss(const void* logits, const int* expert_count, float* aux, fl
   }
   router_finish_kernel<<<1, 1024, 0, st>>>(colsum_partial, nullptr, blocks, E, nullptr, const_cast<int*>(expert_count),
                                            aux, aux_grad);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc(blocks > 0 ? 2 : 1);
 }
 
 int smoe_router_backward(void* dlogits, const void* logits, const float* dscores, const float* scores,
@@ -924,7 +924,7 @@ int smoe_router_backward_aux(void* dlogits, const void* logits, const float* dsc
                       : per_lane <= 4 ? (exact ? router_backward_kernel<4, true> : router_backward_kernel<4, false>)
                                       : (exact ? router_backward_kernel<8, true> : router_backward_kernel<8, false>);
   kernel<<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E, K);
-  return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH;
+  return launch_rc();
 }
 
 }  // extern "C"

@@ -20,7 +20,6 @@ constexpr int kMaxSortBlocks = 128;       // chunks the flat index vector is cut
 constexpr int kMaxSmemExperts = 4096;     // histogram bins kept in shared memory
 
 static inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
-static inline int launch_rc() { return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH; }
 
 // ----------------------------------------------------------------------------------------------
 // top-k + softmax over the K winners
@@ -539,6 +538,8 @@ extern "C" {
 
 int smoe_abi_version(void) { return 1; }
 
+long long smoe_kernel_launches(void) { return kernel_launches.load(std::memory_order_relaxed); }
+
 int smoe_topk_softmax(const void* logits, int logits_dtype, float* scores, int* indices, int T, int E, int K,
                       void* stream) {
   if (T < 0 || E <= 0 || K <= 0 || K > E) return SMOE_ERR_SHAPE;
@@ -593,7 +594,7 @@ int smoe_count_cumsum(const void* x, int x_dtype, long long n, int E, int* count
       global_histogram_kernel<long long><<<blocks, 256, 0, st>>>(static_cast<const long long*>(x), n, E, count);
     if (cumsum != nullptr) scan_bins_kernel<<<1, 1024, 0, st>>>(nullptr, 0, E, count, nullptr, cumsum, nullptr);
   }
-  return launch_rc();
+  return launch_rc(E <= kMaxSmemExperts || cumsum != nullptr ? 2 : 1);
 }
 
 size_t smoe_route_metadata_workspace_bytes(int E) { return smoe_count_cumsum_workspace_bytes(E); }
@@ -626,7 +627,7 @@ int smoe_count_cumsum_noalloc(const void* x, int x_dtype, long long n, int E, in
     chunk_histogram_kernel<long long><<<blocks, kSortThreads, E * sizeof(int), st>>>(
         static_cast<const long long*>(x), n, E, hist);
   scan_bins_kernel<<<1, 1024, 0, st>>>(hist, blocks, E, nullptr, count, cumsum, nullptr);
-  return launch_rc();
+  return launch_rc(2);
 }
 
 int smoe_route_metadata(const int* expert_idx, const int* token_idx, long long n, int E, int K, int* expert_count,
@@ -654,7 +655,7 @@ int smoe_route_metadata(const int* expert_idx, const int* token_idx, long long n
     sort_scatter_kernel<<<blocks, kSortThreads, smem, st>>>(expert_idx, n, E, hist, expert_offset, K, token_idx,
                                                             s_scatter_idx, s_reverse_scatter_idx, x_gather_idx);
   }
-  return launch_rc();
+  return launch_rc(n > 0 ? 3 : 2);
 }
 
 int smoe_sorted_offsets(const int* sorted_idx, long long n, int T, int* offsets, void* stream) {

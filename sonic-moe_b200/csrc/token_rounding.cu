@@ -20,6 +20,7 @@
 #include <stdint.h>
 
 #include "../../include/sonicmoe_b200.h"
+#include "device_cache.cuh"
 
 namespace smoe {
 namespace rounding {
@@ -30,7 +31,6 @@ constexpr int kSelectThreads = 1024;
 constexpr int kCountThreads = 256;
 
 static inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
-static inline int launch_rc() { return cudaGetLastError() == cudaSuccess ? SMOE_OK : SMOE_ERR_LAUNCH; }
 
 // larger key = ranked earlier; -0.0 == +0.0
 __device__ __forceinline__ uint32_t order_key(float v) {
@@ -322,6 +322,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(int* __restrict__ v, int n, 
 }  // namespace rounding
 }  // namespace smoe
 
+using namespace smoe;
 using namespace smoe::rounding;
 
 extern "C" size_t smoe_token_rounding_workspace_bytes(int T, int E) {
@@ -343,7 +344,7 @@ extern "C" int smoe_token_rounding_select(const void* scores, int scores_dtype, 
   if (T == 0) {
     cudaMemsetAsync(expert_count, 0, sizeof(int) * E, st);
     cudaMemsetAsync(num_pairs, 0, sizeof(int), st);
-    return launch_rc();
+    return launch_rc(0);
   }
   Layout L;
   carve(L, workspace, T, E);
@@ -358,5 +359,5 @@ extern "C" int smoe_token_rounding_select(const void* scores, int scores_dtype, 
   count_emit_kernel<false><<<blocks, kCountThreads, 0, st>>>(T, E, L, nullptr, nullptr, 0);
   scan_kernel<<<1, 1024, 0, st>>>(L.cnt_block, blocks, num_pairs);
   count_emit_kernel<true><<<blocks, kCountThreads, 0, st>>>(T, E, L, tokens, experts, capacity);
-  return launch_rc();
+  return launch_rc(5);
 }

@@ -33,6 +33,7 @@ P, I, LL = c_void_p, c_int, c_longlong
 # name -> (restype, argtypes); must list every function the header declares.
 SIGNATURES: dict[str, tuple] = {
     "smoe_abi_version": (I, []),
+    "smoe_kernel_launches": (LL, []),
     "smoe_topk_softmax": (I, [P, I, P, P, I, I, I, P]),
     "smoe_softmax_topk_backward": (I, [P, I, P, P, P, I, I, I, P]),
     "smoe_count_cumsum_workspace_bytes": (c_size_t, [I]),
@@ -123,21 +124,14 @@ def _load() -> ctypes.CDLL:
 lib = _load()
 
 
-# kernels one successful entry-point call launches (1 unless listed)
-_KERNELS_PER_CALL = {"route_metadata": 3, "count_cumsum": 2, "router_forward": 2, "switch_loss": 2, "layer_forward": 8}
-_launches = 0
-
-
 def check(rc: int, what: str) -> None:
-    global _launches
     if rc != 0:
         raise SonicMoEError(f"{what} failed: {_ERRORS.get(rc, 'error')} (code {rc})")
-    _launches += _KERNELS_PER_CALL.get(what, 1)
 
 
 def launch_count() -> int:
-    """Kernels of this library launched so far by this process through the Python layer."""
-    return _launches
+    """Kernels of this library launched so far by this process."""
+    return lib.smoe_kernel_launches()
 
 
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor:

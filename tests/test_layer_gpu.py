@@ -413,3 +413,25 @@ def test_training_steps_on_two_streams_at_a_time(built_library):
         for result in got[i]:
             for a, b in zip(result, want[i]):
                 assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T,E,K,kernels", [
+    (1, 32, 1, 7),       # router 2, sort 3, up, down
+    (4, 64, 4, 8),       # and the combine
+    (1030, 128, 8, 10),  # both projections in two launches: 64 rows per expert
+    (9600, 32, 4, 8),    # 256 x 256 tiles alone
+])
+def test_launch_count(built_library, T, E, K, kernels):
+    """The library's own count of its launches, over an inference forward."""
+    import sonicmoe
+    from sonicmoe import _lib
+    from sonicmoe.enums import ActivationType
+
+    m = sonicmoe.MoE(E, K, 256, 128, ActivationType.SWIGLU, False, 0.05).cuda().to(torch.bfloat16)
+    x = torch.randn(T, 256, device="cuda").bfloat16()
+    with torch.no_grad():
+        before = _lib.launch_count()
+        m(x)
+        assert _lib.launch_count() - before == kernels
+    torch.cuda.synchronize()
+    _lib.check_status()
