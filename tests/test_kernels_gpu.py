@@ -697,3 +697,37 @@ def test_few_rows_per_expert(smoe, counts, H, I):
     assert rel(y2[:TK], torch.einsum("ri,rhi->rh", y1[:TK].float().cpu(), w2[expert].float())) < BF16_TOL
     for t in (z, y1, y1b, y2):  # nothing behind the last row
         assert t[TK].isnan().all()
+
+
+@pytest.mark.parametrize("counts", [[1, 5, 0, 33], [40, 64, 3, 20], [128, 90, 129, 7]])
+@pytest.mark.parametrize("H,I", [(192, 64), (1024, 256)])
+def test_few_rows_kernel_agrees_with_tiles(smoe, counts, H, I):
+    """Rows that the kernel for experts with few rows works on, and the same rows beside one expert with so many that the
+    256 x 256 tiles take all: both add up the products of a row in the same order, so the bits are the same.  One token is
+    NaN, and so are its rows alone."""
+    lib = smoe[0].lib
+    few, many, T = sum(counts), 3000, 50
+    g = torch.Generator().manual_seed(H + few)
+    x = torch.randn(T, H, generator=g).bfloat16()
+    x[11] = float("nan")
+    w1 = (torch.randn(5, 2 * I, H, generator=g) * 0.05).bfloat16().cuda()
+    w2 = (torch.randn(5, H, I, generator=g) * 0.05).bfloat16().cuda()
+    tok = torch.randint(0, T, (few + many,), generator=g, dtype=torch.int32)
+    xd, td = x.cuda(), tok.cuda()
+    st = smoe[0].device_state(xd.device).status.data_ptr()
+    s = torch.cuda.current_stream().cuda_stream
+    results = []
+    for E, rows in ((4, few), (5, few + many)):
+        off = torch.tensor([0, *torch.tensor(counts).cumsum(0).tolist(), few + many][: E + 1], dtype=torch.int32).cuda()
+        z, y1, y2 = (torch.empty(rows, n, dtype=torch.bfloat16, device="cuda") for n in (2 * I, I, H))
+        assert lib.smoe_up_projection_forward(xd.data_ptr(), w1.data_ptr(), z.data_ptr(), y1.data_ptr(), off.data_ptr(),
+                                              td.data_ptr(), T, H, I, E, rows, st, s) == 0
+        assert lib.smoe_down_projection_forward(y1.data_ptr(), w2.data_ptr(), y2.data_ptr(), off.data_ptr(), H, I, E, rows,
+                                                st, s) == 0
+        torch.cuda.synchronize()
+        smoe[0].check_status()
+        results.append([t[:few] for t in (z, y1, y2)])
+    bad = (tok[:few] == 11).cuda()
+    for a, b in zip(*results):
+        assert torch.equal(a.isnan().any(1), bad) and torch.equal(b.isnan().any(1), bad)
+        assert torch.equal(a[~bad], b[~bad])

@@ -227,3 +227,25 @@ def test_switch_loss_of_small_probabilities(built_library, E):
         logits[:, 0], logits[:, 1] = 0, -depth
         want = E * torch.softmax(logits[0].double(), 0)[1].item()
         assert abs(fn.switch_loss(logits, freq).item() - want) <= 1.6e-6 * want, depth
+
+
+@pytest.mark.parametrize("H,E,K", [(256, 64, 4), (1024, 128, 8), (512, 256, 16), (192, 32, 1)])
+def test_router_forms_agree(built_library, H, E, K):
+    """The same tokens through the small tiles (up to 9472 tokens) and the large ones (above): the same logits and winners bit
+    for bit, scores to the last bits of their sum; also of tokens with NaN or infinities."""
+    from sonicmoe.functional import _FusedRouter
+
+    T = 9600
+    g = torch.Generator(device="cuda").manual_seed(H + E)
+    x = torch.randn(T, H, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(E, H, generator=g, device="cuda") * 0.05).bfloat16()
+    x[0, 3], x[40], x[41, 0], x[100, H - 1] = float("nan"), float("nan"), float("inf"), -float("inf")
+    large = _FusedRouter.apply(x, w, K)
+    assert large[0][0].isnan().all() and large[2][40].tolist() == list(range(K))
+    for n in (1, 33, 127, 1030, 2049, 4097, 9472):
+        small = _FusedRouter.apply(x[:n], w, K)
+        assert torch.equal(small[0].nan_to_num(7.0), large[0][:n].nan_to_num(7.0))
+        assert torch.equal(small[0].isnan(), large[0][:n].isnan())
+        assert torch.equal(small[2], large[2][:n])
+        assert torch.equal(small[3], torch.bincount(large[2][:n].reshape(-1), minlength=E).int())
+        torch.testing.assert_close(small[1], large[1][:n], rtol=1e-6, atol=0, equal_nan=True)
