@@ -714,16 +714,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
 
   // ---- tear-down ----------------------------------------------------------------------------
-  __syncwarp();  // the MMA role is one lane's: its warp meets again before the barriers that every thread of a warp takes
   if (*abort_flag != 0) {
     const uint64_t t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
-  __syncwarp();  // each lane read the flag for itself
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // neither CTA leaves while the other may still signal its barriers or read its smem
   if (warp == 1) {
+    __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * BN);
   }
