@@ -217,6 +217,14 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// Barriers of the block and of the cluster that the lanes of a warp may reach one by one: without .aligned each thread
+// arrives for itself.
+__device__ __forceinline__ void block_sync_diverged() { asm volatile("barrier.sync 0;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync_diverged() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // shared::cluster address of the same shared-memory offset in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
   uint32_t r;
