@@ -66,8 +66,8 @@ struct GemmParams {
 
 // Whether the experts with more than `limit` rows hold at least half of all rows.  Then the 256 x 256 tiles take all experts
 // and the kernel for experts with few rows finds nothing to do: most of the others have next to none, and a wave of each
-// kernel would cost more than tiles for all of them (T 640, top-8 of 128 experts, loads falling with the square of the rank:
-// up projection 208 us divided, 170 by tiles).  One warp, all lanes; both kernels come to the same answer.
+// kernel would cost more than tiles for all of them (H 4096, I 1024, 5120 rows in 128 experts, loads falling with the square
+// of the rank: up projection 208 us divided, 170 by tiles).  One warp, all lanes; both kernels come to the same answer.
 __device__ __forceinline__ bool tiles_take_all(const GemmParams& p, int limit, int lane) {
   int above = 0;
   for (int e = lane; e < p.E; e += 32) {

@@ -118,10 +118,10 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
     const int doubled = A_GATHER ? p.N : p.M;
     const bool fits = ((doubled + 511) / 512 * 512 - doubled) * 8 <= doubled;
     // The activation-gradient epilogues keep single tiles: with both accumulators belonging to one unit the next
-    // unit's second MMA group waits for the first accumulator's dSwiGLU pass.  Measured at the benchmark shape with
-    // that pass staged through shared memory like the single-tile one: step 17.75-17.97 ms dual against 17.88-18.13 ms
-    // single in alternating runs, the kernel alone 2.26-2.69 against 2.09-2.58 ms -- no gain worth a second variant.  The general forward epilogue is
-    // too long to be worked off from registers, and must not hold accumulators that the next unit needs.
+    // unit's second MMA group waits for the first accumulator's dSwiGLU pass.  Measured with four epilogue warps in the
+    // single form, T 32768, H 4096, I 1024, E 128, K 8: the kernel alone 2.26-2.69 ms dual against 2.09-2.58 single.  Eight
+    // warps made the single form 3 % faster since (2.59 -> 2.51 ms, alternating).  The general forward epilogue is too long
+    // to be worked off from registers, and must not hold accumulators that the next unit needs.
     if constexpr (EPI != EPI_DSWIGLU && epi_base(EPI) != EPI_DACT && epi_base(EPI) != EPI_ACT) {
     if (use_dual_tiles() && fits) {
       constexpr int kDual = A_GATHER ? pair::DUAL_N : pair::DUAL_M;
@@ -150,23 +150,42 @@ static int launch_activation(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   return SMOE_ERR_SHAPE;
 }
 
-// Rows per unit of the kernel for experts with few rows (gemm_skinny.cuh), or 0 for the 256 x 256 tiles.  The line is the
-// mean number of rows per expert, all that the host knows of the load; an expert with more rows than a unit reads its
-// weights again, mostly from L2.  Up / down projection at H 4096, I 1024, E 128, us, units of 32 / 64 / 128 rows / tiles:
-// mean 4 339, 344, 353, 406 / 180, 183, 188, 197; mean 16 350, 350, 360, 409 / 195, 186, 193, 201; mean 32 533, 375, 377,
-// 407 / 234, 191, 195, 205; mean 64 867, 551, 387, 412 / 389, 244, 201, 209; mean 128 1546, 862, 594, 426 / 680, 391,
-// 252, 219.
-static int skinny_rows(int TK, int E) {
-  const double mean = static_cast<double>(TK) / E;
-  return mean <= 12 ? 32 : mean <= 40 ? 64 : mean <= 96 ? 128 : 0;
+// How a forward projection is shared between the kernel for experts with few rows (gemm_skinny.cuh) and the 256 x 256 tiles.
+// The host knows the mean number of rows per expert and not the load, so the choice has to hold for an even load and for one
+// in which all tokens take the same experts.  Measured inside inference layers in a row, us, to the start of the next kernel.
+//   * Rows per unit by the mean: an even load costs least with the smallest unit that holds most experts' rows (more stages of
+//     weights in flight).  H 4096, I 1024, E 128, units of 32 / 64 / 128 rows / tiles, up projection: mean 4 318, 324, 336,
+//     350; mean 16 329, 332, 343, 361; mean 24 367, 346, 354, 364; down projection at mean 4 162, 164, 171, 193.
+//   * An expert with more rows than a unit has its weights streamed again by every further unit, so a load in few experts
+//     costs one pass per wave of units, where the tiles need about one.  One launch therefore takes all experts only where even
+//     all rows in the fewest units give no more than two per SM, if need be with units of twice the rows: 2048 rows in 8 of
+//     256 experts, H 4096, I 1024, up projection 184 with units of 32 rows, 109 with 64, 64 with 128 and 54 by tiles.
+//   * Beyond that experts with more than two units' rows go to the tiles in a second launch, which finds nothing to do in an
+//     even load: 60 for the load above, and even 645 where units alone take 635 and tiles 714.  Layers whose weights do not
+//     outweigh that launch (6 to 9 us: half a GB) take larger units still, or the tiles: H 1536, I 256, E 128, 8192 rows,
+//     divided / units of 128 / tiles, up 55, 49, 51.
+struct FewRows {
+  int unit = 0;      // rows per unit; 0: the tiles take all experts
+  int max_rows = 0;  // experts with more rows are left to the tiles
+};
+static FewRows few_rows(const GemmParams& p) {
+  FewRows f;
+  const double mean = static_cast<double>(p.total_rows) / p.E;
+  if (mean > 96) return f;
+  const int by_mean = mean <= 12 ? 32 : mean <= 40 ? 64 : skinny::MAX_NT;
+  const bool divide = 2.0 * p.E * p.N * p.K >= 0.5e9;
+  const int largest = divide && 2 * by_mean < skinny::MAX_NT ? 2 * by_mean : skinny::MAX_NT;
+  const long long blocks = (p.N + skinny::BM - 1) / skinny::BM, most = 2ll * num_sms();
+  for (f.unit = by_mean; f.unit <= largest; f.unit *= 2) {
+    if ((p.total_rows + f.unit - 1) / f.unit * blocks <= most) {
+      f.max_rows = p.total_rows;
+      return f;
+    }
+  }
+  f.unit = divide ? by_mean : 0;
+  f.max_rows = 2 * by_mean;
+  return f;
 }
-
-// A skewed load has experts with many rows beside many with few: above this many routed rows the experts that take more
-// than two units go to a second launch, of the 256 x 256 tiles (about 4 us when it finds nothing to do).  T 640, top-8 of
-// 128 experts, loads falling with the square of the rank, up / down projection: 166 / 90 us with tiles alone, 299 / 143
-// with units alone (tiles_take_all() gives such a load to the tiles).  Below it, all rows in one expert still cost less than that launch and a wave of its tiles.
-constexpr int SKINNY_ONLY_ROWS = 2048;
-static int skinny_max_rows(int TK, int nt) { return TK > SKINNY_ONLY_ROWS ? 2 * nt : TK; }
 
 template <bool GATHER, bool SWIGLU>
 static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p, int nt, cudaStream_t stream) {
@@ -221,10 +240,11 @@ int smoe_up_projection_forward(const void* x, const void* w1, void* z, void* y1,
   p.out0 = static_cast<__nv_bfloat16*>(z); p.ld0 = 2 * I;
   p.out1 = static_cast<__nv_bfloat16*>(y1); p.ld1 = I;
   p.status = status;
-  if (const int nt = skinny_rows(TK, E)) {
-    p.max_rows = p.min_rows = skinny_max_rows(TK, nt);
-    SMOE_TRY((launch_skinny<true, true>(tmB, tmA, p, nt, static_cast<cudaStream_t>(stream))));
-    if (p.max_rows == TK) return SMOE_OK;
+  const FewRows few = few_rows(p);
+  if (few.unit > 0) {
+    p.max_rows = p.min_rows = few.max_rows;
+    SMOE_TRY((launch_skinny<true, true>(tmB, tmA, p, few.unit, static_cast<cudaStream_t>(stream))));
+    if (few.max_rows >= TK) return SMOE_OK;
   }
   return launch<false, true, false, false, false, EPI_SWIGLU>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
 }
@@ -241,12 +261,13 @@ int smoe_down_projection_forward(const void* y1, const void* w2, void* y2, const
   p.off = expert_offset;
   p.out0 = static_cast<__nv_bfloat16*>(y2); p.ld0 = H;
   p.status = status;
-  if (const int nt = skinny_rows(TK, E)) {
+  const FewRows few = few_rows(p);
+  if (few.unit > 0) {
     CUtensorMap tmX;
     SMOE_TRY(encode_2d(&tmX, y1, TK, I, I, skinny::BOX_ROWS, BK));
-    p.max_rows = p.min_rows = skinny_max_rows(TK, nt);
-    SMOE_TRY((launch_skinny<false, false>(tmB, tmX, p, nt, static_cast<cudaStream_t>(stream))));
-    if (p.max_rows == TK) return SMOE_OK;
+    p.max_rows = p.min_rows = few.max_rows;
+    SMOE_TRY((launch_skinny<false, false>(tmB, tmX, p, few.unit, static_cast<cudaStream_t>(stream))));
+    if (few.max_rows >= TK) return SMOE_OK;
   }
   return launch<false, false, false, false, false, EPI_STORE>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
 }

@@ -731,3 +731,54 @@ def test_few_rows_kernel_agrees_with_tiles(smoe, counts, H, I):
     for a, b in zip(*results):
         assert torch.equal(a.isnan().any(1), bad) and torch.equal(b.isnan().any(1), bad)
         assert torch.equal(a[~bad], b[~bad])
+
+
+@pytest.mark.parametrize("rows,launches", [
+    (4, (1, 1)),    # 512 rows: at most 256 units of 32 (up) or 64 rows (down), two per SM
+    (9, (1, 2)),    # 1152: 288 units of 64 in the up projection; experts above two units go to the tiles in the other
+    (18, (1, 2)),   # 2304: 288 units of 128
+    (19, (2, 2)),
+    (41, (2, 2)),   # 128-row units
+    (97, (1, 1)),   # above 96 rows per expert the tiles take all
+])
+@pytest.mark.parametrize("hot", [0, 300, 1024])
+def test_few_rows_kernel_beside_tiles(smoe, rows, launches, hot):
+    """Weights of a size at which the two kernels share a load: as many launches as the rule says, and the bits of the tiles
+    alone (the same rows beside one more expert that has most of them).  hot: rows of one expert (1024: above half of the
+    smaller loads, where the tiles take all)."""
+    lib = smoe[0].lib
+    E, H, I, T, many = 128, 4096, 1024, 3000, 16000
+    few = 128 * rows
+    hot = min(hot, few)
+    counts = torch.full((E,), (few - hot) // E)
+    spread = min(5, int(counts[0]))
+    counts[0] += hot
+    counts[::3] += spread
+    counts[1::3] -= spread
+    counts[E - 1] += few - counts.sum()
+    assert counts.min() >= 0 and counts.sum() == few
+    g = torch.Generator(device="cuda").manual_seed(rows + hot)
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    x = torch.empty(T, H, **bf).normal_(generator=g)
+    w1 = torch.empty(E + 1, 2 * I, H, **bf).normal_(0, 0.02, generator=g)
+    w2 = torch.empty(E + 1, H, I, **bf).normal_(0, 0.02, generator=g)
+    tok = torch.randint(0, T, (few + many,), generator=g, dtype=torch.int32, device="cuda")
+    off = torch.tensor([0, *counts.cumsum(0).tolist(), few + many], dtype=torch.int32, device="cuda")
+    st = smoe[0].device_state(x.device).status.data_ptr()
+    s = torch.cuda.current_stream().cuda_stream
+    results, seen = [], []
+    for e, n in ((E, few), (E + 1, few + many)):
+        y1, y2 = torch.empty(n, I, **bf), torch.empty(n, H, **bf)
+        before = smoe[0].launch_count()
+        assert lib.smoe_up_projection_forward(x.data_ptr(), w1.data_ptr(), None, y1.data_ptr(), off.data_ptr(),
+                                              tok.data_ptr(), T, H, I, e, n, st, s) == 0
+        between = smoe[0].launch_count()
+        assert lib.smoe_down_projection_forward(y1.data_ptr(), w2.data_ptr(), y2.data_ptr(), off.data_ptr(), H, I, e, n, st,
+                                                s) == 0
+        seen.append((between - before, smoe[0].launch_count() - between))
+        torch.cuda.synchronize()
+        smoe[0].check_status()
+        results.append([t[:few] for t in (y1, y2)])
+    assert seen == [launches, (1, 1)]
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
