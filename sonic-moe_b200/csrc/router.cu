@@ -745,10 +745,13 @@ static int encode_rows(CUtensorMap* map, const void* base, uint64_t rows, uint64
 
 // Tile of router_forward_small_kernel: what a CTA loads per k-block is (rows + E / split) lines, so the smallest such tile
 // whose CTAs all fit on the chip at once; one with the large kernel's 128 rows and all experts means that kernel (from
-// 9473 tokens on at 148 SMs, where tiles of half its traffic would take a second wave).
+// 9473 tokens on at 148 SMs, where tiles of half its traffic would take a second wave).  With 32 experts the large kernel's
+// thread is done with a token's list sooner than a warp here, which no longer pays from about 2048 tokens on (T 1000 / 2500 /
+// 7000 / 9472, H 1536, large 23.6, 25.7, 29.7, 29.7 us, small 23.5, 27.6, 33.8, 33.9).
 static void small_tile(int T, int E, int sms, int& rows, int& split) {
   rows = BM;
   split = 1;
+  if (E == 32 && T > 2048) return;
   int best = BM + E;
   for (int r = 32; r <= BM; r *= 2) {
     for (int s = 1; s <= 8 && s <= r; s *= 2) {
