@@ -149,12 +149,13 @@ def _route_metadata(expert_idx: torch.Tensor, token_idx: torch.Tensor | None, E:
         off = torch.empty(E + 1, dtype=torch.int32, device=dev)
         idx3 = torch.empty(3, n, dtype=torch.int32, device=dev)
         ws = _lib.workspace(lib.smoe_route_metadata_workspace_bytes(E), dev)
+        s_scatter, s_reverse, x_gather = idx3.unbind(0)
         rc = lib.smoe_route_metadata(
             expert_idx.data_ptr(), ptr(token_idx), n, E, max(K, 1), freq.data_ptr(), off.data_ptr(),
-            idx3[0].data_ptr(), idx3[1].data_ptr(), idx3[2].data_ptr(), ws.data_ptr(), stream_ptr(dev),
+            s_scatter.data_ptr(), s_reverse.data_ptr(), x_gather.data_ptr(), ws.data_ptr(), stream_ptr(dev),
         )
         check(rc, "route_metadata")
-    return Route(freq, off, idx3[2], idx3[0], idx3[1], None, K)
+    return Route(freq, off, x_gather, s_scatter, s_reverse, None, K)
 
 
 def TC_topk_router_metadata(topk_router_indices: torch.Tensor, expert_frequency_offset: torch.Tensor, K: int):

@@ -131,8 +131,8 @@ class MoE(nn.Module):
             raise ValueError(f"kernel backend {kernel_backend_moe} is not provided by this build")
 
         out = out.view(original_shape)
-        replaced = getattr(self._compute_switch_loss, "__func__", None) is not MoE._compute_switch_loss
-        if aux_loss is None and kernel_backend_moe == KernelBackendMoE.sonicmoe and not replaced:
+        if (aux_loss is None and kernel_backend_moe == KernelBackendMoE.sonicmoe
+                and getattr(self._compute_switch_loss, "__func__", None) is MoE._compute_switch_loss):
             aux_loss = switch_loss(router_logits, expert_frequency)
         if aux_loss is None:
             aux_loss = self._compute_switch_loss(
