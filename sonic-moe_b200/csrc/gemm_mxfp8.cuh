@@ -72,7 +72,7 @@ struct SharedStorage {
   int m_tile_prefix[MAX_EXPERTS + 1];
 };
 
-// Output staging: 32 rows x 80 bytes per epilogue warp, so that bf16 outputs leave as 64-byte row segments (8 rows
+// Output staging: 32 rows x 64 bytes per epilogue warp, so that bf16 outputs leave as 64-byte row segments (8 rows
 // per store instruction) instead of one row per lane (see warp_store_rows64 in epilogue.cuh).
 constexpr int STAGE_OUT_BYTES = EPI_WARPS * STAGE_ROWS_BYTES;  // 16 KiB
 constexpr int SMEM_BYTES = 1024 + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + SF_SETS * SF_SET_BYTES +

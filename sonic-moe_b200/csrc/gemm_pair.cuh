@@ -118,9 +118,9 @@ __device__ __forceinline__ void order_experts(const GemmParams& p, SharedStorage
 // Ragged-K with a skewed load: a unit is as long as its expert's token count, so the experts go in descending order of
 // their counts and every other round is dealt out in reverse, which evens out the clusters' sums: at 65536 tokens, top-4 of
 // 64 experts, loads falling with the square of the rank, the longest cluster has 1379 k-blocks (dW2) where the mean is
-// 1336 and plain round-robin gave 2356; dW2 1489 -> 1040 us, dW1 1818 -> 1315 us.  Even loads keep the plain order, which
-// is 3 % faster there (dW1 of the 128-expert benchmark layer 3560 against 3666 us): the line is a largest count of twice
-// the mean, below which round-robin is at most one such unit off.
+// 1336 and plain round-robin gave 2356; dW2 1342 -> 922 us, dW1 1642 -> 1199 us (alternating; the eight-warp epilogue is in
+// it).  Even loads keep the plain order, which is 3 % faster there (dW1 of the 128-expert benchmark layer 3560 against
+// 3666 us): the line is a largest count of twice the mean, below which round-robin is at most one such unit off.
 template <bool RAGGED_K, int DUAL>
 struct UnitWalker {
   static constexpr int UNIT_N = DUAL == DUAL_N ? 2 * BN : BN;
