@@ -657,12 +657,12 @@ def test_general_epilogues_at_tile_edges(smoe, act, I):
 
 
 @pytest.mark.parametrize("counts", [
-    [0, 1, 3, 4, 5, 16, 17, 31, 32, 33, 70, 0],   # mean below 20: 32-row units, experts with several of them
-    [0, 1, 15, 63, 64, 65, 130, 20],              # 64
-    [0, 127, 128, 129, 33, 97, 250, 1],           # 128
-    [0, 1500, 63, 128, 129, 64, 300, 1] + [2] * 70,  # above 2048 rows, most of them in few experts: tiles for all
-    [0, 500, 63, 128, 129, 64, 200, 1] + [25] * 70,  # those above two units go to the tiles
-    [1],
+    [0, 1, 3, 4, 5, 16, 17, 31, 32, 33, 70, 0],   # mean 18: 64-row units
+    [0, 1, 15, 63, 64, 65, 130, 20],              # mean 45: 128
+    [0, 127, 128, 129, 33, 97, 250, 1],           # 128, experts with several of them
+    [0, 1500, 63, 128, 129, 64, 300, 1] + [2] * 70,  # 64-row units, one expert with 24 of them
+    [0, 500, 63, 128, 129, 64, 200, 1] + [25] * 70,  # 64
+    [1],                                          # 32
 ])
 @pytest.mark.parametrize("H,I", [(192, 64), (512, 192), (64, 128)])
 def test_few_rows_per_expert(smoe, counts, H, I):
