@@ -1,5 +1,4 @@
 // Host side of the grouped GEMMs: tensor-map construction and the C-ABI launchers.
-#include "device_cache.cuh"
 #include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
 
@@ -91,19 +90,8 @@ static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   }
   const int sms = num_sms();
   if (sms < 2) return SMOE_ERR_DRIVER;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1), 1, 1);
-  cfg.blockDim = dim3(pair::threads(GW, kSplit), 1, 1);
-  cfg.dynamicSmemBytes = pair::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return launched(cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p));
+  return launched(launch_chained(kernel, dim3(static_cast<unsigned>(sms & ~1)), pair::threads(GW, kSplit),
+                                 pair::SMEM_BYTES, stream, 2, tmA, tmB, p));
 }
 
 // Kernels without a gathered operand work on single tiles, kernels with one on dual tiles where they pay.
@@ -201,8 +189,8 @@ static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, const G
   const int sms = num_sms();
   if (sms <= 0) return SMOE_ERR_DRIVER;
   const int stages = skinny::num_stages(nt);
-  kernel<<<sms, skinny::threads(GATHER), skinny::smem_bytes(nt, stages), stream>>>(tmW, tmX, p, nt, stages);
-  return launch_rc();
+  return launched(launch_chained(kernel, dim3(static_cast<unsigned>(sms)), skinny::threads(GATHER),
+                                 skinny::smem_bytes(nt, stages), stream, 1, tmW, tmX, p, nt, stages));
 }
 
 // An empty batch (T == 0, hence TK == 0) is valid: the entry points return at once (weight-gradient entry points

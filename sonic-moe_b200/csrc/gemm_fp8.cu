@@ -1,6 +1,5 @@
 // FP8 (E4M3) entry points: quantisation kernels and the launchers of the FP8 grouped GEMMs, for fp32 block
 // scales (amax / 448, applied in software) and for power-of-two UE8M0 block scales (applied by the tensor cores).
-#include "device_cache.cuh"
 #include "gemm_fp8.cuh"
 #include "gemm_mxfp8.cuh"
 
@@ -68,19 +67,8 @@ static int launch_kernel(Kernel kernel, PerDeviceFlag& configured, int smem_byte
   }
   const int sms = num_sms();
   if (sms < 2) return SMOE_ERR_DRIVER;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1), 1, 1);
-  cfg.blockDim = dim3(THREADS, 1, 1);
-  cfg.dynamicSmemBytes = smem_bytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return launched(cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, p, sc));
+  return launched(launch_chained(kernel, dim3(static_cast<unsigned>(sms & ~1)), THREADS, smem_bytes, stream, 2, tmA,
+                                 tmB, p, sc));
 }
 
 template <bool A_GATHER, bool B_MN, int EPI>
@@ -123,9 +111,10 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
 // group are one 32-bit word of the padded scale row (ld bytes per row, ld % 4 == 0, padding = 2^0); otherwise fp32
 // scales amax / 448, one per block (ld = blocks per row).
 template <bool POW2>
-__global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16* __restrict__ x,
-                                                            uint8_t* __restrict__ q, void* __restrict__ scale,
+__global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16* x, uint8_t* q, void* scale,
                                                             long long rows, int cols, int ld) {
+  release_next();
+  wait_for_previous();
   const int nblk = cols >> 7;
   const int groups = (nblk + 3) >> 2;
   const long long w = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -170,9 +159,10 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16*
 // POW2: the scale is a UE8M0 byte (smallest power of two >= amax / 448), else fp32 amax / 448.
 // WIDE: w is 16-byte and q 8-byte aligned; otherwise (a view into a larger buffer) w is 8-byte and q 4-byte aligned.
 template <bool POW2, bool WIDE>
-__global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat16* __restrict__ w,
-                                                              uint8_t* __restrict__ q, void* __restrict__ scale,
-                                                              int rows, int cols) {
+__global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat16* w, uint8_t* q, void* scale, int rows,
+                                                              int cols) {
+  release_next();
+  wait_for_previous();
   __shared__ float warp_max[8];
   const int cb = blockIdx.x, rb = blockIdx.y, e = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -253,8 +243,8 @@ static int quantize_blocks(const void* w, void* q, void* scale, int batch, int r
   if (!POW2 && reinterpret_cast<uintptr_t>(scale) % 4 != 0) return SMOE_ERR_ALIGNMENT;
   const dim3 grid(cols / 128, (rows + 127) / 128, batch);
   const auto kernel = wa % 16 == 0 && qa % 8 == 0 ? quantize_blocks_kernel<POW2, true> : quantize_blocks_kernel<POW2, false>;
-  kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(w),
-                                                              static_cast<uint8_t*>(q), scale, rows, cols);
+  launch_chained(kernel, grid, 256, 0, static_cast<cudaStream_t>(stream), 1, static_cast<const __nv_bfloat16*>(w),
+                 static_cast<uint8_t*>(q), scale, rows, cols);
   return launch_rc();
 }
 
@@ -277,8 +267,9 @@ int smoe_fp8_quantize_rows(const void* x, void* q, float* scale, long long rows,
   if (rows == 0) return SMOE_OK;
   const int nblk = cols / 128;
   const long long warps = rows * ((nblk + 3) / 4);
-  quantize_rows_kernel<false><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale, rows, cols, nblk);
+  launch_chained(quantize_rows_kernel<false>, static_cast<unsigned>((warps + 7) / 8), 256, 0,
+                 static_cast<cudaStream_t>(stream), 1, static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q),
+                 scale, rows, cols, nblk);
   return launch_rc();
 }
 
@@ -373,8 +364,9 @@ int smoe_mxfp8_quantize_rows(const void* x, void* q, void* scale, long long rows
   if ((reinterpret_cast<uintptr_t>(scale) & 3u) != 0) return SMOE_ERR_ALIGNMENT;
   const int ld = smoe_mxfp8_scale_row_bytes(cols);
   const long long warps = rows * (ld / 4);
-  quantize_rows_kernel<true><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scale, rows, cols, ld);
+  launch_chained(quantize_rows_kernel<true>, static_cast<unsigned>((warps + 7) / 8), 256, 0,
+                 static_cast<cudaStream_t>(stream), 1, static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q),
+                 scale, rows, cols, ld);
   return launch_rc();
 }
 

@@ -13,6 +13,7 @@
 // Registers are moved from the light warps to the promotion warps with setmaxnreg.
 #pragma once
 #include "epilogue.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace smoe {
@@ -152,6 +153,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     tmem_alloc(smem_u32(&ss.tmem_base), 2 * BN);
     tmem_relinquish();
   }
+  wait_for_previous();
   if (warp == 2) {
     int running = 0;
     for (int base = 0; base < p.E; base += 32) {
@@ -172,6 +174,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
+  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 

@@ -159,6 +159,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     tmem_alloc(smem_u32(&ss.tmem_base), TMEM_COLS);
     tmem_relinquish();
   }
+  wait_for_previous();
   if (warp == 2) {
     int running = 0;
     for (int base = 0; base < p.E; base += 32) {
@@ -179,6 +180,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
+  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 

@@ -24,6 +24,7 @@
 // bounded (ptx.cuh).
 #pragma once
 #include "epilogue.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace smoe {
@@ -261,6 +262,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     tmem_alloc(smem_u32(&ss.tmem_base), 2 * BN);  // all 512 columns: both CTAs get the same base
     tmem_relinquish();
   }
+  wait_for_previous();
   for (int e = threadIdx.x; e <= p.E; e += blockDim.x) ss.off[e] = p.off[e];
   if constexpr (RAGGED_K) {
     if (threadIdx.x == 0) ss.most_rows = 0;
@@ -292,6 +294,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // the other CTA's barriers are initialised before anything can arrive on them
+  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 

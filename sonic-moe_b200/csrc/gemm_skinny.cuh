@@ -16,6 +16,7 @@
 // staging rows turn these words into 64-byte row segments.
 #pragma once
 #include "epilogue.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace smoe {
@@ -157,6 +158,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     tmem_alloc(smem_u32(&ss.tmem_base), 2 * MAX_NT);
     tmem_relinquish();
   }
+  wait_for_previous();
   for (int e = threadIdx.x; e <= p.E; e += blockDim.x) ss.off[e] = p.off[e];
   if (warp == 2) {
     const int max_rows = p.max_rows < p.total_rows && tiles_take_all(p, p.max_rows, lane) ? 0 : p.max_rows;
@@ -178,6 +180,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
+  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
   bool ok = true;

@@ -22,7 +22,7 @@
 #include <mutex>
 
 #include "../../include/sonicmoe_b200.h"
-#include "device_cache.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace smoe {
@@ -128,8 +128,10 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     tmem_alloc(smem_u32(&ss.tmem_base), 2 * p.acc_cols);
     tmem_relinquish();
   }
+  wait_for_previous();
   tc_fence_before();
   __syncthreads();
+  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 
@@ -360,9 +362,11 @@ router_forward_small_kernel(const __grid_constant__ CUtensorMap tmX, const __gri
     tmem_alloc(smem_u32(&ss.tmem_base), p.acc_cols);
     tmem_relinquish();
   }
+  wait_for_previous();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // every CTA of the cluster runs before anything is written to its shared memory
+  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 
@@ -522,10 +526,11 @@ router_forward_small_kernel(const __grid_constant__ CUtensorMap tmX, const __gri
 // over its share of the CTAs); without hist_partial, count is an input.  With `aux` also the load-balancing loss E <mean, share>, mean = colsum / sum(colsum) and
 // share = count / sum(count) (denominators at least 1e-12), and its gradient by colsum, E (share - <mean, share>) /
 // sum(colsum): two norms, divisions and a product over E values that took ten launches forward and fifteen backward.
-__global__ void __launch_bounds__(1024) router_finish_kernel(const float* __restrict__ colsum_partial,
-                                                             const int* __restrict__ hist_partial, int blocks, int E,
-                                                             float* __restrict__ colsum, int* __restrict__ count,
-                                                             float* __restrict__ aux, float* __restrict__ aux_grad) {
+__global__ void __launch_bounds__(1024) router_finish_kernel(const float* colsum_partial, const int* hist_partial,
+                                                             int blocks, int E, float* colsum, int* count, float* aux,
+                                                             float* aux_grad) {
+  release_next();
+  wait_for_previous();
   __shared__ float part_s[4][MAX_E];
   __shared__ int part_c[4][MAX_E];
   __shared__ float red[3][8];
@@ -587,8 +592,10 @@ __global__ void __launch_bounds__(1024) router_finish_kernel(const float* __rest
 // accurate exponential and division: the fast ones are off by |x| 2^-24 of a probability, which shows in the loss when the
 // tokens go to experts of small probability.
 template <int PER_LANE>
-__global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16* __restrict__ logits, int rows, int E,
-                                                             float* __restrict__ colsum_partial) {
+__global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16* logits, int rows, int E,
+                                                             float* colsum_partial) {
+  release_next();
+  wait_for_previous();
   __shared__ float sums[8][MAX_E];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float colsum[PER_LANE];
@@ -633,16 +640,13 @@ __global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16
 // One warp per row; the row's probabilities are recomputed from the saved bf16 logits, with the exponential that the forward
 // pass used: the fast one behind the router kernels, the accurate one (EXACT) behind softmax_colsum_kernel.
 template <int PER_LANE, bool EXACT>
-__global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* __restrict__ dlogits,
-                                                              const __nv_bfloat16* __restrict__ logits,
-                                                              const float* __restrict__ dscore,
-                                                              const float* __restrict__ score,
-                                                              const int* __restrict__ indices,
-                                                              const float* __restrict__ g_colsum,
-                                                              const __nv_bfloat16* __restrict__ g_logits,
-                                                              const float* __restrict__ g_aux,
-                                                              const float* __restrict__ aux_grad, int rows, int E,
-                                                              int K) {
+__global__ void __launch_bounds__(256) router_backward_kernel(__nv_bfloat16* dlogits, const __nv_bfloat16* logits,
+                                                              const float* dscore, const float* score,
+                                                              const int* indices, const float* g_colsum,
+                                                              const __nv_bfloat16* g_logits, const float* g_aux,
+                                                              const float* aux_grad, int rows, int E, int K) {
+  release_next();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -838,19 +842,7 @@ int smoe_router_forward_aux(const void* x, const void* router_w, void* logits, f
           return SMOE_ERR_LAUNCH;
         configured.set(dev);
       }
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-      cfg.blockDim = dim3(THREADS, 1, 1);
-      cfg.dynamicSmemBytes = SmallLayout(p.tile_rows, p.split, E, p.stages).total;
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = static_cast<unsigned>(p.split);
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (cudaLaunchKernelEx(&cfg, kernel, tmX, tmW, p) != cudaSuccess) return SMOE_ERR_LAUNCH;
+      launch_chained(kernel, grid, THREADS, SmallLayout(p.tile_rows, p.split, E, p.stages).total, st, p.split, tmX, tmW, p);
     } else if (K <= 8) {
       if (!configured8.test(dev)) {
         if (cudaFuncSetAttribute(router_forward_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
@@ -858,7 +850,7 @@ int smoe_router_forward_aux(const void* x, const void* router_w, void* logits, f
           return SMOE_ERR_LAUNCH;
         configured8.set(dev);
       }
-      router_forward_kernel<8><<<grid, THREADS, smem, st>>>(tmX, tmW, p);
+      launch_chained(router_forward_kernel<8>, grid, THREADS, smem, st, 1, tmX, tmW, p);
     } else {
       if (!configured16.test(dev)) {
         if (cudaFuncSetAttribute(router_forward_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) !=
@@ -866,12 +858,12 @@ int smoe_router_forward_aux(const void* x, const void* router_w, void* logits, f
           return SMOE_ERR_LAUNCH;
         configured16.set(dev);
       }
-      router_forward_kernel<16><<<grid, THREADS, smem, st>>>(tmX, tmW, p);
+      launch_chained(router_forward_kernel<16>, grid, THREADS, smem, st, 1, tmX, tmW, p);
     }
     if (cudaGetLastError() != cudaSuccess) return SMOE_ERR_LAUNCH;
   }
-  router_finish_kernel<<<1, 1024, 0, st>>>(colsum_partial, hist_partial, T > 0 ? grid : 0, E, prob_colsum, expert_count,
-                                           aux, aux_grad);
+  launch_chained(router_finish_kernel, 1, 1024, 0, st, 1, colsum_partial, hist_partial,
+                 T > 0 ? grid : 0, E, prob_colsum, expert_count, aux, aux_grad);
   return launch_rc(T > 0 ? 2 : 1);
 }
 
@@ -888,15 +880,15 @@ int smoe_switch_loss(const void* logits, const int* expert_count, float* aux, fl
   if (blocks > 0) {
     const int per_lane = (E + 31) / 32;
     if (per_lane <= 1)
-      softmax_colsum_kernel<1><<<blocks, 256, 0, st>>>(l, T, E, colsum_partial);
+      launch_chained(softmax_colsum_kernel<1>, blocks, 256, 0, st, 1, l, T, E, colsum_partial);
     else if (per_lane <= 4)
-      softmax_colsum_kernel<4><<<blocks, 256, 0, st>>>(l, T, E, colsum_partial);
+      launch_chained(softmax_colsum_kernel<4>, blocks, 256, 0, st, 1, l, T, E, colsum_partial);
     else
-      softmax_colsum_kernel<8><<<blocks, 256, 0, st>>>(l, T, E, colsum_partial);
+      launch_chained(softmax_colsum_kernel<8>, blocks, 256, 0, st, 1, l, T, E, colsum_partial);
     if (cudaGetLastError() != cudaSuccess) return SMOE_ERR_LAUNCH;
   }
-  router_finish_kernel<<<1, 1024, 0, st>>>(colsum_partial, nullptr, blocks, E, nullptr, const_cast<int*>(expert_count),
-                                           aux, aux_grad);
+  launch_chained(router_finish_kernel, 1, 1024, 0, st, 1, colsum_partial, nullptr, blocks, E, nullptr,
+                 const_cast<int*>(expert_count), aux, aux_grad);
   return launch_rc(blocks > 0 ? 2 : 1);
 }
 
@@ -926,7 +918,7 @@ int smoe_router_backward_aux(void* dlogits, const void* logits, const float* dsc
   const auto kernel = per_lane <= 2   ? (exact ? router_backward_kernel<2, true> : router_backward_kernel<2, false>)
                       : per_lane <= 4 ? (exact ? router_backward_kernel<4, true> : router_backward_kernel<4, false>)
                                       : (exact ? router_backward_kernel<8, true> : router_backward_kernel<8, false>);
-  kernel<<<grid, 256, 0, st>>>(d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E, K);
+  launch_chained(kernel, grid, 256, 0, st, 1, d, l, dscores, scores, indices, g_colsum, g, g_aux, aux_grad, T, E, K);
   return launch_rc();
 }
 

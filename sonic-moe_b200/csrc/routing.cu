@@ -10,7 +10,7 @@
 #include <mutex>
 
 #include "../../include/sonicmoe_b200.h"
-#include "device_cache.cuh"
+#include "launch.cuh"
 
 namespace smoe {
 
@@ -46,8 +46,10 @@ __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return
 
 // One warp per row; lane l keeps columns l, l+32, ... in registers (PER_LANE of them).
 template <typename T, int PER_LANE>
-__global__ void __launch_bounds__(256) topk_softmax_kernel(const T* __restrict__ logits, float* __restrict__ scores,
-                                                           int* __restrict__ indices, int rows, int E, int K) {
+__global__ void __launch_bounds__(256) topk_softmax_kernel(const T* logits, float* scores, int* indices, int rows,
+                                                           int E, int K) {
+  release_next();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -90,10 +92,10 @@ __global__ void __launch_bounds__(256) topk_softmax_kernel(const T* __restrict__
 
 // Any E: K passes over the row, each finding the best key below the previous winner.
 template <typename T>
-__global__ void __launch_bounds__(256) topk_softmax_generic_kernel(const T* __restrict__ logits,
-                                                                   float* __restrict__ scores,
-                                                                   int* __restrict__ indices, int rows, int E,
-                                                                   int K) {
+__global__ void __launch_bounds__(256) topk_softmax_generic_kernel(const T* logits, float* scores, int* indices,
+                                                                   int rows, int E, int K) {
+  release_next();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -133,32 +135,31 @@ static int launch_topk(const void* logits, float* scores, int* indices, int rows
   const unsigned grid = (rows + warps - 1) / warps;
   const int per_lane = (E + 31) / 32;
   if (K > 32) {
-    topk_softmax_generic_kernel<T><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_generic_kernel<T>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   } else if (per_lane <= 1) {
-    topk_softmax_kernel<T, 1><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_kernel<T, 1>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   } else if (per_lane <= 2) {
-    topk_softmax_kernel<T, 2><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_kernel<T, 2>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   } else if (per_lane <= 4) {
-    topk_softmax_kernel<T, 4><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_kernel<T, 4>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   } else if (per_lane <= 8) {
-    topk_softmax_kernel<T, 8><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_kernel<T, 8>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   } else if (per_lane <= 16) {
-    topk_softmax_kernel<T, 16><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_kernel<T, 16>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   } else if (per_lane <= 32) {
-    topk_softmax_kernel<T, 32><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_kernel<T, 32>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   } else {
-    topk_softmax_generic_kernel<T><<<grid, warps * 32, 0, st>>>(src, scores, indices, rows, E, K);
+    launch_chained(topk_softmax_generic_kernel<T>, grid, warps * 32, 0, st, 1, src, scores, indices, rows, E, K);
   }
   return launch_rc();
 }
 
 // dlogits[t, idx[t,k]] = s_k * (g_k - sum_j g_j s_j); every other column of the row is written as zero.
 template <typename T>
-__global__ void __launch_bounds__(256) softmax_topk_bwd_kernel(T* __restrict__ dlogits,
-                                                               const float* __restrict__ dscore,
-                                                               const float* __restrict__ score,
-                                                               const int* __restrict__ indices, int rows, int E,
-                                                               int K) {
+__global__ void __launch_bounds__(256) softmax_topk_bwd_kernel(T* dlogits, const float* dscore, const float* score,
+                                                               const int* indices, int rows, int E, int K) {
+  release_next();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -179,8 +180,10 @@ __global__ void __launch_bounds__(256) softmax_topk_bwd_kernel(T* __restrict__ d
 // histogram + prefix sum
 // ----------------------------------------------------------------------------------------------
 template <typename IdxT>
-__global__ void __launch_bounds__(kSortThreads) chunk_histogram_kernel(const IdxT* __restrict__ idx, long long n,
-                                                                       int E, int* __restrict__ block_hist) {
+__global__ void __launch_bounds__(kSortThreads) chunk_histogram_kernel(const IdxT* idx, long long n, int E,
+                                                                       int* block_hist) {
+  release_next();
+  wait_for_previous();
   extern __shared__ int hist[];
   for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
   __syncthreads();
@@ -211,9 +214,10 @@ __global__ void __launch_bounds__(256) global_histogram_kernel(const IdxT* __res
 //   count[e]   = total of bin e               (optional)
 //   cumsum[e]  = count[0] + ... + count[e]    (optional)
 //   offset[e]  = exclusive scan, E+1 entries  (optional)
-__global__ void __launch_bounds__(1024) scan_bins_kernel(int* __restrict__ block_hist, int num_blocks, int E,
-                                                         const int* __restrict__ count_in, int* __restrict__ count,
-                                                         int* __restrict__ cumsum, int* __restrict__ offset) {
+__global__ void __launch_bounds__(1024) scan_bins_kernel(int* block_hist, int num_blocks, int E, const int* count_in,
+                                                         int* count, int* cumsum, int* offset) {
+  release_next();
+  wait_for_previous();
   __shared__ int warp_sums[32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -282,13 +286,12 @@ __global__ void __launch_bounds__(1024) scan_bins_kernel(int* __restrict__ block
 //   r = offset[e] + block_hist[b][e] + (slots of bin e earlier in the chunk)
 // Outputs: s_scatter[r] = p, s_reverse[p] = r, x_gather[r] = token of slot p
 // (p / K for a fixed K per token, token_idx[p] when the caller lists the pairs).
-__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* __restrict__ idx, long long n, int E,
-                                                                    const int* __restrict__ block_hist,
-                                                                    const int* __restrict__ offset, int K,
-                                                                    const int* __restrict__ token_idx,
-                                                                    int* __restrict__ s_scatter,
-                                                                    int* __restrict__ s_reverse,
-                                                                    int* __restrict__ x_gather) {
+__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* idx, long long n, int E,
+                                                                    const int* block_hist, const int* offset, int K,
+                                                                    const int* token_idx, int* s_scatter,
+                                                                    int* s_reverse, int* x_gather) {
+  release_next();
+  wait_for_previous();
   extern __shared__ int sm[];
   int* running = sm;                 // [E] slots of each bin already placed by this chunk (plus bases)
   int* warp_cnt = sm + E;            // [kSortWarps][E]
@@ -330,8 +333,9 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const int* _
 }
 
 // offsets[t] = first position p with sorted_idx[p] >= t, for t = 0..T (offsets[T] = n).
-__global__ void sorted_offsets_kernel(const int* __restrict__ sorted_idx, long long n, int T,
-                                      int* __restrict__ offsets) {
+__global__ void sorted_offsets_kernel(const int* sorted_idx, long long n, int T, int* offsets) {
+  release_next();
+  wait_for_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t > T) return;
   long long lo = 0, hi = n;
@@ -349,10 +353,11 @@ __global__ void sorted_offsets_kernel(const int* __restrict__ sorted_idx, long l
 // tok_off == nullptr means a fixed K rows per token: p in [t*K, (t+1)*K).
 // One thread per 8 consecutive columns of one token, fp32 accumulation.
 template <typename W, bool ADD_FP32>
-__global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* __restrict__ src,
-                                                         __nv_bfloat16* __restrict__ out, const W* __restrict__ w,
-                                                         const int* __restrict__ rev, const int* __restrict__ tok_off,
-                                                         const float* __restrict__ add, int T, int H, int K) {
+__global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* src, __nv_bfloat16* out, const W* w,
+                                                         const int* rev, const int* tok_off, const float* add, int T,
+                                                         int H, int K) {
+  release_next();
+  wait_for_previous();
   const int vec_per_row = H >> 3;
   const long long g = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (g >= static_cast<long long>(T) * vec_per_row) return;
@@ -407,9 +412,10 @@ __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restr
 
 // ds[s_scatter[r]] = sum_c ds_partial[c, r]
 template <typename OutT>
-__global__ void __launch_bounds__(256) ds_reduce_kernel(const float* __restrict__ ds_partial,
-                                                        const int* __restrict__ s_scatter, OutT* __restrict__ ds,
-                                                        int TK, int ncols) {
+__global__ void __launch_bounds__(256) ds_reduce_kernel(const float* ds_partial, const int* s_scatter, OutT* ds, int TK,
+                                                        int ncols) {
+  release_next();
+  wait_for_previous();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= TK) return;
   float acc = 0.f;
@@ -446,12 +452,12 @@ static int noalloc_scratch(int** out) {
 // took 36 us for 32764 rows of 1024 columns in 32 experts, now 15).
 constexpr int kColumnSumThreads = 1024;
 template <typename ScoreT>
-__global__ void __launch_bounds__(kColumnSumThreads) expert_column_sum_kernel(const __nv_bfloat16* __restrict__ src, long long ld,
-                                                                const int* __restrict__ gather,
-                                                                const ScoreT* __restrict__ scores,
-                                                                const int* __restrict__ s_scatter,
-                                                                const int* __restrict__ off,
-                                                                __nv_bfloat16* __restrict__ out, int N) {
+__global__ void __launch_bounds__(kColumnSumThreads) expert_column_sum_kernel(const __nv_bfloat16* src, long long ld,
+                                                                              const int* gather, const ScoreT* scores,
+                                                                              const int* s_scatter, const int* off,
+                                                                              __nv_bfloat16* out, int N) {
+  release_next();
+  wait_for_previous();
   constexpr int WARPS = kColumnSumThreads / 32;
   __shared__ float part[WARPS][256];
   const int e = blockIdx.x;
@@ -489,11 +495,11 @@ __global__ void __launch_bounds__(kColumnSumThreads) expert_column_sum_kernel(co
 // ds[s_scatter[r]] += <dout[gather[r], :], b2[e(r), :]>: the part of the score gradient that comes from the
 // down-projection bias.  One warp per grouped row; the expert of a row by binary search in the offsets.
 template <typename DsT>
-__global__ void __launch_bounds__(256) ds_bias_term_kernel(const __nv_bfloat16* __restrict__ dout,
-                                                           const __nv_bfloat16* __restrict__ b2,
-                                                           const int* __restrict__ off, const int* __restrict__ gather,
-                                                           const int* __restrict__ s_scatter, DsT* __restrict__ ds,
-                                                           int E, int H, int TK) {
+__global__ void __launch_bounds__(256) ds_bias_term_kernel(const __nv_bfloat16* dout, const __nv_bfloat16* b2,
+                                                           const int* off, const int* gather, const int* s_scatter,
+                                                           DsT* ds, int E, int H, int TK) {
+  release_next();
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= TK) return;
@@ -555,11 +561,11 @@ int smoe_softmax_topk_backward(void* dlogits, int dlogits_dtype, const float* ds
   if (T == 0) return SMOE_OK;
   const unsigned grid = (T + 7) / 8;
   if (dlogits_dtype == SMOE_F32) {
-    softmax_topk_bwd_kernel<float><<<grid, 256, 0, S(stream)>>>(static_cast<float*>(dlogits), dscore, score, indices,
-                                                                 T, E, K);
+    launch_chained(softmax_topk_bwd_kernel<float>, grid, 256, 0, S(stream), 1, static_cast<float*>(dlogits), dscore,
+                   score, indices, T, E, K);
   } else if (dlogits_dtype == SMOE_BF16) {
-    softmax_topk_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(static_cast<__nv_bfloat16*>(dlogits), dscore,
-                                                                         score, indices, T, E, K);
+    launch_chained(softmax_topk_bwd_kernel<__nv_bfloat16>, grid, 256, 0, S(stream), 1,
+                   static_cast<__nv_bfloat16*>(dlogits), dscore, score, indices, T, E, K);
   } else {
     return SMOE_ERR_DTYPE;
   }
@@ -580,11 +586,12 @@ int smoe_count_cumsum(const void* x, int x_dtype, long long n, int E, int* count
     int* hist = static_cast<int*>(workspace);
     const int blocks = sort_blocks(n);
     if (x_dtype == SMOE_I32)
-      chunk_histogram_kernel<int><<<blocks, kSortThreads, E * sizeof(int), st>>>(static_cast<const int*>(x), n, E, hist);
+      launch_chained(chunk_histogram_kernel<int>, blocks, kSortThreads, E * sizeof(int), st, 1,
+                     static_cast<const int*>(x), n, E, hist);
     else
-      chunk_histogram_kernel<long long><<<blocks, kSortThreads, E * sizeof(int), st>>>(
-          static_cast<const long long*>(x), n, E, hist);
-    scan_bins_kernel<<<1, 1024, 0, st>>>(hist, blocks, E, nullptr, count, cumsum, nullptr);
+      launch_chained(chunk_histogram_kernel<long long>, blocks, kSortThreads, E * sizeof(int), st, 1,
+                     static_cast<const long long*>(x), n, E, hist);
+    launch_chained(scan_bins_kernel, 1, 1024, 0, st, 1, hist, blocks, E, nullptr, count, cumsum, nullptr);
   } else {
     if (cudaMemsetAsync(count, 0, sizeof(int) * E, st) != cudaSuccess) return SMOE_ERR_LAUNCH;
     const int blocks = static_cast<int>(n / 1024 + 1 < 1184 ? n / 1024 + 1 : 1184);
@@ -592,7 +599,8 @@ int smoe_count_cumsum(const void* x, int x_dtype, long long n, int E, int* count
       global_histogram_kernel<int><<<blocks, 256, 0, st>>>(static_cast<const int*>(x), n, E, count);
     else
       global_histogram_kernel<long long><<<blocks, 256, 0, st>>>(static_cast<const long long*>(x), n, E, count);
-    if (cumsum != nullptr) scan_bins_kernel<<<1, 1024, 0, st>>>(nullptr, 0, E, count, nullptr, cumsum, nullptr);
+    if (cumsum != nullptr)
+      launch_chained(scan_bins_kernel, 1, 1024, 0, st, 1, nullptr, 0, E, count, nullptr, cumsum, nullptr);
   }
   return launch_rc(E <= kMaxSmemExperts || cumsum != nullptr ? 2 : 1);
 }
@@ -622,11 +630,12 @@ int smoe_count_cumsum_noalloc(const void* x, int x_dtype, long long n, int E, in
   cudaStream_t st = S(stream);
   const int blocks = sort_blocks(n);
   if (x_dtype == SMOE_I32)
-    chunk_histogram_kernel<int><<<blocks, kSortThreads, E * sizeof(int), st>>>(static_cast<const int*>(x), n, E, hist);
+    launch_chained(chunk_histogram_kernel<int>, blocks, kSortThreads, E * sizeof(int), st, 1,
+                   static_cast<const int*>(x), n, E, hist);
   else
-    chunk_histogram_kernel<long long><<<blocks, kSortThreads, E * sizeof(int), st>>>(
-        static_cast<const long long*>(x), n, E, hist);
-  scan_bins_kernel<<<1, 1024, 0, st>>>(hist, blocks, E, nullptr, count, cumsum, nullptr);
+    launch_chained(chunk_histogram_kernel<long long>, blocks, kSortThreads, E * sizeof(int), st, 1,
+                   static_cast<const long long*>(x), n, E, hist);
+  launch_chained(scan_bins_kernel, 1, 1024, 0, st, 1, hist, blocks, E, nullptr, count, cumsum, nullptr);
   return launch_rc(2);
 }
 
@@ -639,8 +648,8 @@ int smoe_route_metadata(const int* expert_idx, const int* token_idx, long long n
   cudaStream_t st = S(stream);
   int* hist = static_cast<int*>(workspace);
   const int blocks = sort_blocks(n);
-  chunk_histogram_kernel<int><<<blocks, kSortThreads, E * sizeof(int), st>>>(expert_idx, n, E, hist);
-  scan_bins_kernel<<<1, 1024, 0, st>>>(hist, blocks, E, nullptr, expert_count, nullptr, expert_offset);
+  launch_chained(chunk_histogram_kernel<int>, blocks, kSortThreads, E * sizeof(int), st, 1, expert_idx, n, E, hist);
+  launch_chained(scan_bins_kernel, 1, 1024, 0, st, 1, hist, blocks, E, nullptr, expert_count, nullptr, expert_offset);
   if (n > 0) {
     const size_t smem = static_cast<size_t>(E) * (1 + kSortWarps) * sizeof(int);
     static PerDeviceFlag configured;
@@ -652,15 +661,15 @@ int smoe_route_metadata(const int* expert_idx, const int* token_idx, long long n
         return SMOE_ERR_LAUNCH;
       configured.set(dev);
     }
-    sort_scatter_kernel<<<blocks, kSortThreads, smem, st>>>(expert_idx, n, E, hist, expert_offset, K, token_idx,
-                                                            s_scatter_idx, s_reverse_scatter_idx, x_gather_idx);
+    launch_chained(sort_scatter_kernel, blocks, kSortThreads, smem, st, 1, expert_idx, n, E, hist, expert_offset, K,
+                   token_idx, s_scatter_idx, s_reverse_scatter_idx, x_gather_idx);
   }
   return launch_rc(n > 0 ? 3 : 2);
 }
 
 int smoe_sorted_offsets(const int* sorted_idx, long long n, int T, int* offsets, void* stream) {
   if (n < 0 || T < 0) return SMOE_ERR_SHAPE;
-  sorted_offsets_kernel<<<(T + 1 + 255) / 256, 256, 0, S(stream)>>>(sorted_idx, n, T, offsets);
+  launch_chained(sorted_offsets_kernel, (T + 1 + 255) / 256, 256, 0, S(stream), 1, sorted_idx, n, T, offsets);
   return launch_rc();
 }
 
@@ -674,11 +683,11 @@ int smoe_gather_sum(const void* src, void* out, const void* weights, int weights
   const __nv_bfloat16* s = static_cast<const __nv_bfloat16*>(src);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   if (weights == nullptr || weights_dtype == SMOE_F32) {
-    gather_sum_kernel<float, false><<<grid, 256, 0, S(stream)>>>(s, o, static_cast<const float*>(weights), reverse_idx,
-                                                                 token_offset, nullptr, T, H, K);
+    launch_chained(gather_sum_kernel<float, false>, grid, 256, 0, S(stream), 1, s, o,
+                   static_cast<const float*>(weights), reverse_idx, token_offset, nullptr, T, H, K);
   } else if (weights_dtype == SMOE_BF16) {
-    gather_sum_kernel<__nv_bfloat16, false><<<grid, 256, 0, S(stream)>>>(
-        s, o, static_cast<const __nv_bfloat16*>(weights), reverse_idx, token_offset, nullptr, T, H, K);
+    launch_chained(gather_sum_kernel<__nv_bfloat16, false>, grid, 256, 0, S(stream), 1, s, o,
+                   static_cast<const __nv_bfloat16*>(weights), reverse_idx, token_offset, nullptr, T, H, K);
   } else {
     return SMOE_ERR_DTYPE;
   }
@@ -702,11 +711,11 @@ int smoe_expert_column_sum(const void* src, long long ld, const int* gather_idx,
   const __nv_bfloat16* s = static_cast<const __nv_bfloat16*>(src);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   if (scores == nullptr || scores_dtype == SMOE_F32)
-    expert_column_sum_kernel<float><<<grid, kColumnSumThreads, 0, S(stream)>>>(s, ld, gather_idx, static_cast<const float*>(scores),
-                                                                 s_scatter_idx, expert_offset, o, N);
+    launch_chained(expert_column_sum_kernel<float>, grid, kColumnSumThreads, 0, S(stream), 1, s, ld, gather_idx,
+                   static_cast<const float*>(scores), s_scatter_idx, expert_offset, o, N);
   else if (scores_dtype == SMOE_BF16)
-    expert_column_sum_kernel<__nv_bfloat16><<<grid, kColumnSumThreads, 0, S(stream)>>>(
-        s, ld, gather_idx, static_cast<const __nv_bfloat16*>(scores), s_scatter_idx, expert_offset, o, N);
+    launch_chained(expert_column_sum_kernel<__nv_bfloat16>, grid, kColumnSumThreads, 0, S(stream), 1, s, ld, gather_idx,
+                   static_cast<const __nv_bfloat16*>(scores), s_scatter_idx, expert_offset, o, N);
   else
     return SMOE_ERR_DTYPE;
   return launch_rc();
@@ -720,11 +729,11 @@ int smoe_ds_add_bias_term(const void* dout, const void* b2, const int* expert_of
   const __nv_bfloat16* d = static_cast<const __nv_bfloat16*>(dout);
   const __nv_bfloat16* b = static_cast<const __nv_bfloat16*>(b2);
   if (ds_dtype == SMOE_F32)
-    ds_bias_term_kernel<float><<<grid, 256, 0, S(stream)>>>(d, b, expert_offset, x_gather_idx, s_scatter_idx,
-                                                            static_cast<float*>(ds), E, H, TK);
+    launch_chained(ds_bias_term_kernel<float>, grid, 256, 0, S(stream), 1, d, b, expert_offset, x_gather_idx,
+                   s_scatter_idx, static_cast<float*>(ds), E, H, TK);
   else if (ds_dtype == SMOE_BF16)
-    ds_bias_term_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(d, b, expert_offset, x_gather_idx, s_scatter_idx,
-                                                                    static_cast<__nv_bfloat16*>(ds), E, H, TK);
+    launch_chained(ds_bias_term_kernel<__nv_bfloat16>, grid, 256, 0, S(stream), 1, d, b, expert_offset, x_gather_idx,
+                   s_scatter_idx, static_cast<__nv_bfloat16*>(ds), E, H, TK);
   else
     return SMOE_ERR_DTYPE;
   return launch_rc();
@@ -736,10 +745,11 @@ int smoe_ds_reduce(const float* ds_partial, const int* s_scatter_idx, void* ds, 
   if (TK == 0) return SMOE_OK;
   const unsigned grid = (TK + 255) / 256;
   if (ds_dtype == SMOE_F32)
-    ds_reduce_kernel<float><<<grid, 256, 0, S(stream)>>>(ds_partial, s_scatter_idx, static_cast<float*>(ds), TK, ncols);
+    launch_chained(ds_reduce_kernel<float>, grid, 256, 0, S(stream), 1, ds_partial, s_scatter_idx,
+                   static_cast<float*>(ds), TK, ncols);
   else if (ds_dtype == SMOE_BF16)
-    ds_reduce_kernel<__nv_bfloat16><<<grid, 256, 0, S(stream)>>>(ds_partial, s_scatter_idx,
-                                                                 static_cast<__nv_bfloat16*>(ds), TK, ncols);
+    launch_chained(ds_reduce_kernel<__nv_bfloat16>, grid, 256, 0, S(stream), 1, ds_partial, s_scatter_idx,
+                   static_cast<__nv_bfloat16*>(ds), TK, ncols);
   else
     return SMOE_ERR_DTYPE;
   return launch_rc();

@@ -435,3 +435,52 @@ def test_launch_count(built_library, T, E, K, kernels):
         assert _lib.launch_count() - before == kernels
     torch.cuda.synchronize()
     _lib.check_status()
+
+
+@pytest.mark.parametrize("T,E,K", [(3, 64, 4), (300, 32, 2), (9600, 32, 4)])
+def test_chained_launches_under_graph_capture(built_library, T, E, K):
+    """The launches may begin before the kernel in front of them has ended: a captured forward pass and training step, replayed
+    back to back on changing inputs, give the bits of the same passes run one by one with a synchronisation after each."""
+    import sonicmoe
+    from sonicmoe import _lib
+    from sonicmoe.enums import ActivationType
+
+    H, I, rounds = 256, 128, 6
+    m = sonicmoe.MoE(E, K, H, I, ActivationType.SWIGLU, False, 0.05).cuda().to(torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    inputs = [torch.randn(T, H, device="cuda", generator=g).bfloat16() for _ in range(rounds)]
+    dout = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    x = inputs[0].clone().requires_grad_(True)
+
+    def step():
+        with torch.no_grad():
+            o = m(x, is_inference_mode=True)[0]
+        y, aux = m(x)
+        return [o, y.detach(), *torch.autograd.grad([y, aux], [x, *m.parameters()], [dout, torch.ones_like(aux)])]
+
+    want = []
+    for v in inputs:
+        with torch.no_grad():
+            x.copy_(v)
+        torch.cuda.synchronize()
+        want.append([t.clone() for t in step()])
+        torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    got = []
+    for v in inputs:
+        with torch.no_grad():
+            x.copy_(v)
+        graph.replay()
+        got.append([t.clone() for t in captured])
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for a, b in zip(got, want):
+        for s, t in zip(a, b):
+            assert torch.equal(s, t)
