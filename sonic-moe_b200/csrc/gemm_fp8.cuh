@@ -123,7 +123,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   uint8_t* sB = smem + STAGES * A_STAGE_BYTES;
   SharedStorage& ss = *reinterpret_cast<SharedStorage*>(smem + STAGES * (A_STAGE_BYTES + B_STAGE_BYTES));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -182,6 +182,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     reg_dec<56>();
     // ---- TMA producer ------------------------------------------------------------------------
     if (warp == 0) {
+      const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -190,9 +191,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         for (int kb = 0; kb < tile.num_kb; ++kb) {
           if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
-          if (leader && lane == 0) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
-          __syncwarp();
-          if (lane == 0) {
+          if (elected) {
+            if (leader) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
             const int k0 = kb * BK;
             if constexpr (!A_GATHER) tma_load_2d_pair(&tmA, bar, smem_u32(sA + stage * A_STAGE_BYTES), k0, tile.row0);
             const int nb = tile.n0 + static_cast<int>(rank) * BN_CTA;
@@ -200,6 +200,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             if constexpr (!B_MN) tma_load_2d_pair(&tmB, bar, b_dst, k0, tile.e * p.b_rows_per_expert + nb);
             else tma_load_2d_pair(&tmB, bar, b_dst, nb, tile.e * p.b_rows_per_expert + k0);
           }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -207,6 +208,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
     // ---- MMA issuer ----------------------------------------------------------------------------
     else if (warp == 1 && leader) {
+      const bool elected = elect_one();
       constexpr uint32_t idesc = make_idesc_e4m3(2 * BM, BN, false, B_MN);
       constexpr uint32_t b_lbo = B_MN ? B_STAGE_BYTES : 16;
       constexpr uint32_t b_kstep = B_MN ? (UMMA_K * 128) : UMMA_K;  // bytes per 32 reduction elements
@@ -221,7 +223,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           if (!mbar_wait(smem_u32(&ss.part_empty[buf]), buf_phase ^ 1u, abort_flag)) { ok = false; break; }
           if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          if (lane == 0) {
+          if (elected) {
             const uint64_t a_desc = make_smem_desc(smem_u32(sA + stage * A_STAGE_BYTES), 16, 1024);
             const uint64_t b_desc = make_smem_desc(smem_u32(sB + stage * B_STAGE_BYTES), b_lbo, 1024);
             const uint32_t d_tmem = tmem_base + buf * BN;

@@ -127,7 +127,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   SharedStorage& ss = *reinterpret_cast<SharedStorage*>(sSF + SF_SETS * SF_SET_BYTES);
   uint8_t* stage_out = reinterpret_cast<uint8_t*>(&ss) + ((sizeof(SharedStorage) + 127) & ~127);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -188,6 +188,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     fp8::reg_dec<56>();
     // ---- TMA producer ------------------------------------------------------------------------
     if (warp == 0) {
+      const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -196,9 +197,8 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         for (int kb = 0; kb < tile.num_kb; ++kb) {
           if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
-          if (leader && lane == 0) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
-          __syncwarp();
-          if (lane == 0) {
+          if (elected) {
+            if (leader) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
             const int k0 = kb * BK;
             if constexpr (!A_GATHER) tma_load_2d_pair(&tmA, bar, smem_u32(sA + stage * A_STAGE_BYTES), k0, tile.row0);
             const int nb = tile.n0 + static_cast<int>(rank) * BN_CTA;
@@ -206,6 +206,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
             if constexpr (!B_MN) tma_load_2d_pair(&tmB, bar, b_dst, k0, tile.e * p.b_rows_per_expert + nb);
             else tma_load_2d_pair(&tmB, bar, b_dst, nb, tile.e * p.b_rows_per_expert + k0);
           }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -213,6 +214,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     }
     // ---- MMA issuer ----------------------------------------------------------------------------
     else if (warp == 1 && leader) {
+      const bool elected = elect_one();
       constexpr uint32_t b_lbo = B_MN ? B_STAGE_BYTES : 16;
       constexpr uint32_t b_kstep = B_MN ? (UMMA_K * 128) : UMMA_K;  // bytes per 32 reduction elements
       int stage = 0;
@@ -235,7 +237,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
             tc_fence_after();
             tsfa = tmem_base + TMEM_SF_COL + set * TMEM_SF_SET_COLS;
             tsfb = tsfa + TMEM_SFB_OFFSET;
-            if (lane == 0) {
+            if (elected) {
               const uint32_t s_sf = smem_u32(sSF + set * SF_SET_BYTES);
               tmem_cp_sf_pair(tsfa, make_sf_desc(s_sf));
               tmem_cp_sf_pair(tsfb, make_sf_desc(s_sf + SFA_BYTES));
@@ -247,7 +249,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
           }
           if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          if (lane == 0) {
+          if (elected) {
             const uint32_t idesc = make_idesc_mx(2 * BM, BN, B_MN, static_cast<uint32_t>(kb & (KB_PER_GROUP - 1)));
             const uint64_t a_desc = make_smem_desc(smem_u32(sA + stage * A_STAGE_BYTES), 16, 1024);
             const uint64_t b_desc = make_smem_desc(smem_u32(sB + stage * B_STAGE_BYTES), b_lbo, 1024);

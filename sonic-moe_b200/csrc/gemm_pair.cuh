@@ -204,6 +204,12 @@ struct UnitWalker {
   }
 };
 
+// An MN-major operand tile of one stage: 64-column chunks of BK rows.
+__device__ __forceinline__ void load_mn_tile(const CUtensorMap* tm, uint32_t bar, uint32_t dst, int col, int row) {
+#pragma unroll
+  for (int c = 0; c < BM / 64; ++c) tma_load_2d_pair(tm, bar, dst + c * CHUNK_BYTES, col + 64 * c, row);
+}
+
 template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI_CODE, int GW,
           int DUAL = DUAL_NONE>
 __global__ void __launch_bounds__(threads(GW, splits_registers(EPI_CODE, DUAL)), 1)
@@ -224,7 +230,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   SharedStorage& ss = *reinterpret_cast<SharedStorage*>(smem + NSTAGES * (A_STAGE_BYTES + B_STAGE_BYTES + X_STAGE_BYTES));
   uint8_t* stage_out = reinterpret_cast<uint8_t*>(&ss) + ((sizeof(SharedStorage) + 127) & ~127);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const bool leader = rank == 0;
@@ -306,6 +312,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   // ---- TMA producer -------------------------------------------------------------------------
   if (warp == 0) {
     if constexpr (kTmaBytesPerCta > 0) {
+      const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -317,42 +324,29 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);  // the leader's barrier
           const uint32_t a_dst = smem_u32(sA + stage * A_STAGE_BYTES);
           const uint32_t b_dst = smem_u32(sB + stage * B_STAGE_BYTES);
-          if (leader && lane == 0) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
-          __syncwarp();
-          const int k0 = RAGGED_K ? (tile.k_begin + kb * BK) : kb * BK;
-          if constexpr (!A_GATHER) {
-            if constexpr (!A_MN) {
+          [[maybe_unused]] const uint32_t x_dst = smem_u32(sX + stage * X_STAGE_BYTES);
+          if (elected) {
+            if (leader) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
+            const int k0 = RAGGED_K ? (tile.k_begin + kb * BK) : kb * BK;
+            if constexpr (!A_GATHER && !A_MN) {
               // no rows at all in this CTA's half of the tile: read past the tensor's end, which delivers zeros
-              if (lane == 0)
-                tma_load_2d_pair(&tmA, bar, a_dst, k0, tile.row0 < tile.row_end ? tile.row0 : p.total_rows);
-            } else {
-              if (lane < BM / 64) tma_load_2d_pair(&tmA, bar, a_dst + lane * CHUNK_BYTES, tile.row0 + 64 * lane, k0);
+              tma_load_2d_pair(&tmA, bar, a_dst, k0, tile.row0 < tile.row_end ? tile.row0 : p.total_rows);
             }
-          }
-          if constexpr (!B_GATHER) {
-            const int nb = tile.n0 + static_cast<int>(rank) * BN_CTA;  // this CTA's half of the B rows
-            if constexpr (!B_MN) {
-              if (lane == 0) tma_load_2d_pair(&tmB, bar, b_dst, k0, tile.e * p.b_rows_per_expert + nb);
-            } else {
+            if constexpr (!A_GATHER && A_MN) load_mn_tile(&tmA, bar, a_dst, tile.row0, k0);
+            if constexpr (!B_GATHER) {
+              const int nb = tile.n0 + static_cast<int>(rank) * BN_CTA;  // this CTA's half of the B rows
               const int krow = RAGGED_K ? k0 : (tile.e * p.b_rows_per_expert + k0);
-              if (lane < BN_CTA / 64) tma_load_2d_pair(&tmB, bar, b_dst + lane * CHUNK_BYTES, nb + 64 * lane, krow);
+              if constexpr (!B_MN) tma_load_2d_pair(&tmB, bar, b_dst, k0, tile.e * p.b_rows_per_expert + nb);
+              else load_mn_tile(&tmB, bar, b_dst, nb, krow);
+              if constexpr (DUAL == DUAL_N) {  // the unit's second B tile: columns n0 + 256 ...
+                if constexpr (!B_MN) tma_load_2d_pair(&tmB, bar, x_dst, k0, tile.e * p.b_rows_per_expert + nb + BN);
+                else load_mn_tile(&tmB, bar, x_dst, nb + BN, krow);
+              }
             }
+            // the unit's second A tile: rows row0 + 256 ...
+            if constexpr (DUAL == DUAL_M) load_mn_tile(&tmA, bar, x_dst, tile.row0 + 2 * BM, k0);
           }
-          if constexpr (DUAL == DUAL_N) {  // the unit's second B tile: columns n0 + 256 ...
-            const uint32_t x_dst = smem_u32(sX + stage * X_STAGE_BYTES);
-            const int nb = tile.n0 + BN + static_cast<int>(rank) * BN_CTA;
-            if constexpr (!B_MN) {
-              if (lane == 0) tma_load_2d_pair(&tmB, bar, x_dst, k0, tile.e * p.b_rows_per_expert + nb);
-            } else {
-              const int krow = RAGGED_K ? k0 : (tile.e * p.b_rows_per_expert + k0);
-              if (lane < BN_CTA / 64) tma_load_2d_pair(&tmB, bar, x_dst + lane * CHUNK_BYTES, nb + 64 * lane, krow);
-            }
-          }
-          if constexpr (DUAL == DUAL_M) {  // the unit's second A tile: rows row0 + 256 ...
-            const uint32_t x_dst = smem_u32(sX + stage * X_STAGE_BYTES);
-            if (lane < BM / 64)
-              tma_load_2d_pair(&tmA, bar, x_dst + lane * CHUNK_BYTES, tile.row0 + 2 * BM + 64 * lane, k0);
-          }
+          __syncwarp();
           if (++stage == NSTAGES) { stage = 0; phase ^= 1u; }
         }
       }
@@ -361,7 +355,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   }
   // ---- MMA issuer (leader) / gather relay (other CTA) ----------------------------------------
   else if (warp == 1) {
-    if (leader && lane == 0) {  // one thread: nothing in this loop is warp-wide
+    if (leader && elect_one()) {  // one thread: nothing in this loop is warp-wide
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       constexpr uint32_t a_lbo = A_MN ? CHUNK_BYTES : 16;
       constexpr uint32_t b_lbo = B_MN ? CHUNK_BYTES : 16;

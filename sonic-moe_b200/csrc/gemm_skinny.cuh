@@ -135,7 +135,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int stage_size = stage_bytes(nt);
   uint8_t* stage_out = smem + stages * stage_size;
   Shared& ss = *reinterpret_cast<Shared*>(stage_out + EPI_WARPS * STAGE_ROWS_BYTES);
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   volatile int* abort_flag = &ss.abort_flag;
   const int num_kb = p.K / BK;
@@ -189,6 +189,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     // ---- TMA producer -------------------------------------------------------------------------
+    const bool elected = elect_one();
     int stage = 0;
     uint32_t phase = 0;
     while (ok && walk.next(u)) {
@@ -198,25 +199,26 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
         const uint32_t bar = smem_u32(&ss.full[stage]);
         const uint32_t dst = smem_u32(smem + stage * stage_size);
-        if (lane == 0) {
+        if (elected) {
           mbar_arrive_expect_tx(bar, bytes);
           tma_load_2d(&tmW, bar, dst, kb * BK, u.e * p.b_rows_per_expert + u.f0);
+          if constexpr (!GATHER) {
+            for (int b = 0; b < boxes; ++b)
+              tma_load_2d(&tmX, bar, dst + W_STAGE_BYTES + b * (BOX_ROWS * BK * 2), kb * BK, u.row0 + b * BOX_ROWS);
+          }
         }
         __syncwarp();
-        if constexpr (!GATHER) {
-          if (lane < boxes)
-            tma_load_2d(&tmX, bar, dst + W_STAGE_BYTES + lane * (BOX_ROWS * BK * 2), kb * BK, u.row0 + lane * BOX_ROWS);
-        }
         if (++stage == stages) { stage = 0; phase ^= 1u; }
       }
     }
     if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
   } else if (warp == 1) {
     // ---- MMA issuer ---------------------------------------------------------------------------
+    const bool elected = elect_one();
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     while (ok && walk.next(u)) {
-      if (lane == 0) {
+      if (elected) {
         const uint32_t idesc = make_idesc_bf16(BM, (u.rows + 15) & ~15, false, false);
         ok = mbar_wait(smem_u32(&ss.acc_empty[acc]), acc_phase ^ 1u, abort_flag);
         tc_fence_after();

@@ -99,7 +99,7 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   const int b_stage_bytes = p.E * BK * 2;
   const int stage_bytes = A_STAGE_BYTES + b_stage_bytes;  // E is a multiple of 32: stages stay 1024-byte aligned
   Shared& ss = *reinterpret_cast<Shared*>(smem + p.stages * stage_bytes);
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   volatile int* abort_flag = &ss.abort_flag;
   const int num_tiles = (p.T + BM - 1) / BM;
@@ -137,13 +137,14 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 
   if (warp == 0) {
     // ---- TMA producer -------------------------------------------------------------------------------------
+    const bool elected = elect_one();
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
-        if (lane == 0) {
+        if (elected) {
           const uint32_t bar = smem_u32(&ss.full[stage]);
           const uint32_t a_dst = smem_u32(smem + stage * stage_bytes);
           mbar_arrive_expect_tx(bar, stage_bytes);
@@ -157,6 +158,7 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     if (!ok && lane == 0 && p.status) atomicCAS(p.status, SMOE_ST_OK, SMOE_ST_TIMEOUT_PRODUCER);
   } else if (warp == 1) {
     // ---- MMA issuer ---------------------------------------------------------------------------------------
+    const bool elected = elect_one();
     const uint32_t idesc = make_idesc_bf16(BM, p.E, false, false);
     int stage = 0;
     uint32_t phase = 0;
@@ -170,7 +172,7 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        if (lane == 0) {
+        if (elected) {
           const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
           const uint64_t a_desc = make_smem_desc(a_addr, 16, 1024);
           const uint64_t b_desc = make_smem_desc(a_addr + A_STAGE_BYTES, 16, 1024);
@@ -184,7 +186,7 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         if (++stage == p.stages) { stage = 0; phase ^= 1u; }
       }
       if (!ok) break;
-      if (lane == 0) umma_commit(smem_u32(&ss.acc_full[acc]));
+      if (elected) umma_commit(smem_u32(&ss.acc_full[acc]));
       __syncwarp();
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
@@ -337,7 +339,7 @@ router_forward_small_kernel(const __grid_constant__ CUtensorMap tmX, const __gri
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const SmallLayout lay(p.tile_rows, p.split, p.E, p.stages);
   Shared& ss = *reinterpret_cast<Shared*>(smem + lay.shared);
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   volatile int* abort_flag = &ss.abort_flag;
   const int rank = static_cast<int>(cluster_ctarank());
@@ -372,7 +374,7 @@ router_forward_small_kernel(const __grid_constant__ CUtensorMap tmX, const __gri
 
   bool ok = true;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -387,7 +389,7 @@ router_forward_small_kernel(const __grid_constant__ CUtensorMap tmX, const __gri
       if (!ok && p.status) atomicCAS(p.status, SMOE_ST_OK, SMOE_ST_TIMEOUT_PRODUCER);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(BM, cols, false, false);
       int stage = 0;
       uint32_t phase = 0;
