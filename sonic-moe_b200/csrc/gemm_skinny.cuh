@@ -142,7 +142,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
-      mbar_init(smem_u32(&ss.full[s]), 1);
+      mbar_init(smem_u32(&ss.full[s]), 1 + (GATHER ? GATHER_WARPS : 0));
       mbar_init(smem_u32(&ss.empty[s]), 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -260,6 +260,10 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           if (mine)
             tma_gather4(&tmX, smem_u32(&ss.full[stage]), smem_u32(smem + stage * stage_size) + W_STAGE_BYTES + j * 512,
                         kb * BK, r4[0], r4[1], r4[2], r4[3]);
+          __syncwarp();
+          // A stage is not full without this warp, also where the warp has no rows: it waits by parity, and a warp that the
+          // ring could overtake twice would take an old phase for the one it waits for.
+          if (lane == 0) mbar_arrive(smem_u32(&ss.full[stage]));
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
