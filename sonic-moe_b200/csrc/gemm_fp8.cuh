@@ -243,31 +243,35 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
   } else if (warp >= FIRST_GATHER_WARP) {
     reg_dec<56>();
-    // ---- row gather with TMA gather4: 8 issuing threads per warp, 4 rows x 128 B each ----------
+    // ---- row gather with TMA gather4: one issuing thread per warp, 8 operations of 4 rows x 128 B per stage ----
     if constexpr (A_GATHER) {
-      const int gt = threadIdx.x - 32 * FIRST_GATHER_WARP;  // 0..127
-      const bool issuer = (gt & 3) == 0;
-      const int j = gt >> 2;  // 0..31
+      const int gw = warp - FIRST_GATHER_WARP;
+      const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       Tile tile;
       for (long long t = first_tile; ok && decode_tile(p, ss, t, num_n, rank, tile); t += tile_step) {
-        int r4[4];
+        const int r = tile.row0 + 32 * gw + lane;  // lane l fetches the index of the warp's row l
+        const int mine = r < tile.row_end ? p.gather[r] : p.gather_rows;  // rows that do not exist: zeros
+        int rows[32];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = tile.row0 + 4 * j + i;
-          r4[i] = (r < p.total_rows) ? p.gather[r] : 0;
+        for (int i = 0; i < 32; ++i) rows[i] = __shfl_sync(0xffffffffu, mine, i);
+        if (elected) {
+          for (int kb = 0; kb < tile.num_kb; ++kb) {
+            if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+            const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
+            const uint32_t dst = smem_u32(sA + stage * A_STAGE_BYTES) + gw * 4096;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              tma_gather4_pair(&tmA, bar, dst + q * 512, kb * BK, rows[4 * q], rows[4 * q + 1], rows[4 * q + 2],
+                               rows[4 * q + 3]);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          }
         }
-        for (int kb = 0; kb < tile.num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
-          if (issuer)
-            tma_gather4_pair(&tmA, map_to_cta(smem_u32(&ss.full[stage]), 0),
-                             smem_u32(sA + stage * A_STAGE_BYTES) + j * 512, kb * BK, r4[0], r4[1], r4[2], r4[3]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-        }
+        ok = __all_sync(0xffffffffu, ok);
       }
-      if (!ok && (gt & 31) == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
+      if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
     }
   } else {
     reg_inc<200>();

@@ -213,58 +213,53 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
       if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
     }
     // ---- MMA issuer ----------------------------------------------------------------------------
-    else if (warp == 1 && leader) {
-      const bool elected = elect_one();
-      constexpr uint32_t b_lbo = B_MN ? B_STAGE_BYTES : 16;
-      constexpr uint32_t b_kstep = B_MN ? (UMMA_K * 128) : UMMA_K;  // bytes per 32 reduction elements
-      int stage = 0;
-      uint32_t phase = 0;
-      int set = 0;
-      uint32_t set_phase = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      // the issuer only needs the number of work units and of k-blocks (a constant): no per-tile decode on its path
-      const long long total_units = static_cast<long long>(ss.m_tile_prefix[p.E]) * num_n;
-      const int num_kb = p.K / BK;
-      for (long long t = first_tile; ok && t < total_units; t += tile_step) {
-        // the epilogue warps of both CTAs have copied the previous tile out of tensor memory
-        if (!mbar_wait(smem_u32(&ss.acc_empty), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
-        acc_phase ^= 1u;
-        uint32_t tsfa = 0, tsfb = 0;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if ((kb & (KB_PER_GROUP - 1)) == 0) {
-            if (!mbar_wait(smem_u32(&ss.sf_full[set]), set_phase, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            tsfa = tmem_base + TMEM_SF_COL + set * TMEM_SF_SET_COLS;
-            tsfb = tsfa + TMEM_SFB_OFFSET;
-            if (elected) {
+    else if (warp == 1) {
+      if (leader && elect_one()) {  // one thread: nothing in this loop is warp-wide
+        constexpr uint32_t b_lbo = B_MN ? B_STAGE_BYTES : 16;
+        constexpr uint32_t b_kstep = B_MN ? (UMMA_K * 128) : UMMA_K;  // bytes per 32 reduction elements
+        int stage = 0;
+        uint32_t phase = 0;
+        int set = 0;
+        uint32_t set_phase = 0;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        // the issuer only needs the number of work units and of k-blocks (a constant): no per-tile decode on its path
+        const long long total_units = static_cast<long long>(ss.m_tile_prefix[p.E]) * num_n;
+        const int num_kb = p.K / BK;
+        for (long long t = first_tile; ok && t < total_units; t += tile_step) {
+          // the epilogue warps of both CTAs have copied the previous tile out of tensor memory
+          if (!mbar_wait(smem_u32(&ss.acc_empty), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
+          acc_phase ^= 1u;
+          uint32_t tsfa = 0, tsfb = 0;
+          for (int kb = 0; kb < num_kb; ++kb) {
+            if ((kb & (KB_PER_GROUP - 1)) == 0) {
+              if (!mbar_wait(smem_u32(&ss.sf_full[set]), set_phase, abort_flag)) { ok = false; break; }
+              tc_fence_after();
+              tsfa = tmem_base + TMEM_SF_COL + set * TMEM_SF_SET_COLS;
+              tsfb = tsfa + TMEM_SFB_OFFSET;
               const uint32_t s_sf = smem_u32(sSF + set * SF_SET_BYTES);
               tmem_cp_sf_pair(tsfa, make_sf_desc(s_sf));
               tmem_cp_sf_pair(tsfb, make_sf_desc(s_sf + SFA_BYTES));
               tmem_cp_sf_pair(tsfb + 4, make_sf_desc(s_sf + SFA_BYTES + 512));
               umma_commit_pair(smem_u32(&ss.sf_empty[set]), 3);  // the words have left shared memory
+              if (++set == SF_SETS) { set = 0; set_phase ^= 1u; }
             }
-            __syncwarp();
-            if (++set == SF_SETS) { set = 0; set_phase ^= 1u; }
-          }
-          if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          if (elected) {
+            if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
+            tc_fence_after();
             const uint32_t idesc = make_idesc_mx(2 * BM, BN, B_MN, static_cast<uint32_t>(kb & (KB_PER_GROUP - 1)));
             const uint64_t a_desc = make_smem_desc(smem_u32(sA + stage * A_STAGE_BYTES), 16, 1024);
             const uint64_t b_desc = make_smem_desc(smem_u32(sB + stage * B_STAGE_BYTES), b_lbo, 1024);
 #pragma unroll
             for (int k4 = 0; k4 < BK / UMMA_K; ++k4)
-              umma_mx_pair(tmem_base, a_desc + ((k4 * UMMA_K) >> 4), b_desc + ((k4 * b_kstep) >> 4), idesc, tsfa,
-                           tsfb, (kb > 0 || k4 > 0) ? 1u : 0u);
+              umma_mx_pair(tmem_base, a_desc + ((k4 * UMMA_K) >> 4), b_desc + ((k4 * b_kstep) >> 4), idesc, tsfa, tsfb,
+                           (kb > 0 || k4 > 0) ? 1u : 0u);
             umma_commit_pair(smem_u32(&ss.empty[stage]), 3);
             if (kb == num_kb - 1) umma_commit_pair(smem_u32(&ss.acc_full), 3);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
-          __syncwarp();
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        if (!ok && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_MMA);
       }
-      if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_MMA);
     }
     // ---- scale-factor words of A (warp 2) and B (warp 3) ----------------------------------------
     else if (warp >= 2) {
@@ -341,31 +336,35 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     }
   } else if (warp >= FIRST_GATHER_WARP) {
     fp8::reg_dec<56>();
-    // ---- row gather with TMA gather4: 8 issuing threads per warp, 4 rows x 128 B each ----------
+    // ---- row gather with TMA gather4: one issuing thread per warp, 8 operations of 4 rows x 128 B per stage ----
     if constexpr (A_GATHER) {
-      const int gt = threadIdx.x - 32 * FIRST_GATHER_WARP;  // 0..127
-      const bool issuer = (gt & 3) == 0;
-      const int j = gt >> 2;  // 0..31
+      const int gw = warp - FIRST_GATHER_WARP;
+      const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       Tile tile;
       for (long long t = first_tile; ok && fp8::decode_tile(p, ss, t, num_n, rank, tile); t += tile_step) {
-        int r4[4];
+        const int r = tile.row0 + 32 * gw + lane;  // lane l fetches the index of the warp's row l
+        const int mine = r < tile.row_end ? p.gather[r] : p.gather_rows;  // rows that do not exist: zeros
+        int rows[32];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = tile.row0 + 4 * j + i;
-          r4[i] = (r < p.total_rows) ? p.gather[r] : 0;
+        for (int i = 0; i < 32; ++i) rows[i] = __shfl_sync(0xffffffffu, mine, i);
+        if (elected) {
+          for (int kb = 0; kb < tile.num_kb; ++kb) {
+            if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+            const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
+            const uint32_t dst = smem_u32(sA + stage * A_STAGE_BYTES) + gw * 4096;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              tma_gather4_pair(&tmA, bar, dst + q * 512, kb * BK, rows[4 * q], rows[4 * q + 1], rows[4 * q + 2],
+                               rows[4 * q + 3]);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          }
         }
-        for (int kb = 0; kb < tile.num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
-          if (issuer)
-            tma_gather4_pair(&tmA, map_to_cta(smem_u32(&ss.full[stage]), 0),
-                             smem_u32(sA + stage * A_STAGE_BYTES) + j * 512, kb * BK, r4[0], r4[1], r4[2], r4[3]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-        }
+        ok = __all_sync(0xffffffffu, ok);
       }
-      if (!ok && (gt & 31) == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
+      if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
     }
   } else {
     fp8::reg_inc<200>();
@@ -542,10 +541,12 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     const uint64_t t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
+  // barriers that the lanes of a warp may reach one by one: the MMA role is one lane's
   tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();
+  block_sync_diverged();
+  cluster_sync_diverged();
   if (warp == 1) {
+    __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }

@@ -15,8 +15,8 @@
 //            on the leader CTA's "full" barrier)
 //   1        leader CTA: MMA issuer.  other CTA: idle
 //   2..      8 epilogue warps (each 32 rows x 128 columns)
-//   10..     GW gather warps (0, 4 or 8): the routed rows of the gathered operand by TMA tile::gather4, issued
-//            from 32 threads spread over these warps (gather4 operations issued by one warp are serialised)
+//   10..     GW gather warps (0, 4 or 8): the routed rows of the gathered operand by TMA tile::gather4, issued by one
+//            thread of each
 //
 // Barriers.  full[s]: leader only; one arrival (the leader's expect_tx), tx = TMA bytes of both CTAs,
 // gathered rows included.  empty[s], acc_full[a]: per CTA, signalled by the leader's multicast
@@ -240,7 +240,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   static_assert(!(A_GATHER && B_GATHER), "at most one operand is gathered");
   static_assert(!kGather || GW > 0, "a gathered operand needs gather warps");
   static_assert(GW == 0 || GW == 4 || GW == 8, "0, 4 or 8 gather warps");
-  constexpr int GATHER_THREADS = 32 * GW;
   constexpr bool SPLIT_REGS = splits_registers(EPI, DUAL);
   constexpr int FIRST_EPI_WARP = SPLIT_REGS ? 4 : 2;
   constexpr int FIRST_GATHER_WARP = FIRST_EPI_WARP + EPI_WARPS;
@@ -431,67 +430,78 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   else if (warp >= FIRST_GATHER_WARP) {
     if constexpr (SPLIT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if constexpr (kGather) {
-      const int gt = threadIdx.x - 32 * FIRST_GATHER_WARP;
+      // One thread of each gather warp issues its share of a stage's 32 gather4 operations (4 rows x 128 B each).  With eight
+      // issuing threads a warp the compiler's loop over active lanes (elect_one) took about 75 cycles an operation, which
+      // with eight of them a stage is more than the 512 cycles of a single tile's MMAs: caller's pairs of 65536 tokens, H 2048,
+      // I 768, top-4 of 64 experts with a skewed load 7580 -> 7220 us a training step, T 24576, H 1536, I 256, E 128, K 8
+      // 2051 -> 2013, inference of 8192 tokens, H 4096, I 1024, E 128, K 8 1959 -> 1935 (alternating).
+      constexpr int OPS = 32 / GW;
+      const int gw = warp - FIRST_GATHER_WARP;
+      const bool elected = elect_one();
+      const CUtensorMap* tm = A_GATHER ? &tmA : &tmB;
+      uint8_t* stage_base = A_GATHER ? sA : sB;
+      constexpr int STAGE_BYTES = A_GATHER ? A_STAGE_BYTES : B_STAGE_BYTES;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       Tile tile;
-      {
-        // 32 issuing threads (every GATHER_THREADS/32-th thread, so they spread over all gather warps), each
-        // fetching 4 rows x 128 B per stage with one gather4.
-        constexpr int STRIDE = GATHER_THREADS / 32;
-        const bool issuer = (gt % STRIDE) == 0;
-        const int j = gt / STRIDE;  // 0..31
-        const CUtensorMap* tm = A_GATHER ? &tmA : &tmB;
-        uint8_t* stage_base = A_GATHER ? sA : sB;
-        constexpr int STAGE_BYTES = A_GATHER ? A_STAGE_BYTES : B_STAGE_BYTES;
-        UnitWalker<RAGGED_K, DUAL> walk(p, ss, lane);
-        while (ok && walk.next(rank, tile)) {
-          if constexpr (!RAGGED_K) {
-            int r4[4];
+      UnitWalker<RAGGED_K, DUAL> walk(p, ss, lane);
+      while (ok && walk.next(rank, tile)) {
+        if constexpr (!RAGGED_K) {
+          // lane l fetches the index of the warp's row l; then every lane has them all, for the whole unit
+          const int r = tile.row0 + 4 * OPS * gw + lane;
+          const int mine = lane < 4 * OPS && r < tile.row_end ? p.gather[r] : p.gather_rows;  // rows that do not exist: zeros
+          // (they cost no traffic and next to no power; multiplying other rows in their place took 2.5 % longer where a
+          // fifth of the tiles' rows do not exist, up projection of 512 rows per expert 980 -> 959 us)
+          int rows[4 * OPS];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int r = tile.row0 + 4 * j + i;
-              r4[i] = (r < tile.row_end) ? p.gather[r] : p.gather_rows;  // rows that do not exist: zeros
-              // (they cost no traffic and next to no power; multiplying other rows in their place took 2.5 % longer where a
-              // fifth of the tiles' rows do not exist, up projection of 512 rows per expert 980 -> 959 us)
-            }
+          for (int i = 0; i < 4 * OPS; ++i) rows[i] = __shfl_sync(0xffffffffu, mine, i);
+          if (elected) {
             for (int kb = 0; kb < tile.num_kb; ++kb) {
-              if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
-              if (issuer)
-                tma_gather4_pair(tm, map_to_cta(smem_u32(&ss.full[stage]), 0),
-                                 smem_u32(stage_base + stage * STAGE_BYTES) + j * 512, kb * BK, r4[0], r4[1], r4[2],
-                                 r4[3]);
-              if (++stage == NSTAGES) { stage = 0; phase ^= 1u; }
-            }
-          } else {
-            const int chunk = j >> 4, tq = j & 15;  // 2 chunks of 64 columns, 16 groups of 4 tokens
-            const int col0 = (A_GATHER ? tile.row0 : tile.n0 + static_cast<int>(rank) * BN_CTA) + 64 * chunk;
-            int cur[4], nxt[4];
-            auto load_idx = [&](int kb, int (&dst_idx)[4]) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int tok = tile.k_begin + kb * BK + 4 * tq + i;
-                dst_idx[i] = (kb < tile.num_kb && tok < tile.k_end) ? p.gather[tok] : p.gather_rows;  // out of range: zeros
-              }
-            };
-            load_idx(0, cur);
-            load_idx(1, nxt);
-            for (int kb = 0; kb < tile.num_kb; ++kb) {  // (nothing here is warp-wide)
               if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
-              if (issuer)
-                tma_gather4_pair(tm, map_to_cta(smem_u32(&ss.full[stage]), 0),
-                                 smem_u32(stage_base + stage * STAGE_BYTES) + chunk * CHUNK_BYTES + tq * 512, col0,
-                                 cur[0], cur[1], cur[2], cur[3]);
+              const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
+              const uint32_t dst = smem_u32(stage_base + stage * STAGE_BYTES) + gw * OPS * 512;
 #pragma unroll
-              for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
-              load_idx(kb + 2, nxt);
+              for (int q = 0; q < OPS; ++q)
+                tma_gather4_pair(tm, bar, dst + q * 512, kb * BK, rows[4 * q], rows[4 * q + 1], rows[4 * q + 2],
+                                 rows[4 * q + 3]);
               if (++stage == NSTAGES) { stage = 0; phase ^= 1u; }
             }
           }
+          ok = __all_sync(0xffffffffu, ok);
+        } else {
+          // 2 chunks of 64 columns x 16 groups of 4 tokens; a warp has OPS / 2 groups of both chunks.  Lane l fetches the
+          // index of its warp's token l, two k-blocks ahead.
+          constexpr int TOKENS = 2 * OPS;
+          const int col0 = A_GATHER ? tile.row0 : tile.n0 + static_cast<int>(rank) * BN_CTA;
+          const auto load_idx = [&](int kb) {
+            const int tok = tile.k_begin + kb * BK + TOKENS * gw + lane;
+            return lane < TOKENS && kb < tile.num_kb && tok < tile.k_end ? p.gather[tok] : p.gather_rows;  // beyond: zeros
+          };
+          int cur = load_idx(0), nxt = load_idx(1);
+          for (int kb = 0; kb < tile.num_kb; ++kb) {
+            if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+            int tokens[TOKENS];
+#pragma unroll
+            for (int i = 0; i < TOKENS; ++i) tokens[i] = __shfl_sync(0xffffffffu, cur, i);
+            if (elected) {
+              const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
+              const uint32_t dst = smem_u32(stage_base + stage * STAGE_BYTES) + gw * (OPS / 2) * 512;
+#pragma unroll
+              for (int q = 0; q < OPS; ++q) {
+                const int g = q % (OPS / 2), chunk = q / (OPS / 2);
+                tma_gather4_pair(tm, bar, dst + chunk * CHUNK_BYTES + g * 512, col0 + 64 * chunk, tokens[4 * g],
+                                 tokens[4 * g + 1], tokens[4 * g + 2], tokens[4 * g + 3]);
+              }
+            }
+            __syncwarp();
+            cur = nxt;
+            nxt = load_idx(kb + 2);
+            if (++stage == NSTAGES) { stage = 0; phase ^= 1u; }
+          }
         }
       }
-      if (!ok && (gt & 31) == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
+      if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
     }
   }
   // ---- epilogue -----------------------------------------------------------------------------
