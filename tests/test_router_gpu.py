@@ -182,6 +182,15 @@ def test_router_forward_small_tiles(built_library, T, H, E, K):
     test_router_forward(built_library, T, H, E, K)
 
 
+@pytest.mark.parametrize("T,H,E,K", [
+    (9600, 64, 32, 1), (9601, 128, 96, 6),          # one tile per CTA at most
+    (18945, 64, 160, 16), (40000, 192, 224, 3), (60001, 64, 256, 16),  # up to four, the last one ragged
+])
+def test_router_forward_large_tiles(built_library, T, H, E, K):
+    """The large form with every width of a lane's row of logits and several tiles per CTA."""
+    test_router_forward(built_library, T, H, E, K)
+
+
 @pytest.mark.parametrize("T,E,fused", [(1, 64, True), (1000, 64, True), (6000, 256, True), (0, 32, True),
                                        (1, 8, False), (777, 8, False), (3001, 40, False), (500, 256, False), (0, 8, False)])
 def test_switch_loss(built_library, T, E, fused):
