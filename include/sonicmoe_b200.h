@@ -394,6 +394,32 @@ int smoe_layer_forward(const void* x, const void* router_w, const void* w1, cons
                        int* expert_count, float* prob_colsum, float* aux, void* scratch, int T, int H, int I, int E,
                        int K, int* status, void* stream);
 
+/* A training pass of the layer (top-K routing, any activation, biases optional) in four calls, with the launches and the
+ * requirements of the entry points above; T > 0.  I: columns of the down projection, N1: rows of the up projection (I, or 2 I
+ * where the activation is gated).
+ * meta: smoe_layer_meta_words(T, E, K) 4-byte words that the forward call writes and the backward calls read.
+ * Forward: with router_w (bf16, where smoe_router_forward_supported) logits, prob_colsum and aux are outputs; without it
+ * logits (T,E) of logits_dtype are an input.  z (T K, N1) may be null where no backward pass follows.
+ * Backward, in this order: _act (dz, y1 s and the scores' gradient into scratch; db1, db2 with b2; dlogits, if not null, from
+ * the scores' gradient and, with fused_router, from g_logits, g_colsum and g_aux, each optional; dout may be null where only
+ * those are given), then _dx (dx = or, with add, += the experts' part; dx_expanded (T K, H) scratch, not needed if K == 1) and
+ * _weights in any order.  scratch: smoe_layer_backward_scratch_bytes, kept between the backward calls. */
+size_t smoe_layer_meta_words(int T, int E, int K);
+size_t smoe_layer_train_forward_scratch_bytes(int T, int H, int I, int E, int K);
+int smoe_layer_train_forward(const void* x, const void* router_w, void* logits, int logits_dtype, const void* w1,
+                             const void* b1, const void* w2, const void* b2, void* o, void* z, void* meta,
+                             int* expert_count, float* prob_colsum, float* aux, void* scratch, int T, int H, int I, int N1,
+                             int E, int K, int activation, int* status, void* stream);
+size_t smoe_layer_backward_scratch_bytes(int T, int I, int N1, int K);
+int smoe_layer_backward_act(const void* dout, const void* w2, const void* b2, const void* z, void* meta,
+                            const void* logits, int logits_dtype, int fused_router, const void* g_logits,
+                            const float* g_colsum, const float* g_aux, void* dlogits, void* db1, void* db2, void* scratch,
+                            int T, int H, int I, int N1, int E, int K, int activation, int* status, void* stream);
+int smoe_layer_backward_dx(const void* w1, void* meta, const void* scratch, void* dx_expanded, void* dx, int add, int T,
+                           int H, int I, int N1, int E, int K, int* status, void* stream);
+int smoe_layer_backward_weights(const void* x, const void* dout, void* meta, const void* scratch, void* dw1, void* dw2,
+                                int T, int H, int I, int N1, int E, int K, int* status, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Expert parallelism over peer memory (one node, NVLink / NVSwitch).  The reference has no distributed
  * code (sonicmoe/moe.py:260 skips even the aux-loss reduction), so these have no counterpart there; they

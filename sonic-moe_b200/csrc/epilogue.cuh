@@ -52,7 +52,8 @@ struct GemmParams {
   float* acc_out;           // EPI_SCATTER: (gather_rows, N) fp32
   int* status;              // device word, 0 = ok
   int accumulate;           // plain-store epilogues: add to what out0 holds (bf16, fp32 sum, one rounding) instead of
-                            // overwriting it -- weight gradients summed over several chunks of tokens
+                            // overwriting it -- weight gradients summed over several chunks of tokens, rows of dx that
+                            // hold the router's part already
   int min_rows;             // ragged-M tiles: experts with at most this many rows are left to another launch
   int max_rows;             // kernel for experts with few rows: those with more are left to another launch
   // general epilogues
@@ -571,7 +572,7 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, int expert, uin
 #pragma unroll
     for (int j = 0; j < 16; ++j) w[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
     if constexpr (EPI == EPI_STORE_ROWS) {
-      warp_store_segments64(stage, lane, w, false, [&](int rr) {
+      warp_store_segments64(stage, lane, w, p.accumulate, [&](int rr) {
         const int row = __shfl_sync(0xffffffffu, dst_row, rr);
         return row_base + rr < row_end ? p.out0 + row * p.ld0 + n : nullptr;
       });

@@ -1,6 +1,7 @@
 // Host side of the grouped GEMMs: tensor-map construction and the C-ABI launchers.
 #include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
+#include "internal.h"
 
 #include <cstdlib>
 #include <mutex>
@@ -395,9 +396,8 @@ int smoe_up_projection_backward_dx(const void* dz, const void* w1, void* dx_expa
   return launch<false, false, false, false, true, EPI_STORE>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
 }
 
-int smoe_up_projection_backward_dx_rows(const void* dz, const void* w1, void* dx, const int* expert_offset,
-                                        const int* x_gather_idx, int H, int I, int E, int TK, int* status,
-                                        void* stream) {
+static int backward_dx_rows(const void* dz, const void* w1, void* dx, const int* expert_offset, const int* x_gather_idx,
+                            int H, int I, int E, int TK, int* status, void* stream, int accumulate) {
   if (bad_shape(H, I, E) || TK < 0) return SMOE_ERR_SHAPE;
   if (TK == 0) return SMOE_OK;
   if (x_gather_idx == nullptr) return SMOE_ERR_SHAPE;
@@ -408,8 +408,14 @@ int smoe_up_projection_backward_dx_rows(const void* dz, const void* w1, void* dx
   p.E = E; p.N = H; p.K = 2 * I; p.total_rows = TK; p.b_rows_per_expert = 2 * I;
   p.off = expert_offset; p.gather = x_gather_idx;
   p.out0 = static_cast<__nv_bfloat16*>(dx); p.ld0 = H;
-  p.status = status;
+  p.status = status; p.accumulate = accumulate;
   return launch<false, false, false, false, true, EPI_STORE_ROWS>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
+}
+
+int smoe_up_projection_backward_dx_rows(const void* dz, const void* w1, void* dx, const int* expert_offset,
+                                        const int* x_gather_idx, int H, int I, int E, int TK, int* status,
+                                        void* stream) {
+  return backward_dx_rows(dz, w1, dx, expert_offset, x_gather_idx, H, I, E, TK, status, stream, 0);
 }
 
 static int down_weight_grad(const void* dout, const void* y1s, void* dw2, const int* expert_offset,
@@ -476,3 +482,9 @@ int smoe_up_projection_weight_grad_accumulate(const void* x, const void* dz, voi
 }
 
 }  // extern "C"
+
+int smoe::up_projection_backward_dx_rows_add(const void* dz, const void* w1, void* dx, const int* expert_offset,
+                                             const int* x_gather_idx, int H, int I, int E, int TK, int* status,
+                                             void* stream) {
+  return backward_dx_rows(dz, w1, dx, expert_offset, x_gather_idx, H, I, E, TK, status, stream, 1);
+}

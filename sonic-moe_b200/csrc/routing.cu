@@ -10,6 +10,7 @@
 #include <mutex>
 
 #include "../../include/sonicmoe_b200.h"
+#include "internal.h"
 #include "launch.cuh"
 
 namespace smoe {
@@ -350,12 +351,11 @@ __global__ void sorted_offsets_kernel(const int* sorted_idx, long long n, int T,
 // gather-and-sum over each token's routed rows
 // ----------------------------------------------------------------------------------------------
 // out[t, :] = sum_{p in [tok_off[t], tok_off[t+1])} w[p] * src[rev[p], :]   (w == nullptr: plain sum)
-// tok_off == nullptr means a fixed K rows per token: p in [t*K, (t+1)*K).
+// tok_off == nullptr means a fixed K rows per token: p in [t*K, (t+1)*K).  ADD: out[t, :] += instead.
 // One thread per 8 consecutive columns of one token, fp32 accumulation.
-template <typename W, bool ADD_FP32>
+template <typename W, bool ADD>
 __global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* src, __nv_bfloat16* out, const W* w,
-                                                         const int* rev, const int* tok_off, const float* add, int T,
-                                                         int H, int K) {
+                                                         const int* rev, const int* tok_off, int T, int H, int K) {
   release_next();
   wait_for_previous();
   const int vec_per_row = H >> 3;
@@ -368,11 +368,16 @@ __global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* sr
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  if constexpr (ADD_FP32) {
-    const float4 a0 = reinterpret_cast<const float4*>(add + static_cast<long long>(t) * H)[2 * c];
-    const float4 a1 = reinterpret_cast<const float4*>(add + static_cast<long long>(t) * H)[2 * c + 1];
-    acc[0] = a0.x; acc[1] = a0.y; acc[2] = a0.z; acc[3] = a0.w;
-    acc[4] = a1.x; acc[5] = a1.y; acc[6] = a1.z; acc[7] = a1.w;
+  uint4* dst = reinterpret_cast<uint4*>(out + static_cast<long long>(t) * H) + c;
+  if constexpr (ADD) {
+    const uint4 v = *dst;
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(h[j]);
+      acc[2 * j] = f.x;
+      acc[2 * j + 1] = f.y;
+    }
   }
 #pragma unroll 4
   for (int p = p0; p < p1; ++p) {
@@ -391,7 +396,7 @@ __global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* sr
   __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
   for (int j = 0; j < 4; ++j) oh[j] = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-  reinterpret_cast<uint4*>(out + static_cast<long long>(t) * H)[c] = o;
+  *dst = o;
 }
 
 // fp32 (T,H) -> bf16 (T,H)
@@ -527,6 +532,17 @@ __global__ void __launch_bounds__(256) ds_bias_term_kernel(const __nv_bfloat16* 
     const int slot = s_scatter[r];
     ds[slot] = static_cast<DsT>(static_cast<float>(ds[slot]) + acc);
   }
+}
+
+int gather_sum_add(const void* src, void* out, const float* weights, const int* reverse_idx, int T, int H, int K,
+                   void* stream) {
+  if (T < 0 || H <= 0 || (H % 8) != 0 || K <= 0) return SMOE_ERR_SHAPE;
+  if (T == 0) return SMOE_OK;
+  const long long total = static_cast<long long>(T) * (H / 8);
+  const unsigned grid = static_cast<unsigned>((total + 255) / 256);
+  return launched(launch_chained(gather_sum_kernel<float, true>, grid, 256, 0, S(stream), 1,
+                                 static_cast<const __nv_bfloat16*>(src), static_cast<__nv_bfloat16*>(out), weights,
+                                 reverse_idx, nullptr, T, H, K));
 }
 
 static int sort_blocks(long long n) {
@@ -684,10 +700,10 @@ int smoe_gather_sum(const void* src, void* out, const void* weights, int weights
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   if (weights == nullptr || weights_dtype == SMOE_F32) {
     launch_chained(gather_sum_kernel<float, false>, grid, 256, 0, S(stream), 1, s, o,
-                   static_cast<const float*>(weights), reverse_idx, token_offset, nullptr, T, H, K);
+                   static_cast<const float*>(weights), reverse_idx, token_offset, T, H, K);
   } else if (weights_dtype == SMOE_BF16) {
     launch_chained(gather_sum_kernel<__nv_bfloat16, false>, grid, 256, 0, S(stream), 1, s, o,
-                   static_cast<const __nv_bfloat16*>(weights), reverse_idx, token_offset, nullptr, T, H, K);
+                   static_cast<const __nv_bfloat16*>(weights), reverse_idx, token_offset, T, H, K);
   } else {
     return SMOE_ERR_DTYPE;
   }

@@ -6,6 +6,7 @@ fails loudly, there is no eager / CPU substitute.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from ctypes import c_int, c_longlong, c_size_t, c_uint, c_void_p
@@ -91,6 +92,13 @@ SIGNATURES: dict[str, tuple] = {
     "smoe_switch_loss": (I, [P, P, P, P, P, I, I, P]),
     "smoe_layer_forward_scratch_bytes": (c_size_t, [I, I, I, I, I]),
     "smoe_layer_forward": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P]),
+    "smoe_layer_meta_words": (c_size_t, [I, I, I]),
+    "smoe_layer_train_forward_scratch_bytes": (c_size_t, [I, I, I, I, I]),
+    "smoe_layer_train_forward": (I, [P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P]),
+    "smoe_layer_backward_scratch_bytes": (c_size_t, [I, I, I, I]),
+    "smoe_layer_backward_act": (I, [P, P, P, P, P, P, I, I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P]),
+    "smoe_layer_backward_dx": (I, [P, P, P, P, P, I, I, I, I, I, I, I, P, P]),
+    "smoe_layer_backward_weights": (I, [P, P, P, P, P, P, I, I, I, I, I, I, P, P]),
     "smoe_peer_alloc": (I, [c_size_t, P]),
     "smoe_peer_free": (I, [P]),
     "smoe_peer_export": (I, [P, P]),
@@ -144,12 +152,23 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
+_HERE_ALREADY = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """`torch.cuda.device(device)`, or nothing where it is the current device."""
+    return _HERE_ALREADY if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+_DTYPE_CODES = {torch.float32: SMOE_F32, torch.bfloat16: SMOE_BF16, torch.int32: SMOE_I32, torch.int64: SMOE_I64}
 
 
 def dtype_code(dt: torch.dtype) -> int:
     try:
-        return {torch.float32: SMOE_F32, torch.bfloat16: SMOE_BF16, torch.int32: SMOE_I32, torch.int64: SMOE_I64}[dt]
+        return _DTYPE_CODES[dt]
     except KeyError:
         raise TypeError(f"unsupported dtype {dt}") from None
 

@@ -398,7 +398,8 @@ _ACT_CODE = {ActivationType.SWIGLU: 0, ActivationType.GEGLU: 1, ActivationType.R
              ActivationType.RELU: 4, ActivationType.GELU: 5, ActivationType.SILU: 6}
 
 
-def _check_experts_args(x, w1, w2, b1, b2, activation_type):
+def _check_experts_args(x, w1, w2, b1, b2, activation_type, expert_major=False):
+    """w1 (N1,H,E) and w2 (H,I,E), or (E,N1,H) and (E,H,I)."""
     if (b1 is None) != (b2 is None):
         raise AssertionError("b1 and b2 has to be None or not None at the same time!")
     if isinstance(activation_type, str):
@@ -410,11 +411,13 @@ def _check_experts_args(x, w1, w2, b1, b2, activation_type):
         raise TypeError("the sm_100a kernels take bf16 activations and weights "
                         f"(got x {x.dtype}, w1 {w1.dtype}, w2 {w2.dtype})")
     H = x.shape[1]
-    n1 = w1.shape[0]
-    gated = is_glu(activation_type)
-    if w1.shape[1] != H or w2.shape[0] != H or w2.shape[1] * (2 if gated else 1) != n1 or w1.shape[2] != w2.shape[2]:
+    if expert_major:
+        (e1, n1, h1), (e2, h2, I) = w1.shape, w2.shape
+    else:
+        (n1, h1, e1), (h2, I, e2) = w1.shape, w2.shape
+    if h1 != H or h2 != H or I * (2 if is_glu(activation_type) else 1) != n1 or e1 != e2:
         raise ValueError(f"inconsistent shapes: x {tuple(x.shape)}, w1 {tuple(w1.shape)}, w2 {tuple(w2.shape)}")
-    if H % 64 != 0 or w2.shape[1] % 64 != 0:
+    if H % 64 != 0 or I % 64 != 0:
         raise ValueError("hidden size and intermediate size must be multiples of 64")
     if (b1 is not None or activation_type != ActivationType.SWIGLU) and n1 % 128 != 0:
         raise ValueError("with a bias or a non-SwiGLU activation the up projection needs a multiple of 128 output rows")
@@ -423,9 +426,9 @@ def _check_experts_args(x, w1, w2, b1, b2, activation_type):
     return activation_type
 
 
-def _check_router_args(x, router_w, w1):
+def _check_router_args(x, router_w, w1, expert_major=False):
     """The kernels take the number of experts from the router and read that many experts' weights."""
-    if router_w.shape != (w1.shape[2], x.shape[1]):
+    if router_w.shape != (w1.shape[0 if expert_major else 2], x.shape[1]):
         raise ValueError(f"inconsistent shapes: x {tuple(x.shape)}, router {tuple(router_w.shape)}, w1 {tuple(w1.shape)}")
 
 
@@ -692,7 +695,9 @@ def moe_TC_softmax_topk_layer_with_router_stats(x, router_w, w1, b1, w2, b2, K, 
                                                 is_inference_mode_enabled=False):
     """`moe_TC_softmax_topk_layer` plus a fourth result: the column sums (E,) fp32 of softmax(router_logits) when the
     fused routing kernel produced them (what the load-balancing loss needs), else None."""
-    return _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inference_mode_enabled)[:4]
+    _check_router_args(x, router_w, w1)
+    return _layer_with_aux(x, router_w, w1.permute(2, 0, 1), b1, w2.permute(2, 0, 1), b2, K, activation_type,
+                           is_inference_mode_enabled)[:4]
 
 
 def _layer_forward(x, router_w, w1, w2, K):
@@ -700,11 +705,9 @@ def _layer_forward(x, router_w, w1, w2, K):
     one call of the library, one piece of scratch."""
     dev = x.device
     T, H = x.shape
-    E = router_w.shape[0]
-    x, router_w = x.contiguous(), router_w.contiguous()
-    w1e, w2e = _expert_major(w1), _expert_major(w2)
-    I = w2e.shape[2]
-    with torch.cuda.device(dev):
+    E, _, I = w2.shape
+    x, router_w, w1, w2 = x.contiguous(), router_w.contiguous(), w1.contiguous(), w2.contiguous()
+    with _lib.on_device(dev):
         o = torch.empty_like(x)
         logits = torch.empty(T, E, dtype=torch.bfloat16, device=dev)
         freq = torch.empty(E, dtype=torch.int32, device=dev)
@@ -712,40 +715,154 @@ def _layer_forward(x, router_w, w1, w2, K):
         aux = torch.empty((), dtype=torch.float32, device=dev)
         scratch = _lib.workspace(lib.smoe_layer_forward_scratch_bytes(T, H, I, E, K), dev)
         check(lib.smoe_layer_forward(
-            x.data_ptr(), router_w.data_ptr(), w1e.data_ptr(), w2e.data_ptr(), o.data_ptr(), logits.data_ptr(),
+            x.data_ptr(), router_w.data_ptr(), w1.data_ptr(), w2.data_ptr(), o.data_ptr(), logits.data_ptr(),
             freq.data_ptr(), colsum.data_ptr(), aux.data_ptr(), scratch.data_ptr(), T, H, I, E, K,
             _lib.device_state(dev).status.data_ptr(), stream_ptr(dev)), "layer_forward")
     return o, logits, freq, colsum, aux
 
 
+class _Layer(torch.autograd.Function):
+    """The whole layer as one node: router (or the top-K of given logits), routing metadata and routed experts, with four
+    calls of the library in a training step where the separate functions make 17 in four nodes.
+
+    Either router_w (the fused router) or logits_in (T,E) is given; training: a backward pass may follow.  Results: o (T,H), expert_frequency (E,) int32, and with
+    router_w the logits, the column sums of their softmax and the load-balancing loss (else None).  The router's part of the
+    gradient of x comes from a library GEMM, the experts' part is added to it by the kernel that adds up each token's rows.
+    Same kernels, results and saved activations as `_FusedRouter` / `topk_softmax` and `_RoutedExperts(General)`."""
+
+    @staticmethod
+    def forward(ctx, x, router_w, logits_in, w1, b1, w2, b2, K: int, act: int, training: bool):
+        dev = x.device
+        x, w1, w2 = x.contiguous(), w1.contiguous(), w2.contiguous()
+        b1 = None if b1 is None else b1.contiguous()
+        b2 = None if b2 is None else b2.contiguous()
+        T, H = x.shape
+        E, n1, _ = w1.shape
+        I = w2.shape[2]
+        with _lib.on_device(dev):
+            if router_w is not None:
+                router_w = router_w.contiguous()
+                logits = torch.empty(T, E, dtype=torch.bfloat16, device=dev)
+                colsum = torch.empty(E, dtype=torch.float32, device=dev)
+                aux = torch.empty((), dtype=torch.float32, device=dev)
+            else:
+                logits = logits_in.contiguous()
+                colsum = aux = None
+            o = torch.empty_like(x)
+            z = torch.empty(T * K, n1, dtype=x.dtype, device=dev) if training else None
+            freq = torch.empty(E, dtype=torch.int32, device=dev)
+            meta = torch.empty(lib.smoe_layer_meta_words(T, E, K), dtype=torch.int32, device=dev)
+            scratch = _lib.workspace(lib.smoe_layer_train_forward_scratch_bytes(T, H, I, E, K), dev)
+            check(lib.smoe_layer_train_forward(
+                x.data_ptr(), ptr(router_w), logits.data_ptr(), _lib.dtype_code(logits.dtype), w1.data_ptr(), ptr(b1),
+                w2.data_ptr(), ptr(b2), o.data_ptr(), ptr(z), meta.data_ptr(), freq.data_ptr(), ptr(colsum), ptr(aux),
+                scratch.data_ptr(), T, H, I, n1, E, K, act, _lib.device_state(dev).status.data_ptr(), stream_ptr(dev)),
+                "layer_train_forward")
+        if training:
+            fused = router_w is not None
+            ctx.save_for_backward(x, w1, w2, b2, z, meta, router_w, logits if fused else None)
+            ctx.layer = (T, H, I, n1, E, K, act, fused, logits.dtype)
+            ctx.mark_non_differentiable(freq)
+            ctx.set_materialize_grads(False)
+        return o, freq, (logits if router_w is not None else None), colsum, aux
+
+    @staticmethod
+    def backward(ctx, dout, _freq, g_logits, g_colsum, g_aux):
+        x, w1, w2, b2, z, meta, router_w, logits = ctx.saved_tensors
+        T, H, I, n1, E, K, act, fused, logits_dtype = ctx.layer
+        need_x, need_router, need_logits, need_w1, _, need_w2 = ctx.needs_input_grad[:6]
+        if dout is None and (not fused or (g_logits is None and g_colsum is None and g_aux is None)):
+            return (None,) * 10
+        dev = x.device
+        if dout is not None:
+            dout = dout.contiguous().to(x.dtype)
+        if g_logits is not None:
+            g_logits = g_logits.contiguous().to(torch.bfloat16)
+        if g_colsum is not None:
+            g_colsum = g_colsum.contiguous().float()
+        if g_aux is not None:
+            g_aux = g_aux.float()
+        dx = dw1 = dw2 = db1 = db2 = dlogits = d_router = None
+        with _lib.on_device(dev):
+            stream = stream_ptr(dev)
+            status = _lib.device_state(dev).status.data_ptr()
+            scratch = None
+            if dout is not None:
+                scratch = _lib.workspace(lib.smoe_layer_backward_scratch_bytes(T, I, n1, K), dev)
+                if b2 is not None:
+                    db1 = torch.empty(E, n1, dtype=x.dtype, device=dev)
+                    db2 = torch.empty(E, H, dtype=x.dtype, device=dev)
+            if need_logits or (fused and (need_x or need_router)):
+                dlogits = torch.empty(T, E, dtype=logits_dtype, device=dev)
+            check(lib.smoe_layer_backward_act(
+                ptr(dout), w2.data_ptr(), ptr(b2), z.data_ptr(), meta.data_ptr(), ptr(logits),
+                _lib.dtype_code(logits_dtype), fused, ptr(g_logits), ptr(g_colsum), ptr(g_aux), ptr(dlogits), ptr(db1),
+                ptr(db2), ptr(scratch), T, H, I, n1, E, K, act, status, stream), "layer_backward_act")
+            if fused:
+                if need_x:
+                    dx = dlogits @ router_w
+                if need_router:
+                    d_router = dlogits.t() @ x
+            if dout is not None:
+                # dX before the weight gradients, so that its rows are given back before those are allocated
+                if need_x:
+                    add = dx is not None
+                    if not add:
+                        dx = torch.empty(T, H, dtype=x.dtype, device=dev)
+                    rows = torch.empty(T * K, H, dtype=x.dtype, device=dev) if K > 1 else None
+                    check(lib.smoe_layer_backward_dx(w1.data_ptr(), meta.data_ptr(), scratch.data_ptr(), ptr(rows),
+                                                     dx.data_ptr(), add, T, H, I, n1, E, K, status, stream),
+                          "layer_backward_dx")
+                    del rows
+                if need_w1 or need_w2:
+                    dw1, dw2 = torch.empty_like(w1), torch.empty_like(w2)
+                    check(lib.smoe_layer_backward_weights(
+                        x.data_ptr(), dout.data_ptr(), meta.data_ptr(), scratch.data_ptr(), dw1.data_ptr(),
+                        dw2.data_ptr(), T, H, I, n1, E, K, status, stream), "layer_backward_weights")
+        return dx, d_router, (None if fused else dlogits), dw1, db1, dw2, db2, None, None, None
+
+
 def _layer_with_aux(x, router_w, w1, b1, w2, b2, K, activation_type, is_inference_mode_enabled):
-    """(o, router_logits, expert_frequency, column sums of softmax(router_logits), load-balancing loss); the last two
-    are None where the fused routing kernel does not apply."""
-    _check_router_args(x, router_w, w1)
-    activation_type = _check_experts_args(x, w1, w2, b1, b2, activation_type)
+    """(o, router_logits, expert_frequency, column sums of softmax(router_logits), load-balancing loss) with w1 (E,N1,H) and
+    w2 (E,H,I); the last two are None where the fused routing kernel does not apply."""
+    _check_router_args(x, router_w, w1, expert_major=True)
+    activation_type = _check_experts_args(x, w1, w2, b1, b2, activation_type, expert_major=True)
     E = router_w.size(0)
     T = x.size(0)
-    inference = is_inference_mode_enabled or not torch.is_grad_enabled()
+    grad = torch.is_grad_enabled()
+    inference = is_inference_mode_enabled or not grad
     fused = fused_router_applies(x, router_w, K)
-    if (fused and T > 0 and b1 is None and activation_type == ActivationType.SWIGLU and not _FUSED_COMBINE
-            and not (torch.is_grad_enabled() and any(t.requires_grad for t in (x, router_w, w1, w2)))
-            and not torch.jit.is_tracing() and forward_ad._current_level < 0):
+    plain = b1 is None and activation_type == ActivationType.SWIGLU
+    one_call = (T > 0 and not _FUSED_COMBINE and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+                and forward_ad._current_level < 0)
+    recorded = grad and any(t is not None and t.requires_grad for t in (x, router_w, w1, b1, w2, b2))
+    if fused and plain and one_call and not recorded:
         return _layer_forward(x, router_w, w1, w2, K)
+    if one_call and not (inference and recorded):
+        act = _ACT_CODE[activation_type]
+        if fused:
+            o, freq, router_logits, colsum, aux = _Layer.apply(x, router_w, None, w1, b1, w2, b2, K, act, recorded)
+            return o, router_logits, freq, colsum, aux
+        router_logits = F.linear(x if x.dtype == router_w.dtype else x.to(router_w.dtype), router_w)
+        if router_logits.dtype in (torch.float32, torch.bfloat16):
+            o, freq, _, _, _ = _Layer.apply(x, None, router_logits, w1, b1, w2, b2, K, act, recorded)
+            return o, router_logits, freq, None, None
     if fused:
         router_logits, scores, indices, _freq, colsum, aux = _FusedRouter.apply(x, router_w, K)
     else:
         colsum = aux = None
         # a router kept in fp32 (an extension over the reference) computes its logits in fp32
         router_logits = F.linear(x if x.dtype == router_w.dtype else x.to(router_w.dtype), router_w)
-        if torch.compiler.is_compiling() and b1 is None and activation_type == ActivationType.SWIGLU:
+        if torch.compiler.is_compiling() and plain:
             # opaque custom ops instead of autograd functions with ctypes calls inside (torch.compile, fullgraph)
             from .compiled_ops import layer_with_custom_ops
 
-            o, freq = layer_with_custom_ops(x, router_logits, w1, w2, K, E, inference)
+            o, freq = layer_with_custom_ops(x, router_logits, w1.permute(1, 2, 0), w2.permute(1, 2, 0), K, E, inference)
             return o, router_logits, freq, None, None
         scores, indices = topk_softmax(router_logits, K)
     route = _route_metadata(indices.reshape(-1), None, E, K)
-    o = _experts(x, w1, b1, w2, b2, scores.reshape(-1), route, T, inference, activation_type)
+    o = _experts(x, w1.permute(1, 2, 0), b1, w2.permute(1, 2, 0), b2, scores.reshape(-1), route, T, inference,
+                 activation_type)
     return o, router_logits, route.expert_frequency, colsum, aux
 
 

@@ -117,9 +117,9 @@ class MoE(nn.Module):
             out, router_logits, expert_frequency, _, aux_loss = _layer_with_aux(
                 hidden_states,
                 self.router.weight,
-                self.c_fc.weight.permute(1, 2, 0),
+                self.c_fc.weight,
                 self.c_fc.bias,
-                self.c_proj.weight.permute(1, 2, 0),
+                self.c_proj.weight,
                 self.c_proj.bias,
                 self.top_k,
                 self.activation_function,

@@ -484,3 +484,83 @@ def test_chained_launches_under_graph_capture(built_library, T, E, K):
     for a, b in zip(got, want):
         for s, t in zip(a, b):
             assert torch.equal(s, t)
+
+
+@pytest.mark.parametrize("T,E,K,act,bias", [
+    (1, 32, 1, "swiglu", False), (333, 64, 4, "swiglu", False), (2050, 32, 1, "swiglu", False),
+    (300, 8, 2, "swiglu", False), (257, 8, 1, "gelu", True), (700, 96, 16, "geglu", True), (130, 32, 1, "relu", False),
+])
+def test_layer_in_one_node_matches_separate_functions(built_library, T, E, K, act, bias):
+    """The layer as one autograd node against the router, the routing metadata and the experts as functions of their own: the
+    same kernels, so the same bits, except for the gradient of x with the fused router and K > 1.  There the experts' part e
+    and the router's r (rounded by its GEMM in both) are added before e is rounded instead of after: s = b(b(e) + r) against
+    t = b(e + r), which differ by u (|e| + |s| + |t|) at most, u = 2^-8 the unit roundoff of bf16 (8 significant bits; 2 % more for
+    the products of two roundings).  Strided inputs,
+    gradients of single outputs, frozen inputs and passes without gradients among them."""
+    from sonicmoe import _lib, functional as fn
+    from sonicmoe.enums import ActivationType, is_glu
+
+    H, I = 256, 128
+    kind = ActivationType(act)
+    n1 = 2 * I if is_glu(kind) else I
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+
+    def normal(*shape, std=0.05):
+        return (torch.randn(*shape, device="cuda", generator=g) * std).bfloat16()
+
+    wide = normal(T, 2 * H, std=1.0)
+    x = wide[:, ::2]                                      # strided
+    router, w1, w2 = normal(E, H), normal(n1, H, E), normal(E, H, I)  # w1 stored as the view that the layer takes
+    b1, b2 = (normal(E, n1), normal(E, H)) if bias else (None, None)
+    dout, gl = normal(T, H, std=1.0).t().contiguous().t(), normal(T, E)
+    ga = torch.full((), 0.3, device="cuda")
+
+    def separate(x, router, w1, b1, w2, b2):
+        if fn.fused_router_applies(x, router, K):
+            logits, scores, indices, _, _, aux = fn._FusedRouter.apply(x, router, K)
+        else:
+            logits = torch.nn.functional.linear(x, router)
+            scores, indices = fn.topk_softmax(logits, K)
+            aux = None
+        route = fn._route_metadata(indices.reshape(-1), None, E, K)
+        o = fn._experts(x, w1, b1, w2, b2, scores.reshape(-1), route, T, False, kind)
+        return o, logits, route.expert_frequency, aux
+
+    def one_node(x, router, w1, b1, w2, b2):
+        o, logits, freq, _, aux = fn._layer_with_aux(x, router, w1.permute(2, 0, 1), b1, w2.permute(2, 0, 1), b2, K, kind,
+                                                     False)
+        return o, logits, freq, aux
+
+    given = [x, router, w1, b1, w2.permute(1, 2, 0), b2]
+    scores, indices = fn.topk_softmax(fn.layer_router_logits(x, router, K), K)
+    xe = x.detach().requires_grad_(True)
+    oe = fn._experts(xe, *given[2:], scores.reshape(-1), fn._route_metadata(indices.reshape(-1), None, E, K), T, False, kind)
+    experts_dx, = torch.autograd.grad(oe, xe, dout)
+    for frozen in ((), (0,), (1,), (2, 4), (0, 1)):
+        results = []
+        for layer in (separate, one_node):
+            inputs = [None if t is None else t.detach().requires_grad_(i not in frozen) for i, t in enumerate(given)]
+            o, logits, freq, aux = layer(*inputs)
+            outputs = [(o, dout), (logits, gl)] + ([(aux, ga)] if aux is not None else [])
+            wanted = [t for t in inputs if t is not None and t.requires_grad]
+            grads = []
+            for chosen in (outputs, outputs[:1], outputs[1:]):
+                chosen = [c for c in chosen if c[0].requires_grad]
+                grads.append(torch.autograd.grad([c[0] for c in chosen], wanted, [c[1] for c in chosen], retain_graph=True,
+                                                 allow_unused=True) if chosen else ())
+            results.append((o, logits, freq, aux, grads, wanted))
+        torch.cuda.synchronize()
+        _lib.check_status()
+        (o, logits, freq, aux, grads, _), (o2, logits2, freq2, aux2, grads2, wanted) = results
+        assert torch.equal(o, o2) and torch.equal(logits, logits2) and torch.equal(freq, freq2)
+        assert aux is None and aux2 is None or torch.equal(aux, aux2)
+        for a, b in zip(grads, grads2):
+            for i, (s, t) in enumerate(zip(a, b)):
+                assert (s is None) == (t is None)
+                if s is not None and i == 0 and 0 not in frozen and K > 1 and aux is not None:
+                    e, s, t = experts_dx.float(), s.float(), t.float()
+                    assert ((s - t).abs() <= 1.02 * 2.0 ** -8 * (e.abs() + s.abs() + t.abs())).all()
+                elif s is not None:
+                    assert torch.equal(s, t), (frozen, i)
+    with torch.no_grad():
+        assert torch.equal(one_node(*given)[0], o)
