@@ -782,3 +782,39 @@ def test_few_rows_kernel_beside_tiles(smoe, rows, launches, hot):
     assert seen == [launches, (1, 1)]
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H", [8, 72, 64, 1040])
+@pytest.mark.parametrize("weights", [None, torch.float32, torch.bfloat16])
+def test_gather_sum_forms(smoe, H, weights):
+    """16-byte and 32-byte loads: rows that are no multiple of 32 bytes (H 8, 72), and the same rows at an address that is not
+    32-byte aligned, with a fixed and a varying number of rows per token (none among them): the same bits, and within one bf16
+    rounding (2^-8) of the sum in 64 bits, up to the rounding of its fp32 terms."""
+    lib, _lib = smoe[0].lib, smoe[0]
+    T, K = 37, 5
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rows = torch.randn(T * K, H, device="cuda", generator=g).bfloat16()
+    rev = torch.randperm(T * K, device="cuda", generator=g).int()
+    counts = torch.randint(0, 2 * K, (T,), device="cuda", generator=g)
+    counts[3] = 0
+    counts = torch.where(counts.cumsum(0) <= T * K, counts, 0)
+    varying = torch.cat([torch.zeros(1, device="cuda", dtype=torch.long), counts.cumsum(0)]).int()
+    w = None if weights is None else torch.rand(T * K, device="cuda", generator=g).to(weights)
+    room = torch.empty(T * K * H + 16, dtype=torch.bfloat16, device="cuda")
+    shifted = room[8:8 + T * K * H].view(T * K, H).copy_(rows)  # 16 bytes off
+    s = torch.cuda.current_stream().cuda_stream
+    for off in (None, varying):
+        outs = []
+        for src in (rows, shifted):
+            out = torch.full((T, H), float("nan"), dtype=torch.bfloat16, device="cuda")
+            assert lib.smoe_gather_sum(src.data_ptr(), out.data_ptr(), None if w is None else w.data_ptr(),
+                                       0 if w is None else _lib.dtype_code(w.dtype), rev.data_ptr(),
+                                       None if off is None else off.data_ptr(), T, H, K, s) == 0
+            outs.append(out)
+        assert torch.equal(*outs)
+        flat = rows[rev.long()].double() * (1.0 if w is None else w.double()[:, None])
+        bounds = (torch.arange(T + 1) * K if off is None else off.cpu()).tolist()
+        for t in range(T):
+            part = flat[bounds[t]:bounds[t + 1]]
+            slack = 2.0 ** -8 * part.sum(0).abs() + 2 * K * 2.0 ** -24 * part.abs().sum(0)
+            assert ((outs[0][t].double() - part.sum(0)).abs() <= 1.01 * slack).all()
