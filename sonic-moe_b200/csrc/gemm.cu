@@ -112,7 +112,16 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
     // warps made the single form 3 % faster since (2.59 -> 2.51 ms, alternating).  The general forward epilogue is too long
     // to be worked off from registers, and must not hold accumulators that the next unit needs.
     if constexpr (EPI != EPI_DSWIGLU && epi_base(EPI) != EPI_DACT && epi_base(EPI) != EPI_ACT) {
-    if (use_dual_tiles() && fits) {
+    // What two tiles per gathered tile save, the rest costs: their accumulators do not alternate between units, so each
+    // unit's hand-over is exposed, and there are half as many units to share out.  Both sides alternating, whole training
+    // steps (single / dual):
+    //   * up projection: reductions up to 2048 go faster as single tiles (T 24576, H 1536, I 256, E 128, K 8 1907 / 1929 us,
+    //     T 8197, H 2048, I 1024, E 64, K 1 780 / 793, T 8000, H 1536, I 512, E 64, K 4 665 / 677), longer ones do not (H 4096, I
+    //     1024, E 128, inference of 8192 tokens 1928 / 1883, step of 2080 2719 / 2701; H 3072 the same either way);
+    //   * weight gradients: their reduction is an expert's rows, and the line lies between a mean of 384 and 500 (dW1, H 1536,
+    //     I 512, E 64, K 4: 256 rows 73 / 91 us, 384 94 / 101, 500 117 / 116; 512 rows, H 4096, I 1024, E 128: 1337 / 1101).
+    const bool pays = RAGGED_K ? p.total_rows >= 480ll * p.E : p.K > 2048;
+    if (use_dual_tiles() && fits && pays) {
       constexpr int kDual = A_GATHER ? pair::DUAL_N : pair::DUAL_M;
       return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 4, kDual>(tmA, tmB, p, stream);
     }

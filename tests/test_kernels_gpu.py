@@ -784,6 +784,24 @@ def test_few_rows_kernel_beside_tiles(smoe, rows, launches, hot):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("T,H,I", [
+    (480, 2112, 960),   # dual tiles in both: the shortest reductions that have them, a second tile that is partly filled
+    (479, 2048, 960),   # single tiles in both
+    (1000, 4096, 256),
+])
+def test_dual_tiles_around_their_rule(smoe, tmp_path, T, H, I):
+    """test_dual_tiles_match_single_tiles where the two forms part: reductions over H of 2048, over an expert's rows of 480."""
+    global _DUAL_SNIPPET
+    snippet = _DUAL_SNIPPET
+    sizes = "T, H, I, E, K = 2048, 1024, 512, 8, 2"
+    assert sizes in snippet
+    try:
+        _DUAL_SNIPPET = snippet.replace(sizes, f"T, H, I, E, K = {T}, {H}, {I}, 2, 2")
+        test_dual_tiles_match_single_tiles(smoe, tmp_path)
+    finally:
+        _DUAL_SNIPPET = snippet
+
+
 @pytest.mark.parametrize("H", [8, 72, 64, 1040])
 @pytest.mark.parametrize("weights", [None, torch.float32, torch.bfloat16])
 def test_gather_sum_forms(smoe, H, weights):
