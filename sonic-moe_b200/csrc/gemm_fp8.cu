@@ -158,8 +158,11 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const __nv_bfloat16*
 // One CTA per 128 x 128 block of a (batch, rows, cols) tensor; rows need not be a multiple of 128.
 // POW2: the scale is a UE8M0 byte (smallest power of two >= amax / 448), else fp32 amax / 448.
 // WIDE: w is 16-byte and q 8-byte aligned; otherwise (a view into a larger buffer) w is 8-byte and q 4-byte aligned.
+// fp32 scales: four blocks per SM, although eleven words a thread spill for it, where the 87 registers that the divisions take
+// leave room for two and one block's loads do not cover another's arithmetic.  32 x 4096 x 7168 values 854 -> 652 us (five blocks
+// 778).  Without divisions the third block that fits already covers it: four are 3 % faster alone, and not in the layer.
 template <bool POW2, bool WIDE>
-__global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat16* w, uint8_t* q, void* scale, int rows,
+__global__ void __launch_bounds__(256, POW2 ? 3 : 4) quantize_blocks_kernel(const __nv_bfloat16* w, uint8_t* q, void* scale, int rows,
                                                               int cols) {
   release_next();
   wait_for_previous();
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat1
   const int nrows = min(128, rows - rb * 128);
   // warp w has rows 16w .. 16w+15 of the block, half a warp per row and load, all of them in flight together; they stay in
   // registers for the conversion.  Bound by memory: 8-byte loads in two dependent passes ran at 4.2 TB/s (1.02 ms for the
-  // weights of 32 experts, H 7168, I 2048; now 0.74 ms, 5.7 TB/s).
+  // weights of 32 experts, H 7168, I 2048; now 0.64 ms).
   const int piece = lane & 15;
   uint4 v[8];
 #pragma unroll
