@@ -396,7 +396,8 @@ int smoe_layer_forward(const void* x, const void* router_w, const void* w1, cons
 
 /* A training pass of the layer (top-K routing, any activation, biases optional) in four calls, with the launches and the
  * requirements of the entry points above; T > 0.  I: columns of the down projection, N1: rows of the up projection (I, or 2 I
- * where the activation is gated).
+ * where the activation is gated).  All sizes, pointers and alignments (meta 4 bytes, scratch 256) are checked before a call's
+ * first launch.
  * meta: smoe_layer_meta_words(T, E, K) 4-byte words that the forward call writes and the backward calls read.
  * Forward: with router_w (bf16, where smoe_router_forward_supported) logits, prob_colsum and aux are outputs; without it
  * logits (T,E) of logits_dtype are an input.  z (T K, N1) may be null where no backward pass follows.

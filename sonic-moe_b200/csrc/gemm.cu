@@ -14,6 +14,7 @@ using pair::BK;
 using pair::BM;
 using pair::BN;
 using pair::MAX_EXPERTS;
+static_assert(MAX_EXPERTS == kMaxExperts, "checked by the compound entry points");
 
 // cuTensorMapEncodeTiled is fetched through the runtime so that the library links against cudart
 // only and still loads on a machine without a driver.

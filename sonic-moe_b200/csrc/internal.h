@@ -3,6 +3,9 @@
 
 namespace smoe {
 
+constexpr int kMaxExperts = 1024;  // experts whose offsets the grouped GEMMs keep in shared memory
+constexpr int kMaxRouterExperts = 256;  // experts of the router kernels
+
 // smoe_gather_sum with fp32 weights or none whose result is added to `out` (bf16) instead of replacing it: one rounding of the sum.
 int gather_sum_add(const void* src, void* out, const float* weights, const int* reverse_idx, int T, int H, int K,
                    void* stream);

@@ -6,7 +6,10 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include "../../include/sonicmoe_b200.h"
+#include "epilogue.cuh"
 #include "internal.h"
 
 namespace {
@@ -84,15 +87,41 @@ struct BackwardScratch {
   }
 };
 
-constexpr int kSwiglu = 0;
-
-// Sizes that the training entry points share; the kernels they call check theirs.
+// What the calls below would refuse is refused before the first of them launches something: sizes, pointers and alignment are
+// checked by the compound entry points themselves.
 bool bad_layer(int T, int H, int I, int N1, int E, int K) {
-  return T <= 0 || H <= 0 || I <= 0 || (N1 != I && N1 != 2 * I) || E <= 0 || K <= 0 || K > E ||
-         static_cast<long long>(T) * K > 0x7fffffffll;
+  return T <= 0 || H <= 0 || H % 64 != 0 || I <= 0 || I % 64 != 0 || (N1 != I && N1 != 2 * static_cast<long long>(I)) ||
+         N1 % 128 != 0 || E <= 0 || E > smoe::kMaxExperts || K <= 0 || K > E || static_cast<long long>(T) * K > 0x7fffffffll;
+}
+
+// Scratch and metadata are laid out for N1 rows, and the activation's kernels write as many as it has.
+bool bad_activation_rows(int activation, int I, int N1) {
+  return activation < smoe::ACT_SWIGLU || activation > smoe::ACT_SILU ||
+         N1 != (smoe::act_is_gated(activation) ? 2 : 1) * static_cast<long long>(I);
 }
 
 bool aligned(const void* p, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
+
+int check_given(std::initializer_list<const void*> pointers, uintptr_t bytes) {
+  for (const void* p : pointers) {
+    if (p == nullptr) return SMOE_ERR_SHAPE;
+    if (!aligned(p, bytes)) return SMOE_ERR_ALIGNMENT;
+  }
+  return SMOE_OK;
+}
+
+int check_optional(std::initializer_list<const void*> pointers, uintptr_t bytes) {
+  for (const void* p : pointers)
+    if (!aligned(p, bytes)) return SMOE_ERR_ALIGNMENT;
+  return SMOE_OK;
+}
+
+int check_workspace(const void* p, uintptr_t bytes) {
+  return p == nullptr ? SMOE_ERR_WORKSPACE : aligned(p, bytes) ? SMOE_OK : SMOE_ERR_ALIGNMENT;
+}
+
+// The router's logits (T,E): bytes per value, or 0 for an unknown type.
+int logit_bytes(int dtype) { return dtype == SMOE_F32 ? 4 : dtype == SMOE_BF16 ? 2 : 0; }
 
 }  // namespace
 
@@ -112,22 +141,12 @@ size_t smoe_layer_forward_scratch_bytes(int T, int H, int I, int E, int K) {
 int smoe_layer_forward(const void* x, const void* router_w, const void* w1, const void* w2, void* o, void* logits,
                        int* expert_count, float* prob_colsum, float* aux, void* scratch, int T, int H, int I, int E,
                        int K, int* status, void* stream) {
-  // what any of the calls below would refuse is refused before the first of them launches something
   if (T <= 0 || !smoe_router_forward_supported(H, E, K) || I <= 0 || I % 64 != 0 ||
       static_cast<long long>(T) * K > 0x7fffffffll)
     return SMOE_ERR_SHAPE;
-  const void* const wide[] = {x, router_w, w1, w2, o, logits};  // TMA sources, and rows stored in 16-byte pieces
-  for (const void* ptr : wide) {
-    if (ptr == nullptr) return SMOE_ERR_SHAPE;
-    if (!aligned(ptr, 16)) return SMOE_ERR_ALIGNMENT;
-  }
-  const void* const words[] = {expert_count, prob_colsum, aux};
-  for (const void* ptr : words) {
-    if (ptr == nullptr) return SMOE_ERR_SHAPE;
-    if (!aligned(ptr, 4)) return SMOE_ERR_ALIGNMENT;
-  }
-  if (scratch == nullptr) return SMOE_ERR_WORKSPACE;
-  if (!aligned(scratch, 256)) return SMOE_ERR_ALIGNMENT;
+  SMOE_TRY(check_given({x, router_w, w1, w2, o, logits}, 16));  // TMA sources, and rows stored in 16-byte pieces
+  SMOE_TRY(check_given({expert_count, prob_colsum, aux}, 4));
+  SMOE_TRY(check_workspace(scratch, 256));
   const Scratch at(T, H, I, E, K);
   char* base = static_cast<char*>(scratch);
   const auto ints = [base](size_t o_) { return reinterpret_cast<int*>(base + o_); };
@@ -163,8 +182,20 @@ int smoe_layer_train_forward(const void* x, const void* router_w, void* logits, 
                              const void* b1, const void* w2, const void* b2, void* o, void* z, void* meta,
                              int* expert_count, float* prob_colsum, float* aux, void* scratch, int T, int H, int I, int N1,
                              int E, int K, int activation, int* status, void* stream) {
-  if (bad_layer(T, H, I, N1, E, K)) return SMOE_ERR_SHAPE;
-  if (meta == nullptr || scratch == nullptr) return SMOE_ERR_WORKSPACE;
+  if (bad_layer(T, H, I, N1, E, K) || bad_activation_rows(activation, I, N1)) return SMOE_ERR_SHAPE;
+  if (router_w != nullptr) {
+    if (!smoe_router_forward_supported(H, E, K)) return SMOE_ERR_SHAPE;
+    SMOE_TRY(check_given({router_w, logits}, 16));
+    SMOE_TRY(check_given({expert_count, aux}, 4));
+  } else {
+    if (logit_bytes(logits_dtype) == 0) return SMOE_ERR_DTYPE;
+    SMOE_TRY(check_given({logits}, logit_bytes(logits_dtype)));
+  }
+  SMOE_TRY(check_given({x, w1, w2, o}, 16));
+  SMOE_TRY(check_optional({b1, b2, z}, 16));
+  SMOE_TRY(check_optional({expert_count, prob_colsum}, 4));
+  SMOE_TRY(check_workspace(meta, 4));
+  SMOE_TRY(check_workspace(scratch, 256));
   const int tk = T * K;
   const Meta m(meta, tk, E);
   const ForwardScratch at(T, H, I, E, K);
@@ -176,7 +207,7 @@ int smoe_layer_train_forward(const void* x, const void* router_w, void* logits, 
     SMOE_TRY(smoe_topk_softmax(logits, logits_dtype, m.scores, m.indices, T, E, K, stream));
   SMOE_TRY(smoe_route_metadata(m.indices, nullptr, tk, E, K, expert_count, m.off, m.s_scatter, m.s_reverse, m.x_gather,
                                base + at.route_ws, stream));
-  const bool plain = activation == kSwiglu && b1 == nullptr && b2 == nullptr;
+  const bool plain = activation == smoe::ACT_SWIGLU && b1 == nullptr && b2 == nullptr;
   if (plain)
     SMOE_TRY(smoe_up_projection_forward(x, w1, z, base + at.y1, m.off, m.x_gather, T, H, I, E, tk, status, stream));
   else
@@ -201,8 +232,26 @@ int smoe_layer_backward_act(const void* dout, const void* w2, const void* b2, co
                             const void* logits, int logits_dtype, int fused_router, const void* g_logits,
                             const float* g_colsum, const float* g_aux, void* dlogits, void* db1, void* db2, void* scratch,
                             int T, int H, int I, int N1, int E, int K, int activation, int* status, void* stream) {
-  if (bad_layer(T, H, I, N1, E, K)) return SMOE_ERR_SHAPE;
-  if (meta == nullptr || (dout != nullptr && scratch == nullptr)) return SMOE_ERR_WORKSPACE;
+  if (bad_layer(T, H, I, N1, E, K) || bad_activation_rows(activation, I, N1)) return SMOE_ERR_SHAPE;
+  SMOE_TRY(check_workspace(meta, 4));
+  if (dout != nullptr) {
+    SMOE_TRY(check_given({dout, w2, z}, 16));
+    SMOE_TRY(check_optional({b2}, 16));
+    if (b2 != nullptr) SMOE_TRY(check_given({db1, db2}, 16));
+    SMOE_TRY(check_workspace(scratch, 256));
+  }
+  if (dlogits != nullptr) {
+    if (fused_router) {
+      if (E > smoe::kMaxRouterExperts) return SMOE_ERR_SHAPE;
+      if (g_colsum != nullptr || g_aux != nullptr) SMOE_TRY(check_given({logits}, 2));
+      SMOE_TRY(check_optional({dlogits, g_logits}, 2));
+      SMOE_TRY(check_optional({g_colsum, g_aux}, 4));
+    } else {
+      if (dout == nullptr) return SMOE_ERR_SHAPE;  // nothing else has a gradient by the scores
+      if (logit_bytes(logits_dtype) == 0) return SMOE_ERR_DTYPE;
+      SMOE_TRY(check_optional({dlogits}, logit_bytes(logits_dtype)));
+    }
+  }
   const int tk = T * K;
   const Meta m(meta, tk, E);
   const BackwardScratch at(T, I, N1, K);
@@ -210,7 +259,7 @@ int smoe_layer_backward_act(const void* dout, const void* w2, const void* b2, co
   float* ds = dout != nullptr ? reinterpret_cast<float*>(base + at.ds) : nullptr;
   if (dout != nullptr) {
     float* partial = reinterpret_cast<float*>(base + at.ds_partial);
-    if (activation == kSwiglu && b2 == nullptr)
+    if (activation == smoe::ACT_SWIGLU && b2 == nullptr)
       SMOE_TRY(smoe_down_projection_backward_act(dout, w2, z, m.scores, 0, base + at.dz, base + at.y1s, partial, m.off,
                                                  m.x_gather, m.s_scatter, T, H, I, E, tk, status, stream));
     else
@@ -227,14 +276,16 @@ int smoe_layer_backward_act(const void* dout, const void* w2, const void* b2, co
   if (fused_router)
     return smoe_router_backward_aux(dlogits, logits, ds, m.scores, m.indices, g_colsum, g_logits, g_aux, m.aux_grad, T, E,
                                     K, stream);
-  if (ds == nullptr) return SMOE_ERR_SHAPE;
   return smoe_softmax_topk_backward(dlogits, logits_dtype, ds, m.scores, m.indices, T, E, K, stream);
 }
 
 int smoe_layer_backward_dx(const void* w1, void* meta, const void* scratch, void* dx_expanded, void* dx, int add, int T,
                            int H, int I, int N1, int E, int K, int* status, void* stream) {
-  if (bad_layer(T, H, I, N1, E, K) || N1 % 2 != 0) return SMOE_ERR_SHAPE;
-  if (meta == nullptr || scratch == nullptr || (K > 1 && dx_expanded == nullptr)) return SMOE_ERR_WORKSPACE;
+  if (bad_layer(T, H, I, N1, E, K)) return SMOE_ERR_SHAPE;
+  SMOE_TRY(check_given({w1, dx}, 16));
+  SMOE_TRY(check_workspace(meta, 4));
+  SMOE_TRY(check_workspace(scratch, 256));
+  if (K > 1) SMOE_TRY(check_workspace(dx_expanded, 16));
   const int tk = T * K;
   const Meta m(meta, tk, E);
   const char* dz = static_cast<const char*>(scratch) + BackwardScratch(T, I, N1, K).dz;
@@ -249,8 +300,10 @@ int smoe_layer_backward_dx(const void* w1, void* meta, const void* scratch, void
 
 int smoe_layer_backward_weights(const void* x, const void* dout, void* meta, const void* scratch, void* dw1, void* dw2,
                                 int T, int H, int I, int N1, int E, int K, int* status, void* stream) {
-  if (bad_layer(T, H, I, N1, E, K) || N1 % 2 != 0) return SMOE_ERR_SHAPE;
-  if (meta == nullptr || scratch == nullptr) return SMOE_ERR_WORKSPACE;
+  if (bad_layer(T, H, I, N1, E, K)) return SMOE_ERR_SHAPE;
+  SMOE_TRY(check_given({x, dout, dw1, dw2}, 16));
+  SMOE_TRY(check_workspace(meta, 4));
+  SMOE_TRY(check_workspace(scratch, 256));
   const int tk = T * K;
   const Meta m(meta, tk, E);
   const BackwardScratch at(T, I, N1, K);

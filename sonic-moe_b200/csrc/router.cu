@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "../../include/sonicmoe_b200.h"
+#include "internal.h"
 #include "launch.cuh"
 #include "ptx.cuh"
 
@@ -36,7 +37,7 @@ constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
-constexpr int MAX_E = 256;
+constexpr int MAX_E = kMaxRouterExperts;
 constexpr int THREADS = 512;
 constexpr int FIRST_DRAIN_WARP = 2;   // 4 warps, one per quarter of the tensor-memory lanes
 constexpr int FIRST_TOKEN_WARP = 6;   // the large kernel's warps that work on tokens

@@ -80,3 +80,78 @@ def test_layer_forward_refuses_before_the_first_launch(built_library):
     for name in ("expert_count", "prob_colsum", "aux"):
         assert call(**{name: 4096 + 2}) == -2 and call(**{name: None}) == -1, name
     assert call(scratch=4096 + 16) == -2 and call(scratch=None) == -7
+
+
+def test_layer_training_calls_refuse_before_the_first_launch(built_library):
+    """Sizes that do not fit the activation (the scratch is laid out for N1 rows) or that only a later kernel of the call would
+    refuse, missing and misaligned pointers (the addresses here belong to nothing)."""
+    from sonicmoe._lib import lib
+
+    swiglu, gelu = 0, 5
+    sizes = dict(T=4, H=128, I=64, N1=128, E=32, K=2)
+
+    def forward(fused=True, activation=swiglu, dtype=1, **bad):
+        s = {**sizes, **{k: bad.pop(k) for k in sizes if k in bad}}
+        p = {n: 4096 for n in ("x", "router_w", "logits", "w1", "b1", "w2", "b2", "o", "z", "meta", "expert_count",
+                               "prob_colsum", "aux", "scratch")}
+        p.update(router_w=4096 if fused else None, b1=None, b2=None, **{} if fused else dict(prob_colsum=None, aux=None))
+        p.update(bad)
+        return lib.smoe_layer_train_forward(
+            p["x"], p["router_w"], p["logits"], dtype, p["w1"], p["b1"], p["w2"], p["b2"], p["o"], p["z"], p["meta"],
+            p["expert_count"], p["prob_colsum"], p["aux"], p["scratch"], *s.values(), activation, None, None)
+
+    def act(fused=1, activation=swiglu, dtype=1, **bad):
+        s = {**sizes, **{k: bad.pop(k) for k in sizes if k in bad}}
+        p = {n: 4096 for n in ("dout", "w2", "z", "meta", "logits", "dlogits", "scratch")}
+        p.update(dict.fromkeys(("b2", "g_logits", "g_colsum", "g_aux", "db1", "db2")))
+        p.update(bad)
+        return lib.smoe_layer_backward_act(
+            p["dout"], p["w2"], p["b2"], p["z"], p["meta"], p["logits"], dtype, fused, p["g_logits"], p["g_colsum"],
+            p["g_aux"], p["dlogits"], p["db1"], p["db2"], p["scratch"], *s.values(), activation, None, None)
+
+    def dx(**bad):
+        s = {**sizes, **{k: bad.pop(k) for k in sizes if k in bad}}
+        p = {n: 4096 for n in ("w1", "meta", "scratch", "dx_expanded", "dx")} | bad
+        return lib.smoe_layer_backward_dx(p["w1"], p["meta"], p["scratch"], p["dx_expanded"], p["dx"], 0, *s.values(), None,
+                                          None)
+
+    def weights(**bad):
+        s = {**sizes, **{k: bad.pop(k) for k in sizes if k in bad}}
+        p = {n: 4096 for n in ("x", "dout", "meta", "scratch", "dw1", "dw2")} | bad
+        return lib.smoe_layer_backward_weights(p["x"], p["dout"], p["meta"], p["scratch"], p["dw1"], p["dw2"], *s.values(),
+                                               None, None)
+
+    def unfused(**bad):
+        return forward(fused=False, **bad)
+
+    for call in (forward, unfused, act, dx, weights):
+        for bad in (dict(T=0), dict(T=2 ** 30), dict(H=100), dict(I=100, N1=200), dict(I=0, N1=0), dict(I=192, N1=192),
+                    dict(N1=192), dict(E=0), dict(E=1025), dict(K=0), dict(K=33)):
+            assert call(**bad) == -1, (call.__name__, bad)
+    for call in (forward, unfused, act):
+        assert call(activation=swiglu, I=128, N1=128) == -1 and call(activation=gelu, I=128, N1=256) == -1
+        assert call(activation=7) == -1 and call(activation=-1) == -1
+    assert forward(E=8) == -1 and forward(K=17) == -1              # not the fused router's
+    assert unfused(dtype=2) == -6 and act(fused=0, dtype=2) == -6
+    for call, names in ((forward, ("x", "router_w", "logits", "w1", "w2", "o")), (unfused, ("x", "w1", "w2", "o")),
+                        (act, ("dout", "w2", "z")), (dx, ("w1", "dx")), (weights, ("x", "dout", "dw1", "dw2"))):
+        for name in names:
+            assert call(**{name: 4096 + 8}) == -2, (call.__name__, name)
+            if name not in ("router_w", "dout") or call is weights:  # (None there selects another form)
+                assert call(**{name: None}) == -1, (call.__name__, name)
+        assert call(meta=None) == -7 and call(meta=4096 + 2) == -2
+        assert call(scratch=None) == -7 and call(scratch=4096 + 16) == -2
+    assert unfused(logits=4096 + 1) == -2 and unfused(logits=4096 + 2, dtype=0) == -2 and unfused(logits=None) == -1
+    for name in ("b1", "b2", "z"):
+        assert forward(**{name: 4096 + 8}) == -2, name
+    for name in ("expert_count", "prob_colsum", "aux"):
+        assert forward(**{name: 4096 + 2}) == -2, name
+    assert forward(expert_count=None) == -1 and forward(aux=None) == -1
+    assert act(b2=4096) == -1 and act(b2=4096, db1=4096) == -1 and act(b2=4096, db1=4096, db2=4096 + 8) == -2
+    assert act(b2=4096 + 8, db1=4096, db2=4096) == -2
+    for given in ("g_colsum", "g_aux"):
+        assert act(**{given: 4096}, logits=None) == -1 and act(**{given: 4096 + 2}) == -2
+    assert act(dlogits=4096 + 1) == -2 and act(g_logits=4096 + 1) == -2 and act(fused=0, dtype=0, dlogits=4096 + 2) == -2
+    assert act(E=512) == -1                                        # more experts than the router's backward pass takes
+    assert act(fused=0, dout=None) == -1                           # nothing to derive the logits' gradient from
+    assert dx(dx_expanded=None) == -7 and dx(dx_expanded=4096 + 8) == -2
