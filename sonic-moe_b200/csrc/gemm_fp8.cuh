@@ -189,7 +189,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       Tile tile;
       for (long long t = first_tile; ok && decode_tile(p, ss, t, num_n, rank, tile); t += tile_step) {
         for (int kb = 0; kb < tile.num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
           if (elected) {
             if (leader) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
@@ -207,23 +207,22 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_PRODUCER);
     }
     // ---- MMA issuer ----------------------------------------------------------------------------
-    else if (warp == 1 && leader) {
-      const bool elected = elect_one();
-      constexpr uint32_t idesc = make_idesc_e4m3(2 * BM, BN, false, B_MN);
-      constexpr uint32_t b_lbo = B_MN ? B_STAGE_BYTES : 16;
-      constexpr uint32_t b_kstep = B_MN ? (UMMA_K * 128) : UMMA_K;  // bytes per 32 reduction elements
-      int stage = 0;
-      uint32_t phase = 0;
-      int buf = 0;
-      uint32_t buf_phase = 0;
-      bool ok = true;
-      Tile tile;
-      for (long long t = first_tile; ok && decode_tile(p, ss, t, num_n, rank, tile); t += tile_step) {
-        for (int kb = 0; kb < tile.num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&ss.part_empty[buf]), buf_phase ^ 1u, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          if (elected) {
+    else if (warp == 1) {
+      if (leader && elect_one()) {  // one thread: nothing in this loop is warp-wide
+        constexpr uint32_t idesc = make_idesc_e4m3(2 * BM, BN, false, B_MN);
+        constexpr uint32_t b_lbo = B_MN ? B_STAGE_BYTES : 16;
+        constexpr uint32_t b_kstep = B_MN ? (UMMA_K * 128) : UMMA_K;  // bytes per 32 reduction elements
+        int stage = 0;
+        uint32_t phase = 0;
+        int buf = 0;
+        uint32_t buf_phase = 0;
+        bool ok = true;
+        Tile tile;
+        for (long long t = first_tile; ok && decode_tile(p, ss, t, num_n, rank, tile); t += tile_step) {
+          for (int kb = 0; kb < tile.num_kb; ++kb) {
+            if (!mbar_wait(smem_u32(&ss.part_empty[buf]), buf_phase ^ 1u, abort_flag)) { ok = false; break; }
+            if (!mbar_wait(smem_u32(&ss.full[stage]), phase, abort_flag)) { ok = false; break; }
+            tc_fence_after();
             const uint64_t a_desc = make_smem_desc(smem_u32(sA + stage * A_STAGE_BYTES), 16, 1024);
             const uint64_t b_desc = make_smem_desc(smem_u32(sB + stage * B_STAGE_BYTES), b_lbo, 1024);
             const uint32_t d_tmem = tmem_base + buf * BN;
@@ -233,13 +232,12 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                              k4 > 0 ? 1u : 0u);
             umma_commit_pair(smem_u32(&ss.empty[stage]), 3);
             umma_commit_pair(smem_u32(&ss.part_full[buf]), 3);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+            if (++buf == 2) { buf = 0; buf_phase ^= 1u; }
           }
-          __syncwarp();
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          if (++buf == 2) { buf = 0; buf_phase ^= 1u; }
         }
+        if (!ok && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_MMA);
       }
-      if (!ok && lane == 0 && p.status) atomicCAS(p.status, ST_OK, ST_TIMEOUT_MMA);
     }
   } else if (warp >= FIRST_GATHER_WARP) {
     reg_dec<56>();
@@ -298,7 +296,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       for (int kb = 0; kb < tile.num_kb; ++kb) {
         const float scale = scale_next;
         if (kb + 1 < tile.num_kb) scale_next = a_sc[kb + 1] * b_sc[(kb + 1) * sc.b_k_stride];
-        if (!mbar_wait(smem_u32(&ss.part_full[buf]), buf_phase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(smem_u32(&ss.part_full[buf]), buf_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t t_addr = tmem_base + buf * BN + col_half * 128 + (static_cast<uint32_t>(quad * 32) << 16);
         // two register buffers: the load of the next 32 columns is in flight while this one is accumulated
@@ -352,10 +350,12 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     const uint64_t t0 = global_timer_ns();
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
+  // barriers that the lanes of a warp may reach one by one: the MMA role is one lane's
   tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();
+  block_sync_diverged();
+  cluster_sync_diverged();
   if (warp == 1) {
+    __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * BN);
   }

@@ -195,7 +195,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
       Tile tile;
       for (long long t = first_tile; ok && fp8::decode_tile(p, ss, t, num_n, rank, tile); t += tile_step) {
         for (int kb = 0; kb < tile.num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(smem_u32(&ss.empty[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t bar = map_to_cta(smem_u32(&ss.full[stage]), 0);
           if (elected) {
             if (leader) mbar_arrive_expect_tx(smem_u32(&ss.full[stage]), 2 * kTmaBytesPerCta);
@@ -314,7 +314,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         for (int g = 0; g < groups; ++g) {
           uint4 n0 = w0, n1 = w1;
           if (g + 1 < groups) load_words(g + 1, n0, n1);
-          if (!mbar_wait(smem_u32(&ss.sf_empty[set]), set_phase ^ 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(smem_u32(&ss.sf_empty[set]), set_phase ^ 1u, abort_flag)) { ok = false; break; }
           uint8_t* dst = sSF + set * SF_SET_BYTES;
           if (warp == 2) {
             reinterpret_cast<uint4*>(dst)[lane] = w0;
@@ -386,7 +386,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         if (row_ok && (EPI != EPI_STORE_ROWS || p.scores != nullptr))
           score = load_score(p.scores, p.scores_are_bf16, p.s_scatter[r]);
       }
-      if (!mbar_wait(smem_u32(&ss.acc_full), acc_phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(smem_u32(&ss.acc_full), acc_phase, abort_flag)) { ok = false; break; }
       acc_phase ^= 1u;
       tc_fence_after();
       const uint32_t t_addr = tmem_base + col_half * 128 + (static_cast<uint32_t>(quad * 32) << 16);

@@ -1,9 +1,13 @@
 """Host-side logic that needs no GPU: module surface, state-dict layout, eager backend vs oracle, errors."""
 
+import os
+import re
+
 import numpy as np
 import pytest
 import torch
 
+from conftest import ROOT
 from oracle import moe_oracle as orc
 
 
@@ -269,3 +273,29 @@ def test_own_load_balancing_loss_is_used(built_library, monkeypatch):
     assert m(inp["x"])[1].item() == 2.0
     m._compute_switch_loss = lambda logits, probs, expert_frequency: torch.tensor(3.0)
     assert m(inp["x"])[1].item() == 3.0
+
+
+def test_waits_of_whole_warps_have_one_answer():
+    """A wait on an mbarrier is given up after a time limit, which the lanes of a warp may see at different polls.  Where a whole
+    warp waits (and its loop goes on with warp-wide operations) that has to be by mbar_wait_warp; mbar_wait is for code that a
+    single elected thread runs."""
+    seen = 0
+    csrc = os.path.join(ROOT, "sonic-moe_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if name == "ptx.cuh":  # defines both
+            continue
+        text = open(os.path.join(csrc, name)).read()
+        text = re.sub(r'/\*.*?\*/|//[^\n]*|"[^"\n]*"', lambda m: re.sub(r"[^\n]", " ", m[0]), text, flags=re.S)
+        headers, start = [], 0  # what stands before each open brace
+        for m in re.finditer(r"[{};]|\bmbar_wait\(", text):
+            if m[0] == "mbar_wait(":
+                seen += 1
+                line = text.count("\n", 0, m.start()) + 1
+                assert any(re.search(r"\belect(ed\b|_one\()", h) for h in headers), f"{name}:{line}"
+                continue
+            if m[0] == "{":
+                headers.append(text[start:m.start()])
+            elif m[0] == "}":
+                headers.pop()
+            start = m.end()
+    assert seen > 10
