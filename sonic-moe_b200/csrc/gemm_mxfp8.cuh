@@ -386,7 +386,14 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         if (row_ok && (EPI != EPI_STORE_ROWS || p.scores != nullptr))
           score = load_score(p.scores, p.scores_are_bf16, p.s_scatter[r]);
       }
-      if (!mbar_wait_warp(smem_u32(&ss.acc_full), acc_phase, abort_flag)) { ok = false; break; }
+      ok = mbar_wait_warp(smem_u32(&ss.acc_full), acc_phase, abort_flag);
+      if (!ok) {
+        // the other warp of the quadrant learns of it where the two exchange maxima (below)
+        if constexpr (EPI == EPI_SWIGLU) {
+          if (p.q_out != nullptr) warps_agree(1 + quad, 64, false);
+        }
+        break;
+      }
       acc_phase ^= 1u;
       tc_fence_after();
       const uint32_t t_addr = tmem_base + col_half * 128 + (static_cast<uint32_t>(quad * 32) << 16);
@@ -471,7 +478,8 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
           swiglu_keep(v2, 2);
           swiglu_keep(v3, 3);
           ss.row_amax[col_half][row_in_tile] = (row_ok && cols_ok) ? amax : 0.f;
-          asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
+          ok = warps_agree(1 + quad, 64, true);
+          if (!ok) break;  // the other warp has given up its wait
           amax = fmaxf(amax, ss.row_amax[col_half ^ 1][row_in_tile]);
           asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");  // the slots may be rewritten for the next tile
           if (row_ok && cols_ok) {

@@ -106,6 +106,23 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// Whether `v` holds for all `threads` threads (whole warps) that meet at this named barrier.  Warps that exchange something
+// behind a wait have to decide together whether it was abandoned: one that left would keep the others in their next barrier.
+__device__ __forceinline__ bool warps_agree(int barrier, int threads, bool v) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
+      "}\n"
+      : "=r"(all)
+      : "r"(static_cast<uint32_t>(v)), "r"(barrier), "r"(threads)
+      : "memory");
+  return all != 0;
+}
+
 // 16-byte shared-memory accesses by shared-space address
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");

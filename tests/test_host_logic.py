@@ -299,3 +299,14 @@ def test_waits_of_whole_warps_have_one_answer():
                 headers.pop()
             start = m.end()
     assert seen > 10
+
+
+def test_warps_that_meet_at_a_named_barrier_give_up_together():
+    """Behind a wait that may be abandoned, warps that will meet at a named barrier decide together whether it was."""
+    csrc = os.path.join(ROOT, "sonic-moe_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, name)).read()
+        for m in re.finditer(r"\bbar\.sync %\d", text):
+            before = text[:m.start()]
+            wait = before.rfind("mbar_wait_warp(")
+            assert "warps_agree(" in before[wait:], f"{name}:{before.count(chr(10)) + 1}"
