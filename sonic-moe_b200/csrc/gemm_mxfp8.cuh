@@ -180,7 +180,6 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
-  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 

@@ -299,7 +299,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // the other CTA's barriers are initialised before anything can arrive on them
-  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 

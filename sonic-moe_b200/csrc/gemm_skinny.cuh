@@ -180,7 +180,6 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
   bool ok = true;

@@ -262,7 +262,6 @@ router_forward_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   wait_for_previous();
   tc_fence_before();
   __syncthreads();
-  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
   float colsum[PER_LANE];
@@ -436,7 +435,6 @@ router_forward_small_kernel(const __grid_constant__ CUtensorMap tmX, const __gri
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // every CTA of the cluster runs before anything is written to its shared memory
-  release_next();
   tc_fence_after();
   const uint32_t tmem_base = ss.tmem_base;
 
@@ -596,7 +594,6 @@ __global__ void __launch_bounds__(1024) router_finish_kernel(const float* colsum
 template <int PER_LANE>
 __global__ void __launch_bounds__(256) softmax_colsum_kernel(const __nv_bfloat16* logits, int rows, int E,
                                                              float* colsum_partial) {
-  release_next();
   wait_for_previous();
   __shared__ float sums[8][MAX_E];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -564,3 +564,43 @@ def test_layer_in_one_node_matches_separate_functions(built_library, T, E, K, ac
                     assert torch.equal(s, t), (frozen, i)
     with torch.no_grad():
         assert torch.equal(one_node(*given)[0], o)
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_second_stream_gets_on_beside_the_launch_chain(built_library, train):
+    """A row of small kernels on a second stream, enqueued behind passes of the layer, ends long before these: a kernel of the chain
+    must not stand in front of them while it waits for room itself, or each of them waits for the end of one of the layer's."""
+    import sonicmoe
+    from sonicmoe import _lib
+    from sonicmoe.enums import ActivationType
+
+    T, H, I, E, K = 16384, 4096, 1024, 32, 8  # about 5 (15) ms of kernels and 0.1 (0.5) ms of launches a pass
+    passes = 4 if train else 10  # fewer kernels than the second stream has
+    m = sonicmoe.MoE(E, K, H, I, ActivationType.SWIGLU, False, 0.02).cuda().to(torch.bfloat16)
+    x = torch.randn(T, H, device="cuda").bfloat16().requires_grad_(train)
+    dout = torch.randn(T, H, device="cuda").bfloat16()
+    small = torch.zeros(1 << 20, device="cuda")
+    side = torch.cuda.Stream()
+
+    def layer():
+        with torch.set_grad_enabled(train):
+            o, _ = m(x, is_inference_mode=not train)
+            if train:
+                torch.autograd.grad(o, [x, *m.parameters()], dout)
+
+    for _ in range(2):
+        layer()
+        small.add_(1.0)
+    torch.cuda.synchronize()
+    begin, end, side_end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    begin.record()
+    for _ in range(passes):
+        layer()
+    end.record()
+    with torch.cuda.stream(side):
+        for _ in range(300):
+            small.add_(1.0)
+        side_end.record()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert begin.elapsed_time(side_end) < 0.7 * begin.elapsed_time(end)
