@@ -800,7 +800,7 @@ class _Layer(torch.autograd.Function):
                 ptr(db2), ptr(scratch), T, H, I, n1, E, K, act, status, stream), "layer_backward_act")
             if fused:
                 if need_x:
-                    dx = dlogits @ router_w
+                    dx = (dlogits @ router_w).to(x.dtype)  # autocast may choose another type, and the experts' part is added below
                 if need_router:
                     d_router = dlogits.t() @ x
             if dout is not None:

@@ -604,3 +604,31 @@ def test_second_stream_gets_on_beside_the_launch_chain(built_library, train):
     torch.cuda.synchronize()
     _lib.check_status()
     assert begin.elapsed_time(side_end) < 0.7 * begin.elapsed_time(end)
+
+
+@pytest.mark.parametrize("K", [1, 4])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_backward_pass_under_autocast(built_library, K, dtype):
+    """A backward pass that runs inside an autocast region: the router's GEMMs may come out in the region's type, and the experts'
+    part of the gradient of x is added to the router's.  Three roundings of at most 2^-8 (bf16 has 8 significant bits; fp16 more) of
+    parts no larger than the gradient tell the two apart: 3 2^-8 < 2^-6 of the norm."""
+    import sonicmoe
+    from sonicmoe import _lib
+    from sonicmoe.enums import ActivationType
+
+    T, H, I, E = 300, 256, 128, 32
+    m = sonicmoe.MoE(E, K, H, I, ActivationType.SWIGLU, False, 0.05).cuda().to(torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16().requires_grad_(True)
+    dout = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    wanted = [x, *m.parameters()]
+    o, aux = m(x)
+    outputs, grads = [o, aux], [dout, torch.ones_like(aux)]
+    plain = torch.autograd.grad(outputs, wanted, grads, retain_graph=True)
+    with torch.autocast("cuda", dtype=dtype):
+        cast = torch.autograd.grad(outputs, wanted, grads)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for p, c in zip(plain, cast):
+        assert p.dtype == c.dtype == torch.bfloat16
+        assert (p.double() - c.double()).norm() <= 2.0 ** -6 * p.double().norm()
