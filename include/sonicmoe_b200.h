@@ -407,6 +407,8 @@ int smoe_layer_forward(const void* x, const void* router_w, const void* w1, cons
  * _weights in any order.  scratch: smoe_layer_backward_scratch_bytes, kept between the backward calls. */
 size_t smoe_layer_meta_words(int T, int E, int K);
 size_t smoe_layer_train_forward_scratch_bytes(int T, int H, int I, int E, int K);
+/* What SwiGLU without biases needs of it (with K == 1 the rows of the down projection go straight to o). */
+size_t smoe_layer_train_forward_plain_scratch_bytes(int T, int H, int I, int E, int K);
 int smoe_layer_train_forward(const void* x, const void* router_w, void* logits, int logits_dtype, const void* w1,
                              const void* b1, const void* w2, const void* b2, void* o, void* z, void* meta,
                              int* expert_count, float* prob_colsum, float* aux, void* scratch, int T, int H, int I, int N1,

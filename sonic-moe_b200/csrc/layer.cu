@@ -61,16 +61,16 @@ struct Meta {
 
 size_t round256(size_t bytes) { return (bytes + 255) & ~static_cast<size_t>(255); }
 
-// Scratch of the training forward pass.
+// Scratch of the training forward pass.  y2 comes last: the plain kernels' combine of one row per token has none.
 struct ForwardScratch {
-  size_t y1, y2, route_ws, router_ws, total;
+  size_t y1, route_ws, router_ws, y2, total;
   ForwardScratch(int T, int H, int I, int E, int K) {
     const size_t tk = static_cast<size_t>(T) * K;
     y1 = 0;
-    y2 = y1 + round256(tk * I * 2);
-    route_ws = y2 + round256(tk * H * 2);
+    route_ws = y1 + round256(tk * I * 2);
     router_ws = route_ws + round256(smoe_route_metadata_workspace_bytes(E));
-    total = router_ws + round256(smoe_router_forward_workspace_bytes(E));
+    y2 = router_ws + round256(smoe_router_forward_workspace_bytes(E));
+    total = y2 + round256(tk * H * 2);
   }
 };
 
@@ -176,6 +176,12 @@ size_t smoe_layer_meta_words(int T, int E, int K) {
 size_t smoe_layer_train_forward_scratch_bytes(int T, int H, int I, int E, int K) {
   if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || K <= 0) return 0;
   return ForwardScratch(T, H, I, E, K).total;
+}
+
+size_t smoe_layer_train_forward_plain_scratch_bytes(int T, int H, int I, int E, int K) {
+  if (T <= 0 || H <= 0 || I <= 0 || E <= 0 || K <= 0) return 0;
+  const ForwardScratch at(T, H, I, E, K);
+  return K == 1 ? at.y2 : at.total;
 }
 
 int smoe_layer_train_forward(const void* x, const void* router_w, void* logits, int logits_dtype, const void* w1,

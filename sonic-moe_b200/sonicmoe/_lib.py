@@ -94,6 +94,7 @@ SIGNATURES: dict[str, tuple] = {
     "smoe_layer_forward": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P]),
     "smoe_layer_meta_words": (c_size_t, [I, I, I]),
     "smoe_layer_train_forward_scratch_bytes": (c_size_t, [I, I, I, I, I]),
+    "smoe_layer_train_forward_plain_scratch_bytes": (c_size_t, [I, I, I, I, I]),
     "smoe_layer_train_forward": (I, [P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P]),
     "smoe_layer_backward_scratch_bytes": (c_size_t, [I, I, I, I]),
     "smoe_layer_backward_act": (I, [P, P, P, P, P, P, I, I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P]),

@@ -752,7 +752,9 @@ class _Layer(torch.autograd.Function):
             z = torch.empty(T * K, n1, dtype=x.dtype, device=dev) if training else None
             freq = torch.empty(E, dtype=torch.int32, device=dev)
             meta = torch.empty(lib.smoe_layer_meta_words(T, E, K), dtype=torch.int32, device=dev)
-            scratch = _lib.workspace(lib.smoe_layer_train_forward_scratch_bytes(T, H, I, E, K), dev)
+            scratch_bytes = (lib.smoe_layer_train_forward_plain_scratch_bytes if b1 is None and act == 0
+                             else lib.smoe_layer_train_forward_scratch_bytes)
+            scratch = _lib.workspace(scratch_bytes(T, H, I, E, K), dev)
             check(lib.smoe_layer_train_forward(
                 x.data_ptr(), ptr(router_w), logits.data_ptr(), _lib.dtype_code(logits.dtype), w1.data_ptr(), ptr(b1),
                 w2.data_ptr(), ptr(b2), o.data_ptr(), ptr(z), meta.data_ptr(), freq.data_ptr(), ptr(colsum), ptr(aux),

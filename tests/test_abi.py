@@ -155,3 +155,16 @@ def test_layer_training_calls_refuse_before_the_first_launch(built_library):
     assert act(E=512) == -1                                        # more experts than the router's backward pass takes
     assert act(fused=0, dout=None) == -1                           # nothing to derive the logits' gradient from
     assert dx(dx_expanded=None) == -7 and dx(dx_expanded=4096 + 8) == -2
+
+
+def test_training_forward_scratch_without_rows_that_nothing_writes(built_library):
+    """SwiGLU without biases writes the down projection's rows of top-1 routing straight to the output."""
+    from sonicmoe._lib import lib
+
+    T, H, I, E = 1000, 192, 64, 8
+    for K in (1, 2):
+        every = lib.smoe_layer_train_forward_scratch_bytes(T, H, I, E, K)
+        plain = lib.smoe_layer_train_forward_plain_scratch_bytes(T, H, I, E, K)
+        rows = -(-T * K * H * 2 // 256) * 256
+        assert every - plain == (rows if K == 1 else 0) and plain >= T * K * I * 2
+    assert lib.smoe_layer_train_forward_plain_scratch_bytes(0, H, I, E, 1) == 0
