@@ -327,6 +327,9 @@ int smoe_down_projection_backward_act(const void* dout, const void* w2, const vo
 }
 
 // ---- general activations and biases ---------------------------------------------
+// Biases are read in 16-byte pieces; unlike the tensor maps' operands nothing else looks at their address.
+static bool bad_bias(const void* b) { return (reinterpret_cast<uintptr_t>(b) & 15u) != 0; }
+
 static bool bad_activation(int a) { return a < ACT_SWIGLU || a > ACT_SILU; }
 
 int smoe_up_projection_forward_act(const void* x, const void* w1, const void* b1, void* z, void* y1,
@@ -336,6 +339,7 @@ int smoe_up_projection_forward_act(const void* x, const void* w1, const void* b1
       E > MAX_EXPERTS || bad_tokens(T, TK))
     return SMOE_ERR_SHAPE;
   if (TK == 0) return SMOE_OK;
+  if (bad_bias(b1)) return SMOE_ERR_ALIGNMENT;
   CUtensorMap tmA, tmB;
   SMOE_TRY(encode_2d(&tmA, x, T, H, H, 1, BK));
   SMOE_TRY(encode_2d(&tmB, w1, (uint64_t)E * N1, H, H, pair::BN_CTA, BK));
@@ -354,6 +358,7 @@ int smoe_down_projection_forward_bias(const void* y1, const void* w2, const void
                                       void* stream) {
   if (bad_shape(H, I, E) || TK < 0) return SMOE_ERR_SHAPE;
   if (TK == 0) return SMOE_OK;
+  if (bad_bias(b2)) return SMOE_ERR_ALIGNMENT;
   CUtensorMap tmA, tmB;
   SMOE_TRY(encode_2d(&tmA, y1, TK, I, I, BM, BK));
   SMOE_TRY(encode_2d(&tmB, w2, (uint64_t)E * H, I, I, pair::BN_CTA, BK));

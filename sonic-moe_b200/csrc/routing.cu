@@ -762,6 +762,7 @@ int smoe_expert_column_sum(const void* src, long long ld, const int* gather_idx,
                            int scores_dtype, const int* s_scatter_idx, const int* expert_offset, void* out, int E,
                            int N, void* stream) {
   if (E <= 0 || N <= 0 || (N % 8) != 0 || (ld % 8) != 0) return SMOE_ERR_SHAPE;
+  if (reinterpret_cast<uintptr_t>(src) % 16 != 0) return SMOE_ERR_ALIGNMENT;
   const dim3 grid(E, (N + 255) / 256);
   const __nv_bfloat16* s = static_cast<const __nv_bfloat16*>(src);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
@@ -780,6 +781,7 @@ int smoe_ds_add_bias_term(const void* dout, const void* b2, const int* expert_of
                           const int* s_scatter_idx, void* ds, int ds_dtype, int E, int H, int TK, void* stream) {
   if (E <= 0 || H <= 0 || (H % 8) != 0 || TK < 0) return SMOE_ERR_SHAPE;
   if (TK == 0) return SMOE_OK;
+  if (reinterpret_cast<uintptr_t>(dout) % 16 != 0 || reinterpret_cast<uintptr_t>(b2) % 16 != 0) return SMOE_ERR_ALIGNMENT;
   const unsigned grid = (TK + 7) / 8;
   const __nv_bfloat16* d = static_cast<const __nv_bfloat16*>(dout);
   const __nv_bfloat16* b = static_cast<const __nv_bfloat16*>(b2);

@@ -168,3 +168,18 @@ def test_training_forward_scratch_without_rows_that_nothing_writes(built_library
         rows = -(-T * K * H * 2 // 256) * 256
         assert every - plain == (rows if K == 1 else 0) and plain >= T * K * I * 2
     assert lib.smoe_layer_train_forward_plain_scratch_bytes(0, H, I, E, 1) == 0
+
+
+def test_biases_read_in_16_byte_pieces(built_library):
+    """Biases that are a view at another offset of a larger buffer are refused before anything is launched (the addresses here
+    belong to nothing)."""
+    from sonicmoe._lib import lib
+
+    at, off = 4096, 4096 + 8
+    gelu = 5
+    assert lib.smoe_up_projection_forward_act(at, at, off, at, at, at, at, 4, 128, 128, 8, 8, gelu, None, None) == -2
+    assert lib.smoe_down_projection_forward_bias(at, at, off, at, at, 128, 64, 8, 8, None, None) == -2
+    assert lib.smoe_ds_add_bias_term(at, off, at, at, at, at, 0, 8, 128, 8, None) == -2
+    assert lib.smoe_ds_add_bias_term(off, at, at, at, at, at, 0, 8, 128, 8, None) == -2
+    assert lib.smoe_expert_column_sum(off, 128, None, None, 0, None, at, at, 8, 128, None) == -2
+    assert lib.smoe_up_projection_forward_act(at, at, off, at, at, at, at, 4, 128, 128, 8, 0, gelu, None, None) == 0
