@@ -215,6 +215,11 @@ int smoe_up_projection_weight_grad_accumulate(const void* x, const void* dz, voi
                                               const int* x_gather_idx, int T, int H, int I, int E, int TK, int* status,
                                               void* stream);
 
+/* Whether the tiles of these GEMMs go in pairs that share each gathered tile (1) or one by one (0): a matter of speed, the
+ * results are the same bits. */
+enum { SMOE_GEMM_UP = 0 /* smoe_up_projection_forward */, SMOE_GEMM_DW1 = 1, SMOE_GEMM_DW2 = 2 /* the weight gradients */ };
+int smoe_dual_tiles(int gemm, int H, int I, int E, int TK);
+
 /* ---------------------------------------------------------------------------------------------
  * Any activation of the layer, and expert biases.  Activation codes: 0 swiglu, 1 geglu, 2 reglu (gated:
  * W1[e] has 2I rows, gate row 2j / up row 2j+1), 3 relu_sq, 4 relu, 5 gelu (erf), 6 silu (W1[e] has I rows).

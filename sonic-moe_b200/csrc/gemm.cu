@@ -71,6 +71,25 @@ static bool use_dual_tiles() {
   return v;
 }
 
+// What two tiles per gathered tile save, the rest costs: their accumulators do not alternate between units, so each unit's
+// hand-over is exposed, and there are half as many units to share out.  Both sides alternating, whole training steps (single /
+// dual):
+//   * up projection: reductions up to 2048 go faster as single tiles (T 24576, H 1536, I 256, E 128, K 8 1907 / 1929 us, T 8197,
+//     H 2048, I 1024, E 64, K 1 780 / 793, T 8000, H 1536, I 512, E 64, K 4 665 / 677; the kernel alone, H 2048, I 1024, E 64: 128 rows
+//     per expert 148 / 177 us, 512 301 / 343, 4096 1730 / 2061; H 1024 and 1536 like it at every load), longer ones do not (H
+//     4096, I 1024, E 128, inference of 8192 tokens 1928 / 1883, step of 2080 2719 / 2701; H 3072 the same either way);
+//   * weight gradients: their reduction is an expert's rows, and the line lies between a mean of 384 and 500 (dW1, H 1536, I
+//     512, E 64, K 4: 256 rows 73 / 91 us, 384 94 / 101, 500 117 / 116; 512 rows, H 4096, I 1024, E 128: 1337 / 1101).  The kernel
+//     alone is up to a tenth faster as dual tiles from 384 rows on with even loads (H 4096, I 1024, E 32, 448 rows 236 / 216) and
+//     a tenth slower with skewed ones (H 1536, I 512, E 64, 448 rows 151 / 165).
+// Never where the doubled dimension is so far from a multiple of 512 that the half-empty last unit wastes more than an eighth of
+// the MMA work (e.g. N = 768).
+static bool dual_tiles(int doubled, bool pays) {
+  return use_dual_tiles() && pays && ((doubled + 511) / 512 * 512 - doubled) * 8 <= doubled;
+}
+static bool dual_reduction(int K) { return K > 2048; }
+static bool dual_rows(long long total_rows, int E) { return total_rows >= 480ll * E; }
+
 template <bool RAGGED_K, bool A_GATHER, bool A_MN, bool B_GATHER, bool B_MN, int EPI, int GW,
           int DUAL = pair::DUAL_NONE>
 static int launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
@@ -103,29 +122,16 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmPara
   if constexpr (!kGather) {
     return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 0>(tmA, tmB, p, stream);
   } else {
-    // not when the doubled dimension is so far from a multiple of 512 that the half-empty last unit wastes more
-    // than an eighth of the MMA work (e.g. N = 768)
-    const int doubled = A_GATHER ? p.N : p.M;
-    const bool fits = ((doubled + 511) / 512 * 512 - doubled) * 8 <= doubled;
     // The activation-gradient epilogues keep single tiles: with both accumulators belonging to one unit the next
     // unit's second MMA group waits for the first accumulator's dSwiGLU pass.  Measured with four epilogue warps in the
     // single form, T 32768, H 4096, I 1024, E 128, K 8: the kernel alone 2.26-2.69 ms dual against 2.09-2.58 single.  Eight
     // warps made the single form 3 % faster since (2.59 -> 2.51 ms, alternating).  The general forward epilogue is too long
     // to be worked off from registers, and must not hold accumulators that the next unit needs.
     if constexpr (EPI != EPI_DSWIGLU && epi_base(EPI) != EPI_DACT && epi_base(EPI) != EPI_ACT) {
-    // What two tiles per gathered tile save, the rest costs: their accumulators do not alternate between units, so each
-    // unit's hand-over is exposed, and there are half as many units to share out.  Both sides alternating, whole training
-    // steps (single / dual):
-    //   * up projection: reductions up to 2048 go faster as single tiles (T 24576, H 1536, I 256, E 128, K 8 1907 / 1929 us,
-    //     T 8197, H 2048, I 1024, E 64, K 1 780 / 793, T 8000, H 1536, I 512, E 64, K 4 665 / 677), longer ones do not (H 4096, I
-    //     1024, E 128, inference of 8192 tokens 1928 / 1883, step of 2080 2719 / 2701; H 3072 the same either way);
-    //   * weight gradients: their reduction is an expert's rows, and the line lies between a mean of 384 and 500 (dW1, H 1536,
-    //     I 512, E 64, K 4: 256 rows 73 / 91 us, 384 94 / 101, 500 117 / 116; 512 rows, H 4096, I 1024, E 128: 1337 / 1101).
-    const bool pays = RAGGED_K ? p.total_rows >= 480ll * p.E : p.K > 2048;
-    if (use_dual_tiles() && fits && pays) {
-      constexpr int kDual = A_GATHER ? pair::DUAL_N : pair::DUAL_M;
-      return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 4, kDual>(tmA, tmB, p, stream);
-    }
+      if (dual_tiles(A_GATHER ? p.N : p.M, RAGGED_K ? dual_rows(p.total_rows, p.E) : dual_reduction(p.K))) {
+        constexpr int kDual = A_GATHER ? pair::DUAL_N : pair::DUAL_M;
+        return launch_variant<RAGGED_K, A_GATHER, A_MN, B_GATHER, B_MN, EPI, 4, kDual>(tmA, tmB, p, stream);
+      }
     }
     // plain stores leave registers for eight gather warps (four: dW2 at H 1536, I 256, 1536 rows per expert 206 us, eight 175)
     constexpr int kGatherWarps = EPI == EPI_STORE ? 8 : 4;
@@ -470,6 +476,15 @@ static int up_weight_grad(const void* x, const void* dz, void* dw1, const int* e
   p.out0 = static_cast<__nv_bfloat16*>(dw1); p.ld0 = H; p.out0_expert_stride = (long long)2 * I * H;
   p.status = status; p.accumulate = accumulate;
   return launch<true, false, true, true, true, EPI_STORE>(tmA, tmB, p, static_cast<cudaStream_t>(stream));
+}
+
+int smoe_dual_tiles(int gemm, int H, int I, int E, int TK) {
+  switch (gemm) {
+    case SMOE_GEMM_UP: return dual_tiles(2 * I, dual_reduction(H));
+    case SMOE_GEMM_DW1: return dual_tiles(2 * I, dual_rows(TK, E));
+    case SMOE_GEMM_DW2: return dual_tiles(I, dual_rows(TK, E));
+    default: return 0;
+  }
 }
 
 int smoe_down_projection_weight_grad(const void* dout, const void* y1s, void* dw2, const int* expert_offset,

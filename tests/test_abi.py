@@ -183,3 +183,17 @@ def test_biases_read_in_16_byte_pieces(built_library):
     assert lib.smoe_ds_add_bias_term(off, at, at, at, at, at, 0, 8, 128, 8, None) == -2
     assert lib.smoe_expert_column_sum(off, 128, None, None, 0, None, at, at, 8, 128, None) == -2
     assert lib.smoe_up_projection_forward_act(at, at, off, at, at, at, at, 4, 128, 128, 8, 0, gelu, None, None) == 0
+
+
+def test_rule_of_the_dual_tiles(built_library):
+    """The lines of the rule: reductions of the up projection above 2048, weight gradients of 480 rows per expert on average, and
+    no last unit that is half empty."""
+    from sonicmoe._lib import lib
+
+    up, dw1, dw2 = 0, 1, 2
+    assert [lib.smoe_dual_tiles(up, H, 960, 8, 4000) for H in (1024, 2048, 2112, 4096)] == [0, 0, 1, 1]
+    for gemm in (dw1, dw2):
+        assert [lib.smoe_dual_tiles(gemm, 2112, 960, 8, rows) for rows in (256, 3839, 3840, 2 ** 31 - 1)] == [0, 0, 1, 1]
+    assert lib.smoe_dual_tiles(up, 4096, 384, 8, 4000) == 0 and lib.smoe_dual_tiles(up, 4096, 768, 8, 4000) == 1
+    assert lib.smoe_dual_tiles(dw2, 4096, 768, 8, 8000) == 0 and lib.smoe_dual_tiles(dw1, 4096, 768, 8, 8000) == 1
+    assert lib.smoe_dual_tiles(3, 4096, 1024, 8, 8000) == 0

@@ -836,3 +836,82 @@ def test_gather_sum_forms(smoe, H, weights):
             part = flat[bounds[t]:bounds[t + 1]]
             slack = 2.0 ** -8 * part.sum(0).abs() + 2 * K * 2.0 ** -24 * part.abs().sum(0)
             assert ((outs[0][t].double() - part.sum(0)).abs() <= 1.01 * slack).all()
+
+
+# One expert above twice the mean, one without rows, ragged ones: rows of 8 experts with a mean of 500 (both weight gradients as
+# dual tiles), and of 479 (single ones).
+_DUAL_LOADS = {2112: (1700, 900, 500, 300, 200, 0, 257, 143), 2048: (1700, 900, 500, 300, 32, 0, 257, 143)}
+
+
+def _gathered_gemms(H, I, out=None):
+    """(inputs, results, forms) of the kernels with a gathered operand on pairs that a caller supplies."""
+    from sonicmoe import _lib
+
+    lib, T, E, rows = _lib.lib, 1111, 8, _DUAL_LOADS[H]
+    TK = sum(rows)
+    g = torch.Generator(device="cuda").manual_seed(H)
+
+    def rn(*shape, std=1.0):
+        return (torch.randn(*shape, device="cuda", generator=g) * std).bfloat16()
+
+    inp = dict(x=rn(T, H), w1=rn(E, 2 * I, H, std=0.05), dout=rn(T, H), dz=rn(TK, 2 * I), y1s=rn(TK, I), dw1=rn(E, 2 * I, H),
+               dw2=rn(E, H, I), gather=torch.randint(0, T, (TK,), device="cuda", generator=g).int(),
+               off=torch.tensor([0, *rows], device="cuda").cumsum(0).int())
+    p = {k: v.data_ptr() for k, v in inp.items()}
+    res = dict(z=torch.full((TK, 2 * I), float("nan"), dtype=torch.bfloat16, device="cuda"), y1=torch.empty_like(inp["y1s"]),
+               dw1=torch.full_like(inp["dw1"], float("nan")), dw2=torch.full_like(inp["dw2"], float("nan")),
+               dw1_sum=inp["dw1"].clone(), dw2_sum=inp["dw2"].clone())
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tail = (p["off"], p["gather"], T, H, I, E, TK, status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert lib.smoe_up_projection_forward(p["x"], p["w1"], res["z"].data_ptr(), res["y1"].data_ptr(), *tail) == 0
+    assert lib.smoe_up_projection_weight_grad(p["x"], p["dz"], res["dw1"].data_ptr(), *tail) == 0
+    assert lib.smoe_down_projection_weight_grad(p["dout"], p["y1s"], res["dw2"].data_ptr(), *tail) == 0
+    assert lib.smoe_up_projection_weight_grad_accumulate(p["x"], p["dz"], res["dw1_sum"].data_ptr(), *tail) == 0
+    assert lib.smoe_down_projection_weight_grad_accumulate(p["dout"], p["y1s"], res["dw2_sum"].data_ptr(), *tail) == 0
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    forms = [lib.smoe_dual_tiles(gemm, H, I, E, TK) for gemm in range(3)]
+    if out is not None:
+        torch.save((res, forms), out)
+    return inp, res, forms
+
+
+@pytest.mark.parametrize("H,dual", [(2112, 1), (2048, 0)])
+def test_dual_tiles_with_a_skewed_load(smoe, tmp_path, H, dual):
+    """Both sides of the dual tiles' rule with caller-supplied pairs and I 960, whose second tiles are partly filled: the
+    form that the rule names, against 64 bits within one bf16 rounding (2^-8) and the rounding of n fp32 terms (2 n 2^-24 of the sum
+    of their magnitudes; twice for the tensor cores' truncation), and dual against single tiles bit for bit."""
+    import os
+    import subprocess
+    import sys
+
+    I = 960
+    inp, res, forms = _gathered_gemms(H, I)
+    assert forms == [dual] * 3
+    off, gather = inp["off"].tolist(), inp["gather"].long()
+
+    def close(got, a, b, n, start=None):
+        want, size = a @ b, a.abs() @ b.abs()
+        bound = 2.0 ** -8 * want.abs() + 2 * n * 2.0 ** -24 * size
+        if start is not None:  # the product is rounded, and then its sum with what was there
+            want = want + start.double()
+            bound = bound + 2.0 ** -8 * (want.abs() + bound)
+        assert ((got.double() - want).abs() <= 1.01 * bound).all()
+
+    for e, (a, b) in enumerate(zip(off[:-1], off[1:])):
+        x, dout = inp["x"][gather[a:b]].double(), inp["dout"][gather[a:b]].double()
+        dz, y1s, w1 = inp["dz"][a:b].double(), inp["y1s"][a:b].double(), inp["w1"][e].double()
+        close(res["z"][a:b], x, w1.T, H)
+        for start, name in ((None, ""), (inp, "_sum")):
+            close(res["dw1" + name][e], dz.T, x, b - a, start and start["dw1"][e])
+            close(res["dw2" + name][e], dout.T, y1s, b - a, start and start["dw2"][e])
+    if dual:
+        root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+        out = str(tmp_path / "single.pt")
+        code = f"import sys; sys.path[:0] = {[os.path.join(root, d) for d in ('tests', '', 'sonic-moe_b200')]!r}\n" \
+               f"import test_kernels_gpu as t; t._gathered_gemms({H}, {I}, {out!r})"
+        subprocess.run([sys.executable, "-c", code], check=True, env=dict(os.environ, SMOE_DUAL="0"), timeout=300)
+        single, forms = torch.load(out)
+        assert forms == [0, 0, 0]
+        for name, v in single.items():
+            assert torch.equal(v, res[name]), name
