@@ -431,9 +431,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     if constexpr (kGather) {
       // One thread of each gather warp issues its share of a stage's 32 gather4 operations (4 rows x 128 B each).  With eight
       // issuing threads a warp the compiler's loop over active lanes (elect_one) took about 75 cycles an operation, which
-      // with eight of them a stage is more than the 512 cycles of a single tile's MMAs: caller's pairs of 65536 tokens, H 2048,
-      // I 768, top-4 of 64 experts with a skewed load 7580 -> 7220 us a training step, T 24576, H 1536, I 256, E 128, K 8
-      // 2051 -> 2013, inference of 8192 tokens, H 4096, I 1024, E 128, K 8 1959 -> 1935 (alternating).
+      // with eight of them a stage is more than the 512 cycles of a single tile's MMAs: a training step of T 24576, H 1536, I 256,
+      // E 128, K 8 2051 -> 2013 us (alternating, repeated runs within 0.4 %; in power-capped steps no more than their spread).
       constexpr int OPS = 32 / GW;
       const int gw = warp - FIRST_GATHER_WARP;
       const bool elected = elect_one();

@@ -244,7 +244,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     // ---- row gather ---------------------------------------------------------------------------
     if constexpr (GATHER) {
       const int gt = threadIdx.x - 32 * FIRST_GATHER_WARP;
-      const bool issuer = (gt & 3) == 0;  // every fourth thread, so that all four warps issue
+      const bool issuer = (gt & 3) == 0;  // every fourth thread: a warp issues for 32 rows, so units of 128 rows take all four
       const int j = gt >> 2;              // rows 4j .. 4j+3 of the unit
       int stage = 0;
       uint32_t phase = 0;

@@ -23,6 +23,7 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // this and not by their lane number: these instructions take their operands from uniform registers, and only behind
 // elect.sync does the compiler know that a single thread is left.  Otherwise it emits a loop over the active lanes around
 // each of them: a k-block of an MMA loop (wait, fence, four MMAs, commit) then takes 483 cycles to issue, 239 with elect.sync.
+// (The row gathers of the few-row kernel are still issued by lane number.)
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(

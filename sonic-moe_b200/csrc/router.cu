@@ -8,13 +8,15 @@
 //   warp 0      TMA producer: x tile 128 x 64 and router-weight tile E x 64 per stage (128-byte swizzle)
 //   warp 1      MMA issuer: tcgen05.mma M 128 x N E x K 16 into one of two tensor-memory accumulators
 //   warps 2-5   thread = token: the accumulator's row, rounded to bf16, goes to shared memory
-//   warps 6-15  warp = token (finish_token): logits out, the K best, their softmax, the full softmax's column sums, which
+//   warps 6-15  warp = token (finish_tokens): logits out, the K best, their softmax, the full softmax's column sums, which
 //               a warp keeps for all its tokens; the warps' and then the CTAs' sums are added up in a fixed order, so the
 //               column sums are bit-reproducible.
 // With a thread per token that kept its K best in a sorted list, the 128 threads took 28 us a tile (E 128, K 8), more than its
 // loads and multiplications, and nothing of it was hidden.  Event time of the two launches, before and now: T 24576, H 1536,
-// E 128, K 8 77 -> 52 us, T 32768, H 4096, E 128, K 8 101 -> 83, T 65536, H 768, E 256, K 16 322 -> 122.  What is left of a tile
-// is the loads of its x rows and of the whole router weight at 100 GB/s per SM.
+// E 128, K 8 77 -> 52 us, T 32768, H 4096, E 128, K 8 101 -> 83, T 65536, H 768, E 256, K 16 322 -> 122.  What is left depends on
+// the layer: with K 1 in the place of K the first two take 37 of 44 us and 66 of 71 (launches in a row, inputs partly in the L2), so
+// there it is the walk over H, loads and multiplications; the third takes 68 of 115, so there it is the search for 16 winners, by
+// ten warps, beside a walk of 12 k-blocks a tile.
 // The routing decision is taken on the bf16-rounded logits the kernel writes, so it can be checked bit for bit
 // against a stable sort of that output.  Every wait is bounded (ptx.cuh).
 #include <cuda_bf16.h>

@@ -384,8 +384,10 @@ __device__ __forceinline__ void load_once(const __nv_bfloat16* p, uint32_t (&v)[
 // tok_off == nullptr means a fixed K rows per token: p in [t*K, (t+1)*K).  ADD: out[t, :] += instead.
 // One thread per COLS consecutive columns of one token, fp32 accumulation.  Bound by memory: 32 bytes of a row per thread
 // (COLS 16), marked to leave the L2 first, since no row is read twice.  With 16-byte loads that the caches kept like any
-// other T 32768, H 4096, K 8 took 408 us, now 378 (6.4 TB/s), T 24576, H 1536, K 8 126, now 111, T 65536, H 2048, K 4 242, now
-// 220, T 8191, H 1024, K 4 19.5, now 17.  COLS 8 is left for rows that are not a multiple of 32 bytes or not so aligned.
+// other, without and with weights, T 32768, H 4096, K 8 took 410 and 381 us, now 383 both (6.4 TB/s), T 8192, H 4096, K 8 115 and
+// 109, now 104, T 24576, H 1536, K 8 127 and 121, now 117, T 65536, H 2048, K 4 246 and 227, now 227 both, T 1027, H 4096, K 16 39
+// and 37, now 31 (single calls, cold L2).  It is the mark that counts: 32-byte loads without it take as long as the old ones, and
+// 16-byte ones with it are within 1 % of these.  COLS 8 is left for rows that are not a multiple of 32 bytes or not so aligned.
 template <typename W, bool ADD, int COLS>
 __global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* src, __nv_bfloat16* out, const W* w,
                                                          const int* rev, const int* tok_off, int T, int H, int K) {
