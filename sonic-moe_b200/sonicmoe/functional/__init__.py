@@ -423,6 +423,9 @@ def _check_experts_args(x, w1, w2, b1, b2, activation_type, expert_major=False):
         raise ValueError("with a bias or a non-SwiGLU activation the up projection needs a multiple of 128 output rows")
     if b1 is not None and (b1.dtype != x.dtype or b2.dtype != x.dtype):
         raise TypeError("biases must have the activations' dtype")
+    if b1 is not None and (b1.numel() < e1 * n1 or b2.numel() < e1 * H):  # the kernels read that many
+        raise ValueError(f"inconsistent shapes: w1 {tuple(w1.shape)}, w2 {tuple(w2.shape)}, b1 {tuple(b1.shape)}, "
+                         f"b2 {tuple(b2.shape)}")
     return activation_type
 
 

@@ -310,3 +310,24 @@ def test_warps_that_meet_at_a_named_barrier_give_up_together():
             before = text[:m.start()]
             wait = before.rfind("mbar_wait_warp(")
             assert "warps_agree(" in before[wait:], f"{name}:{before.count(chr(10)) + 1}"
+
+
+def test_biases_of_another_size_are_refused(built_library, monkeypatch):
+    """The kernels read E rows of both biases."""
+    from sonicmoe import functional as fn
+
+    monkeypatch.setattr(fn._lib, "require_cuda", lambda *args: None)
+    E, H, I = 4, 64, 128
+
+    def bf(*shape):
+        return torch.zeros(shape, dtype=torch.bfloat16)
+
+    x, w1, w2 = bf(8, H), bf(E, I, H), bf(E, H, I)
+    good, views = (bf(E, I), bf(E, H)), (w1.permute(1, 2, 0), w2.permute(1, 2, 0))
+    fn._check_experts_args(x, w1, w2, *good, "gelu", expert_major=True)
+    fn._check_experts_args(x, *views, *good, "gelu")
+    for b1, b2 in ((bf(E - 1, I), good[1]), (good[0], bf(H)), (bf(E, H), good[1])):
+        with pytest.raises(ValueError):
+            fn._check_experts_args(x, w1, w2, b1, b2, "gelu", expert_major=True)
+        with pytest.raises(ValueError):
+            fn._check_experts_args(x, *views, b1, b2, "gelu")
