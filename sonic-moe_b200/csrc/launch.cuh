@@ -14,8 +14,9 @@
 //     stay for many pieces (the GEMMs, the router): their end releases the next one.  A grid that is released before its blocks
 //     find room stands in front of the other streams' grids, and with a release at the start of every GEMM a second stream
 //     did not get on until the chain ended: 40 small kernels beside a training step of T 32768, H 4096, I 1024, E 128, K 8 took
-//     20 ms, the whole step, instead of 1.2.  The release at the end costs nothing: one token 55 -> 54 us, 1027 tokens, H 4096, I 512,
-//     E 256, K 16 730 -> 724, T 24576, H 1536, I 256, E 128, K 8 training 1998 -> 1995 (means of three alternating runs).
+//     20 ms, the whole step, instead of 1.2.  The release at the end costs next to nothing: one token 55 -> 54 us, 1027 tokens, H 4096, I
+//     512, E 256, K 16 730 -> 724, training steps of T 24576, H 1536, I 256, E 128, K 8 1998 -> 1995 and of T 8197, H 2048, I 1024, E 64,
+//     K 1 763 -> 767 (means of three to five alternating runs).
 // Pointers that such a kernel loads from are not __restrict__: loads that the compiler takes to be of constant memory could
 // move in front of the wait.
 #pragma once
